@@ -108,6 +108,7 @@ SIGNATURES = {
     "smeg_matmul_q4_partial_dev": (_i, [_vp, _vp, _vp, _sz, _vp]),
     "smeg_kv_append_dev": (_i, [_vp, _vp, _vp, _sz, _sz, _sz, _sz, _sz, _sz, _vp]),
     "smeg_attn_kv_causal_dev": (_i, [_vp, _vp, _i, _sz, _vp, _vp, _sz, _sz, _sz, _sz, _sz, C.c_float, _vp]),
+    "smeg_attn_kv_causal_f16_dev": (_i, [_vp, _vp, _i, _sz, _vp, _vp, _sz, _sz, _sz, _sz, _sz, C.c_float, _vp]),
     "smeg_mlp_finish_dev": (_i, [_vp, _vp, _sz, _vp]),
     "smeg_mlp_reduce_finish_dev": (_i, [_vp, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64), _i, _i, _sz, _u32, _i, _vp]),
     "smeg_mlp_partial_push_dev": (_i, [_vp, _vp, C.POINTER(C.c_uint64), _i, _i, _sz, _vp]),

@@ -1164,8 +1164,8 @@ int smeg_kv_append_dev(uint16_t* k_cache, uint16_t* v_cache, const uint16_t* src
     if (!dev_state()) return -5;
     return kv_append_launch(k_cache, v_cache, src, src_stride, k_off, v_off, row_len, pos, rows, (cudaStream_t)stream) == cudaSuccess ? 0 : -6;
 }
-int smeg_attn_kv_causal_dev(float* out, const void* q, int q_f32, size_t q_stride, const uint16_t* k, const uint16_t* v, size_t start,
-                            size_t rows, size_t heads, size_t kv_heads, size_t head_dim, float scale, void* stream) {
+static int attn_dev(void* out, int out16, const void* q, int q_f32, size_t q_stride, const uint16_t* k, const uint16_t* v, size_t start,
+                    size_t rows, size_t heads, size_t kv_heads, size_t head_dim, float scale, void* stream) {
     if (rows == 0) return 0;
     // the reference's panics (src/kernels/kv_attention.rs:171-199) as rc -4
     if (!out || !q || !k || !v) return -4;
@@ -1173,14 +1173,23 @@ int smeg_attn_kv_causal_dev(float* out, const void* q, int q_f32, size_t q_strid
     if (kv_heads == 0 || heads == 0 || heads % kv_heads != 0 || q_stride < heads * head_dim) return -4;
     if (((uintptr_t)k & 15) != 0 || ((uintptr_t)v & 15) != 0) return -4;
     if (start + rows > 0x7fffffffu || heads > 65535 || rows > 65535) return -3;
-    if (!dev_state()) return -5;
+    DeviceState* ds = dev_state();
+    if (!ds) return -5;
     AttnArgs a;
     memset(&a, 0, sizeof(a));
-    a.out = out; a.q = q; a.q_stride = q_stride; a.k = k; a.v = v;
+    a.out = out; a.out16 = out16; a.q = q; a.q_stride = q_stride; a.k = k; a.v = v;
     a.start = (int)start; a.rows = (int)rows; a.heads = (int)heads; a.kv_heads = (int)kv_heads; a.head_dim = (int)head_dim;
-    a.scale = scale;
-    const cudaError_t e = attn_kv_causal_launch(a, q_f32, (cudaStream_t)stream);
+    a.scale = scale; a.status = ds->status;
+    const cudaError_t e = attn_kv_causal_launch(a, q_f32, ds->sm_count, (cudaStream_t)stream);
     return e == cudaSuccess ? 0 : (e == cudaErrorInvalidValue ? -3 : -6);
+}
+int smeg_attn_kv_causal_dev(float* out, const void* q, int q_f32, size_t q_stride, const uint16_t* k, const uint16_t* v, size_t start,
+                            size_t rows, size_t heads, size_t kv_heads, size_t head_dim, float scale, void* stream) {
+    return attn_dev(out, 0, q, q_f32, q_stride, k, v, start, rows, heads, kv_heads, head_dim, scale, stream);
+}
+int smeg_attn_kv_causal_f16_dev(uint16_t* out, const void* q, int q_f32, size_t q_stride, const uint16_t* k, const uint16_t* v, size_t start,
+                                size_t rows, size_t heads, size_t kv_heads, size_t head_dim, float scale, void* stream) {
+    return attn_dev(out, 1, q, q_f32, q_stride, k, v, start, rows, heads, kv_heads, head_dim, scale, stream);
 }
 
 int smeg_mlp_create(const smeg_q4* gate_up, const smeg_q4* down, uint32_t gate_act, smeg_mlp** out) {

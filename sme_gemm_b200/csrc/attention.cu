@@ -1,122 +1,513 @@
 // Causal attention against an f16 key/value cache, and the append into that cache (sm_100a) -- the attention step of
 // SelfAttention::accumulate (src/self_attention.rs:189-231) between its two projections:
 //   attention_kv_causal_f16 / attention_kv_f16 (src/kernels/kv_attention.rs:29-331): query row i of a block attends to
-//   keys 0..=start+i; per head softmax(f16(q * scale) . k) @ v, f32 sums in key / depth order, f32 probabilities
-//   exp(s - max), the division by their sum last.  Query head h uses KV head h / (heads / kv_heads).
+//   keys 0..=start+i; per head softmax(f16(q * scale) . k) @ v, f32 sums, f32 probabilities exp(s - max), the division by
+//   their sum last.  Query head h uses KV head h / (heads / kv_heads).
 //   KvCache::extend (:499-520): a block's key and value rows copied to the cache's next positions.
 //
-// One CTA per (query row, head).  A thread owns keys t, t + 128, ...: its score is the depth-ordered f32 sum the scalar
-// statement forms (separately rounded multiply and add), so scores -- and the maximum -- are the reference's bits; the
-// probabilities differ from libm's by the device expf, their sum by summation order.  The value pass gives every thread
-// one depth and walks the keys in order (the reference's order again), lanes reading consecutive depths of a row.  This is
-// the plain form for decode steps and moderate prompts: scores of one (row, head) live in shared memory (up to ~50 k
-// keys), nothing is tiled for the tensor cores.
+// attn_tc_kernel forms both products on the 5th-generation tensor cores.  The query rows of one KV head -- every row of the
+// block times every head of the group -- are the M dimension, 128 to a tile, so that grouped queries share one read of the
+// keys and values; a key block is 128 keys.  Two passes over the keys of a tile:
+//   1. S = Q K^T into tensor memory, the row maxima from it;
+//   2. S again (not where both blocks of a short range are still in tensor memory), p = exp(s - max), O += P V.
+// With the exact maximum known first, a probability is the reference's exp(s - max) whatever the order of the blocks, and the
+// accumulator in tensor memory is never rescaled; the second Q K^T costs a quarter of the tensor work, and the tensor pipe
+// waits for the exponentials anyway.  Operands are exact: q and k are f16 already, and the f32 probability travels as the sum
+// of two f16 numbers (p * 2^15 = hi + lo: 22 significant bits down to probabilities of 2^-29), two MMAs per step of P V.
+//
+// Roles (320 threads): warps 0-7 (softmax; warp = 32 rows x 64 keys of a block, a thread one row), warp 8 (TMA: K and V
+// blocks as three-dimensional boxes, so that a head of less than 64 depths and the rows past the last key read as zero),
+// warp 9 (MMA).  P goes back into the S columns it was read from (A operand in tensor memory), V is taken as it lies in the
+// cache ([key][depth]: an MN-major B operand).
+//
+// What bounds it: the exponentials -- about 14 instructions for each of a block's 16384 scores, ~1900 cycles per block on
+// the four schedulers against ~1500 cycles of tensor time.  A short prompt or a decode step has too few (tile, KV head)
+// pairs for the machine: there a cluster of 2, 4 or 8 CTAs shares one tile's key blocks, each against the maximum of its own
+// range, and the parts meet over distributed shared memory (out = sum_c e^(m_c - m) O_c / sum_c e^(m_c - m) l_c, in rank
+// order).
 #include "common.cuh"
 #include "kernels.h"
+#include "tc_common.cuh"
 
 namespace smeg {
 namespace {
 
-constexpr int kAttnThreads = 128;
+constexpr int kAtThreads = 320;
+constexpr int kAtKeys = 128;                      // keys of a block
+constexpr int kAtChunk = 128 * 128;               // bytes of 128 rows x 64 depths
+constexpr int kAtMaxSlots = 8;
+constexpr uint32_t kAtOCol = 256;                 // tensor memory: S / P buffers at columns 0 and 128, O behind them
+constexpr float kAtPScale = 32768.0f;             // probabilities are scaled by 2^15 on their way into two f16 parts
 
-__device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const float u = __shfl_xor_sync(0xffffffffu, v, o);
-        v = is_max ? fmaxf(v, u) : v + u;
-    }
-    __syncthreads();                                   // red may still be read from the previous reduction
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    float r = red[0];
-    for (int w = 1; w < kAttnThreads / 32; ++w) r = is_max ? fmaxf(r, red[w]) : r + red[w];
-    return r;
+// D[tmem] (+)= A[tmem] * B[smem desc], kind::f16
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+        : "memory");
+}
+// MN-major tile stored as rows of 64 MN elements (128 bytes, 128-byte swizzle) per K index: 8-row groups along K 1024 bytes
+// apart, 64-element chunks along MN one kAtChunk apart.
+__device__ __forceinline__ uint64_t umma_desc_sw128_mn(uint32_t smem_addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((smem_addr >> 4) & 0x3fffu);
+    d |= (uint64_t)(kAtChunk >> 4) << 16;         // leading byte offset: next 64 elements along MN
+    d |= (uint64_t)(1024 >> 4) << 32;             // stride byte offset: next 8 rows along K
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* tmap, int x, int y, int z, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ float ld_dsmem_f32(uint32_t cluster_addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t cluster_addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_addr) : "memory");
+    return v;
 }
 
-template <int QF32>
-__global__ void __launch_bounds__(kAttnThreads) attn_kv_causal_kernel(const __grid_constant__ AttnArgs p) {
-    extern __shared__ __align__(16) float smem_f[];
-    const int h = blockIdx.x, i = blockIdx.y, tid = threadIdx.x;
-    const int hd = p.head_dim, ld = p.kv_heads * hd, group = p.heads / p.kv_heads;
-    const int off = (h / group) * hd;
-    const int len = p.start + i + 1;
-    float* qh = smem_f;                                // [hd] f16-rounded scaled query
-    float* red = qh + hd;                              // [4]
-    float* scores = red + 8;                           // [len]
-    for (int d = tid; d < hd; d += kAttnThreads) {
-        float x;
-        if (QF32) x = reinterpret_cast<const float*>(p.q)[(size_t)i * p.q_stride + (size_t)h * hd + d];
-        else x = __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(p.q)[(size_t)i * p.q_stride + (size_t)h * hd + d]));
-        qh[d] = __half2float(__float2half_rn(__fmul_rn(x, p.scale)));
-    }
-    __syncthreads();
-    // ---- scores: s_t = sum_d qh[d] * k[t][d], d ascending ----
-    float mx = -INFINITY;
-    for (int t = tid; t < len; t += kAttnThreads) {
-        const uint4* kr = reinterpret_cast<const uint4*>(p.k + (size_t)t * ld + off);      // head_dim % 8 == 0: 16-byte vectors
-        float s = 0.0f;
-        for (int c = 0; c < hd / 8; ++c) {
-            const uint4 kv = kr[c];
-            const uint32_t w[4] = {kv.x, kv.y, kv.z, kv.w};
+// Largest of a warp's 64 scores per row; keys from `lim` on do not count.
+template <bool MASK>
+__device__ __forceinline__ float block_max(uint32_t taddr, int lim, float mx) {
+    uint32_t r[2][32];
+    tmem_ld32(taddr, r[0]);
+    tmem_ld32(taddr + 32, r[1]);
+    tmem_ld_wait();
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-                s = __fadd_rn(s, __fmul_rn(qh[8 * c + 2 * e], f.x));
-                s = __fadd_rn(s, __fmul_rn(qh[8 * c + 2 * e + 1], f.y));
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const float s = __uint_as_float(r[h][i]);
+            mx = (!MASK || 32 * h + i < lim) ? fmaxf(mx, s) : mx;
+        }
+    return mx;
+}
+
+// p = exp(s - mx) of a warp's 64 scores per row, added to `sum`, and written over them as two f16 parts: columns 0..31 of
+// the 64 hold the high parts (two keys to a column), 32..63 the low ones.
+template <bool MASK>
+__device__ __forceinline__ float block_exp(uint32_t taddr, int lim, float mx, float sum) {
+    uint32_t r[2][32];
+    tmem_ld32(taddr, r[0]);
+    tmem_ld32(taddr + 32, r[1]);
+    tmem_ld_wait();
+    uint32_t hi[2][16], lo[2][16];
+    float sum2 = 0.0f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+            float e0 = expf(__uint_as_float(r[h][i]) - mx), e1 = expf(__uint_as_float(r[h][i + 1]) - mx);
+            if (MASK) {
+                e0 = 32 * h + i < lim ? e0 : 0.0f;
+                e1 = 32 * h + i + 1 < lim ? e1 : 0.0f;
+            }
+            sum += e0;
+            sum2 += e1;
+            e0 *= kAtPScale;
+            e1 *= kAtPScale;
+            const uint32_t p = pack2_t<0>(e0, e1);
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&p));
+            hi[h][i / 2] = p;
+            lo[h][i / 2] = pack2_t<0>(e0 - f.x, e1 - f.y);
+        }
+    tmem_st16(taddr, hi[0]);
+    tmem_st16(taddr + 16, hi[1]);
+    tmem_st16(taddr + 32, lo[0]);
+    tmem_st16(taddr + 48, lo[1]);
+    tmem_st_wait();
+    return sum + sum2;
+}
+
+template <int OUT16>
+__device__ __forceinline__ void store8(const AttnArgs& p, size_t off, const float (&v)[8]) {
+    if (OUT16) {
+        uint4 o;
+        o.x = pack2_t<0>(v[0], v[1]); o.y = pack2_t<0>(v[2], v[3]); o.z = pack2_t<0>(v[4], v[5]); o.w = pack2_t<0>(v[6], v[7]);
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + off) = o;
+    } else {
+        float* d = reinterpret_cast<float*>(p.out) + off;
+        *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(d + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    }
+}
+
+// Grid: (CTAs per tile, tiles of 128 query rows x heads of a group, KV heads); the CTAs of a tile are a cluster.
+template <int QF32, int OUT16>
+__global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
+                                                                const __grid_constant__ AttnArgs p) {
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
+    __shared__ __align__(8) uint64_t bars[2 * kAtMaxSlots + 9];
+    __shared__ float red_m[2][128], red_l[2][128];             // per half of the softmax warps and row: maximum, sum
+    __shared__ float part_m[128], part_l[128];                 // of this CTA's key range
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_word;
+    volatile int* abort_flag = &abort_word;
+    uint64_t *full = bars, *empty = full + kAtMaxSlots, *q_full = empty + kAtMaxSlots, *s_full = q_full + 1, *s_free = s_full + 2,
+             *p_full = s_free + 2, *pv_done = p_full + 2;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int hd = p.head_dim, group = p.heads / p.kv_heads, kvh = blockIdx.z;
+    const int tile = gridDim.y - 1 - blockIdx.y;               // the tiles with the most keys first
+    const int splits = gridDim.x, rank = blockIdx.x;
+    const int row0 = tile * 128, nrow = min(128, p.rows * group - row0);
+    const int nch = (hd + 63) >> 6, tile_bytes = nch * kAtChunk, hd16 = (hd + 15) & ~15;
+    const int nslots = p.slots;
+    // key blocks of the tile, and this CTA's share of them
+    const int keys = p.start + (row0 + nrow - 1) / group + 1;
+    const int nblk = (keys + kAtKeys - 1) / kAtKeys, per = (nblk + splits - 1) / splits;
+    const int blk0 = min(rank * per, nblk), nb = min(per, nblk - blk0);
+    const bool resident = nb <= 2;                             // both S buffers keep their block from pass 1 to pass 2
+    unsigned char* q_s = smem;
+    unsigned char* ring = smem + tile_bytes;
+
+    if (tid == 0) {
+        abort_word = 0;
+        for (int i = 0; i < nslots; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        mbar_init(q_full, 256);
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 8); mbar_init(&p_full[i], 8); mbar_init(&pv_done[i], 1); }
+        fence_barrier_init();
+    }
+    pdl_wait();                                                // (before the allocation: the kernel ahead may still hold tensor memory)
+    if (warp == 9) {
+        tmem_alloc(&tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_launch_dependents();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == 8) {                                           // ---- K and V blocks ----
+        if (elect_one()) {
+            int n = 0;
+            auto load = [&](const CUtensorMap* map, int j) {
+                const int slot = n % nslots, round = n / nslots;
+                ++n;
+                if (round && !mbar_wait(&empty[slot], (round - 1) & 1, abort_flag, p.status)) return;
+                mbar_expect_tx(&full[slot], tile_bytes);
+                for (int c = 0; c < nch; ++c)
+                    tma_load_3d(ring + (size_t)slot * tile_bytes + c * kAtChunk, map, c * 64, kvh, (blk0 + j) * kAtKeys, &full[slot]);
+            };
+            for (int j = 0; j < nb; ++j) load(&tk, j);
+            if (!resident && nb) load(&tk, 0);
+            for (int j = 0; j < nb; ++j) {
+                if (!resident && j + 1 < nb) load(&tk, j + 1);
+                load(&tv, j);
             }
         }
-        scores[t] = s;
-        mx = fmaxf(mx, s);
+        __syncwarp();
+    } else if (warp == 9) {                                    // ---- MMA ----
+        const uint32_t idesc_s = umma_idesc(0, 128, kAtKeys);
+        const uint32_t idesc_o = umma_idesc(0, 128, hd16) | (1u << 16);          // B is MN-major
+        const int ksteps = hd16 >> 4;
+        const uint32_t q_a = smem_u32(q_s), ring_a = smem_u32(ring);
+        int n = 0;
+        bool ok = nb > 0 && __all_sync(0xffffffffu, mbar_wait(q_full, 0, abort_flag, p.status));
+        auto take = [&](uint32_t& addr, int& slot) {
+            slot = n % nslots;
+            addr = ring_a + (uint32_t)slot * tile_bytes;
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(&full[slot], (n / nslots) & 1, abort_flag, p.status));
+            ++n;
+            tc_fence_after();
+        };
+        auto issue_s = [&](int b) {
+            uint32_t addr;
+            int slot;
+            take(addr, slot);
+            if (!ok) return;
+            if (elect_one()) {
+                for (int s = 0; s < ksteps; ++s) {
+                    const uint32_t off = (uint32_t)((s >> 2) * kAtChunk + (s & 3) * 32);
+                    umma_f16(tmem + 128 * b, umma_desc_sw128(q_a + off), umma_desc_sw128(addr + off), idesc_s, s > 0);
+                }
+                umma_commit(&empty[slot]);
+                umma_commit(&s_full[b]);
+            }
+            __syncwarp();
+        };
+        for (int j = 0; ok && j < nb; ++j) {
+            const int b = j & 1;
+            if (j >= 2) ok = __all_sync(0xffffffffu, mbar_wait(&s_free[b], ((j >> 1) - 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            if (ok) { tc_fence_after(); issue_s(b); }
+        }
+        // pass 2: the scores of block j + 1 are formed while the softmax warps work on block j
+        auto again = [&](int j) {
+            const int b = j & 1, used = (nb - b + 1) >> 1;                       // uses of buffer b in pass 1
+            if (j < 2) ok = ok && __all_sync(0xffffffffu, mbar_wait(&s_free[b], (used - 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            else ok = ok && __all_sync(0xffffffffu, mbar_wait(&pv_done[b], ((j >> 1) - 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            if (ok) { tc_fence_after(); issue_s(b); }
+        };
+        if (!resident) again(0);
+        for (int j = 0; ok && j < nb; ++j) {
+            if (!resident && j + 1 < nb) again(j + 1);
+            const int b = j & 1;
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(&p_full[b], (j >> 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            uint32_t addr;
+            int slot;
+            take(addr, slot);
+            if (!ok) break;
+            if (elect_one()) {
+                for (int s = 0; s < kAtKeys / 16; ++s) {
+                    const uint32_t a = tmem + 128 * b + (s >> 2) * 64 + (s & 3) * 8;
+                    const uint64_t bd = umma_desc_sw128_mn(addr + s * 2048);
+                    umma_f16_ts(tmem + kAtOCol, a, bd, idesc_o, j > 0 || s > 0);
+                    umma_f16_ts(tmem + kAtOCol, a + 32, bd, idesc_o, 1);
+                }
+                umma_commit(&empty[slot]);
+                umma_commit(&pv_done[b]);
+            }
+            __syncwarp();
+        }
+    } else {                                                   // ---- softmax ----
+        const int q4 = warp & 3, half = warp >> 2, row = q4 * 32 + lane;
+        // the tile's queries: f16(q * scale), K-major with the 128-byte swizzle (rows past the tile's last are never read)
+        for (int it = tid; it < nrow * nch * 8; it += 256) {
+            const int r = it / (nch * 8), c = it - r * (nch * 8);                // row, run of 8 depths
+            const int i = (row0 + r) / group, g = (row0 + r) - i * group;
+            uint4 o = make_uint4(0, 0, 0, 0);
+            if (c * 8 < hd) {
+                const size_t src = (size_t)i * p.q_stride + (size_t)(kvh * group + g) * hd + c * 8;
+                float x[8];
+                if (QF32) {
+                    const float* q = reinterpret_cast<const float*>(p.q) + src;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = q[e];
+                } else if (p.q_vec) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.q) + src);
+                    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                        x[2 * e] = f.x;
+                        x[2 * e + 1] = f.y;
+                    }
+                } else {
+                    const uint16_t* q = reinterpret_cast<const uint16_t*>(p.q) + src;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = __half2float(__ushort_as_half(q[e]));
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = __fmul_rn(x[e], p.scale);
+                o.x = pack2_t<0>(x[0], x[1]); o.y = pack2_t<0>(x[2], x[3]); o.z = pack2_t<0>(x[4], x[5]); o.w = pack2_t<0>(x[6], x[7]);
+            }
+            *reinterpret_cast<uint4*>(q_s + (c >> 3) * kAtChunk + r * 128 + (((c & 7) ^ (r & 7)) << 4)) = o;
+        }
+        fence_proxy_async();
+        mbar_arrive(q_full);
+
+        const bool live = q4 * 32 < nrow;                                        // does the warp hold rows of the tile?
+        const uint32_t t_s = tmem + ((uint32_t)(q4 * 32) << 16) + 64 * half;
+        const int len = row < nrow ? p.start + (row0 + row) / group + 1 : 0;     // keys this row attends to
+        const int len_all = p.start + row0 / group + 1;                          // keys that every row of the tile attends to
+        bool ok = true;
+        float mx = -INFINITY;
+        for (int j = 0; ok && j < nb; ++j) {
+            const int b = j & 1, key0 = (blk0 + j) * kAtKeys + 64 * half;
+            ok = __all_sync(0xffffffffu, mbar_wait(&s_full[b], (j >> 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            if (!ok) break;
+            tc_fence_after();
+            if (live) mx = key0 + 64 <= len_all ? block_max<false>(t_s + 128 * b, 0, mx) : block_max<true>(t_s + 128 * b, len - key0, mx);
+            if (!resident) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_free[b]);
+            }
+        }
+        red_m[half][row] = mx;
+        named_barrier_sync(1, 256);
+        mx = fmaxf(mx, red_m[half ^ 1][row]);
+        const float mx_e = mx == -INFINITY ? 0.0f : mx;                          // no key of this range counts for the row
+        float sum = 0.0f;
+        for (int j = 0; ok && j < nb; ++j) {
+            const int b = j & 1, key0 = (blk0 + j) * kAtKeys + 64 * half;
+            if (!resident) {
+                const int used = (nb - b + 1) >> 1;
+                ok = __all_sync(0xffffffffu, mbar_wait(&s_full[b], (used + (j >> 1)) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+                if (!ok) break;
+                tc_fence_after();
+            }
+            if (live) sum = key0 + 64 <= len_all ? block_exp<false>(t_s + 128 * b, 0, mx_e, sum) : block_exp<true>(t_s + 128 * b, len - key0, mx_e, sum);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_full[b]);
+        }
+        red_l[half][row] = sum;
+        if (nb > 0) ok = ok && __all_sync(0xffffffffu, mbar_wait(&pv_done[(nb - 1) & 1], ((nb - 1) >> 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+        tc_fence_after();
+        named_barrier_sync(1, 256);
+        sum = red_l[0][row] + red_l[1][row];
+        // the two halves of the warps take a half of the depths each
+        const int c_begin = half ? ((hd / 8 + 1) / 2) * 8 : 0, c_end = half ? hd : ((hd / 8 + 1) / 2) * 8;
+        if (splits == 1) {
+            const int i = (row0 + row) / group, g = (row0 + row) - i * group;
+            const size_t dst = (size_t)i * p.heads * hd + (size_t)(kvh * group + g) * hd;
+            for (int c = c_begin; ok && live && c < c_end; c += 8) {
+                uint32_t r[8];
+                tmem_ld8(tmem + ((uint32_t)(q4 * 32) << 16) + kAtOCol + c, r);
+                tmem_ld_wait();
+                float v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(__uint_as_float(r[e]) * (1.0f / kAtPScale), sum);
+                if (row < nrow) store8<OUT16>(p, dst + c, v);
+            }
+        } else {
+            if (half == 0) { part_m[row] = nb > 0 ? mx : -INFINITY; part_l[row] = sum; }
+            float* o_s = reinterpret_cast<float*>(smem);                         // the operands are not needed any more
+            for (int c = c_begin; live && c < c_end; c += 8) {
+                uint32_t r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                if (nb > 0) {
+                    tmem_ld8(tmem + ((uint32_t)(q4 * 32) << 16) + kAtOCol + c, r);
+                    tmem_ld_wait();
+                }
+                if (row < nrow) {
+                    *reinterpret_cast<uint4*>(o_s + (size_t)row * (hd + 4) + c) = make_uint4(r[0], r[1], r[2], r[3]);
+                    *reinterpret_cast<uint4*>(o_s + (size_t)row * (hd + 4) + c + 4) = make_uint4(r[4], r[5], r[6], r[7]);
+                }
+            }
+        }
     }
-    mx = block_reduce(mx, red, true);
-    float sum = 0.0f;
-    for (int t = tid; t < len; t += kAttnThreads) {
-        const float e = expf(__fsub_rn(scores[t], mx));
-        scores[t] = e;
-        sum += e;
+    if (splits > 1) {                                          // ---- the parts of a cluster meet ----
+        cluster_sync_all();
+        const uint32_t o_a = smem_u32(smem), m_a = smem_u32(part_m), l_a = smem_u32(part_l);
+        const int items = nrow * (hd / 8);
+        for (int it = rank * kAtThreads + tid; it < items && *abort_flag == 0; it += splits * kAtThreads) {
+            const int r = it / (hd / 8), c = (it - r * (hd / 8)) * 8;
+            float m[8], l[8];
+            float4 o[8][2];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                if (s >= splits) break;
+                m[s] = ld_dsmem_f32(mapa_shared(m_a + r * 4, s));
+                l[s] = ld_dsmem_f32(mapa_shared(l_a + r * 4, s));
+                const uint32_t oa = mapa_shared(o_a + (uint32_t)(r * (hd + 4) + c) * 4, s);
+                o[s][0] = ld_dsmem_f32x4(oa);
+                o[s][1] = ld_dsmem_f32x4(oa + 16);
+            }
+            float mx = -INFINITY;
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if (s < splits) mx = fmaxf(mx, m[s]);
+            float sum = 0.0f, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {
+                if (s >= splits || m[s] == -INFINITY) continue;
+                const float f = expf(m[s] - mx);
+                sum = fmaf(f, l[s], sum);
+                v[0] = fmaf(f, o[s][0].x, v[0]); v[1] = fmaf(f, o[s][0].y, v[1]); v[2] = fmaf(f, o[s][0].z, v[2]); v[3] = fmaf(f, o[s][0].w, v[3]);
+                v[4] = fmaf(f, o[s][1].x, v[4]); v[5] = fmaf(f, o[s][1].y, v[5]); v[6] = fmaf(f, o[s][1].z, v[6]); v[7] = fmaf(f, o[s][1].w, v[7]);
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(v[e] * (1.0f / kAtPScale), sum);
+            const int i = (row0 + r) / group, g = (row0 + r) - i * group;
+            store8<OUT16>(p, (size_t)i * p.heads * hd + (size_t)(kvh * group + g) * hd + c, v);
+        }
+        tc_fence_before();
+        cluster_sync_all();                                    // nobody leaves while its shared memory is read
+    } else {
+        tc_fence_before();
+        __syncthreads();
     }
-    sum = block_reduce(sum, red, false);               // (its barriers also publish the probabilities)
-    // ---- values: out[d] = (sum_t p_t * v[t][d]) / sum, t ascending ----
-    for (int d = tid; d < hd; d += kAttnThreads) {
-        const uint16_t* vc = p.v + off + d;
-        float o = 0.0f;
-        for (int t = 0; t < len; ++t) o = __fadd_rn(o, __fmul_rn(scores[t], __half2float(__ushort_as_half(vc[(size_t)t * ld]))));
-        p.out[(size_t)i * p.heads * hd + (size_t)h * hd + d] = __fdiv_rn(o, sum);
+    if (warp == 9) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
     }
 }
 
-// rows x row_len f16 values from a strided source (the k or v part of projected [q | k | v] rows) to cache rows pos...
+// rows x row_len f16 values from a strided source (the k or v part of projected [q | k | v] rows) to cache rows pos...; a
+// thread moves 8 values of each (VEC: every address involved is 16-byte aligned) or one.
+template <int VEC>
 __global__ void kv_append_kernel(uint16_t* __restrict__ kc, uint16_t* __restrict__ vc, const uint16_t* __restrict__ src, size_t stride,
                                  size_t k_off, size_t v_off, size_t row_len, size_t pos, size_t rows) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= rows * row_len) return;
-    const size_t r = idx / row_len, c = idx - r * row_len;
-    kc[(pos + r) * row_len + c] = src[r * stride + k_off + c];
-    vc[(pos + r) * row_len + c] = src[r * stride + v_off + c];
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t per = row_len / VEC, idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= rows * per) return;
+    const size_t r = idx / per, c = (idx - r * per) * VEC;
+    if (VEC == 8) {
+        *reinterpret_cast<uint4*>(kc + (pos + r) * row_len + c) = *reinterpret_cast<const uint4*>(src + r * stride + k_off + c);
+        *reinterpret_cast<uint4*>(vc + (pos + r) * row_len + c) = *reinterpret_cast<const uint4*>(src + r * stride + v_off + c);
+    } else {
+        kc[(pos + r) * row_len + c] = src[r * stride + k_off + c];
+        vc[(pos + r) * row_len + c] = src[r * stride + v_off + c];
+    }
+}
+
+template <int QF32, int OUT16>
+cudaError_t attn_tc_launch(const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
+    auto kern = attn_tc_kernel<QF32, OUT16>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kAtThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = grid.x;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kern, tk, tv, a);
 }
 
 }  // namespace
 
-cudaError_t attn_kv_causal_launch(const AttnArgs& a, int q_f32, cudaStream_t stream) {
-    const size_t smem = ((size_t)a.head_dim + 8 + (size_t)(a.start + a.rows)) * sizeof(float);
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e;
-    if (q_f32) e = cudaFuncSetAttribute(attn_kv_causal_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    else e = cudaFuncSetAttribute(attn_kv_causal_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (e != cudaSuccess) return e;
-    const dim3 grid(a.heads, a.rows);
-    if (q_f32) attn_kv_causal_kernel<1><<<grid, kAttnThreads, smem, stream>>>(a);
-    else attn_kv_causal_kernel<0><<<grid, kAttnThreads, smem, stream>>>(a);
-    return cudaGetLastError();
+cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream) {
+    TensorMapEncodeFn enc = tensor_map_encoder();
+    if (!enc) return cudaErrorNotSupported;
+    // [depth][KV head][position], a box = 64 depths of one head at 128 positions
+    const size_t len = (size_t)a.start + a.rows, row = (size_t)a.kv_heads * a.head_dim;
+    const cuuint64_t dim[3] = {(cuuint64_t)a.head_dim, (cuuint64_t)a.kv_heads, (cuuint64_t)len};
+    const cuuint64_t stride[2] = {(cuuint64_t)a.head_dim * 2, (cuuint64_t)row * 2};
+    const cuuint32_t box[3] = {64, 1, (cuuint32_t)kAtKeys}, estr[3] = {1, 1, 1};
+    CUtensorMap tk, tv;
+    if (enc(&tk, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)a.k, dim, stride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
+        enc(&tv, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, (void*)a.v, dim, stride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorInvalidValue;
+    const size_t tiles = ((size_t)a.rows * (a.heads / a.kv_heads) + 127) / 128, blocks = (len + kAtKeys - 1) / kAtKeys;
+    if (tiles > 65535) return cudaErrorInvalidValue;
+    // a cluster shares a tile's key blocks while the machine has SMs to spare and every CTA keeps a block
+    unsigned splits = 1;
+    while (splits < 8 && splits * 2 <= blocks && tiles * a.kv_heads * splits * 2 <= (size_t)sm_count) splits *= 2;
+    // ring of K / V blocks beside the query tile: at least two slots (heads of 256 depths)
+    const int tile_bytes = ((a.head_dim + 63) / 64) * kAtChunk;
+    a.slots = (216 * 1024 - tile_bytes) / tile_bytes;
+    if (a.slots > kAtMaxSlots) a.slots = kAtMaxSlots;
+    size_t smem = 1024 + (size_t)tile_bytes * (1 + a.slots);
+    const size_t parts = 1024 + 128 * (size_t)(a.head_dim + 4) * 4;              // what a cluster's CTAs exchange lies over the operands
+    if (splits > 1 && smem < parts) smem = parts;
+    a.q_vec = a.q_stride % 8 == 0 && ((uintptr_t)a.q & 15) == 0;
+    const dim3 grid(splits, (unsigned)tiles, (unsigned)a.kv_heads);
+    if (a.out16) return q_f32 ? attn_tc_launch<1, 1>(tk, tv, a, grid, smem, stream) : attn_tc_launch<0, 1>(tk, tv, a, grid, smem, stream);
+    return q_f32 ? attn_tc_launch<1, 0>(tk, tv, a, grid, smem, stream) : attn_tc_launch<0, 0>(tk, tv, a, grid, smem, stream);
 }
 
 cudaError_t kv_append_launch(uint16_t* kc, uint16_t* vc, const uint16_t* src, size_t stride, size_t k_off, size_t v_off, size_t row_len,
                              size_t pos, size_t rows, cudaStream_t stream) {
-    const size_t total = rows * row_len;
-    if (total == 0) return cudaSuccess;
-    kv_append_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(kc, vc, src, stride, k_off, v_off, row_len, pos, rows);
-    return cudaGetLastError();
+    if (rows * row_len == 0) return cudaSuccess;
+    const bool vec = row_len % 8 == 0 && stride % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 &&
+                     (((uintptr_t)kc | (uintptr_t)vc | (uintptr_t)src) & 15) == 0;
+    const size_t threads = rows * row_len / (vec ? 8 : 1);
+    const dim3 grid((unsigned)((threads + 255) / 256));
+    if (vec) return launch_pdl(kv_append_kernel<8>, grid, dim3(256), 0, stream, kc, vc, src, stride, k_off, v_off, row_len, pos, rows);
+    return launch_pdl(kv_append_kernel<1>, grid, dim3(256), 0, stream, kc, vc, src, stride, k_off, v_off, row_len, pos, rows);
 }
 
 }  // namespace smeg

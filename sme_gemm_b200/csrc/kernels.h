@@ -214,7 +214,8 @@ constexpr int kTpMaxGrid = 160;                                    // most CTAs 
 constexpr int kTpFlagWords = kTpReadyWords + 8 * kTpMaxGrid;       // "done" from owner s, CTA b at [8 + s * kTpMaxGrid + b]
 // ---- causal attention against an f16 KV cache (attention.cu) ----
 struct AttnArgs {
-    float* out;            // [rows][heads][head_dim] f32
+    void* out;             // [rows][heads][head_dim] f32, or f16 bits
+    int out16;
     const void* q;         // rows of heads * head_dim queries, f16 bits or f32, q_stride elements apart
     size_t q_stride;
     const uint16_t* k;     // cache rows of kv_heads * head_dim f16 bits
@@ -222,8 +223,10 @@ struct AttnArgs {
     int start, rows;       // query row i attends to keys 0..=start+i
     int heads, kv_heads, head_dim;
     float scale;
+    unsigned* status;
+    int slots, q_vec;      // launcher-filled: K / V ring slots, rows of f16 queries are 16-byte aligned
 };
-cudaError_t attn_kv_causal_launch(const AttnArgs& a, int q_f32, cudaStream_t stream);
+cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream);
 cudaError_t kv_append_launch(uint16_t* kc, uint16_t* vc, const uint16_t* src, size_t stride, size_t k_off, size_t v_off, size_t row_len,
                              size_t pos, size_t rows, cudaStream_t stream);
 

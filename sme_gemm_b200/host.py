@@ -1070,9 +1070,9 @@ class KvCache:
 
     def _attend(self, q, q_stride: int, rows: int, out) -> None:
         q_f32 = 1 if q.dtype == torch.float32 else 0
-        check("smeg_attn_kv_causal_dev",
-              lib().smeg_attn_kv_causal_dev(_ptr(out), _ptr(q), q_f32, q_stride, _ptr(self._k), _ptr(self._v), self._len - rows, rows,
-                                            self._heads, self._kv_heads, self._head_dim, self._scale, _stream()))
+        name = "smeg_attn_kv_causal_f16_dev" if out.dtype == torch.float16 else "smeg_attn_kv_causal_dev"
+        check(name, getattr(lib(), name)(_ptr(out), _ptr(q), q_f32, q_stride, _ptr(self._k), _ptr(self._v), self._len - rows, rows,
+                                         self._heads, self._kv_heads, self._head_dim, self._scale, _stream()))
 
     def attend(self, q, out) -> None:
         """One query row of heads * head_dim (f32 or f16) against every cached position; out f32."""
@@ -1125,11 +1125,9 @@ class SelfAttention:
         qkv = torch.empty((m, w), dtype=torch.float16, device=x.device)
         self.qkv.forward(x, qkv, m)
         cache.extend_from(qkv, w, q_len, q_len + kv_len, m)
-        att = torch.empty((m, q_len), dtype=torch.float32, device=x.device)
+        att = torch.empty((m, q_len), dtype=torch.float16, device=x.device)
         cache._attend(qkv, w, m, att)                       # the queries are the first q_len values of each projected row
-        att16 = torch.empty((m, q_len), dtype=torch.float16, device=x.device)
-        check("smeg_f32_to_f16_dev", lib().smeg_f32_to_f16_dev(_ptr(att16), _ptr(att), m * q_len, _stream()))
-        return att16
+        return att
 
     def accumulate(self, x, cache: KvCache, y, m: int) -> None:
         """y (m x out.n f32) += out(attention(qkv(x))) for m rows of f16 x at the cache's next positions, which this appends."""

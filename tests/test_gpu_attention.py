@@ -238,3 +238,39 @@ def test_partial_product_is_the_projection_before_its_rounding(m):
     one.accumulate(x, one.cache(128), y2, m)
     torch.cuda.synchronize()
     assert torch.equal(y1, y2) and sg.last_status() == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd,start,rows,q_f32,pad", [
+    (4, 2, 64, 127, 1, False, 0), (4, 2, 64, 128, 1, True, 0), (8, 2, 128, 1023, 1, False, 16), (8, 1, 128, 4095, 1, False, 0),
+    (6, 2, 72, 300, 5, False, 8), (4, 4, 256, 600, 3, True, 0), (6, 2, 200, 130, 70, False, 3), (1, 1, 64, 0, 129, False, 0),
+    (12, 4, 64, 250, 200, False, 64), (5, 1, 48, 511, 77, True, 0), (32, 8, 128, 0, 512, False, 2048), (32, 8, 128, 385, 130, False, 0)])
+def test_attention_tiles_splits_and_ragged_key_blocks(heads, kv_heads, hd, start, rows, q_f32, pad):
+    """Edges of the 128-key blocks and 128-row tiles, heads that are no multiple of 64 depths, key ranges shared by the CTAs
+    of a cluster (with and without a range for every CTA), query rows inside wider projected rows, and the f16 result."""
+    rng = np.random.default_rng(heads * 7 + hd + start + rows)
+    cache = sg.KvCache(heads, kv_heads, hd, start + rows + 200)
+    cache._k.fill_(7.0)                                    # what lies past the last row must not count
+    cache._v.fill_(-9.0)
+    k16 = (rng.standard_normal((start + rows, kv_heads * hd)) * 0.7).astype(np.float16)
+    v16 = rng.standard_normal((start + rows, kv_heads * hd)).astype(np.float16)
+    cache.extend(torch.from_numpy(k16).cuda(), torch.from_numpy(v16).cuda())
+    q32 = rng.standard_normal((rows, heads * hd)).astype(np.float32)
+    if not q_f32:
+        q32 = q32.astype(np.float16).astype(np.float32)
+    q = torch.zeros((rows, heads * hd + pad), dtype=torch.float32 if q_f32 else torch.float16, device="cuda")
+    q[:, :heads * hd] = torch.from_numpy(q32).cuda()
+    out = torch.full((rows, heads * hd), 3.0, dtype=torch.float32, device="cuda")
+    out16 = torch.full((rows, heads * hd), 3.0, dtype=torch.float16, device="cuda")
+    cache._attend(q, heads * hd + pad, rows, out)
+    cache._attend(q, heads * hd + pad, rows, out16)
+    # the scalar statement in 64 bits (its f32 sums are within 1e-6 of it); the queries are rounded to f16 after the scale
+    qh = (q32 * np.float32(cache.scale())).astype(np.float16).astype(np.float64).reshape(rows, kv_heads, heads // kv_heads, hd)
+    kd, vd = (x.astype(np.float64).reshape(start + rows, kv_heads, hd) for x in (k16, v16))
+    s = np.einsum("ikgd,tkd->kgit", qh, kd)
+    s[:, :, np.arange(start + rows)[None, :] > start + np.arange(rows)[:, None]] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = (np.einsum("kgit,tkd->ikgd", p, vd) / p.sum(-1).transpose(2, 0, 1)[..., None]).reshape(rows, heads * hd)
+    # f32 scores of magnitude ~10 carry 1e-6, probabilities and their sums a few 2^-24 each
+    assert max_rel(out.cpu().numpy(), want) <= 2e-5
+    assert torch.equal(out16, out.half())
+    assert sg.last_status() == 0
