@@ -668,14 +668,24 @@ static bool q4_takes_direct(const smeg_q4* w, const uint16_t* a, size_t m, int b
     return q4_direct_supported(g, bf16);
 }
 
+// A whose rows TMA and the bulk copies cannot take (k no multiple of 8, or a base off a 16-byte boundary) in a zero-padded
+// copy [m][kd] out of the stream's pool; *out = nullptr where A is fine as it is.
+static int padded_rows(const uint16_t* a, size_t m, size_t k, size_t kd, cudaStream_t stream, uint16_t** out) {
+    *out = nullptr;
+    if (k == 0 || (k % 8 == 0 && ((uintptr_t)a & 15) == 0)) return 0;
+    if (cudaMallocAsync(out, m * kd * 2, stream) != cudaSuccess) return -2;
+    if (pad_rows_launch(*out, a, m, k, kd, stream) != cudaSuccess) { cudaFreeAsync(*out, stream); *out = nullptr; return -6; }
+    return 0;
+}
+
 // glu / yacc: the fused forms of the MLP block (the tensor-core GEMM, and the one-wave decode kernel at up to four rows).
 struct TpPush { float* bufs[8]; int world, rank, rows; };
 static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, const ep_desc16* ep, int bf16,
                   cudaStream_t stream, float* c32 = nullptr, int glu = 0, float* yacc = nullptr, const TpPush* push = nullptr) {
     if (!w) return -4;
-    const size_t n = w->d.n, k = w->d.k;
+    const size_t n = w->d.n, k0 = w->d.k;
     if (m == 0 || n == 0) return 0;
-    if ((!c && !c32 && !yacc) || (k && !a) || m > 0x7fffffffu || n > 0x7fffffffu || k > 0x7fffffffu) return -4;
+    if ((!c && !c32 && !yacc) || (k0 && !a) || m > 0x7fffffffu || n > 0x7fffffffu || k0 > 0x7fffffffu) return -4;
     if (w->affine) {
         if (c32 || glu || yacc) return -3;                       // the fused forms of the MLP block take Q4_0 weights
         const smeg_dense* t = nullptr;
@@ -687,11 +697,22 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     if (push && (!c32 || !q4_uses_tc(w, a, m))) return -3;
     DeviceState* ds = dev_state();
     if (!ds) return -5;
+    // Rows that are not whole 16-byte words: one or two rows are read as they are by the decode kernels; every other call
+    // moves A by TMA or bulk copies and takes a padded copy, a pass of ~2 us.  2051 x 1500 f16, us without and with it:
+    // 8 rows 8.4 / 5.5, 64 rows 67 / 16, 300 rows 299 / 20 (the kernel that reads A by halves walks the weights once per 16
+    // rows); 5001 x 4097 bf16: 1 row 17.6 / 20.3, 4 rows 23.3 / 21.6, 64 rows 478 / 27.
+    uint16_t* a_pad = nullptr;
+    size_t k = k0;
+    if (m > 2 && !q4_takes_direct(w, a, m, bf16, glu)) {
+        const int prc = padded_rows(a, m, k0, (k0 + 7) / 8 * 8, stream, &a_pad);
+        if (prc) return prc;
+        if (a_pad) { a = a_pad; k = (k0 + 7) / 8 * 8; }
+    }
     Q4GemvArgs g;
     memset(&g, 0, sizeof(g));
     EpNodeDev* ext = nullptr;
     int rc = make_ep(ep, n, &g.ep, stream, &ext);
-    if (rc) { if (ext) cudaFreeAsync(ext, stream); return rc; }
+    if (rc) { if (ext) cudaFreeAsync(ext, stream); if (a_pad) cudaFreeAsync(a_pad, stream); return rc; }
     g.codes = w->codes; g.scales = w->scales; g.a = a; g.c = c; g.c32 = c32;
     g.m = (int)m; g.n = (int)n; g.k = (int)k;
     g.n16 = (int)w->d.n16; g.k64 = (int)w->d.ku; g.nb = (int)w->d.nb;
@@ -699,7 +720,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     g.a_vec_ok = (k % 8 == 0) && ((uintptr_t)a % 16 == 0);
     g.status = ds->status;
     cudaError_t e;
-    if (q4_uses_tc(w, a, m)) {
+    if ((int)m > g_tc_min_rows && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a)) {
         GemmTcArgs t;
         memset(&t, 0, sizeof(t));
         t.codes = w->codes; t.scales = w->scales; t.a = a; t.c = c; t.c32 = c32; t.glu = glu; t.yacc = yacc;
@@ -717,6 +738,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         TcScratch sc;
         if (ws_floats && tc_scratch(stream, ws_floats, ncounters, &sc)) {
             if (ext) cudaFreeAsync(ext, stream);
+            if (a_pad) cudaFreeAsync(a_pad, stream);
             return -2;
         }
         t.ws = sc.ws;
@@ -732,6 +754,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
             TcScratch sc;
             if (tc_scratch(stream, ws_floats, ncounters, &sc)) {
                 if (ext) cudaFreeAsync(ext, stream);
+                if (a_pad) cudaFreeAsync(a_pad, stream);
                 return -2;
             }
             g.ws = sc.ws;
@@ -740,6 +763,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         e = q4_gemv_launch(g, bf16, ds->sm_count, stream);
     }
     if (ext) cudaFreeAsync(ext, stream);
+    if (a_pad) cudaFreeAsync(a_pad, stream);
     return e == cudaSuccess ? 0 : -6;
 }
 
@@ -1000,12 +1024,8 @@ int smeg_gemm_dense_dev(const smeg_dense* w, const uint16_t* a, uint16_t* c, siz
     // the token tile travels by TMA: rows of 16-byte multiples at a 16-byte aligned base.  Any other A is
     // staged through a zero-padded copy [m][kd] (the weights are already padded to kd along K)
     uint16_t* a_pad = nullptr;
-    if (k % 8 != 0 || ((uintptr_t)a & 15) != 0) {
-        if (cudaMallocAsync(&a_pad, m * w->kd * 2, stream) != cudaSuccess) return -2;
-        cudaError_t ce = cudaMemsetAsync(a_pad, 0, m * w->kd * 2, stream);
-        if (ce == cudaSuccess) ce = cudaMemcpy2DAsync(a_pad, w->kd * 2, a, k * 2, k * 2, m, cudaMemcpyDeviceToDevice, stream);
-        if (ce != cudaSuccess) { cudaFreeAsync(a_pad, stream); return -6; }
-    }
+    const int prc = padded_rows(a, m, k, w->kd, stream, &a_pad);
+    if (prc) return prc;
     const uint16_t* a_run = a_pad ? a_pad : a;
     const size_t k_run = a_pad ? w->kd : k;
     if (!gemm_tc_supported(16, (int)m, (int)k_run, 5, a_run)) { if (a_pad) cudaFreeAsync(a_pad, stream); return -3; }

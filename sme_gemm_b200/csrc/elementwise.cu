@@ -55,6 +55,25 @@ __global__ void f16_to_f32_kernel(float* __restrict__ dst, const uint16_t* __res
     if (idx < n) dst[idx] = __half2float(__ushort_as_half(src[idx]));
 }
 
+// rows x k 16-bit values to rows of kd (a multiple of 8), zeros behind the k-th: an activation matrix whose rows are no
+// multiple of 16 bytes, or that starts off a 16-byte boundary, as TMA takes it.  A thread forms one 16-byte store; its
+// eight 2-byte loads share their sectors with its neighbours' (m * k is at most a few MB: the pass is one launch, ~2 us).
+__global__ void __launch_bounds__(256) pad_rows_kernel(uint4* __restrict__ dst, const uint16_t* __restrict__ src, size_t rows, size_t k, size_t kd) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t idx = (size_t)blockIdx.x * 256 + threadIdx.x, per = kd / 8;
+    if (idx >= rows * per) return;
+    const size_t r = idx / per, d = (idx - r * per) * 8;
+    const uint16_t* s = src + r * k;
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const size_t i = d + 2 * e;
+        w[e] = (i < k ? (uint32_t)s[i] : 0u) | (i + 1 < k ? (uint32_t)s[i + 1] << 16 : 0u);
+    }
+    dst[idx] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
 // Sum over the 256 threads of a CTA (every thread gets it).
 __device__ __forceinline__ float cta_sum(float v, float* sh) {
 #pragma unroll
@@ -121,6 +140,10 @@ inline unsigned blocks_for(size_t n) { return (unsigned)((n + 255) / 256); }
 cudaError_t glu_launch(uint16_t* out, const uint16_t* both, size_t m, size_t n, uint32_t act, cudaStream_t s) {
     if (m * n == 0) return cudaSuccess;
     return launch_pdl(glu_kernel, dim3(blocks_for(m * n)), dim3(256), 0, s, out, both, m, n, act);
+}
+cudaError_t pad_rows_launch(uint16_t* dst, const uint16_t* src, size_t rows, size_t k, size_t kd, cudaStream_t s) {
+    if (rows * kd == 0) return cudaSuccess;
+    return launch_pdl(pad_rows_kernel, dim3(blocks_for(rows * (kd / 8))), dim3(256), 0, s, reinterpret_cast<uint4*>(dst), src, rows, k, kd);
 }
 cudaError_t add_f16_to_f32_launch(float* dst, const uint16_t* src, size_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;

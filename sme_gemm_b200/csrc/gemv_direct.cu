@@ -125,6 +125,18 @@ __global__ void __launch_bounds__(kDThreads, M <= 2 ? 3 : 2) q4_direct_kernel(co
     pdl_wait();                                                    // the activations may come from the kernel ahead
 
     // ---- stage the activation rows (zero past k) ----
+    if (!p.a_vec_ok) {
+        // rows that are no whole 16-byte words, or start off a 16-byte boundary: a half at a time, eight loads in flight
+        for (int r = 0; r < M; ++r)
+            for (int d0 = tid; d0 < kpad; d0 += kDThreads * 8) {
+                uint16_t v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = d0 + e * kDThreads < p.k ? p.a[(size_t)r * p.k + d0 + e * kDThreads] : (uint16_t)0;
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (d0 + e * kDThreads < kpad) As[(size_t)r * a_stride + d0 + e * kDThreads] = v[e];
+            }
+    } else
 #pragma unroll
     for (int r = 0; r < M; ++r)
     for (int d = tid * 8; d < kpad; d += kDThreads * 8) {
@@ -508,7 +520,6 @@ int direct_grid(int n16, int sm_count, int max_groups, int* cpc, int per_sm) {
 // ---- Q4 ----
 bool q4_direct_supported(const Q4GemvArgs& a, int bf16) {
     if (bf16 || a.m < 1 || a.m > 4 || a.log2_block < 5 || a.k64 < 1) return false;
-    if (a.k % 8 != 0 || !a.a_vec_ok) return false;                // 128-bit activation loads
     const size_t smem = kQ4RingBytes + (size_t)a.m * ((size_t)a.k64 * 64 + 8) * 2;
     return smem <= 100 * 1024;
 }

@@ -199,6 +199,7 @@ cudaError_t lowbit_to_dense_launch(const LowbitToQ4Args& a, uint16_t* dst, size_
 
 // ---- element-wise model ops (elementwise.cu) ----
 cudaError_t glu_launch(uint16_t* out, const uint16_t* both, size_t m, size_t n, uint32_t act, cudaStream_t s);
+cudaError_t pad_rows_launch(uint16_t* dst, const uint16_t* src, size_t rows, size_t k, size_t kd, cudaStream_t s);
 cudaError_t add_f16_to_f32_launch(float* dst, const uint16_t* src, size_t n, cudaStream_t s);
 cudaError_t act_f16_launch(uint16_t* dst, const uint16_t* src, size_t n, uint32_t act, cudaStream_t s);
 cudaError_t f32_to_f16_launch(uint16_t* dst, const float* src, size_t n, cudaStream_t s);

@@ -298,3 +298,25 @@ def test_affine_with_zero_minima_equals_the_scale_form_and_the_library_quantiser
     want = orc.matmul_q4(bits_of(a), qo, so, mo, n, k, block, m)
     sg.matmul_q4(a, wq, c1, m)
     assert max_rel(c1.float().cpu().numpy(), orc.f16_bits_to_f32(want).reshape(m, n)) <= TOL
+
+
+@pytest.mark.parametrize("m,n,k,off", [(1, 33, 9, 0), (4, 130, 1027, 0), (2, 70, 96, 1), (3, 40, 515, 0), (9, 65, 1501, 0), (16, 130, 64, 1),
+                                       (17, 2051, 1500, 0), (65, 129, 1027, 0), (130, 300, 513, 0), (300, 140, 2049, 0)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_rows_off_the_16_byte_grid(m, n, k, off, bf16):
+    """Depths that are no multiple of 8 and matrices that start off a 16-byte boundary, on every kernel: what lies around A
+    (and between the rows' ends and the next 16-byte boundary) is non-finite and must not be read into the sums."""
+    rng = np.random.default_rng(m + n + k)
+    q, s = q4_logical(rng, n, k, 32)
+    w = sg.Q4Weights.with_params(q, s, None, n, k, sg.Q4Params(32))
+    a32 = rng.standard_normal((m, k)).astype(np.float32)
+    a_bits = (orc.f32_to_bf16_bits if bf16 else orc.f32_to_f16_bits)(a32)
+    room = torch.full((m * k + 64,), float("nan"), dtype=torch.bfloat16 if bf16 else torch.float16, device="cuda")
+    a = room[off:off + m * k]
+    a.copy_((bf16_bits_dev if bf16 else f16_bits_dev)(a_bits).reshape(-1))
+    c = torch.full((m, n), 9.0, dtype=a.dtype, device="cuda")
+    (sg.matmul_q4_bf16 if bf16 else sg.matmul_q4)(a, w, c, m)
+    torch.cuda.synchronize()
+    want = orc.matmul_q4(a_bits, q, s, None, n, k, 32, m, None, bf16)
+    assert sg.last_status() == 0
+    assert max_rel(orc.t_bits_to_f32(bits_of(c), bf16), orc.t_bits_to_f32(want, bf16)) <= TOL
