@@ -48,7 +48,8 @@ int g_tc_min_rows = []() {
 }();
 
 // Rows up to which the decode calls take the direct kernels of gemv_direct.cu (plain loads, packed
-// f16 / dp4a arithmetic); 0 keeps them on the ring-staged kernels.  SMEG_DIRECT_ROWS is a tuning knob.
+// f16 / dp4a arithmetic; Q4 at most two rows: from three on its arithmetic per row costs more than q4_mma_kernel's
+// instructions); 0 keeps them on the other kernels.  SMEG_DIRECT_ROWS is a tuning knob.
 int g_direct_rows = []() {
     const char* e = getenv("SMEG_DIRECT_ROWS");
     const int v = e ? atoi(e) : 4;
@@ -591,9 +592,21 @@ int smeg_host_q1_quantize(const float* w, int layout, size_t n, size_t k, size_t
 // ---------------------------------------------------------------------------
 // device-pointer compute
 // ---------------------------------------------------------------------------
-// Whether an m-row call on these weights runs on the tensor-core GEMM (else the decode kernel).
+// Rows of the one-wave Q4 kernel.
+static int q4_direct_rows() { return g_direct_rows < 2 ? g_direct_rows : 2; }
+
+// Whether an m-row call on these weights is better off on the tensor-core GEMM than on the warp-level kernels.  Up to 16
+// rows never; up to 64 it depends on the matrix: q4_mma_kernel takes about 1.6 us and 0.29 us per 1000 units (16 columns x
+// 64 depths) and 16 rows, the GEMM about 11 us and 0.33 us per 1000 units, whatever the rows.  Measured, us, mma / tc:
+// 1536 x 1152 at 17 and 64 rows 4 / 14, 4 / 14; 4096 x 4096 at 17 rows 12 / 15; 4096 x 14336 at 17 rows 33 / 31.
+static bool q4_rows_want_tc(const smeg_q4* w, size_t m) {
+    if ((int)m <= g_tc_min_rows) return false;
+    if (m > 64 || w->d.log2_block < 5) return true;
+    const size_t units = div_up(w->d.n, 16) * w->d.ku;
+    return units * (29 * div_up(m, 16) - 33) >= 900000;
+}
 static bool q4_uses_tc(const smeg_q4* w, const uint16_t* a, size_t m) {
-    return (int)m > g_tc_min_rows && gemm_tc_supported(4, (int)m, (int)w->d.k, w->d.log2_block, a);
+    return q4_rows_want_tc(w, m) && gemm_tc_supported(4, (int)m, (int)w->d.k, w->d.log2_block, a);
 }
 
 static float half_bits_to_float(uint16_t h) {
@@ -659,13 +672,19 @@ static int q4_affine_twin(const smeg_q4* w, int bf16, const smeg_dense** out) {
 // Does a call of m rows run on the one-wave decode kernel (gemv_direct.cu)?  With glu: also that the matrix interleaves
 // whole 32-column gate / up chunks.
 static bool q4_takes_direct(const smeg_q4* w, const uint16_t* a, size_t m, int bf16, int glu) {
-    if (w->affine || q4_uses_tc(w, a, m) || g_direct_rows <= 0 || (int)m > g_direct_rows) return false;
+    if (w->affine || q4_uses_tc(w, a, m) || (int)m > q4_direct_rows()) return false;
     if (glu && w->d.n % 64 != 0) return false;
     Q4GemvArgs g;
     memset(&g, 0, sizeof(g));
     g.m = (int)m; g.n = (int)w->d.n; g.k = (int)w->d.k; g.k64 = (int)w->d.ku; g.log2_block = w->d.log2_block;
     g.a_vec_ok = (w->d.k % 8 == 0) && ((uintptr_t)a % 16 == 0);
     return q4_direct_supported(g, bf16);
+}
+
+// Can a call of m rows carry the fused stores of the MLP block (gated product, residual add) on a decode kernel?
+static bool q4_fuses_decode(const smeg_q4* w, const uint16_t* a, size_t m, int bf16, int glu) {
+    if (q4_takes_direct(w, a, m, bf16, glu)) return true;
+    return !w->affine && !q4_rows_want_tc(w, m) && w->d.log2_block >= 5 && w->d.ku >= 1 && !(glu && w->d.n % 64 != 0);
 }
 
 // A whose rows TMA and the bulk copies cannot take (k no multiple of 8, or a base off a 16-byte boundary) in a zero-padded
@@ -693,7 +712,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         if (rc) return rc;
         return smeg_gemm_dense_dev(t, a, c, m, bf16 ? 0x3f80 : 0x3c00 /* beta = 1 */, 0, ep, stream);
     }
-    if ((glu || yacc) && !q4_uses_tc(w, a, m) && !q4_takes_direct(w, a, m, bf16, glu)) return -4;
+    if ((glu || yacc) && !q4_uses_tc(w, a, m) && !q4_fuses_decode(w, a, m, bf16, glu)) return -4;
     if (push && (!c32 || !q4_uses_tc(w, a, m))) return -3;
     DeviceState* ds = dev_state();
     if (!ds) return -5;
@@ -703,7 +722,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     // rows); 5001 x 4097 bf16: 1 row 17.6 / 20.3, 4 rows 23.3 / 21.6, 64 rows 478 / 27.
     uint16_t* a_pad = nullptr;
     size_t k = k0;
-    if (m > 2 && !q4_takes_direct(w, a, m, bf16, glu)) {
+    if (!q4_takes_direct(w, a, m, bf16, glu)) {
         const int prc = padded_rows(a, m, k0, (k0 + 7) / 8 * 8, stream, &a_pad);
         if (prc) return prc;
         if (a_pad) { a = a_pad; k = (k0 + 7) / 8 * 8; }
@@ -720,7 +739,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     g.a_vec_ok = (k % 8 == 0) && ((uintptr_t)a % 16 == 0);
     g.status = ds->status;
     cudaError_t e;
-    if ((int)m > g_tc_min_rows && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a)) {
+    if (q4_rows_want_tc(w, m) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a)) {
         GemmTcArgs t;
         memset(&t, 0, sizeof(t));
         t.codes = w->codes; t.scales = w->scales; t.a = a; t.c = c; t.c32 = c32; t.glu = glu; t.yacc = yacc;
@@ -744,9 +763,12 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         t.ws = sc.ws;
         t.counters = sc.counters;
         e = gemm_tc_launch(t, bf16, grid, smem, stream);
-    } else if (g_direct_rows > 0 && (int)m <= g_direct_rows && q4_direct_supported(g, bf16)) {
+    } else if ((int)m <= q4_direct_rows() && q4_direct_supported(g, bf16)) {
         g.glu = glu; g.yacc = yacc;
         e = q4_direct_launch(g, ds->sm_count, stream);
+    } else if (q4_mma_supported(g)) {
+        g.glu = glu; g.yacc = yacc;
+        e = q4_mma_launch(g, bf16, ds->sm_count, stream);
     } else {
         size_t ws_floats = 0, ncounters = 0;
         q4_gemv_stream_plan(g, bf16, ds->sm_count, &ws_floats, &ncounters);
@@ -1224,6 +1246,15 @@ int smeg_mlp_create(const smeg_q4* gate_up, const smeg_q4* down, uint32_t gate_a
 }
 void smeg_mlp_destroy(smeg_mlp* mlp) { delete mlp; }
 
+// y += f32(f16(a @ W)): the residual add in the store of the product where a kernel has that form, else behind it through
+// `out` (m x n f16).
+static int q4_accumulate(const smeg_q4* w, const uint16_t* a, float* y, uint16_t* out, size_t m, cudaStream_t stream) {
+    if (!w->affine && (q4_uses_tc(w, a, m) || q4_fuses_decode(w, a, m, 0, 0))) return q4_dev(w, a, nullptr, m, nullptr, 0, stream, nullptr, 0, y);
+    const int rc = q4_dev(w, a, out, m, nullptr, 0, stream);
+    if (rc) return rc;
+    return add_f16_to_f32_launch(y, out, m * w->d.n, stream) == cudaSuccess ? 0 : -6;
+}
+
 // both = x @ gate_up (f16), hid = glu(both), then the down projection either
 // rounded to f16 and added into y (partial == nullptr) or left as f32 partial sums.
 static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, size_t m, cudaStream_t stream, const TpPush* push = nullptr) {
@@ -1237,8 +1268,8 @@ static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, s
     // prefill-sized batches: the gated product is formed in the gate/up GEMM's drain and the residual add in the
     // down GEMM's, with the arithmetic of the separate passes (two launches instead of four)
     if (push && !(m > 64)) return -3;
-    const bool fuse = m > 64 && h % 32 == 0 && mlp->gate_up->d.n == 2 * h && q4_uses_tc(mlp->gate_up, x, m) &&
-                      mlp->down->d.k % 8 == 0 && (int)m > g_tc_min_rows && mlp->down->d.log2_block >= 3;
+    const bool fuse = h % 32 == 0 && mlp->gate_up->d.n == 2 * h && q4_uses_tc(mlp->gate_up, x, m) &&
+                      q4_uses_tc(mlp->down, (const uint16_t*)nullptr, m);
     if (cudaMallocAsync(&ws, (fuse ? 0 : both_bytes) + hid_bytes + out_bytes, stream) != cudaSuccess) return -2;
     uint16_t* hid = (uint16_t*)ws;
     uint16_t* out = (uint16_t*)(ws + hid_bytes);
@@ -1248,8 +1279,8 @@ static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, s
         rc = q4_dev(mlp->gate_up, x, hid, m, nullptr, 0, stream, nullptr, (int)mlp->act);
         if (!rc) rc = partial ? q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, partial, 0, nullptr, push)
                               : q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, nullptr, 0, y);
-    } else if (q4_takes_direct(mlp->gate_up, x, m, 0, (int)mlp->act) && q4_takes_direct(mlp->down, hid, m, 0, 0) && mlp->gate_up->d.n == 2 * h) {
-        // decode-sized steps on the one-wave kernels: the gated product is formed where the gate/up projection's sums
+    } else if (q4_fuses_decode(mlp->gate_up, x, m, 0, (int)mlp->act) && q4_fuses_decode(mlp->down, hid, m, 0, 0) && mlp->gate_up->d.n == 2 * h) {
+        // decode-sized steps: the gated product is formed where the gate/up projection's sums
         // meet and the residual add where the down projection's do (two launches instead of four, the same arithmetic)
         rc = q4_dev(mlp->gate_up, x, hid, m, nullptr, 0, stream, nullptr, (int)mlp->act);
         if (!rc) rc = partial ? q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, partial)
@@ -1261,8 +1292,7 @@ static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, s
             if (partial) {
                 rc = push ? -3 : q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, partial);
             } else {
-                rc = q4_dev(mlp->down, hid, out, m, nullptr, 0, stream);
-                if (!rc) rc = add_f16_to_f32_launch(y, out, m * d_out, stream) == cudaSuccess ? 0 : -6;
+                rc = q4_accumulate(mlp->down, hid, y, out, m, stream);
             }
         }
     }

@@ -44,6 +44,10 @@ cudaError_t q4_gemv_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t st
 bool q4_direct_supported(const Q4GemvArgs& a, int bf16);
 cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream);
 
+// A handful of rows (row tiles beyond 32), f16 or bf16, K-blocks of 32 and up: warp-level MMAs (q4_mma.cu).
+bool q4_mma_supported(const Q4GemvArgs& a);
+cudaError_t q4_mma_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t stream);
+
 // Launch with programmatic stream serialisation allowed: when the kernel ahead in the stream has let
 // its dependents go (griddepcontrol.launch_dependents in every CTA, or its end), this kernel's CTAs
 // may start while that one drains.  Every kernel launched this way executes griddepcontrol.wait

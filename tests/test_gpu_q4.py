@@ -320,3 +320,38 @@ def test_rows_off_the_16_byte_grid(m, n, k, off, bf16):
     want = orc.matmul_q4(a_bits, q, s, None, n, k, 32, m, None, bf16)
     assert sg.last_status() == 0
     assert max_rel(orc.t_bits_to_f32(bits_of(c), bf16), orc.t_bits_to_f32(want, bf16)) <= TOL
+
+
+@pytest.mark.parametrize("m,n,k,block", [(1, 16, 64, 32), (3, 17, 72, 32), (8, 33, 520, 64), (5, 4800, 128, 32), (9, 1152, 1536, 128), (16, 9500, 264, 32),
+                                         (13, 100, 8200, 256), (17, 65, 4096, 32), (33, 640, 1000, 32), (64, 1152, 1536, 64)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_warp_level_kernel(m, n, k, block, bf16):
+    """Row tiles of 8 and 16 with rows missing, passes of one and two column groups with a group missing, depths that leave
+    warps without a unit or end inside one, an epilogue on the product."""
+    got, want, (q, s, a_bits) = run_q4(m, n, k, block, bf16, bias_relu, from_f32=False)
+    assert max_rel(got, want) <= (2e-2 if bf16 else TOL)       # one bf16 place of the product can flip through the epilogue
+    # the product itself: f32 sums of unrounded weights, so nearer to the exact product than half a place of the store
+    got, want, _ = run_q4(m, n, k, block, bf16, None)
+    assert max_rel(got, want) <= TOL
+
+
+@pytest.mark.parametrize("m", [3, 8, 16, 17, 40, 64])
+@pytest.mark.parametrize("d,f", [(256, 640), (1024, 3072)])
+def test_gated_block_in_two_launches_is_its_separate_passes(m, d, f):
+    """The gated product and the residual add in the stores of the products, at every row count that fuses them: the bits of
+    product, gate pass, product, add."""
+    rng = np.random.default_rng(m + d)
+    w = [(rng.standard_normal((f, d)) * 0.05).astype(np.float32) for _ in range(2)]
+    up = sg.GatedLinear.quantize(w[0], w[1], sg.WeightLayout.OutIn, f, d, sg.Gate.Silu)
+    down = sg.Linear.quantize((rng.standard_normal((d, f)) * 0.05).astype(np.float32), sg.WeightLayout.OutIn, d, f)
+    x = torch.from_numpy(rng.standard_normal((m, d)).astype(np.float16)).cuda()
+    y = torch.from_numpy(rng.standard_normal((m, d)).astype(np.float32)).cuda()
+    want = y.clone()
+    sg.Mlp.gated(up, down).accumulate(x, y, m)
+    hid = torch.empty((m, f), dtype=torch.float16, device="cuda")
+    up.forward(x, hid, m)
+    out = torch.empty((m, d), dtype=torch.float16, device="cuda")
+    down.forward(hid, out, m)
+    want += out.float()
+    torch.cuda.synchronize()
+    assert sg.last_status() == 0 and torch.equal(y, want)
