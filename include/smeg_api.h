@@ -285,6 +285,29 @@ void smeg_mlp_destroy(smeg_mlp *mlp);
  * x is m x k f16. */
 int smeg_mlp_accumulate_dev(smeg_mlp *mlp, const uint16_t *x, float *y, size_t m, void *stream);
 int smeg_mlp_accumulate(smeg_mlp *mlp, const uint16_t *x, float *y, size_t m);
+/* Linear::accumulate (src/linear.rs:425-432) on Q4 weights: y (m x n, f32) += f32(f16(A @ dequant(W))). */
+int smeg_matmul_q4_accumulate_dev(const smeg_q4 *w, const uint16_t *a, float *y, size_t m, void *stream);
+/* Block::accumulate (src/block.rs:90-106) as one call: x (rows x width, f32) += attn(norm1(x)), then x += mlp(norm2(x)),
+ * the new positions' keys and values at cache rows pos .. pos + rows (the caller checks the capacity).  Q4 weights
+ * without biases; mlp: the gated block, or NULL and up / down / act the plain form.  norm*_b may be NULL;
+ * norm*_rms selects rms_norm.  The same passes and bits as the single calls. */
+typedef struct smeg_block_args {
+    float *x;
+    size_t rows, width;
+    const float *norm1_w, *norm1_b;
+    const float *norm2_w, *norm2_b;
+    float norm1_eps, norm2_eps;
+    int norm1_rms, norm2_rms;
+    const smeg_q4 *qkv, *out;
+    size_t heads, kv_heads, head_dim;
+    uint16_t *k_cache, *v_cache;
+    size_t pos;
+    smeg_mlp *mlp;
+    const smeg_q4 *up, *down;
+    float scale;
+    uint32_t act;
+} smeg_block_args;
+int smeg_block_accumulate_dev(const smeg_block_args *b, void *stream);
 /* Tensor-parallel halves of the same step: `partial` (m x d, f32) receives this
  * rank's un-rounded down-projection partial sums (its rows of W_down); after the
  * ranks' partials are summed, finish applies the f16 store rounding and the

@@ -35,6 +35,17 @@ class EpDesc16(C.Structure):
     _fields_ = [("n_nodes", C.c_uint32), ("nodes", C.POINTER(EpNode))]
 
 
+class BlockArgs(C.Structure):
+    """smeg_block_args, include/smeg_api.h."""
+
+    _fields_ = [("x", C.c_void_p), ("rows", C.c_size_t), ("width", C.c_size_t), ("norm1_w", C.c_void_p), ("norm1_b", C.c_void_p),
+                ("norm2_w", C.c_void_p), ("norm2_b", C.c_void_p), ("norm1_eps", C.c_float), ("norm2_eps", C.c_float),
+                ("norm1_rms", C.c_int), ("norm2_rms", C.c_int), ("qkv", C.c_void_p), ("out", C.c_void_p), ("heads", C.c_size_t),
+                ("kv_heads", C.c_size_t), ("head_dim", C.c_size_t), ("k_cache", C.c_void_p), ("v_cache", C.c_void_p),
+                ("pos", C.c_size_t), ("mlp", C.c_void_p), ("up", C.c_void_p), ("down", C.c_void_p), ("scale", C.c_float),
+                ("act", C.c_uint32)]
+
+
 assert C.sizeof(EpNode) == 32 and EpNode.ptr.offset == 16 and EpNode.ld.offset == 24
 
 _sz, _vp, _u32, _i = C.c_size_t, C.c_void_p, C.c_uint32, C.c_int
@@ -106,6 +117,8 @@ SIGNATURES = {
     "smeg_mlp_accumulate": (_i, [_vp, _vp, _vp, _sz]),
     "smeg_mlp_partial_dev": (_i, [_vp, _vp, _vp, _sz, _vp]),
     "smeg_matmul_q4_partial_dev": (_i, [_vp, _vp, _vp, _sz, _vp]),
+    "smeg_matmul_q4_accumulate_dev": (_i, [_vp, _vp, _vp, _sz, _vp]),
+    "smeg_block_accumulate_dev": (_i, [C.POINTER(BlockArgs), _vp]),
     "smeg_kv_append_dev": (_i, [_vp, _vp, _vp, _sz, _sz, _sz, _sz, _sz, _sz, _vp]),
     "smeg_attn_kv_causal_dev": (_i, [_vp, _vp, _i, _sz, _vp, _vp, _sz, _sz, _sz, _sz, _sz, C.c_float, _vp]),
     "smeg_attn_kv_causal_f16_dev": (_i, [_vp, _vp, _i, _sz, _vp, _vp, _sz, _sz, _sz, _sz, _sz, C.c_float, _vp]),

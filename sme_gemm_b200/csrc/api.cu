@@ -1300,6 +1300,56 @@ static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, s
     return rc;
 }
 
+int smeg_block_accumulate_dev(const smeg_block_args* b, void* stream_v) {
+    if (!b || !b->x || !b->qkv || !b->out || !b->k_cache || !b->v_cache || !b->norm1_w || !b->norm2_w || (!b->mlp && (!b->up || !b->down))) return -4;
+    const size_t m = b->rows, d = b->width, q_len = b->heads * b->head_dim, kv_len = b->kv_heads * b->head_dim, w = q_len + 2 * kv_len;
+    if (m == 0) return 0;
+    const smeg_q4 *up = b->mlp ? b->mlp->gate_up : b->up, *down = b->mlp ? b->mlp->down : b->down;
+    const size_t hidden = down->d.k;
+    if (b->qkv->d.k != d || b->qkv->d.n != w || b->out->d.k != q_len || b->out->d.n != d || up->d.k != d || down->d.n != d) return -4;
+    if (!b->mlp && (up->d.n != hidden || (b->act != SMEG_ACT_GELU && b->act != SMEG_ACT_SILU))) return -4;
+    cudaStream_t stream = (cudaStream_t)stream_v;
+    // one allocation for the passes between the products: rows of the norms, of [q | k | v] (later of the hidden layer) and of
+    // the attention (later of a product that is added behind its store)
+    auto pad = [](size_t halves) { return (halves * 2 + 255) / 256 * 256; };
+    const size_t h_bytes = pad(m * d), qkv_bytes = pad(m * (b->mlp ? w : (w > hidden ? w : hidden))), att_bytes = pad(m * q_len), out_bytes = pad(m * d);
+    char* ws = nullptr;
+    if (cudaMallocAsync(&ws, h_bytes + qkv_bytes + att_bytes + out_bytes, stream) != cudaSuccess) return -2;
+    uint16_t *h = (uint16_t*)ws, *qkv = (uint16_t*)(ws + h_bytes), *att = (uint16_t*)(ws + h_bytes + qkv_bytes), *out = (uint16_t*)(ws + h_bytes + qkv_bytes + att_bytes);
+    int rc = smeg_norm_rows_dev(h, nullptr, b->x, b->norm1_w, b->norm1_b, m, d, b->norm1_eps, b->norm1_rms, stream);
+    if (!rc) rc = q4_dev(b->qkv, h, qkv, m, nullptr, 0, stream);
+    if (!rc) rc = smeg_kv_append_dev(b->k_cache, b->v_cache, qkv, w, q_len, q_len + kv_len, kv_len, b->pos, m, stream);
+    if (!rc) rc = smeg_attn_kv_causal_f16_dev(att, qkv, 0, w, b->k_cache, b->v_cache, b->pos, m, b->heads, b->kv_heads, b->head_dim, b->scale, stream);
+    if (!rc) rc = q4_accumulate(b->out, att, b->x, out, m, stream);
+    if (!rc) rc = smeg_norm_rows_dev(h, nullptr, b->x, b->norm2_w, b->norm2_b, m, d, b->norm2_eps, b->norm2_rms, stream);
+    if (!rc) {
+        if (b->mlp) {
+            rc = mlp_run(b->mlp, h, b->x, nullptr, m, stream);
+        } else {
+            EpNode node;
+            memset(&node, 0, sizeof(node));
+            node.op = 8; node.aux = b->act;                                     // the activation alone
+            const ep_desc16 ep = {1, &node};
+            rc = q4_dev(up, h, qkv, m, &ep, 0, stream);
+            if (!rc) rc = q4_accumulate(down, qkv, b->x, out, m, stream);
+        }
+    }
+    cudaFreeAsync(ws, stream);
+    return rc;
+}
+
+int smeg_matmul_q4_accumulate_dev(const smeg_q4* w, const uint16_t* a, float* y, size_t m, void* stream_v) {
+    if (!w || !y) return -4;
+    if (m == 0 || w->d.n == 0) return 0;
+    cudaStream_t stream = (cudaStream_t)stream_v;
+    const bool fused = !w->affine && (q4_uses_tc(w, a, m) || q4_fuses_decode(w, a, m, 0, 0));
+    uint16_t* out = nullptr;
+    if (!fused && cudaMallocAsync(&out, m * w->d.n * 2, stream) != cudaSuccess) return -2;
+    const int rc = q4_accumulate(w, a, y, out, m, stream);
+    if (out) cudaFreeAsync(out, stream);
+    return rc;
+}
+
 int smeg_mlp_accumulate_dev(smeg_mlp* mlp, const uint16_t* x, float* y, size_t m, void* stream) {
     return mlp_run(mlp, x, y, nullptr, m, (cudaStream_t)stream);
 }

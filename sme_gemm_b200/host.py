@@ -19,7 +19,7 @@ from enum import IntEnum
 
 import numpy as np
 
-from ._lib import EpDesc16, EpNode, SmegError, check, lib
+from ._lib import BlockArgs, EpDesc16, EpNode, SmegError, check, lib
 
 try:  # torch is plumbing for device memory and streams only
     import torch
@@ -109,8 +109,13 @@ def _ptr(x) -> int:
     return x.ctypes.data
 
 
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+if torch is not None and hasattr(torch._C, "_cuda_getCurrentRawStream"):
+    def _stream() -> int:
+        """The handle of torch's current stream on the current device (without building a Stream object: 2 us a call)."""
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+else:
+    def _stream() -> int:
+        return torch.cuda.current_stream().cuda_stream
 
 
 def _numel(x) -> int:
@@ -125,6 +130,7 @@ class Q4Weights:
 
     def __init__(self, handle, params: Q4Params):
         self._h, self._params = handle, params
+        self._n, self._k = lib().smeg_q4_n(handle), lib().smeg_q4_k(handle)      # fixed for the handle's life
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -172,10 +178,10 @@ class Q4Weights:
         return Q4Weights(h, p)
 
     def n(self) -> int:
-        return lib().smeg_q4_n(self._h)
+        return self._n
 
     def k(self) -> int:
-        return lib().smeg_q4_k(self._h)
+        return self._k
 
     def params(self) -> Q4Params:
         return self._params
@@ -196,6 +202,7 @@ class Q4Weights:
 class _LowbitWeights:
     def __init__(self, handle):
         self._h = handle
+        self._n, self._k = lib().smeg_lowbit_n(handle), lib().smeg_lowbit_k(handle)
 
     def __del__(self):
         h, self._h = getattr(self, "_h", None), None
@@ -203,10 +210,10 @@ class _LowbitWeights:
             lib().smeg_lowbit_destroy(h)
 
     def n(self) -> int:
-        return lib().smeg_lowbit_n(self._h)
+        return self._n
 
     def k(self) -> int:
-        return lib().smeg_lowbit_k(self._h)
+        return self._k
 
     def block(self) -> int:
         return lib().smeg_lowbit_block(self._h)
@@ -830,6 +837,11 @@ class Linear:
     def accumulate(self, x, y, m: int) -> None:
         """y (f32) += f32(forward(x)) -- Linear::accumulate, src/linear.rs:425-432.  Device tensors."""
         assert _is_torch(x) and _numel(y) == m * self.n(), "y is m*n"
+        if (self.q4 is not None and self.bias is None and self.rms_eps is None and y.is_contiguous() and y.dtype == torch.float32
+                and x.is_cuda and x.is_contiguous() and x.dtype == torch.float16):
+            assert _numel(x) == m * self.k(), "a is m*k"
+            check("smeg_matmul_q4_accumulate_dev", lib().smeg_matmul_q4_accumulate_dev(self.q4._h, _ptr(x), _ptr(y), m, _stream()))
+            return
         out = torch.empty((m, self.n()), dtype=torch.float16, device=x.device)
         self.forward(x, out, m)
         check("smeg_add_f16_to_f32_dev", lib().smeg_add_f16_to_f32_dev(_ptr(y), _ptr(out), m * self.n(), _stream()))
@@ -1159,10 +1171,38 @@ class Block:
     def cache(self, capacity: int) -> KvCache:
         return self.attn.cache(capacity)
 
+    def _accumulate_native(self, x, cache, rows: int) -> bool:
+        """The whole layer as one library call, for the forms that has (Q4 projections without biases or folded norms, one
+        device); False leaves every other form to its parts.  The same kernels in the same order, without a Python call and
+        an allocation around each: a 384-wide layer at one row is 8 launches of 2-3 us."""
+        n1, attn, n2, mlp = self.norm1, self.attn, self.norm2, self.mlp
+        if type(attn) is not SelfAttention or type(mlp) is not Mlp or type(n1) is not Norm or type(n2) is not Norm:
+            return False
+        up = mlp.up.inner if type(mlp.up) is GatedLinear else mlp.up
+        for lin in (attn.qkv, attn.out, up, mlp.down):
+            if type(lin) is not Linear or lin.q4 is None or lin.bias is not None or lin.rms_eps is not None:
+                return False
+        if (mlp.up is not up and mlp._h is None) or not (x.is_cuda and x.is_contiguous()) or rows <= 0:
+            return False
+        d = self.width()
+        heads, kv_heads, hd = attn._heads, attn._kv_heads, attn._head_dim
+        if n1.weight.numel() != d or type(cache) is not KvCache:
+            return False
+        assert cache._heads == heads and cache._kv_heads == kv_heads and cache._head_dim == hd, "the cache's heads match the block's"
+        assert cache._len + rows <= cache._capacity, f"{rows} rows do not fit in the cache"
+        args = BlockArgs(x.data_ptr(), rows, d, n1.weight.data_ptr(), _ptr(n1.bias), n2.weight.data_ptr(), _ptr(n2.bias), n1.eps, n2.eps,
+                         n1.is_rms, n2.is_rms, attn.qkv.q4._h, attn.out.q4._h, heads, kv_heads, hd, cache._k.data_ptr(), cache._v.data_ptr(),
+                         cache._len, mlp._h if mlp.up is not up else None, up.q4._h, mlp.down.q4._h, cache._scale, int(mlp.act or 0))
+        check("smeg_block_accumulate_dev", lib().smeg_block_accumulate_dev(C.byref(args), _stream()))
+        cache._len += rows
+        return True
+
     def accumulate(self, x, *args) -> None:
         """accumulate(x, cache, rows): both halves at the cache's next positions; accumulate(x, rows): the MLP half."""
         cache, rows = (None, args[0]) if len(args) == 1 else args
         assert _is_torch(x) and x.dtype == torch.float32 and x.numel() == rows * self.width(), "x is rows * width"
+        if cache is not None and self._accumulate_native(x, cache, rows):
+            return
         h = torch.empty((rows, self.width()), dtype=torch.float16, device=x.device)
         if cache is not None:
             assert self.attn is not None, "this block was built without its attention half"
