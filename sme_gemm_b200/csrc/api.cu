@@ -848,7 +848,7 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
             probe.qh = (const uint16_t*)1; probe.sa = (const float*)1; probe.qsum = (const int32_t*)1;   // set below
             mma = lowbit_mma_supported(probe, ds->sm_count);
         }
-        const size_t mpad = (m + 127) / 128 * 128;                     // whole row tiles of the tensor-core kernel (up to 128 rows)
+        const size_t mpad = (m + 159) / 32 * 32;                       // a row tile of the tensor-core kernel may end 127 rows past m
         const size_t q_bytes = (m * kq + 255) / 256 * 256, sa_bytes = (m * nb * 4 + 255) / 256 * 256;
         const size_t t_bytes = tc ? (mpad * nb * 4 + 255) / 256 * 256 : 0, qh_bytes = (tc || mma) ? ((m + 7) / 8 * 8 * kq * 2 + 255) / 256 * 256 : 0;
         if (cudaMallocAsync(&ws, q_bytes + 2 * sa_bytes + 2 * t_bytes + qh_bytes + 256, stream) != cudaSuccess) {
@@ -884,7 +884,7 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
                 t.m = (int)m; t.n = (int)n; t.k = (int)k; t.kq = (int)kq;
                 t.n16 = (int)w->d.n16; t.ku = (int)w->d.ku; t.nb = (int)nb; t.nb_real = (int)w->d.nb_real;
                 t.log2_block = w->d.log2_block; t.bits = w->bits; t.lut = w->lut ^ 0x80808080u; t.status = ds->status; t.ep = g.ep;
-                e = lowbit_tc_launch(t, stream);
+                e = lowbit_tc_launch(t, ds->sm_count, stream);
             } else if (mma) e = lowbit_mma_launch(g, w->bits, ds->sm_count, stream);
             else if ((int)m <= g_direct_rows && lowbit_direct_supported(g, false)) e = lowbit_direct_launch(g, w->bits, ds->sm_count, stream);
             else e = lowbit_gemv_launch(g, w->bits, ds->sm_count, stream);

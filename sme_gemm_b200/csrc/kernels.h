@@ -126,7 +126,7 @@ struct LowbitTcArgs {
     const uint16_t* qh;           // m x kq activation codes as f16 integers (act_quant_kernel)
     const float* sa_t;            // nb x mpad activation scales, block-major
     const float* qsum_t;          // nb x mpad per-block sums of q, as floats
-    int mpad;                     // m rounded up to a multiple of 128
+    int mpad;                     // row length of sa_t and qsum_t: whole row tiles of up to 128 rows from any row below m
     uint16_t* c;                  // m x n f16 bits
     int32_t* sums_out;            // optional debug: m x n x nb_real exact block sums
     int m, n, k, kq;
@@ -137,7 +137,7 @@ struct LowbitTcArgs {
     EpParams ep;
 };
 bool lowbit_tc_supported(int bits, int m, int k, int log2_block);
-cudaError_t lowbit_tc_launch(LowbitTcArgs a, cudaStream_t stream);
+cudaError_t lowbit_tc_launch(LowbitTcArgs a, int sm_count, cudaStream_t stream);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point lookup (gemm_tc.cu); null if unavailable.
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,

@@ -39,10 +39,9 @@
 //                       warp ever waits for a global load.
 //   warps 8-15 (fold)   thread = weight column: read a finished run per row (tcgen05.ld), release
 //                       the accumulator, and at the end of a K-block fold the block's integer into
-//                       the running f32 total with the block's scale (K-blocks of one run: without
-//                       leaving floating point, the integer being exact there; 128-row tiles: totals
-//                       in tensor memory); after the last block the epilogue graph runs on the
-//                       f16-rounded product and C is stored.
+//                       the running f32 total with the block's scale; after the last block the
+//                       epilogue graph runs on the f16-rounded product and C is stored.
+// K-blocks of one run take lowbit_tc_block_kernel, further down.
 // Every wait is bounded; a timed-out wait raises the status word and the kernel drains and exits.
 #include "epilogue.cuh"
 #include "kernels.h"
@@ -69,17 +68,13 @@ __device__ __forceinline__ uint32_t prmt2(uint32_t a, uint32_t b, uint32_t sel) 
 __device__ __forceinline__ uint2 widen4(uint32_t v) { return make_uint2(prmt2(v, 0u, 0x4140u), prmt2(v, 0u, 0x4342u)); }
 // TPW = rows one fold warp takes (16 or 32), DW = fold warps per lane quarter (1 or 2): the row
 // tile of a CTA is TPW * DW rows.
-// FAST: K-blocks of one run (256 depths or fewer) and no debug output -- the fold stays in floating point.
-// FAST == 2 (TPW 32, DW 2): a tile of 128 rows, so that the weights are expanded half as often; a fold warp then takes
-// 32 rows of either 64-row half, and the running totals live in tensor memory (columns 384..511: lane = weight column,
-// column = row) beside three accumulators instead of in registers.
-template <int BITS, int TPW, int DW, int FAST>
+// The general form: K-blocks of several runs (more than 256 depths), and the debug output of the block sums.
+template <int BITS, int TPW, int DW>
 __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ LowbitTcArgs p) {
-    constexpr int NT = FAST == 2 ? 128 : TPW * DW;             // rows per CTA tile
+    constexpr int NT = TPW * DW;                               // rows per CTA tile
     constexpr int ACC_STRIDE = NT < 32 ? 32 : NT;              // tensor-memory columns between accumulators
-    constexpr int NACC = FAST == 2 ? 3 : 512 / ACC_STRIDE;
-    constexpr int TOT_COL = 384;                               // FAST == 2: first column of the running totals
-    constexpr int NA = FAST == 2 ? 5 : kLtNA, NB = NA;         // ring depths: operand, rows (both tiles are 16 KB at 128 rows)
+    constexpr int NACC = 512 / ACC_STRIDE;
+    constexpr int NA = kLtNA, NB = kLtNB;                      // ring depths: operand, rows
     constexpr int UPS = BITS == 2 ? 4 : 2;                     // packed units per slot and column group (512 depths)
     constexpr int SPU = BITS == 2 ? 2 : 4;                     // stages per unit
     constexpr int KSLOT = 8 * UPS * kUnitBytes;                // bytes of a packed slot
@@ -293,84 +288,6 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
             // what turns an accumulator into S = sum u q: 2-bit sums are scaled by 2^-24, 1-bit by 2^-16 (columns g of a
             // column group) or 2^-15 (columns g + 8)
             const float unscale = BITS == 2 ? 16777216.0f : ((cl & 8) ? 32768.0f : 65536.0f);
-            if (FAST == 2) {
-                // ---- 128 rows: rows 32 part .. 32 part + 31 of either 64-row half, totals in tensor memory ----
-                const uint32_t acc_base = tmem_base + ((uint32_t)(32 * q) << 16);
-                const uint32_t tot_base = acc_base + (uint32_t)TOT_COL;
-                {
-                    const uint32_t z[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-#pragma unroll
-                    for (int pass = 0; pass < 2; ++pass)
-#pragma unroll
-                        for (int j0 = 0; j0 < 32; j0 += 8) tmem_st8(tot_base + (uint32_t)(64 * pass + 32 * part + j0), z);
-                    tmem_st_wait();
-                }
-                bool ok = true;
-                for (int blk = 0; blk < p.nb_real && ok; ++blk) {              // one run per block: run counter = blk
-                    const int fs = blk % kLtNF, buf = blk % NACC;
-                    ok = mbar_wait_poll(&acc_full[buf], (blk / NACC) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT);
-                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-                    ok = mbar_wait_poll(&f_full[fs], (blk / kLtNF) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT);
-                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-                    tc_fence_after();
-                    const unsigned char* fo = ring_f + (size_t)fs * FSLOT;
-                    const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off)));
-#pragma unroll
-                    for (int pass = 0; pass < 2; ++pass) {
-                        const int ro = 64 * pass + 32 * part;                  // first row of this pass within the tile
-                        const float* sa = reinterpret_cast<const float*>(fo) + ro;
-                        const float* qf = reinterpret_cast<const float*>(fo + NT * 4) + ro;
-#pragma unroll
-                        for (int hf = 0; hf < 2; ++hf) {
-                            // sixteen accumulator values and their totals: two loads in flight, one wait
-                            uint32_t av[16], tt[16];
-                            if (pass == 0 && hf == 0) tmem_st_wait();              // the totals stored in the block before
-                            tmem_ld16(acc_base + (uint32_t)(buf * ACC_STRIDE + ro + 16 * hf), av);
-                            tmem_ld16(tot_base + (uint32_t)(ro + 16 * hf), tt);
-                            tmem_ld_wait();
-                            if (pass == 1 && hf == 1) {
-                                // the accumulator has been read: hand it back to the MMA warp
-                                tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) mbar_arrive(&acc_empty[buf]);
-                            }
-#pragma unroll
-                            for (int j0 = 0; j0 < 16; j0 += 4) {
-                                const float4 s0 = *reinterpret_cast<const float4*>(sa + 16 * hf + j0);
-                                const float4 q0 = *reinterpret_cast<const float4*>(qf + 16 * hf + j0);
-                                const float sv[4] = {s0.x, s0.y, s0.z, s0.w};
-                                const float qv[4] = {q0.x, q0.y, q0.z, q0.w};
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const float a = __uint_as_float(av[j0 + j]);
-                                    const float sumf = BITS == 1 ? fmaf(a, 2.0f * unscale, -qv[j]) : fmaf(a, unscale, __fmul_rn(qv[j], -128.0f));
-                                    tt[j0 + j] = __float_as_uint(fmaf(sumf, __fmul_rn(scale, sv[j]), __uint_as_float(tt[j0 + j])));
-                                }
-                            }
-                            tmem_st16(tot_base + (uint32_t)(ro + 16 * hf), tt);
-                        }
-                    }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&f_empty[fs]);
-                }
-                tmem_st_wait();
-                if (ok) {                                                      // (warp-uniform: the tensor-memory loads take whole warps)
-#pragma unroll
-                    for (int pass = 0; pass < 2; ++pass)
-#pragma unroll
-                        for (int j0 = 0; j0 < 32; j0 += 8) {
-                            uint32_t tt[8];
-                            tmem_ld8(tot_base + (uint32_t)(64 * pass + 32 * part + j0), tt);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const int row = tok0 + 64 * pass + 32 * part + j0 + j;
-                                if (row < p.m && col < p.n)
-                                    p.c[(size_t)row * p.n + col] = ep_store_value<0>(p.ep, __uint_as_float(tt[j]), (size_t)row, (size_t)col);
-                            }
-                        }
-                }
-            } else {
             float tot[TPW];
 #pragma unroll
             for (int j = 0; j < TPW; ++j) tot[j] = 0.0f;
@@ -379,51 +296,6 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
             int ri = 0;                                                     // run counter
             for (int blk = 0; blk < p.nb_real && ok; ++blk) {
                 const int fs = blk % kLtNF;
-                if (FAST) {
-                    // One run per block: the accumulator holds S / unscale exactly, so the block's integer sum as a
-                    // float -- what (float)sum is -- comes from one exact fused multiply-add, without the two
-                    // conversions: 2 S - sum(q) = fma(acc, 2 unscale, -sum(q)); S - 128 sum(q) = fma(acc, unscale, -128 sum(q)).
-                    const int buf = ri % NACC;
-                    ok = mbar_wait_poll(&acc_full[buf], (ri / NACC) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT);
-                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-                    tc_fence_after();
-                    uint32_t av[TPW];                                          // every load in flight before the one wait
-                    if constexpr (TPW == 32) {
-                        tmem_ld32(lane_base + (uint32_t)(buf * ACC_STRIDE), av);
-                    } else {
-#pragma unroll
-                        for (int j0 = 0; j0 < TPW; j0 += 8) {
-                            uint32_t r[8];
-                            tmem_ld8(lane_base + (uint32_t)(buf * ACC_STRIDE + j0), r);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) av[j0 + j] = r[j];
-                        }
-                    }
-                    tmem_ld_wait();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[buf]);
-                    ++ri;
-                    ok = mbar_wait_poll(&f_full[fs], (blk / kLtNF) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT);
-                    if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
-                    const unsigned char* fo = ring_f + (size_t)fs * FSLOT;
-                    const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off)));
-                    const float* sa = reinterpret_cast<const float*>(fo) + part * TPW;
-                    const float* qf = reinterpret_cast<const float*>(fo + NT * 4) + part * TPW;
-#pragma unroll
-                    for (int j0 = 0; j0 < TPW; j0 += 4) {
-                        const float4 s0 = *reinterpret_cast<const float4*>(sa + j0);
-                        const float4 q0 = *reinterpret_cast<const float4*>(qf + j0);
-                        const float sv[4] = {s0.x, s0.y, s0.z, s0.w};
-                        const float qv[4] = {q0.x, q0.y, q0.z, q0.w};
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float a = __uint_as_float(av[j0 + j]);
-                            const float sumf = BITS == 1 ? fmaf(a, 2.0f * unscale, -qv[j]) : fmaf(a, unscale, __fmul_rn(qv[j], -128.0f));
-                            tot[j0 + j] = fmaf(sumf, __fmul_rn(scale, sv[j]), tot[j0 + j]);
-                        }
-                    }
-                } else {
                 int sblk[TPW];                                              // the block's integer sums
 #pragma unroll
                 for (int j = 0; j < TPW; ++j) sblk[j] = 0;
@@ -470,7 +342,6 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
                         tot[j0 + j] = fmaf((float)sum, __fmul_rn(scale, sv[j]), tot[j0 + j]);
                     }
                 }
-                }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&f_empty[fs]);
             }
@@ -480,7 +351,6 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
                     const int row = row0 + j;
                     if (row < p.m) p.c[(size_t)row * p.n + col] = ep_store_value<0>(p.ep, tot[j], (size_t)row, (size_t)col);
                 }
-            }
             }
         }
     }
@@ -492,9 +362,324 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
     }
 }
 
-template <int BITS, int TPW, int DW, int FAST>
+// ------------------------------------------------------------------------------------------------------------------
+// K-blocks of one run (16 to 256 depths), the form every model's call takes.  The roles are those above; what differs is
+// the cost per depth of the single-warp chains.  Measured at one 64-deep stage per hand-off the MMA warp took ~1080 cycles
+// a stage whatever the tile (each wait ~120, four instructions and two commits ~310, ring arithmetic ~340), everything
+// else waiting for it.  Here a stage is 128 depths, its operand and row tiles share one pair of barriers (a wait and a
+// commit each), accumulators are asked for only where a run begins, and ring positions are counters.
+//   warps 0-7 (expand)  two groups of four warps take alternate stages, a warp two column groups; lanes of odd column
+//                       write the two 32-deep steps of a tile in the other order, so that stores are free of bank conflicts
+//   warps 8-23 (fold)   four warps per lane quarter, NT / 4 rows each, totals in registers; two rows per instruction
+//                       (f32x2), the block's integer from one exact fused multiply-add
+// NT rows per CTA are chosen by the launcher.  1-bit 512 x 4096 x 14336: 219 us with 64-deep stages.
+constexpr int kLbThreads = 32 * 28;
+constexpr int kLbNK = 3, kLbNF = 6;               // ring depths: packed slots (two units a column group), fold operands
+constexpr int kLbKSlot = 8 * 2 * kUnitBytes;
+__host__ __device__ constexpr int lb_slots(int nt) { return nt >= 96 ? 3 : 4; }
+__host__ __device__ constexpr int lb_nacc(int nt) { return nt >= 96 ? 4 : 8; }
+__host__ __device__ constexpr size_t lb_smem(int nt) {
+    return 1024 + (size_t)lb_slots(nt) * (2 * kLtATile + nt * 256) + (size_t)kLbNK * kLbKSlot + 1024 + (size_t)kLbNF * (nt * 8 + 256);
+}
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack_f32x2(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack_f32x2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+struct LbRing {
+    int slot = 0;
+    unsigned phase = 0;
+    bool wrapped = false;
+    __device__ __forceinline__ void next(int n) {
+        if (++slot == n) { slot = 0; phase ^= 1u; wrapped = true; }
+    }
+};
+
+template <int BITS, int NT>
+__global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ LowbitTcArgs p) {
+    constexpr int NS = lb_slots(NT), NACC = lb_nacc(NT), ACC_STRIDE = 512 / NACC;
+    constexpr int TPW = NT / 4;                                // rows of a fold warp
+    constexpr int BTILE = NT * 128;                            // row tile of 64 depths
+    constexpr int SLOT = 2 * kLtATile + 2 * BTILE;
+    constexpr int SPK = BITS == 2 ? 2 : 4;                     // stages per packed slot
+    constexpr int FSLOT = NT * 8 + 256;
+    extern __shared__ unsigned char smem_dyn[];
+    unsigned char* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
+    unsigned char* ring_k = smem + (size_t)NS * SLOT;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ring_k + (size_t)kLbNK * kLbKSlot);
+    unsigned char* ring_f = reinterpret_cast<unsigned char*>(bars) + 1024;
+    uint64_t *full = bars, *empty = full + NS, *k_full = empty + NS, *k_empty = k_full + kLbNK, *acc_full = k_empty + kLbNK, *acc_empty = acc_full + NACC,
+             *f_full = acc_empty + NACC, *f_empty = f_full + kLbNF;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(f_empty + kLbNF);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int col0 = blockIdx.x * 128, cg0 = blockIdx.x * 8, tok0 = blockIdx.y * NT;
+    // depths that belong to a real K-block and are staged (>= k: what lies past k multiplies zero activations)
+    const int k_end = (int)min((long long)p.nb_real << p.log2_block, (long long)p.kq);
+    const int stages = (k_end + 127) >> 7;
+
+    if (tid == 0) {
+        for (int s = 0; s < NS; ++s) { mbar_init(&full[s], 5); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < kLbNK; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 4 * SPK); }
+        for (int s = 0; s < NACC; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 16); }
+        for (int s = 0; s < kLbNF; ++s) { mbar_init(&f_full[s], 1); mbar_init(&f_empty[s], 16); }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    pdl_launch_dependents();
+    pdl_wait();                                                // (before the allocation: the kernel ahead may still hold tensor memory)
+    if (warp == 25) {
+        tmem_alloc(tmem_slot, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 24) {                                          // ---- row tiles ----
+        if (lane == 0) {
+            tma_prefetch_desc(&tmap_q);
+            LbRing r;
+            for (int i = 0; i < stages; ++i, r.next(NS)) {
+                if (r.wrapped && !mbar_wait(&empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT)) break;
+                unsigned char* b = smem + (size_t)r.slot * SLOT + 2 * kLtATile;
+                mbar_expect_tx(&full[r.slot], 2 * BTILE);
+                tma_load_2d(b, &tmap_q, i * 128, tok0, &full[r.slot]);
+                tma_load_2d(b + BTILE, &tmap_q, i * 128 + 64, tok0, &full[r.slot]);
+            }
+        }
+    } else if (warp == 26) {                                   // ---- packed weights: lane c = column group c ----
+        LbRing r;
+        const size_t cgi = (size_t)min(cg0 + (lane & 7), p.n16 - 1);             // a tail group re-reads the last one
+        for (int u0 = 0; u0 * (BITS == 2 ? kQ2UnitDepth : kQ1UnitDepth) < k_end; u0 += 2, r.next(kLbNK)) {
+            if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&k_empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+            const int units = min(2, p.ku - u0);
+            if (lane == 0) mbar_expect_tx(&k_full[r.slot], (unsigned)(8 * units * kUnitBytes));
+            __syncwarp();
+            if (lane < 8)
+                bulk_g2s(ring_k + (size_t)r.slot * kLbKSlot + (size_t)lane * 2 * kUnitBytes, p.codes + (cgi * p.ku + (size_t)u0) * kUnitBytes,
+                         units * kUnitBytes, &k_full[r.slot]);
+            __syncwarp();
+        }
+    } else if (warp == 27) {                                   // ---- fold operands: lane 0 the rows' scales, 1 their code sums, 2-9 scale rows ----
+        LbRing r;
+        const size_t cgi = (size_t)min(cg0 + max(lane - 2, 0), p.n16 - 1);
+        for (int blk = 0; blk < p.nb_real; ++blk, r.next(kLbNF)) {
+            if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&f_empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+            unsigned char* dst = ring_f + (size_t)r.slot * FSLOT;
+            if (lane == 0) mbar_expect_tx(&f_full[r.slot], (unsigned)(NT * 8 + 8 * 32));
+            __syncwarp();
+            if (lane == 0) bulk_g2s(dst, p.sa_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
+            else if (lane == 1) bulk_g2s(dst + NT * 4, p.qsum_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
+            else if (lane < 10) bulk_g2s(dst + NT * 8 + (lane - 2) * 32, p.scales + (cgi * p.nb + (size_t)blk) * 16, 32, &f_full[r.slot]);
+            __syncwarp();
+        }
+    } else if (warp == 25) {                                   // ---- MMA ----
+        const uint32_t idesc = umma_idesc(0, 128, NT);
+        const uint64_t a_first = umma_desc_sw128(smem_u32(smem)), b_first = umma_desc_sw128(smem_u32(smem) + 2 * kLtATile);
+        LbRing r, acc;
+        const int L = p.log2_block;
+        if (L >= 7) {
+            // one accumulator per 128 or 256 depths
+            const int mask = (1 << (L - 7)) - 1;
+            for (int i = 0; i < stages; ++i, r.next(NS)) {
+                const bool first = (i & mask) == 0, last = ((i + 1) & mask) == 0 || i == stages - 1;
+                if (first && acc.wrapped && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(&full[r.slot], r.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+                tc_fence_after();
+                const uint64_t ad = a_first + (uint64_t)(r.slot * (SLOT >> 4)), bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
+                const uint32_t d = tmem + (uint32_t)(acc.slot * ACC_STRIDE);
+                if (elect_one()) {
+                    if (k_end - i * 128 >= 128) {
+#pragma unroll
+                        for (int ks = 0; ks < 8; ++ks)
+                            umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > 0 || !first);
+                    } else {
+                        for (int ks = 0; i * 128 + 16 * ks < k_end; ++ks)
+                            umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > 0 || !first);
+                    }
+                    umma_commit(&empty[r.slot]);
+                    if (last) umma_commit(&acc_full[acc.slot]);
+                }
+                __syncwarp();
+                if (last) acc.next(NACC);
+            }
+        } else {
+            // several runs per stage: an accumulator each, asked for as its run begins (the runs before it are on their way
+            // to the fold warps by then, however few accumulators there are)
+            const int steps = 1 << (L - 4);
+            bool ok = true;
+            for (int i = 0; ok && i < stages; ++i, r.next(NS)) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&full[r.slot], r.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+                if (!ok) break;
+                const uint64_t ad = a_first + (uint64_t)(r.slot * (SLOT >> 4)), bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
+                for (int k0 = 0; k0 < 8 && i * 128 + 16 * k0 < k_end; k0 += steps, acc.next(NACC)) {
+                    if (acc.wrapped) ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t d = tmem + (uint32_t)(acc.slot * ACC_STRIDE);
+                    if (elect_one()) {
+                        for (int ks = k0; ks < k0 + steps && i * 128 + 16 * ks < k_end; ++ks)
+                            umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > k0);
+                        umma_commit(&acc_full[acc.slot]);
+                    }
+                    __syncwarp();
+                }
+                if (!ok) break;
+                if (elect_one()) umma_commit(&empty[r.slot]);
+                __syncwarp();
+            }
+        }
+    } else if (warp < 8) {                                     // ---- expand ----
+        const int g = lane >> 2, t = lane & 3, group = warp >> 2, wg = warp & 3, odd = g & 1;
+        // a lane's 16 bytes of 32-deep step s land in chunk 4 s + t of rows g (low) and g + 8 (high) of a column group; lanes
+        // of odd g take step 1 first
+        const uint32_t base = smem_u32(smem) + (uint32_t)(2 * wg * 2048 + g * 128);
+        const uint32_t o0 = (uint32_t)(((4 * odd + t) ^ g) << 4), o1 = (uint32_t)(((4 * (odd ^ 1) + t) ^ g) << 4);
+        const uint32_t pk = smem_u32(ring_k) + (uint32_t)(2 * wg * 2 * kUnitBytes + lane * 16);
+        auto sts = [](uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+        };
+        LbRing r, kr;
+        if (group) r.next(NS);
+        for (int i = group; i < stages; i += 2, r.next(NS), r.next(NS)) {
+            const int part = i & (SPK - 1);                    // stage within its packed slot
+            if (i >= SPK && part == group) kr.next(kLbNK);
+            if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(&k_full[kr.slot], kr.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+            const uint32_t at = base + (uint32_t)(r.slot * SLOT);
+            // 2-bit: a unit is the stage; 1-bit: words 0, 1 or 2, 3 of a unit
+            const uint32_t src = pk + (uint32_t)(kr.slot * kLbKSlot + (BITS == 2 ? part : part >> 1) * kUnitBytes);
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+                uint32_t w[4];
+                if (BITS == 2) {
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(src + cc * 2 * kUnitBytes) : "memory");
+                } else {
+                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(src + cc * 2 * kUnitBytes + (uint32_t)(part & 1) * 8) : "memory");
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {                  // 64-deep tile
+                    const uint32_t dst = at + (uint32_t)(cc * 2048 + h * kLtATile);
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {              // step s ^ odd
+                        const uint32_t lo = dst + (s ? o1 : o0), hi = lo + 1024;
+                        if (BITS == 1) {
+                            // A sign bit stays where it lies in its half word: bit b of an f16 is the number 2^(b-24) for
+                            // b < 12, and act_quant_kernel has left the codes of a run of eight depths in the order
+                            // 0 2 1 3 4 6 5 7, scaled by 2^8 2^8 1 1 2^6 2^6 2^-2 2^-2: every product of column g is
+                            // u q 2^-16 and of column g + 8 (one bit higher) u q 2^-15.  One AND per register.
+                            const uint32_t v = w[h] >> (4 * (s ^ odd));
+                            sts(lo, v & 0x00010001u, v & 0x01000100u, v & 0x00040004u, v & 0x04000400u);
+                            sts(hi, v & 0x00020002u, v & 0x02000200u, v & 0x00080008u, v & 0x08000800u);
+                        } else {
+                            const uint32_t x = (s ^ odd) ? w[2 * h + 1] : w[2 * h];
+                            const uint32_t e = x & 0x33333333u, o = (x >> 2) & 0x33333333u;
+                            const uint2 l0 = widen4(prmt2(p.lut, 0u, e)), l1 = widen4(prmt2(p.lut, 0u, e >> 16));
+                            const uint2 h0 = widen4(prmt2(p.lut, 0u, o)), h1 = widen4(prmt2(p.lut, 0u, o >> 16));
+                            sts(lo, l0.x, l0.y, l1.x, l1.y);
+                            sts(hi, h0.x, h0.y, h1.x, h1.y);
+                        }
+                    }
+                }
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&full[r.slot]);
+                mbar_arrive(&k_empty[kr.slot]);
+            }
+        }
+    } else {                                                   // ---- fold: thread = weight column, registers = rows ----
+        const int dw = warp - 8, q = dw & 3, part = dw >> 2;
+        const int cl = 32 * q + lane, col = col0 + cl;
+        const uint32_t acc_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(part * TPW);
+        const int sc_off = NT * 8 + (cl >> 4) * 32 + scale_slot(cl & 15) * 2;    // this column's scale inside a fold slot
+        // An accumulator is S = sum u q times 2^-24 (2-bit), 2^-16 or 2^-15 (1-bit, columns g and g + 8), exactly; the block's
+        // integer is 2 S - sum(q) (1-bit) or S - 128 sum(q).  nsum = fma(acc, mul, sum(q)) is minus that (2-bit: a 128th of
+        // it), exactly, and its factor carries the sign (and the 128) back: nsum * -(scale * sa) is the reference's product.
+        const float mul = BITS == 2 ? -131072.0f : ((cl & 8) ? -65536.0f : -131072.0f);
+        const f32x2 mul2 = pack_f32x2(mul, mul);
+        f32x2 tot[TPW / 2];
+#pragma unroll
+        for (int j = 0; j < TPW / 2; ++j) tot[j] = 0ull;
+        LbRing acc, fr;
+        bool ok = true;
+        for (int blk = 0; blk < p.nb_real; ++blk, acc.next(NACC), fr.next(kLbNF)) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&f_full[fr.slot], fr.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            if (!ok) break;
+            const unsigned char* fo = ring_f + (size_t)fr.slot * FSLOT;
+            const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off)));
+            const float ns = BITS == 2 ? -128.0f * scale : -scale;
+            const f32x2 ns2 = pack_f32x2(ns, ns);
+            const ulonglong2* sa = reinterpret_cast<const ulonglong2*>(fo + part * TPW * 4);
+            const ulonglong2* qf = reinterpret_cast<const ulonglong2*>(fo + NT * 4 + part * TPW * 4);
+            ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc.slot], acc.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            if (!ok) break;
+            tc_fence_after();
+            constexpr int CH = TPW < 16 ? 8 : (TPW == 24 ? 8 : 16);              // accumulator values read at a time
+#pragma unroll
+            for (int c0 = 0; c0 < TPW; c0 += CH) {
+                uint32_t av[CH];
+                if constexpr (CH == 16) tmem_ld16(acc_base + (uint32_t)(acc.slot * ACC_STRIDE + c0), av);
+                else tmem_ld8(acc_base + (uint32_t)(acc.slot * ACC_STRIDE + c0), av);
+                tmem_ld_wait();
+                if (c0 + CH == TPW) {
+                    // the accumulator has been read: hand it back to the MMA warp
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&acc_empty[acc.slot]);
+                }
+#pragma unroll
+                for (int j = 0; j < CH; j += 4) {
+                    const ulonglong2 s2 = sa[(c0 + j) / 4], q2 = qf[(c0 + j) / 4];
+                    const f32x2 n0 = fma_f32x2(pack_f32x2(__uint_as_float(av[j]), __uint_as_float(av[j + 1])), mul2, q2.x);
+                    const f32x2 n1 = fma_f32x2(pack_f32x2(__uint_as_float(av[j + 2]), __uint_as_float(av[j + 3])), mul2, q2.y);
+                    f32x2* to = tot + (c0 + j) / 2;
+                    to[0] = fma_f32x2(n0, mul_f32x2(ns2, s2.x), to[0]);
+                    to[1] = fma_f32x2(n1, mul_f32x2(ns2, s2.y), to[1]);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&f_empty[fr.slot]);
+        }
+        if (ok && col < p.n) {
+#pragma unroll
+            for (int j = 0; j < TPW; j += 2) {
+                float a, b;
+                unpack_f32x2(tot[j / 2], a, b);
+                const int row = tok0 + part * TPW + j;
+                if (row < p.m) p.c[(size_t)row * p.n + col] = ep_store_value<0>(p.ep, a, (size_t)row, (size_t)col);
+                if (row + 1 < p.m) p.c[(size_t)(row + 1) * p.n + col] = ep_store_value<0>(p.ep, b, (size_t)(row + 1), (size_t)col);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 25) {
+        tc_fence_after();
+        tmem_dealloc(tmem, 512);
+    }
+}
+
+template <int BITS, int TPW, int DW>
 cudaError_t launch_lt(const CUtensorMap& tm, const LowbitTcArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kern = lowbit_tc_kernel<BITS, TPW, DW, FAST>;
+    auto kern = lowbit_tc_kernel<BITS, TPW, DW>;
     static int attr_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -507,6 +692,20 @@ cudaError_t launch_lt(const CUtensorMap& tm, const LowbitTcArgs& a, dim3 grid, s
     return cudaGetLastError();
 }
 
+template <int BITS, int NT>
+cudaError_t launch_lb(const CUtensorMap& tm, const LowbitTcArgs& a, dim3 grid, cudaStream_t stream) {
+    auto kern = lowbit_tc_block_kernel<BITS, NT>;
+    static int attr_dev = -1;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (attr_dev != dev) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lb_smem(NT));
+        if (e != cudaSuccess) return e;
+        attr_dev = dev;
+    }
+    return launch_pdl(kern, grid, dim3(kLbThreads), lb_smem(NT), stream, tm, a);
+}
+
 }  // namespace
 
 bool lowbit_tc_supported(int bits, int m, int k, int log2_block) {
@@ -516,18 +715,21 @@ bool lowbit_tc_supported(int bits, int m, int k, int log2_block) {
     return tensor_map_encoder() != nullptr;
 }
 
-// an MMA of 128 weight columns takes 16 rows or more
-int lowbit_tc_row_tile(int m) { return m <= 16 ? 16 : (m <= 32 ? 32 : 64); }
-// ... and 128 rows where the floating-point fold applies, the rows fill more than one 64-row tile and at most one
-// K-block begins per 64-deep stage: the MMA warp takes the accumulators of every run that begins in a stage before it
-// issues the stage, and the 128-row form has a ring of three (smaller blocks would wait for their own stage)
-static int lt_row_tile(int m, int fast, int log2_block) { return fast && m > 64 && log2_block >= 6 ? 128 : lowbit_tc_row_tile(m); }
-
-cudaError_t lowbit_tc_launch(LowbitTcArgs a, cudaStream_t stream) {
+cudaError_t lowbit_tc_launch(LowbitTcArgs a, int sm_count, cudaStream_t stream) {
     // blocks of one run and no debug output: the floating-point fold
-    const int fast = a.log2_block <= 8 && a.sums_out == nullptr ? 1 : 0;
-    const int nt = lt_row_tile(a.m, fast, a.log2_block);
-    const int nab = nt == 128 ? 5 : kLtNA;                         // ring depths of the kernel's NA, NB
+    const bool one_run = a.log2_block <= 8 && a.sums_out == nullptr;
+    const int col_tiles = (a.n + 127) / 128;
+    // an MMA of 128 weight columns takes 16 rows or more
+    int nt = a.m <= 16 ? 16 : (a.m <= 32 ? 32 : 64);
+    if (one_run) {
+        // rows per CTA: the fewest (waves x time of a tile); a tile costs its expansion whatever its rows, about what 100
+        // rows of fold cost
+        long long best = 0;
+        for (int t : {128, 96, 64, 32}) {
+            const long long tiles = (long long)col_tiles * ((a.m + t - 1) / t), cost = (tiles + sm_count - 1) / sm_count * (100 + t);
+            if (best == 0 || cost < best) { best = cost; nt = t; }
+        }
+    }
     CUtensorMap tm;
     const cuuint64_t gdim[2] = {(cuuint64_t)a.kq, (cuuint64_t)a.m};
     const cuuint64_t gstride[1] = {(cuuint64_t)a.kq * 2};
@@ -536,22 +738,31 @@ cudaError_t lowbit_tc_launch(LowbitTcArgs a, cudaStream_t stream) {
     CUresult r = tensor_map_encoder()(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)a.qh, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    const dim3 grid(col_tiles, (a.m + nt - 1) / nt);
+    if (one_run) {
+        if (a.bits == 2) {
+            if (nt == 32) return launch_lb<2, 32>(tm, a, grid, stream);
+            if (nt == 64) return launch_lb<2, 64>(tm, a, grid, stream);
+            if (nt == 96) return launch_lb<2, 96>(tm, a, grid, stream);
+            return launch_lb<2, 128>(tm, a, grid, stream);
+        }
+        if (nt == 32) return launch_lb<1, 32>(tm, a, grid, stream);
+        if (nt == 64) return launch_lb<1, 64>(tm, a, grid, stream);
+        if (nt == 96) return launch_lb<1, 96>(tm, a, grid, stream);
+        return launch_lb<1, 128>(tm, a, grid, stream);
+    }
     const int ups = a.bits == 2 ? 4 : 2;
     const int bslot = (nt * 128 + 1023) / 1024 * 1024;
-    const size_t smem = 1024 + (size_t)nab * kLtATile + (size_t)nab * bslot + (size_t)kLtNK * 8 * ups * kUnitBytes +
+    const size_t smem = 1024 + (size_t)kLtNA * kLtATile + (size_t)kLtNB * bslot + (size_t)kLtNK * 8 * ups * kUnitBytes +
                         1024 + (size_t)kLtNF * (nt * 8 + 256) + 64;
-    const dim3 grid((a.n + 127) / 128, (a.m + nt - 1) / nt);
-#define SMEG_LT(B, F)                                                                  \
-    if (a.bits == B && fast == F) {                                                    \
-        if (nt == 16) return launch_lt<B, 16, 1, F>(tm, a, grid, smem, stream);        \
-        if (nt == 32) return launch_lt<B, 16, 2, F>(tm, a, grid, smem, stream);        \
-        if (nt == 128) return launch_lt<B, 32, 2, 2 * F>(tm, a, grid, smem, stream);   \
-        return launch_lt<B, 32, 2, F>(tm, a, grid, smem, stream);                      \
+    if (a.bits == 2) {
+        if (nt == 16) return launch_lt<2, 16, 1>(tm, a, grid, smem, stream);
+        if (nt == 32) return launch_lt<2, 16, 2>(tm, a, grid, smem, stream);
+        return launch_lt<2, 32, 2>(tm, a, grid, smem, stream);
     }
-    SMEG_LT(2, 0) SMEG_LT(2, 1)
-    SMEG_LT(1, 0) SMEG_LT(1, 1)
-#undef SMEG_LT
-    return cudaErrorInvalidValue;
+    if (nt == 16) return launch_lt<1, 16, 1>(tm, a, grid, smem, stream);
+    if (nt == 32) return launch_lt<1, 16, 2>(tm, a, grid, smem, stream);
+    return launch_lt<1, 32, 2>(tm, a, grid, smem, stream);
 }
 
 }  // namespace smeg

@@ -225,3 +225,29 @@ def test_many_rows_on_the_tensor_cores_are_the_reference_bits(m, n, k):
         want = orc.lowbit_matmul(a_bits, 1, signs, 0, scales, None, n, k, block, m)
         assert np.array_equal(_canon16(bits_of(c)), _canon16(want)), f"q1 {m}x{n}x{k} block {block}"
     assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k,block", [(17, 129, 256, 16), (33, 300, 1000, 32), (65, 130, 640, 64), (97, 128, 1501, 128), (129, 200, 700, 256),
+                                         (300, 70, 384, 128), (32, 2000, 130, 256), (220, 1100, 2048, 64)])
+@pytest.mark.parametrize("kind", [1, 2])
+def test_row_tiles_of_the_block_kernel(kind, m, n, k, block):
+    """Every row tile (32 to 128 rows) with rows and columns missing, accumulators of one stage, of two and several to a stage,
+    depths that end inside a stage; rows of zeros, infinities and NaN among the others."""
+    rng = np.random.default_rng(m + n + k + kind)
+    nbk = -(-k // block)
+    scales = orc.f32_to_f16_bits((rng.standard_normal(n * nbk) * 0.02).astype(np.float32))
+    scales[:3] = (0x7c00, 0x0001, 0x8000)                        # an infinite, a subnormal and a negative zero scale
+    a32 = rng.standard_normal((m, k)).astype(np.float32) * 3
+    a32[1], a32[3, k // 2], a32[5, 0], a32[m - 1, k - 1] = 0.0, np.nan, np.inf, -65504.0
+    a_bits = orc.f32_to_f16_bits(a32)
+    wbits = rng.integers(0, 256, (k * n * kind + 7) // 8).astype(np.uint8)
+    book = BOOKS[m % 3]
+    w = (sg.Q2Weights.new(wbits, scales, n, k, sg.Q2Params(block).with_codebook(book)) if kind == 2
+         else sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block))
+    c = torch.full((m, n), 9.0, dtype=torch.float16, device="cuda")
+    (sg.matmul_q2 if kind == 2 else sg.matmul_q1)(f16_bits_dev(a_bits), w, c, m)
+    torch.cuda.synchronize()
+    assert sg.last_status() == 0
+    want = orc.lowbit_matmul(a_bits, kind, wbits, 1 if kind == 2 else 0, scales, book if kind == 2 else None, n, k, block, m)
+    want = want[0] if isinstance(want, tuple) else want
+    assert np.array_equal(_canon16(bits_of(c)).reshape(-1), _canon16(want).reshape(-1))
