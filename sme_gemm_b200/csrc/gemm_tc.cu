@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
     if (warp == kDeqWarps) {
         // ===================== token producer =====================
         if (lane == 0) {
+            pdl_wait();                                        // the activations may come from the kernel ahead; the weights never do
             RingPos tp;
             for (int i = 0; i < num_stages; ++i, tp.next(NT)) {
                 const int slot = tp.slot;
@@ -736,6 +737,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
         // the kernel behind in the stream (the depth-split reduce, the tensor-parallel finish) may be scheduled from here
         // on: it waits (griddepcontrol.wait) for this grid to complete before it touches anything
         pdl_launch_dependents();
+        pdl_wait();                                                // C, y and the workspace may still be in use by the kernel ahead
         const int ntok = p.ntok_pad;                               // a multiple of 32
         const int parts = (ntok % 64 == 0) ? 4 : 2;                // every part is whole groups of 16 tokens
         const int splits = (int)gridDim.z;
@@ -904,23 +906,23 @@ cudaError_t launch_tc(const CUtensorMap& tm, const CUtensorMap& tc, const CUtens
         maps.codes = tw;
         maps.scales = ts;
     }
-    if (CG == 2) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(kTcThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 2;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, kern, maps, a);
-    }
-    kern<<<grid, kTcThreads, smem, stream>>>(maps, a);
-    return cudaGetLastError();
+    // launched while the kernel ahead drains: barriers, tensor memory, the first packed slots and their expansion come before
+    // the wait for it
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kTcThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 2;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = CG == 2 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, maps, a);
 }
 
 }  // namespace
