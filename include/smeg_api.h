@@ -263,8 +263,7 @@ int smeg_gemm_dense(const smeg_dense *w, const uint16_t *a, uint16_t *c, size_t 
  * q is f16 bits (q_f32 = 0) or f32 rows of heads * head_dim values q_stride elements apart, out f32 [rows][heads *
  * head_dim].  Per head softmax(f16(q * scale) . k) @ v with f32 sums and f32 probabilities.  head_dim a multiple of 8 in
  * 8..=256 and heads a positive multiple of kv_heads (-4 otherwise, where the reference panics); -3 beyond 65535 rows or
- * heads.  The products are formed 128 keys at a time, so a non-finite value among the next 127 cached rows after the last
- * attended one reaches the row as well (0 * inf).
+ * heads and beyond ~50 k keys.
  * smeg_attn_kv_causal_f16_dev -- the same with the result rounded to f16, as the out projection takes it. */
 int smeg_kv_append_dev(uint16_t *k_cache, uint16_t *v_cache, const uint16_t *src, size_t src_stride, size_t k_off,
                        size_t v_off, size_t row_len, size_t pos, size_t rows, void *stream);

@@ -1215,6 +1215,7 @@ static int attn_dev(void* out, int out16, const void* q, int q_f32, size_t q_str
     if (kv_heads == 0 || heads == 0 || heads % kv_heads != 0 || q_stride < heads * head_dim) return -4;
     if (((uintptr_t)k & 15) != 0 || ((uintptr_t)v & 15) != 0) return -4;
     if (start + rows > 0x7fffffffu || heads > 65535 || rows > 65535) return -3;
+    if (head_dim + 8 + start + rows > 50 * 1024) return -3;                    // about 50 k keys: the bound callers have been given
     DeviceState* ds = dev_state();
     if (!ds) return -5;
     AttnArgs a;

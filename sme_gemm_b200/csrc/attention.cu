@@ -141,6 +141,48 @@ __device__ __forceinline__ void store8(const AttnArgs& p, size_t off, const floa
     }
 }
 
+// Eight depths of one (query row, head) by the scalar statement.  The products above are formed a key block at a time with
+// the probabilities in two parts, so an infinity or NaN among the values reaches rows that do not attend to it (0 * inf) and
+// an infinity turns into NaN (inf * 0 in the low part): a row whose result is not finite is formed again here.
+template <int QF32>
+__device__ __noinline__ void attend_exact8(const AttnArgs& p, int i, int head, int c, float (&v)[8]) {
+    const int hd = p.head_dim, ld = p.kv_heads * hd, off = head / (p.heads / p.kv_heads) * hd, len = p.start + i + 1;
+    const size_t qo = (size_t)i * p.q_stride + (size_t)head * hd;
+    auto score = [&](int t) {
+        const uint16_t* kr = p.k + (size_t)t * ld + off;
+        float s = 0.0f;
+        for (int d = 0; d < hd; ++d) {
+            const float x = QF32 ? reinterpret_cast<const float*>(p.q)[qo + d] : __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(p.q)[qo + d]));
+            s = __fadd_rn(s, __fmul_rn(__half2float(__float2half_rn(__fmul_rn(x, p.scale))), __half2float(__ushort_as_half(kr[d]))));
+        }
+        return s;
+    };
+    float mx = -INFINITY, sum = 0.0f;
+    for (int t = 0; t < len; ++t) mx = fmaxf(mx, score(t));
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+    for (int t = 0; t < len; ++t) {
+        const float pt = expf(__fsub_rn(score(t), mx));
+        sum += pt;
+        const uint4 x = *reinterpret_cast<const uint4*>(p.v + (size_t)t * ld + off + c);
+        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+            v[2 * e] = __fadd_rn(v[2 * e], __fmul_rn(pt, f.x));
+            v[2 * e + 1] = __fadd_rn(v[2 * e + 1], __fmul_rn(pt, f.y));
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(v[e], sum);
+}
+__device__ __forceinline__ bool all_finite(const float (&v)[8]) {
+    bool ok = true;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ok = ok && fabsf(v[e]) <= 3.402823466e38f;
+    return ok;
+}
+
 // Grid: (CTAs per tile, tiles of 128 query rows x heads of a group, KV heads); the CTAs of a tile are a cluster.
 template <int QF32, int OUT16>
 __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
@@ -359,7 +401,10 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 float v[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(__uint_as_float(r[e]) * (1.0f / kAtPScale), sum);
-                if (row < nrow) store8<OUT16>(p, dst + c, v);
+                if (row < nrow) {
+                    if (!all_finite(v)) attend_exact8<QF32>(p, i, kvh * group + g, c, v);
+                    store8<OUT16>(p, dst + c, v);
+                }
             }
         } else {
             if (half == 0) { part_m[row] = nb > 0 ? mx : -INFINITY; part_l[row] = sum; }
@@ -410,6 +455,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(v[e] * (1.0f / kAtPScale), sum);
             const int i = (row0 + r) / group, g = (row0 + r) - i * group;
+            if (!all_finite(v)) attend_exact8<QF32>(p, i, kvh * group + g, c, v);
             store8<OUT16>(p, (size_t)i * p.heads * hd + (size_t)(kvh * group + g) * hd + c, v);
         }
         tc_fence_before();

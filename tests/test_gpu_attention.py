@@ -274,3 +274,38 @@ def test_attention_tiles_splits_and_ragged_key_blocks(heads, kv_heads, hd, start
     assert max_rel(out.cpu().numpy(), want) <= 2e-5
     assert torch.equal(out16, out.half())
     assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd,start,rows", [(4, 2, 64, 100, 9), (8, 2, 128, 700, 1), (2, 2, 32, 0, 140)])
+def test_non_finite_values_stay_with_the_rows_that_attend_to_them(heads, kv_heads, hd, start, rows):
+    """An infinite value at one position: rows before it are as if it were not there, rows from it on have the infinity itself
+    (not NaN) in its depth and their other depths untouched; a NaN key at the last position makes NaN of the last row alone."""
+    rng = np.random.default_rng(heads + start)
+    n = start + rows
+    cache = sg.KvCache(heads, kv_heads, hd, n)
+    k = torch.from_numpy((rng.standard_normal((n, kv_heads * hd)) * 0.5).astype(np.float16)).cuda()
+    v = torch.from_numpy(rng.standard_normal((n, kv_heads * hd)).astype(np.float16)).cuda()
+    q = torch.from_numpy(rng.standard_normal((rows, heads * hd)).astype(np.float16)).cuda()
+    clean, bad = (torch.empty((rows, heads * hd), dtype=torch.float32, device="cuda") for _ in range(2))
+    cache.extend(k, v)
+    cache.attend_causal(q, rows, clean)
+    at = start + rows // 2
+    v[at, 5] = float("inf")                                    # KV head 0, depth 5
+    cache.clear()
+    cache.extend(k, v)
+    cache.attend_causal(q, rows, bad)
+    torch.cuda.synchronize()
+    group = heads // kv_heads
+    want = clean.clone()
+    for h in range(group):
+        want[at - start:, h * hd + 5] = float("inf")
+    assert torch.equal(torch.isinf(bad), torch.isinf(want)) and not torch.isnan(bad).any()
+    fin = torch.isfinite(want)
+    assert max_rel(bad[fin].cpu().numpy(), want[fin].cpu().numpy()) <= 2e-5
+    k[n - 1, 0] = float("nan")
+    cache.clear()
+    cache.extend(k, v)
+    cache.attend_causal(q, rows, bad)
+    torch.cuda.synchronize()
+    assert torch.isnan(bad[rows - 1, :group * hd]).all() and not torch.isnan(bad[:rows - 1]).any() and not torch.isnan(bad[:, group * hd:]).any()
+    assert sg.last_status() == 0
