@@ -596,12 +596,12 @@ int smeg_host_q1_quantize(const float* w, int layout, size_t n, size_t k, size_t
 static int q4_direct_rows() { return g_direct_rows < 2 ? g_direct_rows : 2; }
 
 // Whether an m-row call on these weights is better off on the tensor-core GEMM than on the warp-level kernels.  Up to 16
-// rows never; up to 64 it depends on the matrix: q4_mma_kernel takes about 1.6 us and 0.29 us per 1000 units (16 columns x
-// 64 depths) and 16 rows, the GEMM about 11 us and 0.33 us per 1000 units, whatever the rows.  Measured, us, mma / tc:
-// 1536 x 1152 at 17 and 64 rows 4 / 14, 4 / 14; 4096 x 4096 at 17 rows 12 / 15; 4096 x 14336 at 17 rows 33 / 31.
+// rows never; above, it depends on the matrix: q4_mma_kernel takes about 1.6 us and 0.29 us per 1000 units (16 columns x 64
+// depths) and 16 rows, the GEMM about 11 us and 0.33 us per 1000 units (more from 128 rows up).  Measured, us, mma / tc:
+// 1536 x 1152 at 17 and 64 rows 2.6 / 14, 3.2 / 14; 4096 x 4096 at 17 rows 11 / 15, at 64 rows 19 / 15.6.
 static bool q4_rows_want_tc(const smeg_q4* w, size_t m) {
     if ((int)m <= g_tc_min_rows) return false;
-    if (m > 64 || w->d.log2_block < 5) return true;
+    if (w->d.log2_block < 5) return true;
     const size_t units = div_up(w->d.n, 16) * w->d.ku;
     return units * (29 * div_up(m, 16) - 33) >= 900000;
 }
@@ -713,7 +713,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         return smeg_gemm_dense_dev(t, a, c, m, bf16 ? 0x3f80 : 0x3c00 /* beta = 1 */, 0, ep, stream);
     }
     if ((glu || yacc) && !q4_uses_tc(w, a, m) && !q4_fuses_decode(w, a, m, bf16, glu)) return -4;
-    if (push && (!c32 || !q4_uses_tc(w, a, m))) return -3;
+    if (push && (!c32 || !gemm_tc_supported(4, (int)m, (int)k0, w->d.log2_block, a))) return -3;
     DeviceState* ds = dev_state();
     if (!ds) return -5;
     // Rows that are not whole 16-byte words: one or two rows are read as they are by the decode kernels; every other call
@@ -739,7 +739,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     g.a_vec_ok = (k % 8 == 0) && ((uintptr_t)a % 16 == 0);
     g.status = ds->status;
     cudaError_t e;
-    if (q4_rows_want_tc(w, m) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a)) {
+    if ((push || q4_rows_want_tc(w, m)) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a)) {
         GemmTcArgs t;
         memset(&t, 0, sizeof(t));
         t.codes = w->codes; t.scales = w->scales; t.a = a; t.c = c; t.c32 = c32; t.glu = glu; t.yacc = yacc;
@@ -1266,11 +1266,11 @@ static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, s
     char* ws = nullptr;
     const size_t both_bytes = (m * 2 * h * 2 + 255) / 256 * 256, hid_bytes = (m * h * 2 + 255) / 256 * 256;
     const size_t out_bytes = (m * d_out * 2 + 255) / 256 * 256;
-    // prefill-sized batches: the gated product is formed in the gate/up GEMM's drain and the residual add in the
-    // down GEMM's, with the arithmetic of the separate passes (two launches instead of four)
     if (push && !(m > 64)) return -3;
-    const bool fuse = h % 32 == 0 && mlp->gate_up->d.n == 2 * h && q4_uses_tc(mlp->gate_up, x, m) &&
-                      q4_uses_tc(mlp->down, (const uint16_t*)nullptr, m);
+    // The gated product is formed where the gate/up projection's sums meet, and the residual add where the down
+    // projection's do, with the arithmetic of the separate passes (two launches instead of four), on every kernel that
+    // takes whole gate/up chunks.
+    const bool fuse = mlp->gate_up->d.n == 2 * h && (q4_fuses_decode(mlp->gate_up, x, m, 0, (int)mlp->act) || (h % 32 == 0 && q4_uses_tc(mlp->gate_up, x, m)));
     if (cudaMallocAsync(&ws, (fuse ? 0 : both_bytes) + hid_bytes + out_bytes, stream) != cudaSuccess) return -2;
     uint16_t* hid = (uint16_t*)ws;
     uint16_t* out = (uint16_t*)(ws + hid_bytes);
@@ -1278,25 +1278,11 @@ static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, s
     int rc;
     if (fuse) {
         rc = q4_dev(mlp->gate_up, x, hid, m, nullptr, 0, stream, nullptr, (int)mlp->act);
-        if (!rc) rc = partial ? q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, partial, 0, nullptr, push)
-                              : q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, nullptr, 0, y);
-    } else if (q4_fuses_decode(mlp->gate_up, x, m, 0, (int)mlp->act) && q4_fuses_decode(mlp->down, hid, m, 0, 0) && mlp->gate_up->d.n == 2 * h) {
-        // decode-sized steps: the gated product is formed where the gate/up projection's sums
-        // meet and the residual add where the down projection's do (two launches instead of four, the same arithmetic)
-        rc = q4_dev(mlp->gate_up, x, hid, m, nullptr, 0, stream, nullptr, (int)mlp->act);
-        if (!rc) rc = partial ? q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, partial)
-                              : q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, nullptr, 0, y);
     } else {
         rc = q4_dev(mlp->gate_up, x, both, m, nullptr, 0, stream);
         if (!rc) rc = glu_launch(hid, both, m, h, mlp->act, stream) == cudaSuccess ? 0 : -6;
-        if (!rc) {
-            if (partial) {
-                rc = push ? -3 : q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, partial);
-            } else {
-                rc = q4_accumulate(mlp->down, hid, y, out, m, stream);
-            }
-        }
     }
+    if (!rc) rc = partial ? q4_dev(mlp->down, hid, nullptr, m, nullptr, 0, stream, partial, 0, nullptr, push) : q4_accumulate(mlp->down, hid, y, out, m, stream);
     cudaFreeAsync(ws, stream);
     return rc;
 }

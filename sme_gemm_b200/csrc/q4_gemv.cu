@@ -1,5 +1,7 @@
 // Q4 decode GEMV / small-M GEMM for sm_100a:  C[m][n] = ep( A[m][k] @ dequant(W) ),
-// m small (rows are processed in groups of 8 per tensor-core instruction).
+// m small (rows are processed in groups of 8 per tensor-core instruction), for K-blocks
+// below 32 depths, whose scales change inside an instruction (q4_mma.cu and gemv_direct.cu
+// take the others), and for an empty depth.
 //
 // Replaces the reference's SME Q4 GEMV (run_q4_gemv1 / run_q4_gemv,
 // csrc/gemm_f16f16_q4.h:236-431, and the bf16 twin csrc/gemm_b16b16_q4.h:171-268).
@@ -15,9 +17,7 @@
 //     lane's 16-byte vector is four A fragments of mma.m16n8k16 (16 weight
 //     columns x 16 depths) -- nibbles become f16 pairs with one lop3 each, the
 //     activations are the 8-wide N operand, accumulation is f32;
-//   * per K-block the raw code sums are folded with the f32 block scale
-//     (accumulator-side scaling), or -- for bf16 and for blocks below 32 -- each
-//     weight is dequantised to exactly the reference's rounded value first;
+//   * each weight is dequantised to exactly the reference's rounded value first;
 //   * warps' partial sums are added in a fixed order through shared memory, the
 //     epilogue graph runs on the rounded product, C is stored once.
 #include <algorithm>
@@ -45,27 +45,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
-}
-
-// One packed word (8 nibbles, offset binary) -> the four A registers holding
-// the exact integer codes as f16 pairs.
-__device__ __forceinline__ void decode_word_f16(uint32_t w, uint32_t (&a)[4]) {
-    const uint32_t w8 = w >> 8;
-    uint32_t lo0 = lop3_and_or(w, 0x000f000fu, 0x64006400u);   // 1024 + u
-    uint32_t hi0 = lop3_and_or(w, 0x00f000f0u, 0x64006400u);   // 1024 + 16 u
-    uint32_t lo1 = lop3_and_or(w8, 0x000f000fu, 0x64006400u);
-    uint32_t hi1 = lop3_and_or(w8, 0x00f000f0u, 0x64006400u);
-    const __half2 off = __halves2half2(__ushort_as_half(0x6408), __ushort_as_half(0x6408));      // 1032
-    const __half2 sc16 = __halves2half2(__ushort_as_half(0x2c00), __ushort_as_half(0x2c00));     // 1/16
-    const __half2 off16 = __halves2half2(__ushort_as_half(0xd480), __ushort_as_half(0xd480));    // -72
-    __half2 r0 = __hsub2(*reinterpret_cast<__half2*>(&lo0), off);
-    __half2 r1 = __hsub2(*reinterpret_cast<__half2*>(&lo1), off);
-    __half2 r2 = __hfma2(*reinterpret_cast<__half2*>(&hi0), sc16, off16);
-    __half2 r3 = __hfma2(*reinterpret_cast<__half2*>(&hi1), sc16, off16);
-    a[0] = *reinterpret_cast<uint32_t*>(&r0);
-    a[1] = *reinterpret_cast<uint32_t*>(&r1);
-    a[2] = *reinterpret_cast<uint32_t*>(&r2);
-    a[3] = *reinterpret_cast<uint32_t*>(&r3);
 }
 
 template <int BF16>
@@ -104,7 +83,7 @@ __device__ __forceinline__ void decode_word_scaled(uint32_t w, uint32_t (&a)[4],
     a[3] = pack2<BF16>(v[3], v[7]);   // column g+8, depths +2,+3
 }
 
-template <int BF16, int OPSIDE, int MT>
+template <int BF16, int MT>
 __global__ void __launch_bounds__(kThreads) q4_gemv_kernel(const __grid_constant__ Q4GemvArgs p) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -166,7 +145,6 @@ __global__ void __launch_bounds__(kThreads) q4_gemv_kernel(const __grid_constant
         const int si = lane / per_stage, j = lane % per_stage;
         // activation chunks that start inside the round at st0: one bulk copy per row, one lane each
         auto send_a = [&](int st0) -> bool {
-            if (!p.a_vec_ok) return true;
             for (int st = st0; st < min(num_stages, st0 + round_stages); ++st) {
                 if (st % stages_per_chunk != 0) continue;
                 const int ch = st / stages_per_chunk, buf = ch & 1;
@@ -226,31 +204,19 @@ __global__ void __launch_bounds__(kThreads) q4_gemv_kernel(const __grid_constant
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
             for (int r = 0; r < 4; ++r) total[c][mt][r] = 0.0f;
-    const float zero4[4] = {0.f, 0.f, 0.f, 0.f};
-
     for (int ch = 0; ch < nchunks; ++ch) {
         const int ka0 = ch * p.ka;
         const int chunk = min(p.ka, kpad - ka0);               // depths of this chunk (multiple of 64)
         const int buf = ch & (nbuf - 1);
         uint16_t* Ab = As + buf * a_buf_halves;
         const int valid = min(chunk, p.k - ka0);                // depths that exist in A
-        if (p.a_vec_ok) {
-            if (valid < chunk) {
-                // zero the padded tail (the bulk copy writes only the first `valid` depths)
-                for (int idx = tid; idx < rows_used * (chunk - valid); idx += 32 * kConsumerWarps)
-                    Ab[(size_t)(idx / (chunk - valid)) * a_stride + valid + idx % (chunk - valid)] = 0;
-                asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumerWarps));
-            }
-            mbar_wait(&a_full[buf], (ch >> 1) & 1, abort_flag, p.status);
-        } else {
-            // rows of A are not 16-byte aligned: cooperative copy (zero padded)
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumerWarps));
-            for (int r = 0; r < rows_used; ++r) {
-                const uint16_t* src = p.a + (size_t)(row0 + r) * p.k + ka0;
-                for (int d = tid; d < chunk; d += 32 * kConsumerWarps) Ab[(size_t)r * a_stride + d] = d < valid ? src[d] : (uint16_t)0;
-            }
+        if (valid < chunk) {
+            // zero the padded tail (the bulk copy writes only the first `valid` depths)
+            for (int idx = tid; idx < rows_used * (chunk - valid); idx += 32 * kConsumerWarps)
+                Ab[(size_t)(idx / (chunk - valid)) * a_stride + valid + idx % (chunk - valid)] = 0;
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumerWarps));
         }
+        mbar_wait(&a_full[buf], (ch >> 1) & 1, abort_flag, p.status);
 
         const int st_begin = ch * stages_per_chunk, st_end = min(num_stages, st_begin + stages_per_chunk);
         for (int st = st_begin; st < st_end; ++st) {
@@ -281,43 +247,17 @@ __global__ void __launch_bounds__(kThreads) q4_gemv_kernel(const __grid_constant
                     const uint4 wv = *reinterpret_cast<const uint4*>(sbase + c * code_bytes + warp * kUnitBytes + lane * 16);
                     const uint16_t* sc = reinterpret_cast<const uint16_t*>(sbase + CG * code_bytes + c * scale_bytes);
                     const uint32_t words[4] = {wv.x, wv.y, wv.z, wv.w};
-                    if (OPSIDE) {
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            uint32_t af[4];
-                            const int d_word = d_unit + 32 * (ks >> 1) + 8 * t + 4 * (ks & 1);
-                            decode_word_scaled<BF16>(words[ks], af, sc, g, d_word - (blk0 << p.log2_block), p.log2_block);
+                    for (int ks = 0; ks < 4; ++ks) {
+                        uint32_t af[4];
+                        const int d_word = d_unit + 32 * (ks >> 1) + 8 * t + 4 * (ks & 1);
+                        decode_word_scaled<BF16>(words[ks], af, sc, g, d_word - (blk0 << p.log2_block), p.log2_block);
 #pragma unroll
-                            for (int mt = 0; mt < MT; ++mt) {
-                                const uint4& av = (ks >> 1) ? ahi[mt] : alo[mt];
-                                const uint32_t b0 = (ks & 1) ? av.z : av.x, b1 = (ks & 1) ? av.w : av.y;
-                                if (BF16) mma_bf16(total[c][mt], af, b0, b1, total[c][mt]);
-                                else mma_f16(total[c][mt], af, b0, b1, total[c][mt]);
-                            }
-                        }
-                    } else {
-                        // accumulator-side scaling: raw code sums per 32-deep half unit,
-                        // folded with the f32 block scale (block >= 32 here)
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            uint32_t af0[4], af1[4];
-                            decode_word_f16(words[2 * h], af0);
-                            decode_word_f16(words[2 * h + 1], af1);
-                            const int row = ((d_unit + 32 * h) >> p.log2_block) - blk0;
-                            // one 32-bit read: the scales of columns g and g+8 sit side by side
-                            const uint32_t sp = *reinterpret_cast<const uint32_t*>(sc + row * 16 + 2 * g);
-                            const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&sp));
-#pragma unroll
-                            for (int mt = 0; mt < MT; ++mt) {
-                                const uint4& av = h ? ahi[mt] : alo[mt];
-                                float part[4];
-                                mma_f16(part, af0, av.x, av.y, zero4);
-                                mma_f16(part, af1, av.z, av.w, part);
-                                total[c][mt][0] = fmaf(part[0], sf.x, total[c][mt][0]);
-                                total[c][mt][1] = fmaf(part[1], sf.x, total[c][mt][1]);
-                                total[c][mt][2] = fmaf(part[2], sf.y, total[c][mt][2]);
-                                total[c][mt][3] = fmaf(part[3], sf.y, total[c][mt][3]);
-                            }
+                        for (int mt = 0; mt < MT; ++mt) {
+                            const uint4& av = (ks >> 1) ? ahi[mt] : alo[mt];
+                            const uint32_t b0 = (ks & 1) ? av.z : av.x, b1 = (ks & 1) ? av.w : av.y;
+                            if (BF16) mma_bf16(total[c][mt], af, b0, b1, total[c][mt]);
+                            else mma_f16(total[c][mt], af, b0, b1, total[c][mt]);
                         }
                     }
                 }
@@ -325,7 +265,7 @@ __global__ void __launch_bounds__(kThreads) q4_gemv_kernel(const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[slot]);
         }
-        if (p.a_vec_ok && lane == 0) mbar_arrive(&a_empty[buf]);
+        if (lane == 0) mbar_arrive(&a_empty[buf]);
     }
 
     // ---- fixed-order reduction over the 8 warps, epilogue, store ----
@@ -375,59 +315,25 @@ constexpr int kSThreads = 32 * (kSWarps + 2);   // + producer warp + store warp
 
 // UPW units of one stage at once, the walk over the units innermost: their chains are independent,
 // so the instruction stream alternates between them.
-template <int BF16, int OPSIDE, int MT, int UPW>
+template <int BF16, int MT, int UPW>
 __device__ __forceinline__ void consume_units(const uint4 (&wv)[UPW], const uint16_t* sc, const uint4 (&alo)[UPW][MT],
                                               const uint4 (&ahi)[UPW][MT], int g, int t, const int (&d_unit)[UPW], int blk0,
                                               int log2_block, float (&total)[MT][4]) {
-    const float zero4[4] = {0.f, 0.f, 0.f, 0.f};
-    if (OPSIDE) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
+    for (int ks = 0; ks < 4; ++ks) {
 #pragma unroll
-            for (int u = 0; u < UPW; ++u) {
-                const uint32_t word = ks == 0 ? wv[u].x : (ks == 1 ? wv[u].y : (ks == 2 ? wv[u].z : wv[u].w));
-                uint32_t af[4];
-                const int d_word = d_unit[u] + 32 * (ks >> 1) + 8 * t + 4 * (ks & 1);
-                decode_word_scaled<BF16>(word, af, sc, g, d_word - (blk0 << log2_block), log2_block);
+        for (int u = 0; u < UPW; ++u) {
+            const uint32_t word = ks == 0 ? wv[u].x : (ks == 1 ? wv[u].y : (ks == 2 ? wv[u].z : wv[u].w));
+            uint32_t af[4];
+            const int d_word = d_unit[u] + 32 * (ks >> 1) + 8 * t + 4 * (ks & 1);
+            decode_word_scaled<BF16>(word, af, sc, g, d_word - (blk0 << log2_block), log2_block);
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    const uint4& av = (ks >> 1) ? ahi[u][mt] : alo[u][mt];
-                    const uint32_t b0 = (ks & 1) ? av.z : av.x, b1 = (ks & 1) ? av.w : av.y;
-                    if (BF16) mma_bf16(total[mt], af, b0, b1, total[mt]);
-                    else mma_f16(total[mt], af, b0, b1, total[mt]);
-                }
+            for (int mt = 0; mt < MT; ++mt) {
+                const uint4& av = (ks >> 1) ? ahi[u][mt] : alo[u][mt];
+                const uint32_t b0 = (ks & 1) ? av.z : av.x, b1 = (ks & 1) ? av.w : av.y;
+                if (BF16) mma_bf16(total[mt], af, b0, b1, total[mt]);
+                else mma_f16(total[mt], af, b0, b1, total[mt]);
             }
-        }
-    } else {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float part[UPW][MT][4];
-            float2 sf[UPW];
-#pragma unroll
-            for (int u = 0; u < UPW; ++u) {
-                uint32_t af0[4], af1[4];
-                decode_word_f16(h ? wv[u].z : wv[u].x, af0);
-                decode_word_f16(h ? wv[u].w : wv[u].y, af1);
-                const int row = ((d_unit[u] + 32 * h) >> log2_block) - blk0;
-                // one 32-bit read: the scales of columns g and g+8 sit side by side
-                const uint32_t sp = *reinterpret_cast<const uint32_t*>(sc + row * 16 + 2 * g);
-                sf[u] = __half22float2(*reinterpret_cast<const __half2*>(&sp));
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    const uint4& av = h ? ahi[u][mt] : alo[u][mt];
-                    mma_f16(part[u][mt], af0, av.x, av.y, zero4);
-                    mma_f16(part[u][mt], af1, av.z, av.w, part[u][mt]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < UPW; ++u)
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt) {
-                    total[mt][0] = fmaf(part[u][mt][0], sf[u].x, total[mt][0]);
-                    total[mt][1] = fmaf(part[u][mt][1], sf[u].x, total[mt][1]);
-                    total[mt][2] = fmaf(part[u][mt][2], sf[u].y, total[mt][2]);
-                    total[mt][3] = fmaf(part[u][mt][3], sf[u].y, total[mt][3]);
-                }
         }
     }
 }
@@ -438,7 +344,7 @@ __device__ __forceinline__ int srange_owner(int s, int total, int grid) {
     return (int)((((long long)s + 1) * grid - 1) / total);
 }
 
-template <int BF16, int OPSIDE, int MT, int UPW>
+template <int BF16, int MT, int UPW>
 __global__ void __launch_bounds__(kSThreads, 1) q4_gemv_stream_kernel(const __grid_constant__ Q4GemvArgs p) {
     constexpr int kSU = kSWarps * UPW;                               // units per stage
     constexpr int kSCodeBytes = kSU * kUnitBytes;
@@ -631,7 +537,7 @@ __global__ void __launch_bounds__(kSThreads, 1) q4_gemv_stream_kernel(const __gr
             }
         }
         if (warp < units)
-            consume_units<BF16, OPSIDE, MT, UPW>(wv, reinterpret_cast<const uint16_t*>(sbase + kSCodeBytes), alo, ahi, g, t, d_unit,
+            consume_units<BF16, MT, UPW>(wv, reinterpret_cast<const uint16_t*>(sbase + kSCodeBytes), alo, ahi, g, t, d_unit,
                                                  blk0, p.log2_block, total);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[slot]);
@@ -655,9 +561,9 @@ __global__ void __launch_bounds__(kSThreads, 1) q4_gemv_stream_kernel(const __gr
     }
 }
 
-template <int BF16, int OPSIDE, int MT>
+template <int BF16, int MT>
 cudaError_t launch(const Q4GemvArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kern = q4_gemv_kernel<BF16, OPSIDE, MT>;
+    auto kern = q4_gemv_kernel<BF16, MT>;
     static int attr_dev = -1;   // the opt-in is per device; set it once (to the maximum) per device
     int dev = 0;
     cudaGetDevice(&dev);
@@ -713,9 +619,9 @@ void q4_gemv_stream_plan(Q4GemvArgs& a, int bf16, int sm_count, size_t* ws_float
     *ncounters = (size_t)a.n16;
 }
 
-template <int BF16, int OPSIDE, int MT, int UPW>
+template <int BF16, int MT, int UPW>
 static cudaError_t launch_stream_u(const Q4GemvArgs& a, cudaStream_t stream) {
-    auto kern = q4_gemv_stream_kernel<BF16, OPSIDE, MT, UPW>;
+    auto kern = q4_gemv_stream_kernel<BF16, MT, UPW>;
     static int attr_dev = -1;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -730,19 +636,16 @@ static cudaError_t launch_stream_u(const Q4GemvArgs& a, cudaStream_t stream) {
     return launch_pdl(kern, dim3(a.sgrid), dim3(kSThreads), smem, stream, a);
 }
 
-template <int BF16, int OPSIDE, int MT>
+template <int BF16, int MT>
 static cudaError_t launch_stream(const Q4GemvArgs& a, cudaStream_t stream) {
-    return a.supw == 2 ? launch_stream_u<BF16, OPSIDE, MT, 2>(a, stream) : launch_stream_u<BF16, OPSIDE, MT, 1>(a, stream);
+    return a.supw == 2 ? launch_stream_u<BF16, MT, 2>(a, stream) : launch_stream_u<BF16, MT, 1>(a, stream);
 }
 
 cudaError_t q4_gemv_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t stream) {
-    const int opside = bf16 || a.log2_block < 5;
     if (a.sgrid > 0) {
         if (!a.ws || !a.counters) return cudaErrorInvalidValue;
-        const int smt = a.m <= 8 ? 1 : 2;
-        if (!bf16 && !opside) return smt == 1 ? launch_stream<0, 0, 1>(a, stream) : launch_stream<0, 0, 2>(a, stream);
-        if (!bf16) return smt == 1 ? launch_stream<0, 1, 1>(a, stream) : launch_stream<0, 1, 2>(a, stream);
-        return smt == 1 ? launch_stream<1, 1, 1>(a, stream) : launch_stream<1, 1, 2>(a, stream);
+        if (!bf16) return a.m <= 8 ? launch_stream<0, 1>(a, stream) : launch_stream<0, 2>(a, stream);
+        return a.m <= 8 ? launch_stream<1, 1>(a, stream) : launch_stream<1, 2>(a, stream);
     }
     const int mt = a.m <= 8 ? 1 : (a.m <= 16 ? 2 : 4);
     int cg = 4;
@@ -774,19 +677,15 @@ cudaError_t q4_gemv_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t st
     const size_t smem = 256 + (size_t)ns * stage_bytes + (size_t)nbuf * rows_used * (ka + 8) * 2 +
                         (size_t)kConsumerWarps * cg * mt * 128 * sizeof(float);
     dim3 grid((a.n16 + cg - 1) / cg, (a.m + 8 * mt - 1) / (8 * mt));
-#define SMEG_Q4_LAUNCH(B, O, M) return launch<B, O, M>(a, grid, smem, stream)
-    if (!bf16 && !opside) {
-        if (mt == 1) SMEG_Q4_LAUNCH(0, 0, 1);
-        if (mt == 2) SMEG_Q4_LAUNCH(0, 0, 2);
-        SMEG_Q4_LAUNCH(0, 0, 4);
-    } else if (!bf16) {
-        if (mt == 1) SMEG_Q4_LAUNCH(0, 1, 1);
-        if (mt == 2) SMEG_Q4_LAUNCH(0, 1, 2);
-        SMEG_Q4_LAUNCH(0, 1, 4);
+#define SMEG_Q4_LAUNCH(B, M) return launch<B, M>(a, grid, smem, stream)
+    if (!bf16) {
+        if (mt == 1) SMEG_Q4_LAUNCH(0, 1);
+        if (mt == 2) SMEG_Q4_LAUNCH(0, 2);
+        SMEG_Q4_LAUNCH(0, 4);
     } else {
-        if (mt == 1) SMEG_Q4_LAUNCH(1, 1, 1);
-        if (mt == 2) SMEG_Q4_LAUNCH(1, 1, 2);
-        SMEG_Q4_LAUNCH(1, 1, 4);
+        if (mt == 1) SMEG_Q4_LAUNCH(1, 1);
+        if (mt == 2) SMEG_Q4_LAUNCH(1, 2);
+        SMEG_Q4_LAUNCH(1, 4);
     }
 #undef SMEG_Q4_LAUNCH
 }
