@@ -374,12 +374,14 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
 //                       (f32x2), the block's integer from one exact fused multiply-add
 // NT rows per CTA are chosen by the launcher.  1-bit 512 x 4096 x 14336: 219 us with 64-deep stages.
 constexpr int kLbThreads = 32 * 28;
-constexpr int kLbNK = 3, kLbNF = 6;               // ring depths: packed slots (two units a column group), fold operands
+constexpr int kLbNK = 3, kLbNF = 3;               // ring depths: packed slots (two units a column group), fold operands
 constexpr int kLbKSlot = 8 * 2 * kUnitBytes;
 __host__ __device__ constexpr int lb_slots(int nt) { return nt >= 96 ? 3 : 4; }
-__host__ __device__ constexpr int lb_nacc(int nt) { return nt >= 96 ? 4 : 8; }
+// Accumulators change hands in groups (a wait and an arrival of every fold warp cost ~0.6 us of a K-block whatever its depth):
+// two groups of them, and a fold slot holds the operands of a group's blocks.
+__host__ __device__ constexpr int lb_group(int nt) { return nt >= 96 ? 2 : 4; }
 __host__ __device__ constexpr size_t lb_smem(int nt) {
-    return 1024 + (size_t)lb_slots(nt) * (2 * kLtATile + nt * 256) + (size_t)kLbNK * kLbKSlot + 1024 + (size_t)kLbNF * (nt * 8 + 256);
+    return 1024 + (size_t)lb_slots(nt) * (2 * kLtATile + nt * 256) + (size_t)kLbNK * kLbKSlot + 1024 + (size_t)kLbNF * lb_group(nt) * (nt * 8 + 256);
 }
 
 typedef unsigned long long f32x2;
@@ -411,7 +413,7 @@ struct LbRing {
 
 template <int BITS, int NT>
 __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ LowbitTcArgs p) {
-    constexpr int NS = lb_slots(NT), NACC = lb_nacc(NT), ACC_STRIDE = 512 / NACC;
+    constexpr int NS = lb_slots(NT), G = lb_group(NT), ACC_STRIDE = 256 / G;   // two groups of G accumulators in 512 columns
     constexpr int TPW = NT / 4;                                // rows of a fold warp
     constexpr int BTILE = NT * 128;                            // row tile of 64 depths
     constexpr int SLOT = 2 * kLtATile + 2 * BTILE;
@@ -422,8 +424,8 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
     unsigned char* ring_k = smem + (size_t)NS * SLOT;
     uint64_t* bars = reinterpret_cast<uint64_t*>(ring_k + (size_t)kLbNK * kLbKSlot);
     unsigned char* ring_f = reinterpret_cast<unsigned char*>(bars) + 1024;
-    uint64_t *full = bars, *empty = full + NS, *k_full = empty + NS, *k_empty = k_full + kLbNK, *acc_full = k_empty + kLbNK, *acc_empty = acc_full + NACC,
-             *f_full = acc_empty + NACC, *f_empty = f_full + kLbNF;
+    uint64_t *full = bars, *empty = full + NS, *k_full = empty + NS, *k_empty = k_full + kLbNK, *acc_full = k_empty + kLbNK, *acc_empty = acc_full + 2,
+             *f_full = acc_empty + 2, *f_empty = f_full + kLbNF;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(f_empty + kLbNF);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -435,7 +437,7 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
     if (tid == 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(&full[s], 5); mbar_init(&empty[s], 1); }
         for (int s = 0; s < kLbNK; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 4 * SPK); }
-        for (int s = 0; s < NACC; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 16); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], 16); }
         for (int s = 0; s < kLbNF; ++s) { mbar_init(&f_full[s], 1); mbar_init(&f_empty[s], 16); }
         *abort_flag = 0;
         fence_barrier_init();
@@ -479,31 +481,37 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
     } else if (warp == 27) {                                   // ---- fold operands: lane 0 the rows' scales, 1 their code sums, 2-9 scale rows ----
         LbRing r;
         const size_t cgi = (size_t)min(cg0 + max(lane - 2, 0), p.n16 - 1);
-        for (int blk = 0; blk < p.nb_real; ++blk, r.next(kLbNF)) {
+        for (int blk0 = 0; blk0 < p.nb_real; blk0 += G, r.next(kLbNF)) {
             if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&f_empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
-            unsigned char* dst = ring_f + (size_t)r.slot * FSLOT;
-            if (lane == 0) mbar_expect_tx(&f_full[r.slot], (unsigned)(NT * 8 + 8 * 32));
+            const int blocks = min(G, p.nb_real - blk0);
+            if (lane == 0) mbar_expect_tx(&f_full[r.slot], (unsigned)(blocks * FSLOT));
             __syncwarp();
-            if (lane == 0) bulk_g2s(dst, p.sa_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
-            else if (lane == 1) bulk_g2s(dst + NT * 4, p.qsum_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
-            else if (lane < 10) bulk_g2s(dst + NT * 8 + (lane - 2) * 32, p.scales + (cgi * p.nb + (size_t)blk) * 16, 32, &f_full[r.slot]);
+            for (int j = 0; j < blocks; ++j) {
+                const int blk = blk0 + j;
+                unsigned char* dst = ring_f + (size_t)(r.slot * G + j) * FSLOT;
+                if (lane == 0) bulk_g2s(dst, p.sa_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
+                else if (lane == 1) bulk_g2s(dst + NT * 4, p.qsum_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
+                else if (lane < 10) bulk_g2s(dst + NT * 8 + (lane - 2) * 32, p.scales + (cgi * p.nb + (size_t)blk) * 16, 32, &f_full[r.slot]);
+            }
             __syncwarp();
         }
     } else if (warp == 25) {                                   // ---- MMA ----
         const uint32_t idesc = umma_idesc(0, 128, NT);
         const uint64_t a_first = umma_desc_sw128(smem_u32(smem)), b_first = umma_desc_sw128(smem_u32(smem) + 2 * kLtATile);
-        LbRing r, acc;
+        LbRing r, acc;                                         // acc: group of accumulators; ga: the one in it
+        int ga = 0;
         const int L = p.log2_block;
         if (L >= 7) {
             // one accumulator per 128 or 256 depths
             const int mask = (1 << (L - 7)) - 1;
             for (int i = 0; i < stages; ++i, r.next(NS)) {
                 const bool first = (i & mask) == 0, last = ((i + 1) & mask) == 0 || i == stages - 1;
-                if (first && acc.wrapped && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+                if (ga == 0 && first && acc.wrapped && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
                 if (!__all_sync(0xffffffffu, mbar_wait(&full[r.slot], r.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
                 tc_fence_after();
                 const uint64_t ad = a_first + (uint64_t)(r.slot * (SLOT >> 4)), bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
-                const uint32_t d = tmem + (uint32_t)(acc.slot * ACC_STRIDE);
+                const uint32_t d = tmem + (uint32_t)((acc.slot * G + ga) * ACC_STRIDE);
+                const bool hand = last && (ga == G - 1 || i == stages - 1);
                 if (elect_one()) {
                     if (k_end - i * 128 >= 128) {
 #pragma unroll
@@ -514,35 +522,41 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
                             umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > 0 || !first);
                     }
                     umma_commit(&empty[r.slot]);
-                    if (last) umma_commit(&acc_full[acc.slot]);
+                    if (hand) umma_commit(&acc_full[acc.slot]);
                 }
                 __syncwarp();
-                if (last) acc.next(NACC);
+                if (hand) { ga = 0; acc.next(2); }
+                else if (last) ++ga;
             }
         } else {
-            // several runs per stage: an accumulator each, asked for as its run begins (the runs before it are on their way
-            // to the fold warps by then, however few accumulators there are)
+            // several runs per stage, an accumulator each; a group is asked for as its first run begins (the groups before it
+            // are on their way to the fold warps by then)
             const int steps = 1 << (L - 4);
             bool ok = true;
             for (int i = 0; ok && i < stages; ++i, r.next(NS)) {
                 ok = __all_sync(0xffffffffu, mbar_wait(&full[r.slot], r.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
                 if (!ok) break;
+                tc_fence_after();
                 const uint64_t ad = a_first + (uint64_t)(r.slot * (SLOT >> 4)), bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
-                for (int k0 = 0; k0 < 8 && i * 128 + 16 * k0 < k_end; k0 += steps, acc.next(NACC)) {
-                    if (acc.wrapped) ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t d = tmem + (uint32_t)(acc.slot * ACC_STRIDE);
+                const int left = min(8, (k_end - i * 128) >> 4);                 // K = 16 steps of the stage
+                for (int k0 = 0; k0 < left; k0 += steps) {
+                    if (ga == 0 && acc.wrapped) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
+                    const uint32_t d = tmem + (uint32_t)((acc.slot * G + ga) * ACC_STRIDE);
+                    const bool end = k0 + steps >= left, hand = ga == G - 1 || (end && i == stages - 1);
                     if (elect_one()) {
-                        for (int ks = k0; ks < k0 + steps && i * 128 + 16 * ks < k_end; ++ks)
+                        for (int ks = k0; ks < k0 + steps && ks < left; ++ks)
                             umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > k0);
-                        umma_commit(&acc_full[acc.slot]);
+                        if (hand) umma_commit(&acc_full[acc.slot]);
+                        if (end) umma_commit(&empty[r.slot]);
                     }
                     __syncwarp();
+                    if (hand) { ga = 0; acc.next(2); }
+                    else ++ga;
                 }
-                if (!ok) break;
-                if (elect_one()) umma_commit(&empty[r.slot]);
-                __syncwarp();
             }
         }
     } else if (warp < 8) {                                     // ---- expand ----
@@ -620,39 +634,44 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
         for (int j = 0; j < TPW / 2; ++j) tot[j] = 0ull;
         LbRing acc, fr;
         bool ok = true;
-        for (int blk = 0; blk < p.nb_real; ++blk, acc.next(NACC), fr.next(kLbNF)) {
+        for (int blk0 = 0; blk0 < p.nb_real; blk0 += G, acc.next(2), fr.next(kLbNF)) {
             ok = __all_sync(0xffffffffu, mbar_wait(&f_full[fr.slot], fr.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
             if (!ok) break;
-            const unsigned char* fo = ring_f + (size_t)fr.slot * FSLOT;
-            const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off)));
-            const float ns = BITS == 2 ? -128.0f * scale : -scale;
-            const f32x2 ns2 = pack_f32x2(ns, ns);
-            const ulonglong2* sa = reinterpret_cast<const ulonglong2*>(fo + part * TPW * 4);
-            const ulonglong2* qf = reinterpret_cast<const ulonglong2*>(fo + NT * 4 + part * TPW * 4);
             ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc.slot], acc.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
             if (!ok) break;
             tc_fence_after();
-            constexpr int CH = TPW < 16 ? 8 : (TPW == 24 ? 8 : 16);              // accumulator values read at a time
+            const int blocks = min(G, p.nb_real - blk0);
 #pragma unroll
-            for (int c0 = 0; c0 < TPW; c0 += CH) {
-                uint32_t av[CH];
-                if constexpr (CH == 16) tmem_ld16(acc_base + (uint32_t)(acc.slot * ACC_STRIDE + c0), av);
-                else tmem_ld8(acc_base + (uint32_t)(acc.slot * ACC_STRIDE + c0), av);
-                tmem_ld_wait();
-                if (c0 + CH == TPW) {
-                    // the accumulator has been read: hand it back to the MMA warp
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[acc.slot]);
-                }
+            for (int gi = 0; gi < G; ++gi) {
+                if (gi >= blocks) break;
+                const unsigned char* fo = ring_f + (size_t)(fr.slot * G + gi) * FSLOT;
+                const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off)));
+                const float ns = BITS == 2 ? -128.0f * scale : -scale;
+                const f32x2 ns2 = pack_f32x2(ns, ns);
+                const ulonglong2* sa = reinterpret_cast<const ulonglong2*>(fo + part * TPW * 4);
+                const ulonglong2* qf = reinterpret_cast<const ulonglong2*>(fo + NT * 4 + part * TPW * 4);
+                constexpr int CH = TPW % 16 == 0 ? 16 : 8;                       // accumulator values read at a time
 #pragma unroll
-                for (int j = 0; j < CH; j += 4) {
-                    const ulonglong2 s2 = sa[(c0 + j) / 4], q2 = qf[(c0 + j) / 4];
-                    const f32x2 n0 = fma_f32x2(pack_f32x2(__uint_as_float(av[j]), __uint_as_float(av[j + 1])), mul2, q2.x);
-                    const f32x2 n1 = fma_f32x2(pack_f32x2(__uint_as_float(av[j + 2]), __uint_as_float(av[j + 3])), mul2, q2.y);
-                    f32x2* to = tot + (c0 + j) / 2;
-                    to[0] = fma_f32x2(n0, mul_f32x2(ns2, s2.x), to[0]);
-                    to[1] = fma_f32x2(n1, mul_f32x2(ns2, s2.y), to[1]);
+                for (int c0 = 0; c0 < TPW; c0 += CH) {
+                    uint32_t av[CH];
+                    if constexpr (CH == 16) tmem_ld16(acc_base + (uint32_t)((acc.slot * G + gi) * ACC_STRIDE + c0), av);
+                    else tmem_ld8(acc_base + (uint32_t)((acc.slot * G + gi) * ACC_STRIDE + c0), av);
+                    tmem_ld_wait();
+                    if (c0 + CH == TPW && gi == blocks - 1) {
+                        // the group has been read: hand it back to the MMA warp
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&acc_empty[acc.slot]);
+                    }
+#pragma unroll
+                    for (int j = 0; j < CH; j += 4) {
+                        const ulonglong2 s2 = sa[(c0 + j) / 4], q2 = qf[(c0 + j) / 4];
+                        const f32x2 n0 = fma_f32x2(pack_f32x2(__uint_as_float(av[j]), __uint_as_float(av[j + 1])), mul2, q2.x);
+                        const f32x2 n1 = fma_f32x2(pack_f32x2(__uint_as_float(av[j + 2]), __uint_as_float(av[j + 3])), mul2, q2.y);
+                        f32x2* to = tot + (c0 + j) / 2;
+                        to[0] = fma_f32x2(n0, mul_f32x2(ns2, s2.x), to[0]);
+                        to[1] = fma_f32x2(n1, mul_f32x2(ns2, s2.y), to[1]);
+                    }
                 }
             }
             __syncwarp();
