@@ -809,81 +809,131 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
     }
 }
 
-// Adds the depth slices of a split GEMM in slice order and stores, for splits deep enough that one CTA per
-// tile would spend longer adding than the GEMM spent multiplying.  One block = all columns of a tile x 8 tokens;
-// a thread owns one column (for a gate/up matrix: one hidden unit, i.e. a gate and an up column).
+// Adds the depth slices of a split GEMM in slice order and stores.  A thread owns four consecutive columns (for a gate/up
+// matrix: four hidden units, i.e. four gate and four up columns) of kRedTok tokens, all of a slice's 16-byte loads in flight
+// before the first add; a block is 128 columns (or hidden units) x 8 kRedTok tokens of a tile.  Bound by L2: 512 x 6144, two
+// slices, 17 us with a thread per column and half of a block's threads idle.
+constexpr int kRedTok = 2;
 template <int BF16>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const __grid_constant__ GemmTcArgs p, int splits, int col_tiles) {
     pdl_launch_dependents();
     pdl_wait();                                                    // launched while the GEMM ahead of it drains
-    const int NW = p.nw, ntok = p.ntok_pad;
+    const int NW = p.nw, ntok = p.ntok_pad, ld = NW * 128;
     const int tile_id = blockIdx.x, bx = tile_id % col_tiles, by = tile_id / col_tiles;
-    const int tok0 = by * p.ntok_tile, j0 = blockIdx.y * 8;
-    const int cl = threadIdx.x;                                  // column within the CTA tile
-    const float* ws_tile = p.ws + ((size_t)tile_id * splits) * (size_t)(NW * 128) * ntok;
-    const EpNodeDev* nodes = p.ep.n_nodes <= kMaxInlineNodes ? p.ep.nodes : p.ep.ext;
+    const int cl = ((int)threadIdx.x & 31) * 4;                  // first column within the 128 (blockIdx.z: which 128 of the tile)
+    const int j0 = (int)blockIdx.y * 8 * kRedTok + ((int)threadIdx.x >> 5);
+    const int tok0 = by * p.ntok_tile + j0;
+    const float* src = p.ws + ((size_t)tile_id * splits * ntok + j0) * ld + (int)blockIdx.z * 128 + cl;
+    const size_t slice = (size_t)ntok * ld, step = (size_t)8 * ld;
+    if (tok0 >= p.m) return;
     if (p.glu) {
         const int hn = p.n >> 1, hcol = bx * 128 + cl;
-        if (cl >= 128 || hcol >= hn) return;
-        float ag[8], au[8];
+        if (hcol >= hn) return;
+        float4 ag[kRedTok], au[kRedTok];
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) ag[jj] = au[jj] = 0.0f;
+        for (int t = 0; t < kRedTok; ++t) ag[t] = au[t] = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int z = 0; z < splits; ++z) {
-            const float* src = ws_tile + ((size_t)z * ntok + j0) * (NW * 128) + cl;
-            float vg[8], vu[8];
+            float4 vg[kRedTok], vu[kRedTok];
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) {
-                vg[jj] = __ldcg(src + (size_t)jj * (NW * 128));
-                vu[jj] = __ldcg(src + (size_t)jj * (NW * 128) + 128);
+            for (int t = 0; t < kRedTok; ++t) {
+                vg[t] = __ldcg(reinterpret_cast<const float4*>(src + z * slice + t * step));
+                vu[t] = __ldcg(reinterpret_cast<const float4*>(src + z * slice + t * step + 128));
             }
 #pragma unroll
-            for (int jj = 0; jj < 8; ++jj) { ag[jj] += vg[jj]; au[jj] += vu[jj]; }
+            for (int t = 0; t < kRedTok; ++t) {
+                ag[t].x += vg[t].x; ag[t].y += vg[t].y; ag[t].z += vg[t].z; ag[t].w += vg[t].w;
+                au[t].x += vu[t].x; au[t].y += vu[t].y; au[t].z += vu[t].z; au[t].w += vu[t].w;
+            }
         }
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-            const int tok = tok0 + j0 + jj;
-            const float gv = t_to_f32<BF16>(f32_to_t<BF16>(ag[jj])), uv = t_to_f32<BF16>(f32_to_t<BF16>(au[jj]));
-            const float a = glu_gate((uint32_t)p.glu, gv);
-            if (tok < p.m) p.c[(size_t)tok * hn + hcol] = f32_to_t<BF16>(__fmul_rn(a, uv));
+        for (int t = 0; t < kRedTok; ++t) {
+            const int tok = tok0 + 8 * t;
+            if (tok >= p.m) continue;
+            const float g[4] = {ag[t].x, ag[t].y, ag[t].z, ag[t].w}, u[4] = {au[t].x, au[t].y, au[t].z, au[t].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float gv = t_to_f32<BF16>(f32_to_t<BF16>(g[e])), uv = t_to_f32<BF16>(f32_to_t<BF16>(u[e]));
+                if (hcol + e < hn) p.c[(size_t)tok * hn + hcol + e] = f32_to_t<BF16>(__fmul_rn(glu_gate((uint32_t)p.glu, gv), uv));
+            }
         }
         return;
     }
-    const int col = bx * 128 * NW + cl;
-    if (cl >= NW * 128 || col >= p.n) return;
-    float acc[8], yv[8];
+    const int col = bx * ld + (int)blockIdx.z * 128 + cl;
+    if (col >= p.n) return;
+    float acc[kRedTok][4];
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) acc[jj] = 0.0f;
-    if (p.yacc) {
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) yv[jj] = (tok0 + j0 + jj < p.m) ? p.yacc[(size_t)(tok0 + j0 + jj) * p.n + col] : 0.0f;
-    }
+    for (int t = 0; t < kRedTok; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f;
     for (int z = 0; z < splits; ++z) {
-        const float* src = ws_tile + ((size_t)z * ntok + j0) * (NW * 128) + cl;
-        float v[8];
+        float4 v[kRedTok];
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) v[jj] = __ldcg(src + (size_t)jj * (NW * 128));
+        for (int t = 0; t < kRedTok; ++t) v[t] = __ldcg(reinterpret_cast<const float4*>(src + z * slice + t * step));
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) acc[jj] += v[jj];
+        for (int t = 0; t < kRedTok; ++t) { acc[t][0] += v[t].x; acc[t][1] += v[t].y; acc[t][2] += v[t].z; acc[t][3] += v[t].w; }
     }
-    FastEp fe;
-    if (p.ep_fast) fast_ep_build<BF16>(nodes, p.ep.n_nodes, col, true, fe);
+    if (p.beta != 1.0f) {
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
-        const int tok = tok0 + j0 + jj;
-        if (tok >= p.m) continue;
-        if (p.beta != 1.0f) acc[jj] = __fmul_rn(p.beta, acc[jj]);
-        const size_t ci = p.col_major ? (size_t)col * p.m + tok : (size_t)tok * p.n + col;
-        if (p.c32) {
-            if (p.push_world) {
+        for (int t = 0; t < kRedTok; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[t][e] = __fmul_rn(p.beta, acc[t][e]);
+    }
+    const bool whole = col + 4 <= p.n && p.n % 4 == 0;             // four columns that exist, 16-byte (f32) or 8-byte (T) aligned rows
+    const EpNodeDev* nodes = p.ep.n_nodes <= kMaxInlineNodes ? p.ep.nodes : p.ep.ext;
+    if (p.c32 || p.yacc) {
+#pragma unroll
+        for (int t = 0; t < kRedTok; ++t) {
+            const int tok = tok0 + 8 * t;
+            if (tok >= p.m) continue;
+            float* dst;
+            if (p.yacc) {
+                dst = p.yacc + (size_t)tok * p.n + col;
+            } else if (p.push_world) {
                 const int owner = tok / p.push_rows;
-                p.push[owner][((size_t)p.push_rank * p.push_rows + (size_t)(tok - owner * p.push_rows)) * p.n + col] = acc[jj];
+                dst = p.push[owner] + ((size_t)p.push_rank * p.push_rows + (size_t)(tok - owner * p.push_rows)) * p.n + col;
             } else {
-                p.c32[(size_t)tok * p.n + col] = acc[jj];
+                dst = p.c32 + (size_t)tok * p.n + col;
+            }
+            if (whole && ((uintptr_t)dst & 15) == 0) {
+                float4 o = make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]);
+                if (p.yacc) {
+                    const float4 y = *reinterpret_cast<const float4*>(dst);
+                    const float2 a = round2_t<BF16>(o.x, o.y), b = round2_t<BF16>(o.z, o.w);
+                    o = make_float4(__fadd_rn(y.x, a.x), __fadd_rn(y.y, a.y), __fadd_rn(y.z, b.x), __fadd_rn(y.w, b.y));
+                }
+                *reinterpret_cast<float4*>(dst) = o;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (col + e < p.n) dst[e] = p.yacc ? __fadd_rn(dst[e], t_to_f32<BF16>(f32_to_t<BF16>(acc[t][e]))) : acc[t][e];
             }
         }
-        else if (p.yacc) p.yacc[(size_t)tok * p.n + col] = __fadd_rn(yv[jj], t_to_f32<BF16>(f32_to_t<BF16>(acc[jj])));
-        else if (p.ep_fast) p.c[ci] = fast_ep_store<BF16>(fe, acc[jj]);
-        else p.c[ci] = ep_store_nodes<BF16>(nodes, p.ep.n_nodes, acc[jj], (size_t)tok, (size_t)col);
+        return;
+    }
+    uint16_t v[kRedTok][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (col + e >= p.n) break;
+        FastEp fe;
+        if (p.ep_fast) fast_ep_build<BF16>(nodes, p.ep.n_nodes, col + e, true, fe);
+#pragma unroll
+        for (int t = 0; t < kRedTok; ++t) {
+            const int tok = tok0 + 8 * t;
+            if (tok >= p.m) continue;
+            v[t][e] = p.ep_fast ? fast_ep_store<BF16>(fe, acc[t][e])
+                                : (p.ep.n_nodes == 0 ? f32_to_t<BF16>(acc[t][e]) : ep_store_nodes<BF16>(nodes, p.ep.n_nodes, acc[t][e], (size_t)tok, (size_t)(col + e)));
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < kRedTok; ++t) {
+        const int tok = tok0 + 8 * t;
+        if (tok >= p.m) continue;
+        uint16_t* dst = p.c + (p.col_major ? (size_t)col * p.m + tok : (size_t)tok * p.n + col);
+        if (whole && !p.col_major && ((uintptr_t)dst & 7) == 0) {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(v[t][0] | (uint32_t)v[t][1] << 16, v[t][2] | (uint32_t)v[t][3] << 16);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (col + e < p.n) dst[p.col_major ? (size_t)e * p.m : (size_t)e] = v[t][e];
+        }
     }
 }
 
@@ -1116,7 +1166,7 @@ cudaError_t gemm_tc_launch(GemmTcArgs a, int bf16, dim3 grid, size_t smem, cudaS
     else if (a.us == 2) e = bf16 ? launch_tc<1, 2, 0, 1>(tm, tc, tw, ts, a, grid, smem, stream) : launch_tc<0, 2, 0, 1>(tm, tc, tw, ts, a, grid, smem, stream);
     else e = bf16 ? launch_tc<1, 1, 0, 1>(tm, tc, tw, ts, a, grid, smem, stream) : launch_tc<0, 1, 0, 1>(tm, tc, tw, ts, a, grid, smem, stream);
     if (e != cudaSuccess || !a.defer || grid.z < 2) return e;
-    const dim3 rgrid(grid.x * grid.y, a.ntok_pad / 8);
+    const dim3 rgrid(grid.x * grid.y, a.ntok_pad / (8 * kRedTok), a.glu ? 1 : a.nw);
     if (bf16) return launch_pdl(splitk_reduce_kernel<1>, rgrid, dim3(256), 0, stream, a, (int)grid.z, (int)grid.x);
     return launch_pdl(splitk_reduce_kernel<0>, rgrid, dim3(256), 0, stream, a, (int)grid.z, (int)grid.x);
 }
