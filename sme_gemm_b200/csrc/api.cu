@@ -857,7 +857,7 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
         }
         ActQuantArgs aq;
         memset(&aq, 0, sizeof(aq));
-        aq.a = a; aq.q = (int8_t*)ws; aq.sa = (float*)(ws + q_bytes);
+        aq.a = a; aq.q = (tc || mma) && !q_out ? nullptr : (int8_t*)ws; aq.sa = (float*)(ws + q_bytes);
         aq.qsum = (w->bits == 1 || tc || mma) ? (int32_t*)(ws + q_bytes + sa_bytes) : nullptr;
         aq.m = (int)m; aq.k = (int)k; aq.kq = (int)kq; aq.nbq = (int)nb; aq.log2_block = w->d.log2_block;
         if (tc) {
@@ -870,8 +870,6 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
         if (mma) {
             aq.qh = (uint16_t*)(ws + q_bytes + 2 * sa_bytes + 2 * t_bytes);
             aq.qh_perm = w->bits == 1 ? 2 : 0;                         // 1-bit: fragment order, codes scaled by position
-            // the rows up to the next multiple of eight are zero rows (the kernel's B fragments read whole tiles of eight)
-            if (m % 8 != 0) cudaMemsetAsync(aq.qh + m * kq, 0, (8 - m % 8) * kq * 2, stream);
         }
         e = act_quant_launch(aq, stream);
         g.q = aq.q; g.sa = aq.sa; g.qsum = aq.qsum; g.qh = aq.qh;

@@ -73,7 +73,7 @@ inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
 // ---- activation int8 quantisation + 2-bit / 1-bit GEMV (lowbit_gemv.cu) ----
 struct ActQuantArgs {
     const uint16_t* a;    // m x k f16 bits
-    int8_t* q;            // m x kq int8 (kq = k padded to the unit depth, pad = 0)
+    int8_t* q;            // m x kq int8 (kq = k padded to the unit depth, pad = 0); may be null
     float* sa;            // m x nbq per-block activation scales (amax / 127), padded blocks 0
     int32_t* qsum;        // m x nbq per-block sums of q (1-bit path only; may be null)
     int m, k, kq, nbq, log2_block;
@@ -82,6 +82,7 @@ struct ActQuantArgs {
     float* sa_t;          // optional: the same scales as nbq x mpad (block-major), for the tensor-core kernel
     float* qsum_t;        // optional: the same sums as nbq x mpad floats (exact: |sum| <= 128 * block < 2^24)
     int mpad;
+    int mz, a_vec_ok;     // launcher-filled: rows of qh written (zeros past m), 16-byte loads of a
 };
 cudaError_t act_quant_launch(const ActQuantArgs& a, cudaStream_t stream);
 

@@ -40,7 +40,7 @@ __device__ __forceinline__ uint32_t prmt(uint32_t lut, uint32_t sel) {
 }
 
 // ---------------------------------------------------------------------------
-// Activation quantisation: one CTA per (K-block, row).
+// Activation quantisation: one CTA per (K-block, row), for K-blocks above 1024 depths.
 // quantize_row, src/kernels/lowbit/matmul.rs:354-371.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) act_quant_kernel(ActQuantArgs p) {
@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(128) act_quant_kernel(ActQuantArgs p) {
     const size_t d0 = (size_t)b * block;
     const size_t d1 = min(d0 + block, (size_t)p.kq);
     const uint16_t* ar = p.a + (size_t)row * p.k;
-    int8_t* qr = p.q + (size_t)row * p.kq;
+    int8_t* qr = p.q ? p.q + (size_t)row * p.kq : nullptr;
 
     float mx = 0.0f;
     int has_nan = 0;
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128) act_quant_kernel(ActQuantArgs p) {
             if (r != r) v = 0;
             else v = (int)fminf(fmaxf(r, -128.0f), 127.0f);
         }
-        qr[d] = (int8_t)v;
+        if (p.q) qr[d] = (int8_t)v;
         if (p.qh) {
             // qh_perm: depths of a group of four in the order 0 2 1 3 (the fragment order of lowbit_mma_kernel);
             // 2: also scaled by position in a group of eight -- 2^8 2^8 2^0 2^0 2^6 2^6 2^-2 2^-2, all exact in f16
@@ -109,6 +109,96 @@ __global__ void __launch_bounds__(128) act_quant_kernel(ActQuantArgs p) {
         if (p.qsum) p.qsum[(size_t)row * p.nbq + b] = qsum;
         if (p.sa_t) p.sa_t[(size_t)b * p.mpad + row] = sa;
         if (p.qsum_t) p.qsum_t[(size_t)b * p.mpad + row] = (float)qsum;
+    }
+}
+
+// The same for K-blocks of up to 1024 depths: a lane takes eight consecutive depths (a 16-byte load, 16- and 8-byte stores),
+// 2 to 32 lanes a block, a warp 256 IT consecutive depths of a row.  One CTA per (block, row) as above is 16384 CTAs of two
+// dozen instructions for 512 x 4096 and took 57 us of a 167 us prefill call; this pass moves the same 12 MB in 5.
+// Rows from m to mz are written as zeros to qh (the tiles of eight rows that lowbit_mma_kernel reads).
+template <int IT>
+__global__ void __launch_bounds__(256) act_quant_warp_kernel(const __grid_constant__ ActQuantArgs p, int chunks) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int task = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5);
+    const int row = task / chunks, chunk = task - row * chunks;
+    if (row >= p.mz) return;
+    const int L = p.log2_block, seg = L < 8 ? 1 << (L - 3) : 32;           // lanes of a block
+    uint4 x[IT];
+    float mx = 0.0f;
+    int has_nan = 0;
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+        const int d = (chunk * IT + it) * 256 + lane * 8;
+        x[it] = make_uint4(0, 0, 0, 0);
+        if (row < p.m && d < p.k) {
+            const uint16_t* a = p.a + (size_t)row * p.k + d;
+            if (p.a_vec_ok) {
+                x[it] = *reinterpret_cast<const uint4*>(a);
+            } else {
+                __align__(16) uint16_t h[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) h[e] = d + e < p.k ? a[e] : (uint16_t)0;
+                x[it] = *reinterpret_cast<uint4*>(h);
+            }
+        }
+        const uint32_t w[4] = {x[it].x, x[it].y, x[it].z, x[it].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+            if (f.x != f.x || f.y != f.y) has_nan = 1;
+            mx = fmaxf(mx, fmaxf(fabsf(f.x), fabsf(f.y)));                 // (fmaxf drops a NaN)
+        }
+    }
+    for (int o = seg >> 1; o; o >>= 1) {
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        has_nan |= __shfl_xor_sync(0xffffffffu, has_nan, o);
+    }
+    const float amax = has_nan ? __int_as_float(0x7fc00000) : mx;
+    const float inv = amax > 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+    int local = 0;
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+        const int d = (chunk * IT + it) * 256 + lane * 8;
+        const uint32_t w[4] = {x[it].x, x[it].y, x[it].z, x[it].w};
+        int v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e >> 1]));
+            const float r = rintf(__fmul_rn(e & 1 ? f.y : f.x, inv));
+            v[e] = r != r ? 0 : (int)fminf(fmaxf(r, -128.0f), 127.0f);
+            local += v[e];
+        }
+        if (d >= p.kq) continue;
+        if (p.q && row < p.m) {
+            uint32_t lo = 0, hi = 0;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { lo |= (uint32_t)(v[e] & 0xff) << (8 * e); hi |= (uint32_t)(v[4 + e] & 0xff) << (8 * e); }
+            *reinterpret_cast<uint2*>(p.q + (size_t)row * p.kq + d) = make_uint2(lo, hi);
+        }
+        if (p.qh) {
+            // qh_perm: depths of a group of four in the order 0 2 1 3; 2: and scaled by position (see above)
+            float f[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int src = p.qh_perm ? ((e & ~3) | ((e & 1) << 1) | ((e >> 1) & 1)) : e;
+                f[e] = (float)v[src];
+                if (p.qh_perm == 2) f[e] *= e < 2 ? 256.0f : (e < 4 ? 1.0f : (e < 6 ? 64.0f : 0.25f));
+            }
+            uint4 o;
+            o.x = pack2_t<0>(f[0], f[1]); o.y = pack2_t<0>(f[2], f[3]); o.z = pack2_t<0>(f[4], f[5]); o.w = pack2_t<0>(f[6], f[7]);
+            *reinterpret_cast<uint4*>(p.qh + (size_t)row * p.kq + d) = o;
+        }
+    }
+    for (int o = seg >> 1; o; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
+    const int b = (chunk * IT * 256 + lane * 8) >> L;
+    if ((lane & (seg - 1)) == 0 && b < p.nbq && row < p.m) {
+        const float sa = (b << L) < p.k ? __fdiv_rn(amax, 127.0f) : 0.0f;
+        p.sa[(size_t)row * p.nbq + b] = sa;
+        if (p.qsum) p.qsum[(size_t)row * p.nbq + b] = local;
+        if (p.sa_t) p.sa_t[(size_t)b * p.mpad + row] = sa;
+        if (p.qsum_t) p.qsum_t[(size_t)b * p.mpad + row] = (float)local;
     }
 }
 
@@ -625,6 +715,23 @@ size_t lowbit_smem(int ns, int gpt, int mt, int rows_s, int kc, int kqc, int blo
 
 cudaError_t act_quant_launch(const ActQuantArgs& a, cudaStream_t stream) {
     if (a.m == 0 || a.nbq == 0) return cudaSuccess;
+    if (a.log2_block <= 10 && ((uintptr_t)a.q & 7) == 0) {
+        ActQuantArgs p = a;
+        p.mz = a.qh ? (a.m + 7) / 8 * 8 : a.m;
+        p.a_vec_ok = a.k % 8 == 0 && ((uintptr_t)a.a & 15) == 0;
+        const int it = a.log2_block <= 8 ? 1 : 1 << (a.log2_block - 8);
+        const size_t depth = (size_t)a.nbq << a.log2_block, span = (size_t)256 * it;
+        const int chunks = (int)(((depth > (size_t)a.kq ? depth : (size_t)a.kq) + span - 1) / span);
+        const dim3 grid((unsigned)(((size_t)p.mz * chunks + 7) / 8));
+        if (it == 1) return launch_pdl(act_quant_warp_kernel<1>, grid, dim3(256), 0, stream, p, chunks);
+        if (it == 2) return launch_pdl(act_quant_warp_kernel<2>, grid, dim3(256), 0, stream, p, chunks);
+        return launch_pdl(act_quant_warp_kernel<4>, grid, dim3(256), 0, stream, p, chunks);
+    }
+    if (a.qh && a.m % 8 != 0) {
+        // the rows up to the next multiple of eight are zero rows (lowbit_mma_kernel reads whole tiles of eight)
+        const cudaError_t e = cudaMemsetAsync(a.qh + (size_t)a.m * a.kq, 0, (size_t)(8 - a.m % 8) * a.kq * 2, stream);
+        if (e != cudaSuccess) return e;
+    }
     dim3 grid(a.nbq, a.m);
     return launch_pdl(act_quant_kernel, grid, dim3(128), 0, stream, a);
 }
