@@ -470,6 +470,214 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     }
 }
 
+// ------------------------------------------------------------------------------------------------------------------
+// Decode: query rows x heads of a group up to 16 per KV head.  The tensor-core form above needs ~10 us for it whatever the
+// number of keys -- tensor memory, a query tile of 128 rows, two passes handed from warp to warp.  Here a CTA is 8 warps on a
+// run of keys of one KV head, the (at most 16) query rows are the M of mma.m16n8k16, and there are three barriers:
+//   scores    B fragments straight from the cache, 16 bytes a lane (a lane's eight depths are two instructions' k indices,
+//             the query fragments are taken in the same order), while the values of the run arrive in shared memory
+//   softmax   two rows per warp: exact maximum, exp, the probabilities in two f16 parts as above
+//   values    a warp owns eight depths at a time, ldmatrix.trans makes its B fragments
+// The runs of one KV head are a cluster of up to eight CTAs and meet over distributed shared memory as above.
+constexpr int kAdThreads = 256;
+struct AdSmem {                                    // byte offsets; KC = keys of a CTA, a multiple of 16
+    int q, s, hi, lo, v, o, total;
+};
+__host__ __device__ inline AdSmem ad_smem(int hd, int kc) {
+    AdSmem a;
+    a.q = 0;                                       // [16][hd32 + 8] f16, depths padded to whole runs of 32
+    a.s = a.q + 16 * (((hd + 31) & ~31) + 8) * 2;  // [16][kc + 4] f32
+    a.hi = a.s + 16 * (kc + 4) * 4;                // [16][kc + 8] f16
+    a.lo = a.hi + 16 * (kc + 8) * 2;
+    a.v = a.lo + 16 * (kc + 8) * 2;                // [kc][hd + 8] f16
+    a.o = a.v + kc * (hd + 8) * 2;                 // [16][hd + 4] f32
+    a.total = a.o + 16 * (hd + 4) * 4;
+    return a;
+}
+constexpr int kAdMaxSmem = 226 * 1024;
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int QF32, int OUT16>
+__global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const __grid_constant__ AttnArgs p, int kc) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ float part_m[16], part_l[16];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int hd = p.head_dim, hd32 = (hd + 31) & ~31, group = p.heads / p.kv_heads, kvh = blockIdx.z;
+    const int splits = gridDim.x, rank = blockIdx.x, nrow = p.rows * group;
+    const int len = p.start + p.rows;
+    const int key0 = rank * kc, nk = max(0, min(kc, len - key0)), nk16 = (nk + 15) & ~15;
+    const AdSmem L = ad_smem(hd, kc);
+    uint16_t* q_s = reinterpret_cast<uint16_t*>(smem + L.q);
+    float* s_s = reinterpret_cast<float*>(smem + L.s);
+    uint16_t *hi_s = reinterpret_cast<uint16_t*>(smem + L.hi), *lo_s = reinterpret_cast<uint16_t*>(smem + L.lo), *v_s = reinterpret_cast<uint16_t*>(smem + L.v);
+    float* o_s = reinterpret_cast<float*>(smem + L.o);
+    const size_t ld = (size_t)p.kv_heads * hd;
+    pdl_launch_dependents();
+    pdl_wait();
+    // ---- values on their way, queries in place ----
+    {
+        const int per = hd / 8;
+        const uint16_t* src = p.v + (size_t)key0 * ld + (size_t)kvh * hd;
+        for (int it = tid; it < nk16 * per; it += kAdThreads) {
+            const int r = it / per, c = (it - r * per) * 8;
+            const uint32_t bytes = r < nk ? 16u : 0u;                            // (zeros behind the last key: nothing is read)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(v_s + (size_t)r * (hd + 8) + c)),
+                         "l"(bytes ? src + (size_t)r * ld + c : p.v), "r"(bytes)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int it = tid; it < 16 * hd32; it += kAdThreads) {
+        const int r = it / hd32, d = it - r * hd32;
+        float x = 0.0f;
+        if (r < nrow && d < hd) {
+            const int i = r / group;
+            const size_t off = (size_t)i * p.q_stride + (size_t)(kvh * group + r - i * group) * hd + d;
+            x = QF32 ? reinterpret_cast<const float*>(p.q)[off] : __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(p.q)[off]));
+            x = __fmul_rn(x, p.scale);
+        }
+        q_s[r * (hd32 + 8) + d] = __half_as_ushort(__float2half_rn(x));
+    }
+    __syncthreads();
+    // ---- scores: a warp eight keys at a time ----
+    {
+        // (the next tile's keys are loaded before this one's products: a trip to the cache is most of a short run)
+        const uint16_t* kb = p.k + (size_t)key0 * ld + (size_t)kvh * hd + 8 * t;
+        auto load = [&](int tile, uint4 (&kv)[8]) {
+            const int key = tile * 8 + g;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                kv[c] = make_uint4(0, 0, 0, 0);
+                if (key < nk && 32 * c + 8 * t < hd) kv[c] = *reinterpret_cast<const uint4*>(kb + (size_t)key * ld + 32 * c);
+            }
+        };
+        uint4 kv[8], nx[8];
+        load(warp, kv);
+        for (int tile = warp; tile < nk16 / 8; tile += 8) {
+            load(tile + 8, nx);
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                if (32 * c >= hd) break;
+                const uint4 qa = *reinterpret_cast<const uint4*>(q_s + g * (hd32 + 8) + 32 * c + 8 * t);
+                const uint4 qb = *reinterpret_cast<const uint4*>(q_s + (g + 8) * (hd32 + 8) + 32 * c + 8 * t);
+                mma_16816(acc, qa.x, qb.x, qa.y, qb.y, kv[c].x, kv[c].y);
+                mma_16816(acc, qa.z, qb.z, qa.w, qb.w, kv[c].z, kv[c].w);
+            }
+            *reinterpret_cast<float2*>(s_s + g * (kc + 4) + tile * 8 + 2 * t) = make_float2(acc[0], acc[1]);
+            *reinterpret_cast<float2*>(s_s + (g + 8) * (kc + 4) + tile * 8 + 2 * t) = make_float2(acc[2], acc[3]);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) kv[c] = nx[c];
+        }
+    }
+    __syncthreads();
+    // ---- softmax of the run: two rows per warp ----
+    for (int r = 2 * warp; r < min(2 * warp + 2, nrow); ++r) {
+        const int lim = min(nk, p.start + r / group + 1 - key0);                 // keys of the run this row attends to
+        const float* sr = s_s + r * (kc + 4);
+        float mx = -INFINITY;
+        for (int j = lane; j < lim; j += 32) mx = fmaxf(mx, sr[j]);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float base = mx == -INFINITY ? 0.0f : mx;                          // no key of this run counts for the row
+        float sum = 0.0f;
+        for (int j = lane; j < nk16; j += 32) {
+            float e = j < lim ? expf(sr[j] - base) : 0.0f;
+            sum += e;
+            e *= kAtPScale;
+            const __half hi = __float2half_rn(e);
+            hi_s[r * (kc + 8) + j] = __half_as_ushort(hi);
+            lo_s[r * (kc + 8) + j] = __half_as_ushort(__float2half_rn(e - __half2float(hi)));
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0) { part_m[r] = mx; part_l[r] = sum; }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    // ---- values: a warp eight depths at a time ----
+    for (int n0 = warp * 8; n0 < hd; n0 += 64) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k0 = 0; k0 < nk16; k0 += 16) {
+            uint32_t b0, b1;
+            asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+                         : "=r"(b0), "=r"(b1)
+                         : "r"(smem_u32(v_s + (size_t)(k0 + (lane & 15)) * (hd + 8) + n0))
+                         : "memory");
+            const uint16_t *h = hi_s + g * (kc + 8) + k0 + 2 * t, *l = lo_s + g * (kc + 8) + k0 + 2 * t;
+            const int down = 8 * (kc + 8);
+            auto w = [](const uint16_t* x) { return *reinterpret_cast<const uint32_t*>(x); };
+            mma_16816(acc, w(h), w(h + down), w(h + 8), w(h + down + 8), b0, b1);
+            mma_16816(acc, w(l), w(l + down), w(l + 8), w(l + down + 8), b0, b1);
+        }
+        *reinterpret_cast<float2*>(o_s + g * (hd + 4) + n0 + 2 * t) = make_float2(acc[0], acc[1]);
+        *reinterpret_cast<float2*>(o_s + (g + 8) * (hd + 4) + n0 + 2 * t) = make_float2(acc[2], acc[3]);
+    }
+    // ---- the runs meet ----
+    if (splits > 1) cluster_sync_all();
+    else __syncthreads();
+    const uint32_t o_a = smem_u32(o_s), m_a = smem_u32(part_m), l_a = smem_u32(part_l);
+    for (int it = rank * kAdThreads + tid; it < nrow * (hd / 8); it += splits * kAdThreads) {
+        const int r = it / (hd / 8), c = (it - r * (hd / 8)) * 8;
+        float m[8], l[8], mx = -INFINITY;
+        float4 o[8][2];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            if (s >= splits) break;
+            m[s] = ld_dsmem_f32(mapa_shared(m_a + r * 4, s));
+            l[s] = ld_dsmem_f32(mapa_shared(l_a + r * 4, s));
+            const uint32_t oa = mapa_shared(o_a + (uint32_t)(r * (hd + 4) + c) * 4, s);
+            o[s][0] = ld_dsmem_f32x4(oa);
+            o[s][1] = ld_dsmem_f32x4(oa + 16);
+        }
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+            if (s < splits) mx = fmaxf(mx, m[s]);
+        float sum = 0.0f, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            if (s >= splits || m[s] == -INFINITY) continue;
+            const float f = expf(m[s] - mx);
+            sum = fmaf(f, l[s], sum);
+            v[0] = fmaf(f, o[s][0].x, v[0]); v[1] = fmaf(f, o[s][0].y, v[1]); v[2] = fmaf(f, o[s][0].z, v[2]); v[3] = fmaf(f, o[s][0].w, v[3]);
+            v[4] = fmaf(f, o[s][1].x, v[4]); v[5] = fmaf(f, o[s][1].y, v[5]); v[6] = fmaf(f, o[s][1].z, v[6]); v[7] = fmaf(f, o[s][1].w, v[7]);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(v[e] * (1.0f / kAtPScale), sum);
+        const int i = r / group, head = kvh * group + r - i * group;
+        if (!all_finite(v)) attend_exact8<QF32>(p, i, head, c, v);
+        store8<OUT16>(p, (size_t)i * p.heads * hd + (size_t)head * hd + c, v);
+    }
+    if (splits > 1) cluster_sync_all();                        // nobody leaves while its shared memory is read
+}
+
+template <int QF32, int OUT16>
+cudaError_t attn_decode_launch(const AttnArgs& a, int splits, int kc, cudaStream_t stream) {
+    auto kern = attn_decode_kernel<QF32, OUT16>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAdMaxSmem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits, 1, a.kv_heads);
+    cfg.blockDim = dim3(kAdThreads);
+    cfg.dynamicSmemBytes = ad_smem(a.head_dim, kc).total;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = splits;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kern, a, kc);
+}
+
 // rows x row_len f16 values from a strided source (the k or v part of projected [q | k | v] rows) to cache rows pos...; a
 // thread moves 8 values of each (VEC: every address involved is 16-byte aligned) or one.
 template <int VEC>
@@ -514,6 +722,17 @@ cudaError_t attn_tc_launch(const CUtensorMap& tk, const CUtensorMap& tv, const A
 }  // namespace
 
 cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream) {
+    if (a.rows * (a.heads / a.kv_heads) <= 16) {
+        // runs of 64 keys and up; caches whose runs do not fit shared memory (about 4 k keys at 128 depths) stay below
+        const int total = a.start + a.rows;
+        int runs = 1;
+        while (runs < 8 && total > 64 * runs && a.kv_heads * runs < sm_count) runs *= 2;
+        const int kc = ((total + runs - 1) / runs + 15) & ~15;
+        if (total <= 8 * 4096 && ad_smem(a.head_dim, kc).total <= kAdMaxSmem) {
+            if (a.out16) return q_f32 ? attn_decode_launch<1, 1>(a, runs, kc, stream) : attn_decode_launch<0, 1>(a, runs, kc, stream);
+            return q_f32 ? attn_decode_launch<1, 0>(a, runs, kc, stream) : attn_decode_launch<0, 0>(a, runs, kc, stream);
+        }
+    }
     TensorMapEncodeFn enc = tensor_map_encoder();
     if (!enc) return cudaErrorNotSupported;
     // [depth][KV head][position], a box = 64 depths of one head at 128 positions
