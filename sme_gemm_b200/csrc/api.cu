@@ -699,12 +699,17 @@ static int padded_rows(const uint16_t* a, size_t m, size_t k, size_t kd, cudaStr
 
 // glu / yacc: the fused forms of the MLP block (the tensor-core GEMM, and the one-wave decode kernel at up to four rows).
 struct TpPush { float* bufs[8]; int world, rank, rows; };
+// The passes around a projection that the one-wave decode kernel takes along: its activations as the norm of f32 rows, and
+// the key / value columns of a [q | k | v] projection to the caches' next rows.
+struct NormIn { const float *x, *weight, *bias; float eps; int rms; };
+struct KvOut { uint16_t *k, *v; size_t q_len, kv_len; };
 static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, const ep_desc16* ep, int bf16,
-                  cudaStream_t stream, float* c32 = nullptr, int glu = 0, float* yacc = nullptr, const TpPush* push = nullptr) {
+                  cudaStream_t stream, float* c32 = nullptr, int glu = 0, float* yacc = nullptr, const TpPush* push = nullptr,
+                  const NormIn* norm = nullptr, const KvOut* kv = nullptr) {
     if (!w) return -4;
     const size_t n = w->d.n, k0 = w->d.k;
     if (m == 0 || n == 0) return 0;
-    if ((!c && !c32 && !yacc) || (k0 && !a) || m > 0x7fffffffu || n > 0x7fffffffu || k0 > 0x7fffffffu) return -4;
+    if ((!c && !c32 && !yacc) || (k0 && !a && !norm) || m > 0x7fffffffu || n > 0x7fffffffu || k0 > 0x7fffffffu) return -4;
     if (w->affine) {
         if (c32 || glu || yacc) return -3;                       // the fused forms of the MLP block take Q4_0 weights
         const smeg_dense* t = nullptr;
@@ -714,6 +719,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     }
     if ((glu || yacc) && !q4_uses_tc(w, a, m) && !q4_fuses_decode(w, a, m, bf16, glu)) return -4;
     if (push && (!c32 || !gemm_tc_supported(4, (int)m, (int)k0, w->d.log2_block, a))) return -3;
+    if ((norm || kv) && (c32 || !q4_takes_direct(w, a, m, bf16, glu))) return -3;
     DeviceState* ds = dev_state();
     if (!ds) return -5;
     // Rows that are not whole 16-byte words: one or two rows are read as they are by the decode kernels; every other call
@@ -765,6 +771,8 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         e = gemm_tc_launch(t, bf16, grid, smem, stream);
     } else if ((int)m <= q4_direct_rows() && q4_direct_supported(g, bf16)) {
         g.glu = glu; g.yacc = yacc;
+        if (norm) { g.nx = norm->x; g.nw = norm->weight; g.nbias = norm->bias; g.neps = norm->eps; g.nrms = norm->rms; }
+        if (kv) { g.kc = kv->k; g.vc = kv->v; g.q_len = (int)kv->q_len; g.kv_len = (int)kv->kv_len; }
         e = q4_direct_launch(g, ds->sm_count, stream);
     } else if (q4_mma_supported(g)) {
         g.glu = glu; g.yacc = yacc;
@@ -1256,7 +1264,8 @@ static int q4_accumulate(const smeg_q4* w, const uint16_t* a, float* y, uint16_t
 
 // both = x @ gate_up (f16), hid = glu(both), then the down projection either
 // rounded to f16 and added into y (partial == nullptr) or left as f32 partial sums.
-static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, size_t m, cudaStream_t stream, const TpPush* push = nullptr) {
+static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, size_t m, cudaStream_t stream, const TpPush* push = nullptr,
+                   const NormIn* norm = nullptr) {
     if (!mlp) return -4;
     if (m == 0) return 0;
     const size_t h = mlp->down->d.k, d_out = mlp->down->d.n;
@@ -1275,7 +1284,7 @@ static int mlp_run(smeg_mlp* mlp, const uint16_t* x, float* y, float* partial, s
     uint16_t* both = (uint16_t*)(ws + hid_bytes + out_bytes);
     int rc;
     if (fuse) {
-        rc = q4_dev(mlp->gate_up, x, hid, m, nullptr, 0, stream, nullptr, (int)mlp->act);
+        rc = q4_dev(mlp->gate_up, x, hid, m, nullptr, 0, stream, nullptr, (int)mlp->act, nullptr, nullptr, norm);
     } else {
         rc = q4_dev(mlp->gate_up, x, both, m, nullptr, 0, stream);
         if (!rc) rc = glu_launch(hid, both, m, h, mlp->act, stream) == cudaSuccess ? 0 : -6;
@@ -1301,21 +1310,33 @@ int smeg_block_accumulate_dev(const smeg_block_args* b, void* stream_v) {
     char* ws = nullptr;
     if (cudaMallocAsync(&ws, h_bytes + qkv_bytes + att_bytes + out_bytes, stream) != cudaSuccess) return -2;
     uint16_t *h = (uint16_t*)ws, *qkv = (uint16_t*)(ws + h_bytes), *att = (uint16_t*)(ws + h_bytes + qkv_bytes), *out = (uint16_t*)(ws + h_bytes + qkv_bytes + att_bytes);
-    int rc = smeg_norm_rows_dev(h, nullptr, b->x, b->norm1_w, b->norm1_b, m, d, b->norm1_eps, b->norm1_rms, stream);
-    if (!rc) rc = q4_dev(b->qkv, h, qkv, m, nullptr, 0, stream);
-    if (!rc) rc = smeg_kv_append_dev(b->k_cache, b->v_cache, qkv, w, q_len, q_len + kv_len, kv_len, b->pos, m, stream);
+    // One or two rows: the keys and values go straight to the caches, and narrow layers' norms are formed by the projections
+    // that take them (up to 1024 wide: every CTA repeats the norm, 384 wide 1.5 us less a norm than a launch of its own, 4096
+    // wide 3 us more) -- five launches a layer instead of eight.
+    const NormIn n1 = {b->x, b->norm1_w, b->norm1_b, b->norm1_eps, b->norm1_rms ? 1 : 0}, n2 = {b->x, b->norm2_w, b->norm2_b, b->norm2_eps, b->norm2_rms ? 1 : 0};
+    const bool direct = q4_takes_direct(b->qkv, h, m, 0, 0), norm_in = direct && d <= 1024;
+    int rc = norm_in ? 0 : smeg_norm_rows_dev(h, nullptr, b->x, b->norm1_w, b->norm1_b, m, d, b->norm1_eps, b->norm1_rms, stream);
+    if (direct) {
+        const KvOut kv = {b->k_cache + b->pos * kv_len, b->v_cache + b->pos * kv_len, q_len, kv_len};
+        if (!rc) rc = q4_dev(b->qkv, norm_in ? nullptr : h, qkv, m, nullptr, 0, stream, nullptr, 0, nullptr, nullptr, norm_in ? &n1 : nullptr, &kv);
+    } else {
+        if (!rc) rc = q4_dev(b->qkv, h, qkv, m, nullptr, 0, stream);
+        if (!rc) rc = smeg_kv_append_dev(b->k_cache, b->v_cache, qkv, w, q_len, q_len + kv_len, kv_len, b->pos, m, stream);
+    }
     if (!rc) rc = smeg_attn_kv_causal_f16_dev(att, qkv, 0, w, b->k_cache, b->v_cache, b->pos, m, b->heads, b->kv_heads, b->head_dim, b->scale, stream);
     if (!rc) rc = q4_accumulate(b->out, att, b->x, out, m, stream);
-    if (!rc) rc = smeg_norm_rows_dev(h, nullptr, b->x, b->norm2_w, b->norm2_b, m, d, b->norm2_eps, b->norm2_rms, stream);
+    const bool norm_in_up = d <= 1024 && q4_takes_direct(up, nullptr, m, 0, b->mlp ? (int)b->mlp->act : 0) && (!b->mlp || up->d.n == 2 * hidden);
+    if (!rc && !norm_in_up) rc = smeg_norm_rows_dev(h, nullptr, b->x, b->norm2_w, b->norm2_b, m, d, b->norm2_eps, b->norm2_rms, stream);
     if (!rc) {
+        const NormIn* norm = norm_in_up ? &n2 : nullptr;
         if (b->mlp) {
-            rc = mlp_run(b->mlp, h, b->x, nullptr, m, stream);
+            rc = mlp_run(b->mlp, norm ? nullptr : h, b->x, nullptr, m, stream, nullptr, norm);
         } else {
             EpNode node;
             memset(&node, 0, sizeof(node));
             node.op = 8; node.aux = b->act;                                     // the activation alone
             const ep_desc16 ep = {1, &node};
-            rc = q4_dev(up, h, qkv, m, &ep, 0, stream);
+            rc = q4_dev(up, norm ? nullptr : h, qkv, m, &ep, 0, stream, nullptr, 0, nullptr, nullptr, norm);
             if (!rc) rc = q4_accumulate(down, qkv, b->x, out, m, stream);
         }
     }

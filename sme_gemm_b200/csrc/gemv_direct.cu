@@ -1,5 +1,5 @@
 // Decode GEMV for one to four activation rows, straight from global memory (sm_100a):
-//   q4_direct_kernel      C[m][n] = ep( A[m][k] @ dequant(W) ), Q4 weights, f16, K-blocks of 32 and up
+//   q4_direct_kernel      C[m][n] = ep( A[m][k] @ dequant(W) ), Q4 weights, f16, K-blocks of 32 and up, one or two rows
 //   lowbit_direct_kernel  2-bit / 1-bit weights against int8-quantised activations (matmul_q2 / matmul_q1)
 //
 // They replace the reference's SME GEMV kernels for the batch sizes a decode step has
@@ -66,15 +66,69 @@ __device__ __forceinline__ void q4_codes_h2(uint32_t w, __half2 (&r)[4]) {
 __device__ __forceinline__ __half2 as_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 
 // ---------------------------------------------------------------------------------------------
-// Q4, f16, M rows (1..4), K-blocks >= 32.
+// Q4, f16, M rows (1 or 2), K-blocks >= 32.
 // Shared memory: ring [8 warps][PF][32 lanes] of {16 B codes} then {2 x 4 B scales} | A rows
 // [M][kpad + 8] f16 | the cross-warp exchange [8 warps][CPC][M][16] f32.
 // ---------------------------------------------------------------------------------------------
 constexpr int kQ4PF = 8;                                           // units in flight per warp
 constexpr size_t kQ4RingBytes = (size_t)kDWarps * kQ4PF * 32 * (16 + 8);
 
+// Sum over the 256 threads of a CTA, in the order of the separate norm pass.
+__device__ __forceinline__ float cta_sum(float v, float* sh) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();                       // sh may still be read from the previous call
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    float t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += sh[w];
+    return t;
+}
+
+// One activation row as the norm of an f32 row, in shared memory: the arithmetic and the order of norm_rows_kernel (the
+// same bits), repeated by every CTA -- a row is a few KB out of L2 against a launch of its own in front of the projection.
+__device__ __noinline__ void stage_norm_row(uint16_t* dst, const float* xr, const float* weight, const float* bias, int dim, int kpad, float eps,
+                                            int rms, float* sh) {
+    constexpr int KEEP = 16;               // values a thread keeps in registers between the passes (rows of up to 4096)
+    const int tid = threadIdx.x;
+    float x[KEEP];
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) x[i] = tid + i * kDThreads < dim ? xr[tid + i * kDThreads] : 0.0f;
+    const float fdim = (float)dim;
+    float mean = 0.0f;
+    if (!rms) {
+        float s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i)
+            if (tid + i * kDThreads < dim) s += x[i];
+        for (int j = tid + KEEP * kDThreads; j < dim; j += kDThreads) s += xr[j];
+        mean = __fdiv_rn(cta_sum(s, sh), fdim);
+    }
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+        if (tid + i * kDThreads < dim) {
+            const float d = __fsub_rn(x[i], mean);
+            ss = __fmaf_rn(d, d, ss);
+        }
+    for (int j = tid + KEEP * kDThreads; j < dim; j += kDThreads) {
+        const float d = __fsub_rn(xr[j], mean);
+        ss = __fmaf_rn(d, d, ss);
+    }
+    const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(cta_sum(ss, sh), fdim), eps)));
+    auto put = [&](int j, float v) {
+        dst[j] = __half_as_ushort(__float2half_rn(__fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(v, mean), r), weight[j]), bias ? bias[j] : 0.0f)));
+    };
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+        if (tid + i * kDThreads < dim) put(tid + i * kDThreads, x[i]);
+    for (int j = tid + KEEP * kDThreads; j < dim; j += kDThreads) put(j, xr[j]);
+    for (int j = dim + tid; j < kpad; j += kDThreads) dst[j] = 0;
+}
+
 template <int M>
-__global__ void __launch_bounds__(kDThreads, M <= 2 ? 3 : 2) q4_direct_kernel(const __grid_constant__ Q4GemvArgs p) {
+__global__ void __launch_bounds__(kDThreads, 3) q4_direct_kernel(const __grid_constant__ Q4GemvArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int PF = kQ4PF;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -125,7 +179,10 @@ __global__ void __launch_bounds__(kDThreads, M <= 2 ? 3 : 2) q4_direct_kernel(co
     pdl_wait();                                                    // the activations may come from the kernel ahead
 
     // ---- stage the activation rows (zero past k) ----
-    if (!p.a_vec_ok) {
+    __shared__ float norm_sh[8];
+    if (p.nx) {
+        for (int r = 0; r < M; ++r) stage_norm_row(As + (size_t)r * a_stride, p.nx + (size_t)r * p.k, p.nw, p.nbias, p.k, kpad, p.neps, p.nrms, norm_sh);
+    } else if (!p.a_vec_ok) {
         // rows that are no whole 16-byte words, or start off a 16-byte boundary: a half at a time, eight loads in flight
         for (int r = 0; r < M; ++r)
             for (int d0 = tid; d0 < kpad; d0 += kDThreads * 8) {
@@ -239,6 +296,12 @@ __global__ void __launch_bounds__(kDThreads, M <= 2 ? 3 : 2) q4_direct_kernel(co
         if (col < p.n) {
             if (p.c32) p.c32[(size_t)r * p.n + col] = acc;
             else if (p.yacc) p.yacc[(size_t)r * p.n + col] = __fadd_rn(p.yacc[(size_t)r * p.n + col], __half2float(__float2half_rn(acc)));
+            else if (p.kc && col >= p.q_len) {
+                const int kv = col - p.q_len;
+                const uint16_t v = __half_as_ushort(__float2half_rn(acc));
+                if (kv < p.kv_len) p.kc[(size_t)r * p.kv_len + kv] = v;
+                else p.vc[(size_t)r * p.kv_len + kv - p.kv_len] = v;
+            }
             else p.c[(size_t)r * p.n + col] = ep_store_value<0>(p.ep, acc, (size_t)r, (size_t)col);
         }
     }
@@ -519,7 +582,7 @@ int direct_grid(int n16, int sm_count, int max_groups, int* cpc, int per_sm) {
 
 // ---- Q4 ----
 bool q4_direct_supported(const Q4GemvArgs& a, int bf16) {
-    if (bf16 || a.m < 1 || a.m > 4 || a.log2_block < 5 || a.k64 < 1) return false;
+    if (bf16 || a.m < 1 || a.m > 2 || a.log2_block < 5 || a.k64 < 1) return false;
     const size_t smem = kQ4RingBytes + (size_t)a.m * ((size_t)a.k64 * 64 + 8) * 2;
     return smem <= 100 * 1024;
 }
@@ -529,7 +592,7 @@ cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream) {
     a.n16 = n16;
     // three CTAs per SM when the matrix gives every SM that many, else two (and then never three on one SM
     // while another has one: the shared-memory request is padded past a third of an SM's)
-    const int per_sm = (a.m <= 2 && n16 > 2 * sm_count) ? 3 : 2;
+    const int per_sm = n16 > 2 * sm_count ? 3 : 2;
     int grid_x;
     if (a.glu) {
         // shares are (gate group, up group) pairs: n16 / 2 of them, at most 8 (16 groups) per CTA
@@ -553,7 +616,7 @@ cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream) {
         if (e != cudaSuccess) return e;                                               \
         return launch_pdl(q4_direct_kernel<MM>, grid, dim3(kDThreads), smem, stream, a);
     switch (a.m) {
-        SMEG_QD(1) SMEG_QD(2) SMEG_QD(3) SMEG_QD(4)
+        SMEG_QD(1) SMEG_QD(2)
     default: return cudaErrorInvalidValue;
     }
 #undef SMEG_QD

@@ -20,6 +20,12 @@ struct Q4GemvArgs {
     int glu;                      // SMEG_ACT_SILU / _GELU: W is a gate/up matrix (32 gate columns, 32 up columns, ...) and c (m x n/2)
                                   // receives f16(act(f16(gate)) * f16(up)); a CTA then owns (gate group, up group) pairs
     float* yacc;                  // if set: y[m][n] += f32(f16(acc)) instead of storing c (the residual add)
+    // one-wave kernel only -- the passes around a layer's projections at decode size:
+    const float *nx, *nw, *nbias; // if nx: the activations are norm(nx) (f32 rows of k, weight nw, bias nbias or null), formed by every CTA
+    float neps;
+    int nrms;                     // rms_norm (else layer_norm)
+    uint16_t *kc, *vc;            // if set: columns from q_len on are keys, then values: kv_len of each go to rows of kc / vc instead of c
+    int q_len, kv_len;
     int m, n, k;
     int n16, k64, nb;             // column groups, 64-deep units, staged scale rows per group
     int log2_block;
@@ -40,7 +46,7 @@ struct Q4GemvArgs {
 // scratch the caller must provide in ws / counters).  Leaves sgrid = 0 otherwise.
 void q4_gemv_stream_plan(Q4GemvArgs& a, int bf16, int sm_count, size_t* ws_floats, size_t* ncounters);
 cudaError_t q4_gemv_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t stream);
-// One to four rows, f16, K-blocks of 32 and up: plain 128-bit loads, packed f16 multiply-adds (gemv_direct.cu).
+// One or two rows, f16, K-blocks of 32 and up: plain 128-bit loads, packed f16 multiply-adds (gemv_direct.cu).
 bool q4_direct_supported(const Q4GemvArgs& a, int bf16);
 cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream);
 

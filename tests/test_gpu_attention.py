@@ -309,3 +309,62 @@ def test_non_finite_values_stay_with_the_rows_that_attend_to_them(heads, kv_head
     torch.cuda.synchronize()
     assert torch.isnan(bad[rows - 1, :group * hd]).all() and not torch.isnan(bad[:rows - 1]).any() and not torch.isnan(bad[:, group * hd:]).any()
     assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd,start,rows,q_f32", [
+    (4, 2, 64, 0, 1, False), (4, 2, 64, 63, 1, True), (8, 2, 128, 64, 3, False), (16, 1, 128, 511, 1, False), (6, 6, 40, 200, 2, True), (4, 4, 256, 130, 16, False),
+    (2, 1, 72, 1000, 8, False), (8, 2, 128, 4090, 4, False), (3, 3, 32, 2050, 1, False), (32, 8, 128, 1023, 1, False)])
+def test_decode_attention_runs_and_rows(heads, kv_heads, hd, start, rows, q_f32):
+    """Up to 16 query rows per KV head: one run of keys and clusters of runs (some of them empty or past a row's last key),
+    depths that are no multiple of 32 or 64, caches of one key."""
+    rng = np.random.default_rng(heads + hd + start)
+    n = start + rows
+    cache = sg.KvCache(heads, kv_heads, hd, n + 100)
+    cache._k.fill_(float("nan"))                           # what lies past the last row must not be read
+    cache._v.fill_(float("nan"))
+    k16 = (rng.standard_normal((n, kv_heads * hd)) * 0.7).astype(np.float16)
+    v16 = rng.standard_normal((n, kv_heads * hd)).astype(np.float16)
+    cache.extend(torch.from_numpy(k16).cuda(), torch.from_numpy(v16).cuda())
+    q32 = rng.standard_normal((rows, heads * hd)).astype(np.float32)
+    if not q_f32:
+        q32 = q32.astype(np.float16).astype(np.float32)
+    q = torch.from_numpy(q32).cuda().to(torch.float32 if q_f32 else torch.float16)
+    out = torch.full((rows, heads * hd), 3.0, dtype=torch.float32, device="cuda")
+    cache._attend(q, heads * hd, rows, out)
+    qh = (q32 * np.float32(cache.scale())).astype(np.float16).astype(np.float64).reshape(rows, kv_heads, heads // kv_heads, hd)
+    kd, vd = (x.astype(np.float64).reshape(n, kv_heads, hd) for x in (k16, v16))
+    s = np.einsum("ikgd,tkd->kgit", qh, kd)
+    s[:, :, np.arange(n)[None, :] > start + np.arange(rows)[:, None]] = -np.inf
+    p = np.exp(s - s.max(-1, keepdims=True))
+    want = (np.einsum("kgit,tkd->ikgd", p, vd) / p.sum(-1).transpose(2, 0, 1)[..., None]).reshape(rows, heads * hd)
+    # f32 scores of magnitude ~10 carry 1e-6, probabilities and their sums a few 2^-24 each
+    assert max_rel(out.cpu().numpy(), want) <= 2e-5
+    assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("rms", [True, False])
+@pytest.mark.parametrize("d,heads,kv_heads,hd,rows", [(384, 6, 6, 64, 1), (256, 4, 2, 64, 2), (1152, 9, 3, 128, 1), (320, 5, 1, 64, 3)])
+def test_layer_in_one_call_is_its_parts(rms, d, heads, kv_heads, hd, rows):
+    """Block.accumulate as one library call (norms formed by the projections, keys and values written by the product) against
+    the same layer run part by part: the same bits in the residual stream and in the caches."""
+    rng = np.random.default_rng(d + rows)
+    lin = lambda n, k: sg.Linear.quantize((rng.standard_normal((n, k)) * 0.05).astype(np.float32), sg.WeightLayout.OutIn, n, k)  # noqa: E731
+    wt = lambda: rng.uniform(0.5, 1.5, d).astype(np.float32)  # noqa: E731
+    norm = (lambda: sg.Norm.rms(wt(), 1e-5)) if rms else (lambda: sg.Norm.layer(wt(), wt() - 1, 1e-5))
+    n1, n2 = norm(), norm()
+    attn = sg.SelfAttention.new(lin((heads + 2 * kv_heads) * hd, d), lin(d, heads * hd), heads, kv_heads, hd)
+    mlp = sg.Mlp.new(lin(2 * d, d), sg.Gate.Gelu, lin(d, 2 * d))
+    block = sg.Block.new(n1, attn, n2, mlp)
+    c1, c2 = block.cache(64), block.cache(64)
+    x1 = torch.from_numpy(rng.standard_normal((rows, d)).astype(np.float32)).cuda()
+    x2 = x1.clone()
+    h = torch.empty((rows, d), dtype=torch.float16, device="cuda")
+    for _ in range(3):
+        block.accumulate(x1, c1, rows)
+        n1.forward(x2, h)
+        attn.accumulate(h, c2, x2, rows)
+        n2.forward(x2, h)
+        mlp.accumulate(h, x2, rows)
+    torch.cuda.synchronize()
+    assert torch.equal(x1, x2) and torch.equal(c1.keys(), c2.keys()) and torch.equal(c1.values(), c2.values())
+    assert c1.len() == c2.len() == 3 * rows and sg.last_status() == 0
