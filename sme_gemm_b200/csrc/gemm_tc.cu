@@ -394,6 +394,28 @@ __device__ __noinline__ void drain_tile(const GemmTcArgs& p, uint32_t tmem_base,
     }   // drain warps
 }
 
+// The MMAs of one stage: US 64-deep units, NW accumulator sets, NM token halves (NW * NM <= 2: 512 columns of tensor memory).
+template <int US, int NW, int NM, int CG>
+__device__ __forceinline__ void issue_stage(uint64_t a_st, uint64_t b_st, uint32_t tmem, int tok_bytes, int ntok_box, uint32_t idesc, int units, bool add) {
+#pragma unroll
+    for (int uu = 0; uu < US; ++uu) {
+        if (US > 1 && uu >= units) break;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            const uint64_t a0 = a_st + (uint64_t)((w * US + uu) * (kWTile >> 4));
+#pragma unroll
+            for (int h = 0; h < NM; ++h) {
+                const uint64_t b0 = b_st + (uint64_t)((uint32_t)(uu * tok_bytes + h * (tok_bytes / 2)) >> 4);
+                const uint32_t d = tmem + (uint32_t)((w * NM + h) * ntok_box);
+#pragma unroll
+                for (int ks = 0; ks < kStageK / 16; ++ks)
+                    if (CG == 2) umma_f16_2(d, a0 + 2 * ks, b0 + 2 * ks, idesc, (add || uu > 0 || ks > 0) ? 1u : 0u);
+                    else umma_f16(d, a0 + 2 * ks, b0 + 2 * ks, idesc, (add || uu > 0 || ks > 0) ? 1u : 0u);
+            }
+        }
+    }
+}
+
 template <int BF16, int US, int DENSE, int CG>
 __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_constant__ TcMaps<DENSE> maps, const __grid_constant__ GemmTcArgs p) {
     const CUtensorMap& tmap_tok = maps.tok;
@@ -569,7 +591,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
         // The whole warp walks the stages, converged, and one elected lane issues: the descriptors and barrier addresses
         // are then warp-uniform values.  (A loop run by one lane alone measured 10-25 % slower.)
         const uint32_t idesc = umma_idesc(BF16, 128 * CG, p.ntok_box);
-        const uint32_t tok_half = (uint32_t)(tok_bytes / 2);
         RingPos tq, oq;
         for (int i = 0; i < (leader ? num_stages : 0); ++i, tq.next(NT), oq.next(O)) {
             const int ts = tq.slot, os = oq.slot;
@@ -580,21 +601,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
             const uint32_t w_addr = smem_u32(ring_o + (size_t)os * o_stride);
             const int units = US == 1 ? 1 : min(US, p.ku - (st_begin + i) * US);
             if (elect_one()) {
-#pragma unroll
-                for (int uu = 0; uu < US; ++uu) {
-                    if (uu >= units) break;
-                    for (int w = 0; w < NW; ++w) {
-                        const uint64_t a_desc0 = umma_desc_sw128(w_addr + (w * US + uu) * kWTile);
-                        for (int h = 0; h < p.nmma; ++h) {
-                            const uint64_t b_desc0 = umma_desc_sw128(tok_addr + uu * tok_bytes + h * tok_half);
-                            const uint32_t d_tmem = tmem_base + (uint32_t)((w * p.nmma + h) * p.ntok_box);
-#pragma unroll
-                            for (int ks = 0; ks < kStageK / 16; ++ks)
-                                if (CG == 2) umma_f16_2(d_tmem, a_desc0 + 2 * ks, b_desc0 + 2 * ks, idesc, (i > 0 || uu > 0 || ks > 0) ? 1u : 0u);
-                                else umma_f16(d_tmem, a_desc0 + 2 * ks, b_desc0 + 2 * ks, idesc, (i > 0 || uu > 0 || ks > 0) ? 1u : 0u);
-                        }
-                    }
-                }
+                // (accumulator sets and token halves as constants: the loops unroll and the descriptors are sums of immediates)
+                const uint64_t a_st = umma_desc_sw128(w_addr), b_st = umma_desc_sw128(tok_addr);
+                if (NW == 1 && p.nmma == 1) issue_stage<US, 1, 1, CG>(a_st, b_st, tmem_base, tok_bytes, p.ntok_box, idesc, units, i > 0);
+                else if (NW == 1) issue_stage<US, 1, 2, CG>(a_st, b_st, tmem_base, tok_bytes, p.ntok_box, idesc, units, i > 0);
+                else issue_stage<US, 2, 1, CG>(a_st, b_st, tmem_base, tok_bytes, p.ntok_box, idesc, units, i > 0);
                 if (CG == 2) {
                     umma_commit2(&o_empty[os]);
                     umma_commit2(&t_empty[ts]);
