@@ -127,7 +127,8 @@ __device__ __noinline__ void stage_norm_row(uint16_t* dst, const float* xr, cons
     for (int j = dim + tid; j < kpad; j += kDThreads) dst[j] = 0;
 }
 
-template <int M>
+// GEN: the activations may be the norm of f32 rows (p.nx).
+template <int M, int GEN>
 __global__ void __launch_bounds__(kDThreads, 3) q4_direct_kernel(const __grid_constant__ Q4GemvArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int PF = kQ4PF;
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(kDThreads, 3) q4_direct_kernel(const __grid_co
 
     // ---- stage the activation rows (zero past k) ----
     __shared__ float norm_sh[8];
-    if (p.nx) {
+    if (GEN && p.nx) {
         for (int r = 0; r < M; ++r) stage_norm_row(As + (size_t)r * a_stride, p.nx + (size_t)r * p.k, p.nw, p.nbias, p.k, kpad, p.neps, p.nrms, norm_sh);
     } else if (!p.a_vec_ok) {
         // rows that are no whole 16-byte words, or start off a 16-byte boundary: a half at a time, eight loads in flight
@@ -608,13 +609,17 @@ cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream) {
     a.dupw = (a.k64 + kDWarps - 1) / kDWarps;
     size_t smem = kQ4RingBytes + (size_t)a.m * ((size_t)a.k64 * 64 + 8) * 2 + (size_t)kDWarps * a.cg * a.m * 16 * sizeof(float);
     if (per_sm == 2 && smem < 80 * 1024) smem = 80 * 1024;
+    // A narrow layer's projections all take the form that can norm: a step through such a layer is launches of 2 us, and going
+    // from one kernel's code to another's costs a fetch of it each time (six 384-wide layers 96 us a step, 111 with two kernels)
+    const bool gen = a.nx || (size_t)n16 * a.k64 <= 4096;
     const dim3 grid(grid_x);
     cudaError_t e;
 #define SMEG_QD(MM)                                                                   \
     case MM:                                                                          \
-        e = opt_in_smem(q4_direct_kernel<MM>, smem);                                  \
+        e = gen ? opt_in_smem(q4_direct_kernel<MM, 1>, smem) : opt_in_smem(q4_direct_kernel<MM, 0>, smem); \
         if (e != cudaSuccess) return e;                                               \
-        return launch_pdl(q4_direct_kernel<MM>, grid, dim3(kDThreads), smem, stream, a);
+        if (gen) return launch_pdl(q4_direct_kernel<MM, 1>, grid, dim3(kDThreads), smem, stream, a); \
+        return launch_pdl(q4_direct_kernel<MM, 0>, grid, dim3(kDThreads), smem, stream, a);
     switch (a.m) {
         SMEG_QD(1) SMEG_QD(2)
     default: return cudaErrorInvalidValue;
