@@ -869,11 +869,12 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
         aq.qsum = (w->bits == 1 || tc || mma) ? (int32_t*)(ws + q_bytes + sa_bytes) : nullptr;
         aq.m = (int)m; aq.k = (int)k; aq.kq = (int)kq; aq.nbq = (int)nb; aq.log2_block = w->d.log2_block;
         if (tc) {
+            const bool one_run = lowbit_tc_one_run(w->d.log2_block, sums_out != nullptr);
             aq.sa_t = (float*)(ws + q_bytes + 2 * sa_bytes);
-            aq.qsum_t = (float*)(ws + q_bytes + 2 * sa_bytes + t_bytes);
+            if (!one_run) aq.qsum_t = (float*)(ws + q_bytes + 2 * sa_bytes + t_bytes);
             aq.qh = (uint16_t*)(ws + q_bytes + 2 * sa_bytes + 2 * t_bytes);
             aq.mpad = (int)mpad;
-            aq.qh_perm = w->bits == 1 ? 2 : 0;                         // 1-bit: the order and scaling the kernel's operand tiles take
+            aq.qh_perm = w->bits == 1 ? (one_run ? 1 : 2) : 0;         // 1-bit: the order (and scaling) the kernel's operands take
         }
         if (mma) {
             aq.qh = (uint16_t*)(ws + q_bytes + 2 * sa_bytes + 2 * t_bytes);

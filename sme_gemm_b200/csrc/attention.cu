@@ -39,15 +39,6 @@ constexpr int kAtMaxSlots = 8;
 constexpr uint32_t kAtOCol = 256;                 // tensor memory: S / P buffers at columns 0 and 128, O behind them
 constexpr float kAtPScale = 32768.0f;             // probabilities are scaled by 2^15 on their way into two f16 parts
 
-// D[tmem] (+)= A[tmem] * B[smem desc], kind::f16
-__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
-        : "memory");
-}
 // MN-major tile stored as rows of 64 MN elements (128 bytes, 128-byte swizzle) per K index: 8-row groups along K 1024 bytes
 // apart, 64-element chunks along MN one kAtChunk apart.
 __device__ __forceinline__ uint64_t umma_desc_sw128_mn(uint32_t smem_addr) {

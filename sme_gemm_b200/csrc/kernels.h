@@ -132,7 +132,7 @@ struct LowbitTcArgs {
     const uint16_t* scales;       // f16 bits [n16][nb][16]
     const uint16_t* qh;           // m x kq activation codes as f16 integers (act_quant_kernel)
     const float* sa_t;            // nb x mpad activation scales, block-major
-    const float* qsum_t;          // nb x mpad per-block sums of q, as floats
+    const float* qsum_t;          // nb x mpad per-block sums of q, as floats (not for K-blocks of one run)
     int mpad;                     // row length of sa_t and qsum_t: whole row tiles of up to 128 rows from any row below m
     uint16_t* c;                  // m x n f16 bits
     int32_t* sums_out;            // optional debug: m x n x nb_real exact block sums
@@ -144,6 +144,7 @@ struct LowbitTcArgs {
     EpParams ep;
 };
 bool lowbit_tc_supported(int bits, int m, int k, int log2_block);
+bool lowbit_tc_one_run(int log2_block, bool sums);                 // which form of the kernel (and of its codes) a call takes
 cudaError_t lowbit_tc_launch(LowbitTcArgs a, int sm_count, cudaStream_t stream);
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point lookup (gemm_tc.cu); null if unavailable.

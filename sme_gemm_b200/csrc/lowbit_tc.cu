@@ -48,6 +48,8 @@
 #include "layout.h"
 #include "tc_common.cuh"
 
+#include <type_traits>
+
 namespace smeg {
 namespace {
 
@@ -363,25 +365,26 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// K-blocks of one run (16 to 256 depths), the form every model's call takes.  The roles are those above; what differs is
-// the cost per depth of the single-warp chains.  Measured at one 64-deep stage per hand-off the MMA warp took ~1080 cycles
-// a stage whatever the tile (each wait ~120, four instructions and two commits ~310, ring arithmetic ~340), everything
-// else waiting for it.  Here a stage is 128 depths, its operand and row tiles share one pair of barriers (a wait and a
-// commit each), accumulators are asked for only where a run begins, and ring positions are counters.
-//   warps 0-7 (expand)  two groups of four warps take alternate stages, a warp two column groups; lanes of odd column
-//                       write the two 32-deep steps of a tile in the other order, so that stores are free of bank conflicts
-//   warps 8-23 (fold)   four warps per lane quarter, NT / 4 rows each, totals in registers; two rows per instruction
-//                       (f32x2), the block's integer from one exact fused multiply-add
-// NT rows per CTA are chosen by the launcher.  1-bit 512 x 4096 x 14336: 219 us with 64-deep stages.
+// K-blocks of one run (16 to 256 depths), the form every model's call takes.  The roles are those above; what differs:
+//   * a stage is 128 depths and its operands share one pair of barriers; accumulators change hands in groups (a wait and an
+//     arrival of every fold warp cost ~0.6 us of a K-block whatever its depth) and are asked for only where one begins;
+//   * the expanded weights go to tensor memory (A operand of the MMA; thread = weight column, 128 depths = 64 columns, four
+//     slots), not to shared memory, whose 128 bytes a cycle bound the kernel: written and read there they were half of a
+//     stage's traffic at 128 rows;
+//   * a weight is its value as an f16 number (1-bit: +-1, the packed bit shifted to the sign; 2-bit: a byte-permute lookup of the
+//     codebook's f16 halves), so the accumulator is the K-block's integer itself (|sum| < 2^23, exact) and the fold reads one
+//     operand per row, its activation scale: every lane of 16 warps reads each of them, and with the code sums beside them
+//     these broadcasts were the other half;
+//   * 16 fold warps, four per lane quarter, NT / 4 rows each, totals in registers, two rows per instruction (f32x2).
+// NT rows per CTA are chosen by the launcher.  1-bit 512 x 4096 x 14336: 219 us with 64-deep stages in shared memory.
 constexpr int kLbThreads = 32 * 28;
-constexpr int kLbNK = 3, kLbNF = 3;               // ring depths: packed slots (two units a column group), fold operands
+constexpr int kLbNK = 3, kLbNF = 6;               // ring depths: packed slots (two units a column group), fold operands
 constexpr int kLbKSlot = 8 * 2 * kUnitBytes;
-__host__ __device__ constexpr int lb_slots(int nt) { return nt >= 96 ? 3 : 4; }
-// Accumulators change hands in groups (a wait and an arrival of every fold warp cost ~0.6 us of a K-block whatever its depth):
-// two groups of them, and a fold slot holds the operands of a group's blocks.
-__host__ __device__ constexpr int lb_group(int nt) { return nt >= 96 ? 2 : 4; }
+constexpr int kLbNS = 4;                          // stages in flight: row tiles in shared memory, weights in tensor memory
+constexpr uint32_t kLbACol = 256;                 // tensor memory: two groups of accumulators below, the weights of the stages from here
+__host__ __device__ constexpr int lb_group(int nt) { return nt >= 96 ? 1 : 128 / nt; }
 __host__ __device__ constexpr size_t lb_smem(int nt) {
-    return 1024 + (size_t)lb_slots(nt) * (2 * kLtATile + nt * 256) + (size_t)kLbNK * kLbKSlot + 1024 + (size_t)kLbNF * lb_group(nt) * (nt * 8 + 256);
+    return 1024 + (size_t)kLbNS * nt * 256 + (size_t)kLbNK * kLbKSlot + 1024 + (size_t)kLbNF * lb_group(nt) * (nt * 4 + 256);
 }
 
 typedef unsigned long long f32x2;
@@ -411,14 +414,20 @@ struct LbRing {
     }
 };
 
+// Tensor maps of the four streams, one tiled copy per stage, packed slot or group of K-blocks each (ten bulk copies of 32 to 512
+// bytes per K-block took their warp ~1000 cycles to issue, more than everything else did in that time):
+//   rows    activation codes as f16 [m][kq], 64 depths x NT rows       codes   packed units [n16][ku x 512 B], two units of 8 groups
+//   sa      activation scales [nb][mpad], NT rows of G blocks      scales  [n16][nb x 32 B], G blocks of 8 groups
+struct LbMaps { CUtensorMap rows, codes, sa, scales; };
+
 template <int BITS, int NT>
-__global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ LowbitTcArgs p) {
-    constexpr int NS = lb_slots(NT), G = lb_group(NT), ACC_STRIDE = 256 / G;   // two groups of G accumulators in 512 columns
+__global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __grid_constant__ LbMaps maps, const __grid_constant__ LowbitTcArgs p) {
+    constexpr int NS = kLbNS, G = lb_group(NT), ACC_STRIDE = 128 / G;
     constexpr int TPW = NT / 4;                                // rows of a fold warp
     constexpr int BTILE = NT * 128;                            // row tile of 64 depths
-    constexpr int SLOT = 2 * kLtATile + 2 * BTILE;
+    constexpr int SLOT = 2 * BTILE;
     constexpr int SPK = BITS == 2 ? 2 : 4;                     // stages per packed slot
-    constexpr int FSLOT = NT * 8 + 256;
+    constexpr int FSLOT = G * (NT * 4 + 256);                  // [G][NT] row scales, then [8 column groups][G][16 f16 scales]
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
     unsigned char* ring_k = smem + (size_t)NS * SLOT;
@@ -455,49 +464,43 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
 
     if (warp == 24) {                                          // ---- row tiles ----
         if (lane == 0) {
-            tma_prefetch_desc(&tmap_q);
+            tma_prefetch_desc(&maps.rows);
             LbRing r;
             for (int i = 0; i < stages; ++i, r.next(NS)) {
                 if (r.wrapped && !mbar_wait(&empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT)) break;
-                unsigned char* b = smem + (size_t)r.slot * SLOT + 2 * kLtATile;
+                unsigned char* b = smem + (size_t)r.slot * SLOT;
                 mbar_expect_tx(&full[r.slot], 2 * BTILE);
-                tma_load_2d(b, &tmap_q, i * 128, tok0, &full[r.slot]);
-                tma_load_2d(b + BTILE, &tmap_q, i * 128 + 64, tok0, &full[r.slot]);
+                tma_load_2d(b, &maps.rows, i * 128, tok0, &full[r.slot]);
+                tma_load_2d(b + BTILE, &maps.rows, i * 128 + 64, tok0, &full[r.slot]);
             }
         }
-    } else if (warp == 26) {                                   // ---- packed weights: lane c = column group c ----
-        LbRing r;
-        const size_t cgi = (size_t)min(cg0 + (lane & 7), p.n16 - 1);             // a tail group re-reads the last one
-        for (int u0 = 0; u0 * (BITS == 2 ? kQ2UnitDepth : kQ1UnitDepth) < k_end; u0 += 2, r.next(kLbNK)) {
-            if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&k_empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
-            const int units = min(2, p.ku - u0);
-            if (lane == 0) mbar_expect_tx(&k_full[r.slot], (unsigned)(8 * units * kUnitBytes));
-            __syncwarp();
-            if (lane < 8)
-                bulk_g2s(ring_k + (size_t)r.slot * kLbKSlot + (size_t)lane * 2 * kUnitBytes, p.codes + (cgi * p.ku + (size_t)u0) * kUnitBytes,
-                         units * kUnitBytes, &k_full[r.slot]);
-            __syncwarp();
-        }
-    } else if (warp == 27) {                                   // ---- fold operands: lane 0 the rows' scales, 1 their code sums, 2-9 scale rows ----
-        LbRing r;
-        const size_t cgi = (size_t)min(cg0 + max(lane - 2, 0), p.n16 - 1);
-        for (int blk0 = 0; blk0 < p.nb_real; blk0 += G, r.next(kLbNF)) {
-            if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&f_empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
-            const int blocks = min(G, p.nb_real - blk0);
-            if (lane == 0) mbar_expect_tx(&f_full[r.slot], (unsigned)(blocks * FSLOT));
-            __syncwarp();
-            for (int j = 0; j < blocks; ++j) {
-                const int blk = blk0 + j;
-                unsigned char* dst = ring_f + (size_t)(r.slot * G + j) * FSLOT;
-                if (lane == 0) bulk_g2s(dst, p.sa_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
-                else if (lane == 1) bulk_g2s(dst + NT * 4, p.qsum_t + (size_t)blk * p.mpad + tok0, NT * 4, &f_full[r.slot]);
-                else if (lane < 10) bulk_g2s(dst + NT * 8 + (lane - 2) * 32, p.scales + (cgi * p.nb + (size_t)blk) * 16, 32, &f_full[r.slot]);
+    } else if (warp == 26) {                                   // ---- packed weights ----
+        if (lane == 0) {
+            tma_prefetch_desc(&maps.codes);
+            LbRing r;
+            for (int u0 = 0; u0 * (BITS == 2 ? kQ2UnitDepth : kQ1UnitDepth) < k_end; u0 += 2, r.next(kLbNK)) {
+                if (r.wrapped && !mbar_wait(&k_empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT)) break;
+                // whole boxes always: what lies past the last unit or column group arrives as zeros and is never used
+                mbar_expect_tx(&k_full[r.slot], (unsigned)kLbKSlot);
+                tma_load_2d(ring_k + (size_t)r.slot * kLbKSlot, &maps.codes, u0 * (kUnitBytes / 8), cg0, &k_full[r.slot]);
             }
-            __syncwarp();
+        }
+    } else if (warp == 27) {                                   // ---- fold operands ----
+        if (lane == 0) {
+            tma_prefetch_desc(&maps.sa);
+            tma_prefetch_desc(&maps.scales);
+            LbRing r;
+            for (int blk0 = 0; blk0 < p.nb_real; blk0 += G, r.next(kLbNF)) {
+                if (r.wrapped && !mbar_wait(&f_empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT)) break;
+                unsigned char* dst = ring_f + (size_t)r.slot * FSLOT;
+                mbar_expect_tx(&f_full[r.slot], (unsigned)FSLOT);
+                tma_load_2d(dst, &maps.sa, tok0, blk0, &f_full[r.slot]);
+                tma_load_2d(dst + G * NT * 4, &maps.scales, blk0 * 4, cg0, &f_full[r.slot]);
+            }
         }
     } else if (warp == 25) {                                   // ---- MMA ----
         const uint32_t idesc = umma_idesc(0, 128, NT);
-        const uint64_t a_first = umma_desc_sw128(smem_u32(smem)), b_first = umma_desc_sw128(smem_u32(smem) + 2 * kLtATile);
+        const uint64_t b_first = umma_desc_sw128(smem_u32(smem));
         LbRing r, acc;                                         // acc: group of accumulators; ga: the one in it
         int ga = 0;
         const int L = p.log2_block;
@@ -509,17 +512,18 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
                 if (ga == 0 && first && acc.wrapped && !__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
                 if (!__all_sync(0xffffffffu, mbar_wait(&full[r.slot], r.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
                 tc_fence_after();
-                const uint64_t ad = a_first + (uint64_t)(r.slot * (SLOT >> 4)), bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
+                const uint32_t at = tmem + kLbACol + 64u * (uint32_t)r.slot;
+                const uint64_t bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
                 const uint32_t d = tmem + (uint32_t)((acc.slot * G + ga) * ACC_STRIDE);
                 const bool hand = last && (ga == G - 1 || i == stages - 1);
                 if (elect_one()) {
                     if (k_end - i * 128 >= 128) {
 #pragma unroll
                         for (int ks = 0; ks < 8; ++ks)
-                            umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > 0 || !first);
+                            umma_f16_ts(d, at + 8 * ks, bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > 0 || !first);
                     } else {
                         for (int ks = 0; i * 128 + 16 * ks < k_end; ++ks)
-                            umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > 0 || !first);
+                            umma_f16_ts(d, at + 8 * ks, bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > 0 || !first);
                     }
                     umma_commit(&empty[r.slot]);
                     if (hand) umma_commit(&acc_full[acc.slot]);
@@ -531,88 +535,102 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
         } else {
             // several runs per stage, an accumulator each; a group is asked for as its first run begins (the groups before it
             // are on their way to the fold warps by then)
-            const int steps = 1 << (L - 4);
-            bool ok = true;
-            for (int i = 0; ok && i < stages; ++i, r.next(NS)) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&full[r.slot], r.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t ad = a_first + (uint64_t)(r.slot * (SLOT >> 4)), bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
-                const int left = min(8, (k_end - i * 128) >> 4);                 // K = 16 steps of the stage
-                for (int k0 = 0; k0 < left; k0 += steps) {
-                    if (ga == 0 && acc.wrapped) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
-                        if (!ok) break;
-                        tc_fence_after();
+            auto walk = [&](auto steps_c) {
+                constexpr int STEPS = decltype(steps_c)::value;              // K = 16 steps of a run
+                for (int i = 0; i < stages; ++i, r.next(NS)) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&full[r.slot], r.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) return;
+                    tc_fence_after();
+                    const uint32_t at = tmem + kLbACol + 64u * (uint32_t)r.slot;
+                    const uint64_t bd = b_first + (uint64_t)(r.slot * (SLOT >> 4));
+                    const int left = min(8, (k_end - i * 128) >> 4);             // K = 16 steps of the stage
+#pragma unroll
+                    for (int k0 = 0; k0 < 8; k0 += STEPS) {
+                        if (k0 >= left) break;
+                        if (ga == 0 && acc.wrapped) {
+                            if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[acc.slot], acc.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) return;
+                            tc_fence_after();
+                        }
+                        const uint32_t d = tmem + (uint32_t)((acc.slot * G + ga) * ACC_STRIDE);
+                        const bool end = k0 + STEPS >= left, hand = ga == G - 1 || (end && i == stages - 1);
+                        if (elect_one()) {
+#pragma unroll
+                            for (int ks = k0; ks < k0 + STEPS; ++ks)
+                                if (ks < left) umma_f16_ts(d, at + 8 * ks, bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > k0);
+                            if (hand) umma_commit(&acc_full[acc.slot]);
+                            if (end) umma_commit(&empty[r.slot]);
+                        }
+                        __syncwarp();
+                        if (hand) { ga = 0; acc.next(2); }
+                        else ++ga;
                     }
-                    const uint32_t d = tmem + (uint32_t)((acc.slot * G + ga) * ACC_STRIDE);
-                    const bool end = k0 + steps >= left, hand = ga == G - 1 || (end && i == stages - 1);
-                    if (elect_one()) {
-                        for (int ks = k0; ks < k0 + steps && ks < left; ++ks)
-                            umma_f16(d, ad + (ks >> 2) * (kLtATile >> 4) + 2 * (ks & 3), bd + (ks >> 2) * (BTILE >> 4) + 2 * (ks & 3), idesc, ks > k0);
-                        if (hand) umma_commit(&acc_full[acc.slot]);
-                        if (end) umma_commit(&empty[r.slot]);
-                    }
-                    __syncwarp();
-                    if (hand) { ga = 0; acc.next(2); }
-                    else ++ga;
                 }
-            }
+            };
+            if (L == 6) walk(std::integral_constant<int, 4>());
+            else if (L == 5) walk(std::integral_constant<int, 2>());
+            else walk(std::integral_constant<int, 1>());
         }
     } else if (warp < 8) {                                     // ---- expand ----
-        const int g = lane >> 2, t = lane & 3, group = warp >> 2, wg = warp & 3, odd = g & 1;
-        // a lane's 16 bytes of 32-deep step s land in chunk 4 s + t of rows g (low) and g + 8 (high) of a column group; lanes
-        // of odd g take step 1 first
-        const uint32_t base = smem_u32(smem) + (uint32_t)(2 * wg * 2048 + g * 128);
-        const uint32_t o0 = (uint32_t)(((4 * odd + t) ^ g) << 4), o1 = (uint32_t)(((4 * (odd ^ 1) + t) ^ g) << 4);
-        const uint32_t pk = smem_u32(ring_k) + (uint32_t)(2 * wg * 2 * kUnitBytes + lane * 16);
-        auto sts = [](uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-        };
+        // thread = weight column: group `group` of warps takes every other stage, warp w the lane quarter w % 4
+        const int group = warp >> 2, q = warp & 3, cl = 32 * q + lane, g = cl & 7, hi = (cl >> 3) & 1;
+        const uint32_t at = tmem + ((uint32_t)(32 * q) << 16) + kLbACol;
+        // the column's depths lie in the 16-byte vectors of four lanes of its column group's units (packed for lane (g, t):
+        // columns g and g + 8, runs of eight depths at 8 t)
+        const uint32_t pk = smem_u32(ring_k) + (uint32_t)((cl >> 4) * 2 * kUnitBytes + g * 64);
+        uint32_t lut_lo = 0, lut_hi = 0;                       // 2-bit: low and high bytes of the codebook's values as f16 numbers
+        if (BITS == 2) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t h = __half_as_ushort(__int2half_rn((int)(int8_t)((p.lut ^ 0x80808080u) >> (8 * c))));
+                lut_lo |= (h & 0xffu) << (8 * c);
+                lut_hi |= (h >> 8) << (8 * c);
+            }
+        }
         LbRing r, kr;
         if (group) r.next(NS);
         for (int i = group; i < stages; i += 2, r.next(NS), r.next(NS)) {
             const int part = i & (SPK - 1);                    // stage within its packed slot
             if (i >= SPK && part == group) kr.next(kLbNK);
-            if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
             if (!__all_sync(0xffffffffu, mbar_wait(&k_full[kr.slot], kr.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
-            const uint32_t at = base + (uint32_t)(r.slot * SLOT);
-            // 2-bit: a unit is the stage; 1-bit: words 0, 1 or 2, 3 of a unit
-            const uint32_t src = pk + (uint32_t)(kr.slot * kLbKSlot + (BITS == 2 ? part : part >> 1) * kUnitBytes);
+            // 2-bit: a unit is the stage, word s its 32-deep step s; 1-bit: half a unit, a word two steps
+            const uint32_t src = pk + (uint32_t)(kr.slot * kLbKSlot) + (uint32_t)(BITS == 2 ? part * kUnitBytes : (part >> 1) * kUnitBytes + (part & 1) * 8);
+            uint32_t w[4][BITS == 2 ? 4 : 2];
 #pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-                uint32_t w[4];
-                if (BITS == 2) {
-                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(src + cc * 2 * kUnitBytes) : "memory");
-                } else {
-                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(src + cc * 2 * kUnitBytes + (uint32_t)(part & 1) * 8) : "memory");
-                }
+            for (int t = 0; t < 4; ++t) {
+                if constexpr (BITS == 2)
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[t][0]), "=r"(w[t][1]), "=r"(w[t][2]), "=r"(w[t][3]) : "r"(src + 16 * t) : "memory");
+                else
+                    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(w[t][0]), "=r"(w[t][1]) : "r"(src + 16 * t) : "memory");
+            }
+            if (r.wrapped && !__all_sync(0xffffffffu, mbar_wait(&empty[r.slot], r.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+            tc_fence_after();
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {                  // 64-deep tile
-                    const uint32_t dst = at + (uint32_t)(cc * 2048 + h * kLtATile);
+            for (int s = 0; s < 4; ++s) {                      // 32-deep step: 16 tensor-memory columns
+                uint32_t o[16];
 #pragma unroll
-                    for (int s = 0; s < 2; ++s) {              // step s ^ odd
-                        const uint32_t lo = dst + (s ? o1 : o0), hi = lo + 1024;
-                        if (BITS == 1) {
-                            // A sign bit stays where it lies in its half word: bit b of an f16 is the number 2^(b-24) for
-                            // b < 12, and act_quant_kernel has left the codes of a run of eight depths in the order
-                            // 0 2 1 3 4 6 5 7, scaled by 2^8 2^8 1 1 2^6 2^6 2^-2 2^-2: every product of column g is
-                            // u q 2^-16 and of column g + 8 (one bit higher) u q 2^-15.  One AND per register.
-                            const uint32_t v = w[h] >> (4 * (s ^ odd));
-                            sts(lo, v & 0x00010001u, v & 0x01000100u, v & 0x00040004u, v & 0x04000400u);
-                            sts(hi, v & 0x00020002u, v & 0x02000200u, v & 0x00080008u, v & 0x08000800u);
-                        } else {
-                            const uint32_t x = (s ^ odd) ? w[2 * h + 1] : w[2 * h];
-                            const uint32_t e = x & 0x33333333u, o = (x >> 2) & 0x33333333u;
-                            const uint2 l0 = widen4(prmt2(p.lut, 0u, e)), l1 = widen4(prmt2(p.lut, 0u, e >> 16));
-                            const uint2 h0 = widen4(prmt2(p.lut, 0u, o)), h1 = widen4(prmt2(p.lut, 0u, o >> 16));
-                            sts(lo, l0.x, l0.y, l1.x, l1.y);
-                            sts(hi, h0.x, h0.y, h1.x, h1.y);
+                for (int t = 0; t < 4; ++t) {
+                    if (BITS == 1) {
+                        // the bits of depths (0, 2), (1, 3), (4, 6), (5, 7) -- the order act_quant_kernel leaves the codes in --
+                        // lie 16 apart: one shift brings a pair to the signs of two f16 ones (bit set = +1)
+                        const uint32_t v = w[t][s >> 1] << (1 - hi);
+                        const int up = 14 - 4 * (s & 1);
+                        o[4 * t] = (~(v << up) & 0x80008000u) | 0x3c003c00u;
+                        o[4 * t + 1] = (~(v << (up - 8)) & 0x80008000u) | 0x3c003c00u;
+                        o[4 * t + 2] = (~(v << (up - 2)) & 0x80008000u) | 0x3c003c00u;
+                        o[4 * t + 3] = (~(v << (up - 10)) & 0x80008000u) | 0x3c003c00u;
+                    } else {
+                        const uint32_t e = (w[t][s] >> (2 * hi)) & 0x33333333u;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {          // depths 0-3, 4-7
+                            const uint32_t lo = prmt2(lut_lo, 0u, e >> (16 * h)), up = prmt2(lut_hi, 0u, e >> (16 * h));
+                            o[4 * t + 2 * h] = prmt2(lo, up, 0x5140u);
+                            o[4 * t + 2 * h + 1] = prmt2(lo, up, 0x7362u);
                         }
                     }
                 }
+                tmem_st16(at + (uint32_t)(64 * r.slot + 16 * s), o);
             }
-            fence_proxy_async();
+            tmem_st_wait();
+            tc_fence_before();
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&full[r.slot]);
@@ -623,12 +641,7 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
         const int dw = warp - 8, q = dw & 3, part = dw >> 2;
         const int cl = 32 * q + lane, col = col0 + cl;
         const uint32_t acc_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(part * TPW);
-        const int sc_off = NT * 8 + (cl >> 4) * 32 + scale_slot(cl & 15) * 2;    // this column's scale inside a fold slot
-        // An accumulator is S = sum u q times 2^-24 (2-bit), 2^-16 or 2^-15 (1-bit, columns g and g + 8), exactly; the block's
-        // integer is 2 S - sum(q) (1-bit) or S - 128 sum(q).  nsum = fma(acc, mul, sum(q)) is minus that (2-bit: a 128th of
-        // it), exactly, and its factor carries the sign (and the 128) back: nsum * -(scale * sa) is the reference's product.
-        const float mul = BITS == 2 ? -131072.0f : ((cl & 8) ? -65536.0f : -131072.0f);
-        const f32x2 mul2 = pack_f32x2(mul, mul);
+        const int sc_off = G * NT * 4 + (cl >> 4) * (G * 32) + scale_slot(cl & 15) * 2;   // this column's first scale inside a fold slot
         f32x2 tot[TPW / 2];
 #pragma unroll
         for (int j = 0; j < TPW / 2; ++j) tot[j] = 0ull;
@@ -644,12 +657,10 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
 #pragma unroll
             for (int gi = 0; gi < G; ++gi) {
                 if (gi >= blocks) break;
-                const unsigned char* fo = ring_f + (size_t)(fr.slot * G + gi) * FSLOT;
-                const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off)));
-                const float ns = BITS == 2 ? -128.0f * scale : -scale;
-                const f32x2 ns2 = pack_f32x2(ns, ns);
-                const ulonglong2* sa = reinterpret_cast<const ulonglong2*>(fo + part * TPW * 4);
-                const ulonglong2* qf = reinterpret_cast<const ulonglong2*>(fo + NT * 4 + part * TPW * 4);
+                const unsigned char* fo = ring_f + (size_t)fr.slot * FSLOT;
+                const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off + gi * 32)));
+                const f32x2 scale2 = pack_f32x2(scale, scale);
+                const ulonglong2* sa = reinterpret_cast<const ulonglong2*>(fo + gi * NT * 4 + part * TPW * 4);
                 constexpr int CH = TPW % 16 == 0 ? 16 : 8;                       // accumulator values read at a time
 #pragma unroll
                 for (int c0 = 0; c0 < TPW; c0 += CH) {
@@ -665,12 +676,11 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
                     }
 #pragma unroll
                     for (int j = 0; j < CH; j += 4) {
-                        const ulonglong2 s2 = sa[(c0 + j) / 4], q2 = qf[(c0 + j) / 4];
-                        const f32x2 n0 = fma_f32x2(pack_f32x2(__uint_as_float(av[j]), __uint_as_float(av[j + 1])), mul2, q2.x);
-                        const f32x2 n1 = fma_f32x2(pack_f32x2(__uint_as_float(av[j + 2]), __uint_as_float(av[j + 3])), mul2, q2.y);
+                        // total = fmaf((float)sum, scale * sa, total), the reference's statement, two rows at a time
+                        const ulonglong2 s2 = sa[(c0 + j) / 4];
                         f32x2* to = tot + (c0 + j) / 2;
-                        to[0] = fma_f32x2(n0, mul_f32x2(ns2, s2.x), to[0]);
-                        to[1] = fma_f32x2(n1, mul_f32x2(ns2, s2.y), to[1]);
+                        to[0] = fma_f32x2(pack_f32x2(__uint_as_float(av[j]), __uint_as_float(av[j + 1])), mul_f32x2(scale2, s2.x), to[0]);
+                        to[1] = fma_f32x2(pack_f32x2(__uint_as_float(av[j + 2]), __uint_as_float(av[j + 3])), mul_f32x2(scale2, s2.y), to[1]);
                     }
                 }
             }
@@ -712,7 +722,25 @@ cudaError_t launch_lt(const CUtensorMap& tm, const LowbitTcArgs& a, dim3 grid, s
 }
 
 template <int BITS, int NT>
-cudaError_t launch_lb(const CUtensorMap& tm, const LowbitTcArgs& a, dim3 grid, cudaStream_t stream) {
+cudaError_t launch_lb(const CUtensorMap& rows, const LowbitTcArgs& a, dim3 grid, cudaStream_t stream) {
+    constexpr int G = lb_group(NT);
+    LbMaps maps;
+    maps.rows = rows;
+    const cuuint32_t estr[2] = {1, 1};
+    const cuuint64_t cdim[2] = {(cuuint64_t)a.ku * (kUnitBytes / 8), (cuuint64_t)a.n16}, cstride[1] = {(cuuint64_t)a.ku * kUnitBytes};
+    const cuuint32_t cbox[2] = {2 * kUnitBytes / 8, 8};
+    const cuuint64_t qdim[2] = {(cuuint64_t)a.mpad, (cuuint64_t)a.nb}, qstride[1] = {(cuuint64_t)a.mpad * 4};
+    const cuuint32_t qbox[2] = {NT, (cuuint32_t)G};
+    const cuuint64_t sdim[2] = {(cuuint64_t)a.nb * 4, (cuuint64_t)a.n16}, sstride[1] = {(cuuint64_t)a.nb * 32};
+    const cuuint32_t sbox[2] = {(cuuint32_t)(4 * G), 8};
+    auto map = [&](CUtensorMap* m, CUtensorMapDataType type, const void* base, const cuuint64_t* dim, const cuuint64_t* stride, const cuuint32_t* box) {
+        return tensor_map_encoder()(m, type, 2, (void*)base, dim, stride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                    CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!map(&maps.codes, CU_TENSOR_MAP_DATA_TYPE_UINT64, a.codes, cdim, cstride, cbox) ||
+        !map(&maps.sa, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.sa_t, qdim, qstride, qbox) ||
+        !map(&maps.scales, CU_TENSOR_MAP_DATA_TYPE_UINT64, a.scales, sdim, sstride, sbox))
+        return cudaErrorInvalidValue;
     auto kern = lowbit_tc_block_kernel<BITS, NT>;
     static int attr_dev = -1;
     int dev = 0;
@@ -722,7 +750,7 @@ cudaError_t launch_lb(const CUtensorMap& tm, const LowbitTcArgs& a, dim3 grid, c
         if (e != cudaSuccess) return e;
         attr_dev = dev;
     }
-    return launch_pdl(kern, grid, dim3(kLbThreads), lb_smem(NT), stream, tm, a);
+    return launch_pdl(kern, grid, dim3(kLbThreads), lb_smem(NT), stream, maps, a);
 }
 
 }  // namespace
@@ -734,18 +762,20 @@ bool lowbit_tc_supported(int bits, int m, int k, int log2_block) {
     return tensor_map_encoder() != nullptr;
 }
 
+bool lowbit_tc_one_run(int log2_block, bool sums) { return log2_block <= 8 && !sums; }
+
 cudaError_t lowbit_tc_launch(LowbitTcArgs a, int sm_count, cudaStream_t stream) {
     // blocks of one run and no debug output: the floating-point fold
-    const bool one_run = a.log2_block <= 8 && a.sums_out == nullptr;
+    const bool one_run = lowbit_tc_one_run(a.log2_block, a.sums_out != nullptr);
     const int col_tiles = (a.n + 127) / 128;
     // an MMA of 128 weight columns takes 16 rows or more
     int nt = a.m <= 16 ? 16 : (a.m <= 32 ? 32 : 64);
     if (one_run) {
-        // rows per CTA: the fewest (waves x time of a tile); a tile costs its expansion whatever its rows, about what 100
+        // rows per CTA: the fewest (waves x time of a tile); a tile costs its expansion whatever its rows, about what 60
         // rows of fold cost
         long long best = 0;
         for (int t : {128, 96, 64, 32}) {
-            const long long tiles = (long long)col_tiles * ((a.m + t - 1) / t), cost = (tiles + sm_count - 1) / sm_count * (100 + t);
+            const long long tiles = (long long)col_tiles * ((a.m + t - 1) / t), cost = (tiles + sm_count - 1) / sm_count * (60 + t);
             if (best == 0 || cost < best) { best = cost; nt = t; }
         }
     }
