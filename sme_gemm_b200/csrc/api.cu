@@ -1063,6 +1063,20 @@ int smeg_gemm_dense_dev(const smeg_dense* w, const uint16_t* a, uint16_t* c, siz
     EpNodeDev* ext = nullptr;
     int rc = make_ep(ep, n, &t.ep, stream, &ext);
     if (rc) { if (ext) cudaFreeAsync(ext, stream); if (a_pad) cudaFreeAsync(a_pad, stream); return rc; }
+    if (m <= 8 || div_up(n, 16) * ((k_run + 63) / 64) * div_up(m, 16) <= 20000) {
+        // The warp-level kernel streams the weights once per 16 rows: about 1.6 us and 0.33 us per 1000 units (16 columns x 64
+        // depths) and 16 rows, where the GEMM takes 9 us and more (2048 x 1504 f16, us, GEMM / this: 1 row 9.4 / 2.1, 17 rows
+        // 8.5 / 3.3; 4096 x 2048: 1 row 9.1 / 3.1, 32 rows 11.4 / 7.2).
+        Q4GemvArgs g;
+        memset(&g, 0, sizeof(g));
+        g.wdense = w->w; g.kd = (int)w->kd; g.a = a_run; g.c = c; g.beta = w->bf16 ? __uint_as_float_host((uint32_t)beta_bits << 16) : h2f(beta_bits);
+        g.col_major = col_major ? 1 : 0;
+        g.m = (int)m; g.n = (int)n; g.k = (int)k_run; g.k64 = (int)((k_run + 63) / 64); g.a_vec_ok = 1; g.status = ds->status; g.ep = t.ep;
+        const cudaError_t e = q4_mma_launch(g, w->bf16, ds->sm_count, stream);
+        if (ext) cudaFreeAsync(ext, stream);
+        if (a_pad) cudaFreeAsync(a_pad, stream);
+        return e == cudaSuccess ? 0 : -6;
+    }
     t.wdense = w->w; t.kd = (int)w->kd; t.a = a_run; t.c = c;
     t.beta = w->bf16 ? __uint_as_float_host((uint32_t)beta_bits << 16) : h2f(beta_bits);
     t.col_major = col_major ? 1 : 0;

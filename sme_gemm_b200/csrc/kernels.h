@@ -24,7 +24,11 @@ struct Q4GemvArgs {
     const float *nx, *nw, *nbias; // if nx: the activations are norm(nx) (f32 rows of k, weight nw, bias nbias or null), formed by every CTA
     float neps;
     int nrms;                     // rms_norm (else layer_norm)
-    uint16_t *kc, *vc;            // if set: columns from q_len on are keys, then values: kv_len of each go to rows of kc / vc instead of c
+    // q4_mma_kernel on dense weights
+    const uint16_t* wdense;       // W[n][kd] K-major instead of codes / scales (k = kd, a multiple of 8)
+    int kd, col_major;            // row length of wdense; C column-major: c[i + j * m]
+    float beta;                   // the product is scaled by it before the store rounding
+    uint16_t *kc, *vc;            // (one-wave kernel) if set: columns from q_len on are keys, then values: kv_len of each go to rows of kc / vc instead of c
     int q_len, kv_len;
     int m, n, k;
     int n16, k64, nb;             // column groups, 64-deep units, staged scale rows per group

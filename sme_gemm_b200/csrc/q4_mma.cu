@@ -1,5 +1,6 @@
 // Q4 GEMM for a handful of rows on warp-level tensor-core instructions, straight from global memory (sm_100a):
 //   q4_mma_kernel   C[m][n] = ep( A[m][k] @ dequant(W) ), f16 or bf16, K-blocks of 32 and up
+//                   DENSE: C = ep( T(beta * (A @ W)) ) on K-major 16-bit weights, whose 16-byte pieces are fragments as they lie
 //
 // Replaces the reference's SME Q4 GEMV (run_q4_gemv1 / run_q4_gemv, csrc/gemm_f16f16_q4.h:236-431, and the bf16 twin
 // csrc/gemm_b16b16_q4.h:171-268) above the rows of q4_direct_kernel, and for bf16 from one row.
@@ -90,19 +91,21 @@ __device__ __forceinline__ void word_codes(uint32_t w, uint32_t (&a)[4]) {
     a[2] = *reinterpret_cast<const uint32_t*>(&r2); a[3] = *reinterpret_cast<const uint32_t*>(&r3);
 }
 
-// Ring slot of a warp: [CG] codes, [2 NT] activation pieces, 16 bytes a lane each, then [CG][2 halves] scale words.
-constexpr int mma_slot_bytes(int nt, int cg) { return 512 * cg + 1024 * nt + 256 * cg; }
+// Ring slot of a warp: [CG] codes (dense: [CG][column g, g + 8][2 halves] pieces of weights), [2 NT] activation pieces, 16 bytes a
+// lane each, then [CG][2 halves] scale words.
+constexpr int mma_w_bytes(int dense) { return dense ? 2048 : 512; }
+constexpr int mma_slot_bytes(int nt, int cg, int dense) { return mma_w_bytes(dense) * cg + 1024 * nt + (dense ? 0 : 256 * cg); }
 // As deep as two CTAs per SM leave room for.
-constexpr int mma_ring_slots(int nt, int cg) { return nt == 1 ? (cg == 1 ? 6 : 4) : (cg == 1 ? 4 : 3); }
-constexpr size_t mma_smem(int nt, int cg) {
-    return (size_t)kMWarps * mma_ring_slots(nt, cg) * mma_slot_bytes(nt, cg) + (size_t)kMWarps * cg * nt * 512;
+constexpr int mma_ring_slots(int nt, int cg, int dense) { return dense ? (nt == 1 ? 4 : 3) : (nt == 1 ? (cg == 1 ? 6 : 4) : (cg == 1 ? 4 : 3)); }
+constexpr size_t mma_smem(int nt, int cg, int dense) {
+    return (size_t)kMWarps * mma_ring_slots(nt, cg, dense) * mma_slot_bytes(nt, cg, dense) + (size_t)kMWarps * cg * nt * 512;
 }
 
 // NT = tiles of eight rows per CTA, CG = column groups of a pass.  Grid: (CTAs over the passes, row tiles of 8 NT).
-template <int BF16, int NT, int CG>
+template <int BF16, int NT, int CG, int DENSE>
 __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_constant__ Q4GemvArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int PF = mma_ring_slots(NT, CG), SLOT = mma_slot_bytes(NT, CG), PER = CG * NT * 128;
+    constexpr int PF = mma_ring_slots(NT, CG, DENSE), SLOT = mma_slot_bytes(NT, CG, DENSE), WB = mma_w_bytes(DENSE), PER = CG * NT * 128;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t ring = smem_u32(smem_raw) + (uint32_t)(warp * PF * SLOT);
@@ -123,6 +126,21 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
     // load cursor
     int lu = u_begin, lpass = first;
     auto issue_weights = [&](uint32_t slot, int pass, int u) {
+        if (DENSE) {
+            const int d = u * 64 + 8 * t;                          // (kd is a multiple of 8; columns past n and depths past kd are zeros)
+#pragma unroll
+            for (int c = 0; c < CG; ++c)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const int col = group_of(pass, c) * 16 + g + 8 * j;
+                    const uint16_t* src = p.wdense + (size_t)min(col, p.n - 1) * p.kd + d;
+                    const uint32_t lo = col < p.n && d < p.kd ? 16u : 0u, hi = col < p.n && d + 32 < p.kd ? 16u : 0u;
+                    const uint32_t dst = slot + (uint32_t)(WB * c + 1024 * j + lane * 16);
+                    cp_async16_zfill(dst, lo ? src : p.wdense, lo);
+                    cp_async16_zfill(dst + 512, hi ? src + 32 : p.wdense, hi);
+                }
+            return;
+        }
 #pragma unroll
         for (int c = 0; c < CG; ++c) {
             const size_t grp = (size_t)min(group_of(pass, c), p.n16 - 1);               // a tail pass may be one group short
@@ -145,7 +163,7 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
             const uint32_t lo = d + 8 * t < kend[nt] ? 16u : 0u, hi = d + 32 + 8 * t < kend[nt] ? 16u : 0u;   // k is a multiple of 8
-            const uint32_t dst = slot + (uint32_t)(512 * CG + 1024 * nt + lane * 16);
+            const uint32_t dst = slot + (uint32_t)(WB * CG + 1024 * nt + lane * 16);
             cp_async16_zfill(dst, lo ? arow[nt] + d : p.a, lo);
             cp_async16_zfill(dst + 512, hi ? arow[nt] + d + 32 : p.a, hi);
         }
@@ -183,16 +201,19 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
             uint4 alo[NT], ahi[NT];
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                alo[nt] = lds128(sb + (uint32_t)(512 * CG + 1024 * nt + lane * 16));
-                ahi[nt] = lds128(sb + (uint32_t)(512 * CG + 1024 * nt + 512 + lane * 16));
+                alo[nt] = lds128(sb + (uint32_t)(WB * CG + 1024 * nt + lane * 16));
+                ahi[nt] = lds128(sb + (uint32_t)(WB * CG + 1024 * nt + 512 + lane * 16));
             }
-            uint4 wv[CG];
+            uint4 wv[CG][DENSE ? 4 : 1];                           // dense: column g low, high half, column g + 8 low, high
             uint32_t sw[CG][2];
 #pragma unroll
             for (int c = 0; c < CG; ++c) {
-                wv[c] = lds128(sb + (uint32_t)(512 * c + lane * 16));
-                sw[c][0] = lds32(sb + (uint32_t)(512 * CG + 1024 * NT + 256 * c + lane * 4));
-                sw[c][1] = lds32(sb + (uint32_t)(512 * CG + 1024 * NT + 256 * c + 128 + lane * 4));
+#pragma unroll
+                for (int j = 0; j < (DENSE ? 4 : 1); ++j) wv[c][j] = lds128(sb + (uint32_t)(WB * c + 512 * j + lane * 16));
+                if (!DENSE) {
+                    sw[c][0] = lds32(sb + (uint32_t)(512 * CG + 1024 * NT + 256 * c + lane * 4));
+                    sw[c][1] = lds32(sb + (uint32_t)(512 * CG + 1024 * NT + 256 * c + 128 + lane * 4));
+                }
             }
             // the slot read in the step before is free: the unit PF - 1 steps on goes there
             const int fill = slot == 0 ? PF - 1 : slot - 1;
@@ -208,9 +229,20 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
             for (int h = 0; h < 2; ++h)
 #pragma unroll
                 for (int c = 0; c < CG; ++c) {
+                    if constexpr (DENSE) {
+                        const uint4 lo = wv[c][h], hi = wv[c][2 + h];
+                        const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt) {
+                            const uint4& av = h ? ahi[nt] : alo[nt];
+                            mma16816<BF16>(tot[c][nt], a0, av.x, av.y, tot[c][nt]);
+                            mma16816<BF16>(tot[c][nt], a1, av.z, av.w, tot[c][nt]);
+                        }
+                        continue;
+                    }
                     uint32_t af0[4], af1[4];
-                    word_codes<BF16>(h ? wv[c].z : wv[c].x, af0);
-                    word_codes<BF16>(h ? wv[c].w : wv[c].y, af1);
+                    word_codes<BF16>(h ? wv[c][0].z : wv[c][0].x, af0);
+                    word_codes<BF16>(h ? wv[c][0].w : wv[c][0].y, af1);
                     const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&sw[c][h]));   // columns g, g + 8
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt) {
@@ -263,7 +295,10 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
             const int ln = o & 31, r = (o >> 5) & 3, nt = (o >> 7) % NT, c = o / (128 * NT);
             const int col = (CG * pass + c) * 16 + (ln >> 2) + 8 * (r >> 1), row = row0 + 8 * nt + 2 * (ln & 3) + (r & 1);
             if (col < p.n && row < p.m) {
-                if (p.c32) p.c32[(size_t)row * p.n + col] = acc;
+                if (DENSE) {
+                    if (p.beta != 1.0f) acc = __fmul_rn(p.beta, acc);
+                    p.c[p.col_major ? (size_t)col * p.m + row : (size_t)row * p.n + col] = ep_store_value<BF16>(p.ep, acc, (size_t)row, (size_t)col);
+                } else if (p.c32) p.c32[(size_t)row * p.n + col] = acc;
                 else if (p.yacc) p.yacc[(size_t)row * p.n + col] = __fadd_rn(p.yacc[(size_t)row * p.n + col], t_to_f32<BF16>(f32_to_t<BF16>(acc)));
                 else p.c[(size_t)row * p.n + col] = ep_store_value<BF16>(p.ep, acc, (size_t)row, (size_t)col);
             }
@@ -272,17 +307,17 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
     cp_async_wait<0>();
 }
 
-template <int BF16, int NT, int CG>
+template <int BF16, int NT, int CG, int DENSE>
 cudaError_t launch(const Q4GemvArgs& a, dim3 grid, cudaStream_t stream) {
     static int attr_dev = -1;   // the opt-in is per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(q4_mma_kernel<BF16, NT, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem(NT, CG));
+        const cudaError_t e = cudaFuncSetAttribute(q4_mma_kernel<BF16, NT, CG, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem(NT, CG, DENSE));
         if (e != cudaSuccess) return e;
         attr_dev = dev;
     }
-    return launch_pdl(q4_mma_kernel<BF16, NT, CG>, grid, dim3(kMThreads), mma_smem(NT, CG), stream, a);
+    return launch_pdl(q4_mma_kernel<BF16, NT, CG, DENSE>, grid, dim3(kMThreads), mma_smem(NT, CG, DENSE), stream, a);
 }
 
 }  // namespace
@@ -295,7 +330,7 @@ cudaError_t q4_mma_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t str
     const int ytiles = (a.m + 8 * nt - 1) / (8 * nt);
     // One wave of CTAs.  Passes of two column groups share the reads of the activations; where that leaves CTA slots idle
     // (under 4 groups per SM) a pass is one group and twice as many CTAs run.
-    const int cg = a.glu || (long long)n16 * ytiles > 4ll * sm_count ? 2 : 1;
+    const int cg = a.wdense ? 1 : a.glu || (long long)n16 * ytiles > 4ll * sm_count ? 2 : 1;
     const int passes = (n16 + cg - 1) / cg;                         // (gated form: n is a multiple of 64)
     const int ctas = 2 * sm_count / ytiles, slots = ctas > 0 ? ctas : 1;
     const int grid_x = passes < slots ? passes : slots;
@@ -303,8 +338,12 @@ cudaError_t q4_mma_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t str
     a.dq = passes / grid_x; a.dr = passes % grid_x;
     a.dupw = (a.k64 + kMWarps - 1) / kMWarps;
     const dim3 grid(grid_x, ytiles);
+    if (a.wdense) {
+        if (bf16) return nt == 1 ? launch<1, 1, 1, 1>(a, grid, stream) : launch<1, 2, 1, 1>(a, grid, stream);
+        return nt == 1 ? launch<0, 1, 1, 1>(a, grid, stream) : launch<0, 2, 1, 1>(a, grid, stream);
+    }
 #define SMEG_QM(B, T)                                                                          \
-    if (bf16 == B && nt == T) return cg == 2 ? launch<B, T, 2>(a, grid, stream) : launch<B, T, 1>(a, grid, stream);
+    if (bf16 == B && nt == T) return cg == 2 ? launch<B, T, 2, 0>(a, grid, stream) : launch<B, T, 1, 0>(a, grid, stream);
     SMEG_QM(0, 1) SMEG_QM(0, 2)
     SMEG_QM(1, 1) SMEG_QM(1, 2)
 #undef SMEG_QM

@@ -90,3 +90,26 @@ def test_ragged_depth_runs_through_a_padded_copy(m, n, k):
     want = orc.apply_ep(orc.gemm16(a, b, m, n, k), m, n, orc.Nodes([(8, 1, 0.0, None, 0)]))
     assert max_rel(c.float().cpu().numpy(), orc.f16_bits_to_f32(want).reshape(m, n)) <= 1e-2
     assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 16, 8), (1, 2051, 1501), (3, 33, 72), (8, 640, 4096), (9, 17, 520), (16, 100, 64), (17, 130, 1000), (32, 1500, 264), (70, 300, 300)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_handful_of_rows_on_dense_weights(m, n, k, bf16):
+    """The warp-level kernel: row tiles of 8 and 16 with rows missing, a column group with columns missing, depths that leave
+    warps without work or end inside a fragment, beta, a row operand and column-major output."""
+    a, b, bias = _case(m, n, k, bf16, m * n)
+    tof = orc.bf16_bits_to_f32 if bf16 else orc.f16_bits_to_f32
+    w = (sg.prepack_bf16 if bf16 else sg.prepack_f16)(b, n, k)
+    ad, biasd = ((bf16_bits_dev if bf16 else f16_bits_dev)(x) for x in (a, bias))
+    ad = ad.reshape(m, k)
+    want = orc.gemm16(a, b, m, n, k, bf16)
+    c = torch.full((m, n), 9.0, dtype=ad.dtype, device="cuda")
+    sg.Gemm.new(ad, w, m).run(c)
+    assert max_rel(tof(bits_of(c)).reshape(m, n), tof(want).reshape(m, n)) <= 1e-2
+    half = orc.gemm16_f32(a, b, m, n, k) if not bf16 else None
+    if half is not None:
+        want = orc.apply_ep(orc.f32_to_f16_bits((np.float32(0.5) * half).astype(np.float32)).reshape(m, n), m, n, orc.Nodes([(4, 0, 0.0, bias, 0)]))
+        ccm = torch.zeros((n, m), dtype=ad.dtype, device="cuda")
+        sg.Gemm.new(ad, w, m).beta(0.5).col_major_output().add_col(biasd).run(ccm.view(m, n))
+        assert max_rel(tof(bits_of(ccm)).reshape(n, m).T, tof(want).reshape(m, n)) <= 1e-2
+    assert sg.last_status() == 0
