@@ -57,11 +57,6 @@ constexpr int kTcThreads = 32 * (kDeqWarps + 3);   // + token producer, MMA issu
 constexpr int kStageK = 64;                       // depths per stage (one 128-byte swizzle row)
 constexpr int kWTile = 128 * kStageK * 2;         // one 128-column operand tile per stage: 16 KB
 
-__device__ __forceinline__ uint32_t swz_off(int row, int chunk) {
-    // byte offset of 16-byte chunk `chunk` (0..7) of row `row` in a 128B-swizzled K-major tile
-    return (uint32_t)((row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4));
-}
-
 template <int BF16>
 __device__ __forceinline__ uint4 scale_chunk(const __half2 (&c)[4], __half s) {
     uint4 out;
@@ -98,35 +93,6 @@ __device__ __forceinline__ void q4_word_codes(uint32_t w, __half2 (&r)[4]) {
     r[3] = __hfma2(*reinterpret_cast<__half2*>(&hi1), sc16, off16);
 }
 
-// One packed Q4 unit (16 columns x 64 depths) -> rows 16*cu + {g, g+8} of a swizzled operand tile.
-template <int BF16>
-__device__ __forceinline__ void dequant_unit_q4(unsigned char* tile, int cu, const uint4 wv, const uint16_t* sc, int ra,
-                                                int rb, int g, int t) {
-    __half2 w0[4], w1[4], w2[4], w3[4];
-    q4_word_codes(wv.x, w0);
-    q4_word_codes(wv.y, w1);
-    q4_word_codes(wv.z, w2);
-    q4_word_codes(wv.w, w3);
-    // chunks: (col g, depths 8t..8t+7), (col g, 32+8t..), (col g+8, 8t..), (col g+8, 32+8t..)
-    const __half2 lo_a[4] = {w0[0], w0[2], w1[0], w1[2]};
-    const __half2 lo_b[4] = {w2[0], w2[2], w3[0], w3[2]};
-    const __half2 hi_a[4] = {w0[1], w0[3], w1[1], w1[3]};
-    const __half2 hi_b[4] = {w2[1], w2[3], w3[1], w3[3]};
-    const uint32_t sa = *reinterpret_cast<const uint32_t*>(sc + ra * 16 + 2 * g);   // (col g, col g+8) of block ra
-    const uint32_t sb = *reinterpret_cast<const uint32_t*>(sc + rb * 16 + 2 * g);
-    const __half s_lo_a = __ushort_as_half((uint16_t)(sa & 0xffffu)), s_hi_a = __ushort_as_half((uint16_t)(sa >> 16));
-    const __half s_lo_b = __ushort_as_half((uint16_t)(sb & 0xffffu)), s_hi_b = __ushort_as_half((uint16_t)(sb >> 16));
-    const int row_lo = 16 * cu + g, row_hi = row_lo + 8;
-    // chunk order per store keeps the 8 lanes of a quarter warp on distinct banks
-    const int ca = (g & 1) ? 4 + t : t, cb = (g & 1) ? t : 4 + t;
-    const uint4 v_lo_a = scale_chunk<BF16>(lo_a, s_lo_a), v_lo_b = scale_chunk<BF16>(lo_b, s_lo_b);
-    const uint4 v_hi_a = scale_chunk<BF16>(hi_a, s_hi_a), v_hi_b = scale_chunk<BF16>(hi_b, s_hi_b);
-    *reinterpret_cast<uint4*>(tile + swz_off(row_lo, ca)) = (g & 1) ? v_lo_b : v_lo_a;
-    *reinterpret_cast<uint4*>(tile + swz_off(row_lo, cb)) = (g & 1) ? v_lo_a : v_lo_b;
-    *reinterpret_cast<uint4*>(tile + swz_off(row_hi, ca)) = (g & 1) ? v_hi_b : v_hi_a;
-    *reinterpret_cast<uint4*>(tile + swz_off(row_hi, cb)) = (g & 1) ? v_hi_a : v_hi_b;
-}
-
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
@@ -141,8 +107,9 @@ __device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// The same expansion on addresses the caller keeps per lane (the role loop's per-stage work is then the waits, three
-// loads, the arithmetic and four stores).  `row` = shared address of the 128-byte row of column g in the operand tile
+// One packed Q4 unit (16 columns x 64 depths) -> rows g and g + 8 of a column group's 16 in a swizzled operand tile, on
+// addresses the caller keeps per lane (the role loop's per-stage work is then the waits, three loads, the arithmetic and four
+// stores).  `row` = shared address of the 128-byte row of column g in the operand tile
 // (column g + 8 lies 1024 bytes on), `off_first` / `off_second` = swizzled chunk offsets.  Lanes of odd g take the two
 // halves of the unit in the other order (the caller swaps the words and scale words), so that the eight lanes of a
 // quarter warp hit distinct banks in every store.
@@ -674,72 +641,59 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
                 }
                 if (++iu == PU) { iu = 0; dk.next(NK); }
             }
-        } else
-        for (int i = 0; i < (dense ? 0 : num_stages); ++i, dq.next(O), (++iu == PU ? (iu = 0, dk.next(NK)) : (void)0)) {
-            const int ks = dk.slot;
-            const bool last_of_slot = (iu == PU - 1) || (i == num_stages - 1);
-            if (deq_groups == 2 && (i & 1) != (warp >> 3)) {
-                // not this group's stage; a warp that walks past the end of a packed slot still releases it
+        } else if (US == 2) {
+            // Two units a stage: unit uu of column group c of the CTA and, with two accumulator sets, of group c + 8 -- invariants
+            // as above.  (Index arithmetic per stage and unit had made these stages, of small token tiles, 1.3 times as long.)
+            const int uu = wig & 1, c = wig >> 1;
+            const bool odd = (g & 1) != 0;
+            const uint32_t off_first = (uint32_t)(((odd ? 4 + t : t) ^ g) << 4), off_second = (uint32_t)(((odd ? t : 4 + t) ^ g) << 4);
+            // gate/up matrix: gate column groups go to operand tile 0 and the matching up groups to tile 1, so that a
+            // thread of the drain holds both values of one hidden unit (chunks of [2 gate | 2 up] groups)
+            uint32_t row_off[US], code_off[US], sc_off[US];
+#pragma unroll
+            for (int j = 0; j < US; ++j) {
+                const int cj = c + 8 * j, tw = p.glu ? (cj >> 1) & 1 : cj >> 3, rg = p.glu ? ((cj >> 2) << 1) | (cj & 1) : cj & 7;
+                row_off[j] = (uint32_t)((tw * US + uu) * kWTile + rg * 2048 + g * 128);
+                code_off[j] = (uint32_t)(((cj << kbox_shift) * kUnitBytes) + lane * 16);
+                sc_off[j] = (uint32_t)(8 * NW * k_code + cj * rpg * 32 + 4 * g);
+            }
+            const uint32_t ring_k_a = smem_u32(ring_k), ring_o_a = smem_u32(ring_o);
+            const int L = p.log2_block, box_mask = (1 << kbox_shift) - 1;
+            int du = st_begin * US * kStageK, blk0 = du >> L;  // depth of the stage, first scale row of its packed slot
+            for (int i = 0; i < num_stages; ++i, du += US * kStageK, dq.next(O)) {
+                const int ks = dk.slot;
+                const bool last_of_slot = (iu == PU - 1) || (i == num_stages - 1);
+                if (iu == 0) blk0 = du >> L;
+                const int os = dq.slot;
+                if (dq.wrapped && !__all_sync(0xffffffffu, mbar_wait(&o_empty[os], dq.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(&k_full[ks], dk.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
+                const uint32_t pk = ring_k_a + (uint32_t)(ks * k_stride);
+                const int un = iu * US + uu, d = du + uu * kStageK;          // unit within the packed slot, its depth
+                const uint32_t unit_off = (uint32_t)((un >> kbox_shift) * kbox_bytes + (un & box_mask) * kUnitBytes);
+                const int ra = ((d + 8 * t) >> L) - blk0, rb = ((d + 32 + 8 * t) >> L) - blk0;
+                // (a stage's second unit may lie past the depth: it is not multiplied then)
+                if ((st_begin + i) * US + uu < p.ku) {
+#pragma unroll
+                    for (int j = 0; j < US; ++j) {
+                        if (j >= NW) break;
+                        uint4 wv = lds128(pk + code_off[j] + unit_off);
+                        uint32_t sa = lds32(pk + sc_off[j] + (uint32_t)(ra * 32)), sb = lds32(pk + sc_off[j] + (uint32_t)(rb * 32));
+                        if (odd) {
+                            uint32_t x = wv.x; wv.x = wv.z; wv.z = x;
+                            x = wv.y; wv.y = wv.w; wv.w = x;
+                            x = sa; sa = sb; sb = x;
+                        }
+                        dequant_unit_q4_at<BF16>(ring_o_a + (uint32_t)(os * o_stride) + row_off[j], off_first, off_second, wv, sa, sb);
+                    }
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&o_full[os]);
                 if (last_of_slot) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&k_empty[ks]);
                 }
-                continue;
-            }
-            const int os = dq.slot;
-            if (dq.wrapped && !__all_sync(0xffffffffu, mbar_wait(&o_empty[os], dq.phase ^ 1u, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
-            if (!__all_sync(0xffffffffu, mbar_wait(&k_full[ks], dk.phase, abort_flag, p.status, STATUS_TMEM_TIMEOUT))) break;
-            const int uq = iu * US;                                 // first unit of the stage within the packed slot
-            const int u0 = (st_begin + i) * US;                     // first unit of the stage
-            const int units = min(US, p.ku - u0);
-            const int blk0 = ((st_begin + i - iu) * US * kStageK) >> p.log2_block;    // first scale row of the slot
-            const unsigned char* pk = ring_k + (size_t)ks * k_stride;
-            const uint16_t* scs = reinterpret_cast<const uint16_t*>(pk + (size_t)8 * NW * k_code);
-            unsigned char* ob = ring_o + (size_t)os * o_stride;
-            if (US == 1) {
-                // work item c = w * 8 + column group
-                const int du = u0 * kStageK;                        // depth of the stage
-                const int ra = ((du + 8 * t) >> p.log2_block) - blk0, rb = ((du + 32 + 8 * t) >> p.log2_block) - blk0;
-                for (int c = wig; c < 8 * NW; c += deq_wpg) {
-                    const int cgl = c & 7, w = c >> 3;
-                    const uint4 wv = *reinterpret_cast<const uint4*>(pk + (size_t)(uq >> kbox_shift) * kbox_bytes + (((size_t)c << kbox_shift) + (uq & ((1 << kbox_shift) - 1))) * kUnitBytes + lane * 16);
-                    // gate/up matrix: gate column groups go to operand tile 0 and the matching up groups to tile 1,
-                    // so that a thread of the drain holds both values of one hidden unit
-                    int tw = w, rg = cgl;
-                    if (p.glu) {
-                        tw = (c >> 1) & 1;                         // chunks of [2 gate | 2 up] groups
-                        rg = ((c >> 2) << 1) | (c & 1);
-                    }
-                    dequant_unit_q4<BF16>(ob + tw * kWTile, rg, wv, scs + (size_t)c * rpg * 16, ra, rb, g, t);
-                }
-            } else {
-            // work item = (w * 8 + column group) * US + unit of the stage
-            for (int it = wig; it < 8 * NW * US; it += deq_wpg) {
-                const int uu = it % US, c = it / US, cgl = c & 7, w = c >> 3;
-                if (uu >= units) continue;
-                const int du = (u0 + uu) * kStageK;                 // depth of the unit
-                const int ra = ((du + 8 * t) >> p.log2_block) - blk0, rb = ((du + 32 + 8 * t) >> p.log2_block) - blk0;
-                const int un = uq + uu;
-                const uint4 wv = *reinterpret_cast<const uint4*>(pk + (size_t)(un >> kbox_shift) * kbox_bytes + (((size_t)c << kbox_shift) + (un & ((1 << kbox_shift) - 1))) * kUnitBytes + lane * 16);
-                // gate/up matrix: gate column groups go to operand tile 0 and the matching up groups to tile 1,
-                // so that a thread of the drain holds both values of one hidden unit
-                int tw = w, rg = cgl;
-                if (p.glu) {
-                    tw = (c >> 1) & 1;                             // chunks of [2 gate | 2 up] groups
-                    rg = ((c >> 2) << 1) | (c & 1);
-                }
-                dequant_unit_q4<BF16>(ob + (tw * US + uu) * kWTile, rg, wv, scs + (size_t)c * rpg * 16, ra, rb, g, t);
-            }
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-                if (CG == 2) mbar_arrive_cluster(o_full_lead + 8u * os);
-                else mbar_arrive(&o_full[os]);
-            }
-            if (last_of_slot) {
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&k_empty[ks]);
+                if (++iu == PU) { iu = 0; dk.next(NK); }
             }
         }
 
