@@ -661,27 +661,30 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
                 const float scale = __half2float(__ushort_as_half(*reinterpret_cast<const uint16_t*>(fo + sc_off + gi * 32)));
                 const f32x2 scale2 = pack_f32x2(scale, scale);
                 const ulonglong2* sa = reinterpret_cast<const ulonglong2*>(fo + gi * NT * 4 + part * TPW * 4);
-                constexpr int CH = TPW % 16 == 0 ? 16 : 8;                       // accumulator values read at a time
+                // Eight rows at a time, the next eight on their way while these are folded: a warp takes its rows of every
+                // block one block after the other, so the length of this chain is the time of a K-block.
+                const uint32_t src = acc_base + (uint32_t)((acc.slot * G + gi) * ACC_STRIDE);
+                uint32_t av[2][8];
+                tmem_ld8(src, av[0]);
 #pragma unroll
-                for (int c0 = 0; c0 < TPW; c0 += CH) {
-                    uint32_t av[CH];
-                    if constexpr (CH == 16) tmem_ld16(acc_base + (uint32_t)((acc.slot * G + gi) * ACC_STRIDE + c0), av);
-                    else tmem_ld8(acc_base + (uint32_t)((acc.slot * G + gi) * ACC_STRIDE + c0), av);
+                for (int c = 0; c < TPW / 8; ++c) {
+                    const ulonglong2 s0 = sa[2 * c], s1 = sa[2 * c + 1];
                     tmem_ld_wait();
-                    if (c0 + CH == TPW && gi == blocks - 1) {
+                    if (c + 1 < TPW / 8) {
+                        tmem_ld8(src + 8 * (c + 1), av[(c + 1) & 1]);
+                    } else if (gi == blocks - 1) {
                         // the group has been read: hand it back to the MMA warp
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&acc_empty[acc.slot]);
                     }
-#pragma unroll
-                    for (int j = 0; j < CH; j += 4) {
-                        // total = fmaf((float)sum, scale * sa, total), the reference's statement, two rows at a time
-                        const ulonglong2 s2 = sa[(c0 + j) / 4];
-                        f32x2* to = tot + (c0 + j) / 2;
-                        to[0] = fma_f32x2(pack_f32x2(__uint_as_float(av[j]), __uint_as_float(av[j + 1])), mul_f32x2(scale2, s2.x), to[0]);
-                        to[1] = fma_f32x2(pack_f32x2(__uint_as_float(av[j + 2]), __uint_as_float(av[j + 3])), mul_f32x2(scale2, s2.y), to[1]);
-                    }
+                    // total = fmaf((float)sum, scale * sa, total), the reference's statement, two rows at a time
+                    const uint32_t(&v)[8] = av[c & 1];
+                    f32x2* to = tot + 4 * c;
+                    to[0] = fma_f32x2(pack_f32x2(__uint_as_float(v[0]), __uint_as_float(v[1])), mul_f32x2(scale2, s0.x), to[0]);
+                    to[1] = fma_f32x2(pack_f32x2(__uint_as_float(v[2]), __uint_as_float(v[3])), mul_f32x2(scale2, s0.y), to[1]);
+                    to[2] = fma_f32x2(pack_f32x2(__uint_as_float(v[4]), __uint_as_float(v[5])), mul_f32x2(scale2, s1.x), to[2]);
+                    to[3] = fma_f32x2(pack_f32x2(__uint_as_float(v[6]), __uint_as_float(v[7])), mul_f32x2(scale2, s1.y), to[3]);
                 }
             }
             __syncwarp();
