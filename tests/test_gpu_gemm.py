@@ -105,3 +105,68 @@ def test_mlp_block_m256_sampled_rows():
         orc.mlp_accumulate(xs[r0:r0 + 1], want, 1, d, f, guq, gus, dq, ds)
         assert max_rel(got[r0], want[0]) <= TOL
     orc.set_threads(1)
+
+
+def _big_q4(rng, n, k):
+    """Random 4-bit weights too large for the warp-level kernels' share of rows, and their values in f32 on the device."""
+    nbk = -(-k // 32)
+    quants = rng.integers(0, 256, (k * n + 1) // 2).astype(np.uint8)
+    scales = (rng.uniform(0.5, 1.5, (n, nbk)) * 0.01).astype(np.float16)
+    w = sg.Q4Weights.new(quants, scales.view(np.uint16).reshape(-1), n, k)
+    q = torch.from_numpy(quants).cuda()
+    codes = torch.stack((q & 15, q >> 4), 1).reshape(-1)[:k * n].view(k, n).float()
+    codes = torch.where(codes >= 8, codes - 16, codes)
+    return w, codes * torch.from_numpy(scales.astype(np.float32)).cuda().t().repeat_interleave(32, 0)[:k]
+
+
+@pytest.mark.parametrize("n,k", [(9301, 4104), (4096, 14336)])
+def test_tensor_core_gemm_on_large_matrices(n, k):
+    """Every form of the stage (two units, one unit, pairs of CTAs, one and two accumulator sets and token halves) and of the
+    depth-split reduce, with rows, columns and depths missing: product, bias + gelu, partial sums, accumulated sums."""
+    rng = np.random.default_rng(n)
+    w, dense = _big_q4(rng, n, k)
+    for bf16 in (False, True):
+        dt = torch.bfloat16 if bf16 else torch.float16
+        rounded = dense.to(dt).float()
+        bias = torch.randn(n, device="cuda").mul(0.1).to(dt)
+        for m in (33, 64, 65, 100, 130, 257, 512):
+            a = torch.randn(m, k, device="cuda").to(dt)
+            want = a.float() @ rounded
+            scale = want.abs().mean()
+            c = torch.full((m, n), 9.0, dtype=dt, device="cuda")
+            (sg.matmul_q4_bf16 if bf16 else sg.matmul_q4)(a, w, c, m)
+            # one rounding of the store (2^-11, 2^-8 of the value) and f32 sums in another order
+            assert ((c.float() - want).abs() <= (2.0 ** -8 if bf16 else 2.0 ** -11) * want.abs() + 1e-4 * scale).all(), (m, bf16)
+            (sg.matmul_q4_bf16_ep if bf16 else sg.matmul_q4_ep)(a, w, c, m, sg.Epilogue("bf16" if bf16 else "f16").add_col(bias).gelu())
+            ref = torch.nn.functional.gelu(want.to(dt).float() + bias.float(), approximate="tanh")
+            assert ((c.float() - ref).abs() <= (2.0 ** -6 if bf16 else 2.0 ** -9) * (1 + ref.abs()) * max(1.0, float(scale))).all(), (m, bf16)
+            if bf16:
+                continue
+            part = torch.full((m, n), 9.0, device="cuda")
+            sg.Linear.from_q4(w).partial(a, part, m)
+            assert (part - want).abs().max() <= 1e-4 * max(1.0, float(want.abs().max()))
+            y = torch.ones((m, n), device="cuda")
+            sg.Linear.from_q4(w).accumulate(a, y, m)
+            sg.matmul_q4(a, w, c, m)
+            assert torch.equal(y, 1 + c.float()), m
+    assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("m", [17, 64, 90, 200, 300])
+def test_gated_block_on_large_matrices(m):
+    """Gate and up columns in the two accumulator sets of every token tile, the residual add behind a depth split."""
+    rng = np.random.default_rng(m)
+    d, f = 4096, 9408
+    up, wu = _big_q4(rng, 2 * f, d)
+    down, wd = _big_q4(rng, d, f)
+    x = torch.randn(m, d, device="cuda").half()
+    y = torch.randn(m, d, device="cuda")
+    both = (x.float() @ wu.half().float()).half().float().view(m, f // 32, 2, 32)
+    hid = (torch.nn.functional.silu(both[:, :, 0]) * both[:, :, 1]).reshape(m, f).half()
+    out = (hid.float() @ wd.half().float()).half().float()
+    got = y.clone()
+    sg.Mlp.gated(sg.GatedLinear(sg.Linear.from_q4(up), sg.Gate.Silu), sg.Linear.from_q4(down)).accumulate(x, got, m)
+    torch.cuda.synchronize()
+    # f16 roundings of hidden units flip by one place between the orders of summation: 2^-11 each, averaged over the depth
+    err, ref = (got - y - out).double(), out.double()
+    assert float(err.norm() / ref.norm()) <= 1e-3 and sg.last_status() == 0
