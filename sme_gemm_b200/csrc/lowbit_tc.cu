@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
 //     operand per row, its activation scale: every lane of 16 warps reads each of them, and with the code sums beside them
 //     these broadcasts were the other half;
 //   * 16 fold warps, four per lane quarter, NT / 4 rows each, totals in registers, two rows per instruction (f32x2).
-// NT rows per CTA are chosen by the launcher.  1-bit 512 x 4096 x 14336: 219 us with 64-deep stages in shared memory.
+// NT rows per CTA are chosen by the launcher.  1-bit 512 x 4096 x 14336: 219 us with 64-deep stages in shared memory, 110 now (0.55
+// PFLOP/s; the tensor pipe is busy a quarter of the time, two thirds of the issue slots are taken).
 constexpr int kLbThreads = 32 * 28;
 constexpr int kLbNK = 3, kLbNF = 6;               // ring depths: packed slots (two units a column group), fold operands
 constexpr int kLbKSlot = 8 * 2 * kUnitBytes;
