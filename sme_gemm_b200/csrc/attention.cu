@@ -119,16 +119,29 @@ __device__ __forceinline__ float block_exp(uint32_t taddr, int lim, float mx, fl
     return sum + sum2;
 }
 
+// Eight results: two 16-byte stores (one as f16) where every row of out starts on a 16-byte boundary, else one by one.
 template <int OUT16>
 __device__ __forceinline__ void store8(const AttnArgs& p, size_t off, const float (&v)[8]) {
     if (OUT16) {
         uint4 o;
         o.x = pack2_t<0>(v[0], v[1]); o.y = pack2_t<0>(v[2], v[3]); o.z = pack2_t<0>(v[4], v[5]); o.w = pack2_t<0>(v[6], v[7]);
-        *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.out) + off) = o;
+        uint16_t* d = reinterpret_cast<uint16_t*>(p.out) + off;
+        if (p.out_vec) {
+            *reinterpret_cast<uint4*>(d) = o;
+            return;
+        }
+        const uint32_t w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) d[e] = (uint16_t)(w[e / 2] >> (16 * (e & 1)));
     } else {
         float* d = reinterpret_cast<float*>(p.out) + off;
-        *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
-        *reinterpret_cast<float4*>(d + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        if (p.out_vec) {
+            *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(d + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            return;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) d[e] = v[e];
     }
 }
 
@@ -713,6 +726,7 @@ cudaError_t attn_tc_launch(const CUtensorMap& tk, const CUtensorMap& tv, const A
 }  // namespace
 
 cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream) {
+    a.out_vec = ((uintptr_t)a.out & 15) == 0;                  // (rows are heads * head_dim long: multiples of 16 bytes)
     if (a.rows * (a.heads / a.kv_heads) <= 16) {
         // runs of 64 keys and up; caches whose runs do not fit shared memory (about 4 k keys at 128 depths) stay below
         const int total = a.start + a.rows;

@@ -241,7 +241,7 @@ struct AttnArgs {
     int heads, kv_heads, head_dim;
     float scale;
     unsigned* status;
-    int slots, q_vec;      // launcher-filled: K / V ring slots, rows of f16 queries are 16-byte aligned
+    int slots, q_vec, out_vec;   // launcher-filled: K / V ring slots; rows of f16 queries, rows of out are 16-byte aligned
 };
 cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream);
 cudaError_t kv_append_launch(uint16_t* kc, uint16_t* vc, const uint16_t* src, size_t stride, size_t k_off, size_t v_off, size_t row_len,

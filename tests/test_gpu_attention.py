@@ -368,3 +368,28 @@ def test_layer_in_one_call_is_its_parts(rms, d, heads, kv_heads, hd, rows):
     torch.cuda.synchronize()
     assert torch.equal(x1, x2) and torch.equal(c1.keys(), c2.keys()) and torch.equal(c1.values(), c2.values())
     assert c1.len() == c2.len() == 3 * rows and sg.last_status() == 0
+
+
+@pytest.mark.parametrize("shift", [1, 2, 3])
+@pytest.mark.parametrize("heads,kv_heads,hd,start,rows", [(4, 2, 64, 30, 1), (8, 2, 128, 700, 1), (4, 2, 64, 20, 40), (8, 1, 72, 300, 130)])
+def test_results_go_to_buffers_off_the_16_byte_grid(heads, kv_heads, hd, start, rows, shift):
+    """out may start at any element of a larger buffer (f32 and f16, one run and clusters of runs on both kernels): the bits of
+    the aligned call, and nothing beside them is written."""
+    rng = np.random.default_rng(heads + hd + shift)
+    n, width = start + rows, heads * hd
+    cache = sg.KvCache(heads, kv_heads, hd, n)
+    cache.extend(*(torch.from_numpy(rng.standard_normal((n, kv_heads * hd)).astype(np.float16)).cuda() for _ in range(2)))
+    q = torch.from_numpy(rng.standard_normal((rows, width)).astype(np.float16)).cuda()
+    for dtype in (torch.float32, torch.float16):
+        want = torch.empty((rows, width), dtype=dtype, device="cuda")
+        cache._attend(q, width, rows, want)
+        buf = torch.full((rows * width + 8,), 3.0, dtype=dtype, device="cuda")
+        out = buf[shift:shift + rows * width]
+        if rows == 1 and dtype == torch.float32:
+            cache.attend(q, out)
+        else:
+            cache._attend(q, width, rows, out)
+        torch.cuda.synchronize()
+        assert torch.equal(out.view(rows, width), want)
+        assert (buf[:shift] == 3.0).all() and (buf[shift + rows * width:] == 3.0).all()
+    assert sg.last_status() == 0

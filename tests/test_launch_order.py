@@ -1,0 +1,35 @@
+"""Order of early launches and tensor memory in the kernels' sources.
+
+A kernel that is launched while its predecessor drains may allocate tensor memory before it waits for that predecessor
+(gemm_tc_kernel does).  It then holds columns the predecessor could still be asking for, unless the predecessor lets its
+dependents go only once every CTA of its own holds its columns: two such kernels on one SM would wait for one another."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sme_gemm_b200", "csrc")
+
+
+def _kernels():
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith(".cu"):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^)]*\)\s*)?(\w+)\s*\([^{;]*\)\s*\{", text):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[i], 0)
+                i += 1
+            yield name, m.group(1), text[m.end():i]
+
+
+def test_dependents_are_let_go_only_with_tensor_memory_held():
+    seen = []
+    for name, kernel, body in _kernels():
+        allocs = [m.start() for m in re.finditer(r"\btmem_alloc2?\(", body)]
+        if not allocs:
+            continue
+        seen.append(kernel)
+        for m in re.finditer(r"\bpdl_launch_dependents\(", body):
+            between = body[max(allocs):m.start()] if m.start() > max(allocs) else ""
+            assert re.search(r"__syncthreads\(\)|cluster_sync_all\(\)", between), f"{name}: {kernel} lets its dependents go before its CTAs hold tensor memory"
+    assert {"gemm_tc_kernel", "attn_tc_kernel", "lowbit_tc_kernel", "lowbit_tc_block_kernel"} <= set(seen)
