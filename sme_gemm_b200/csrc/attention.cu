@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             float sum = 0.0f, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
-                if (s >= splits || m[s] == -INFINITY) continue;
+                if (s >= splits || (m[s] == -INFINITY && l[s] == 0.0f)) continue;   // no key of this part counts (a NaN score does: l is NaN)
                 const float f = expf(m[s] - mx);
                 sum = fmaf(f, l[s], sum);
                 v[0] = fmaf(f, o[s][0].x, v[0]); v[1] = fmaf(f, o[s][0].y, v[1]); v[2] = fmaf(f, o[s][0].z, v[2]); v[3] = fmaf(f, o[s][0].w, v[3]);
@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const __grid_co
         float sum = 0.0f, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
-            if (s >= splits || m[s] == -INFINITY) continue;
+            if (s >= splits || (m[s] == -INFINITY && l[s] == 0.0f)) continue;       // no key of this run counts (a NaN score does: l is NaN)
             const float f = expf(m[s] - mx);
             sum = fmaf(f, l[s], sum);
             v[0] = fmaf(f, o[s][0].x, v[0]); v[1] = fmaf(f, o[s][0].y, v[1]); v[2] = fmaf(f, o[s][0].z, v[2]); v[3] = fmaf(f, o[s][0].w, v[3]);

@@ -393,3 +393,30 @@ def test_results_go_to_buffers_off_the_16_byte_grid(heads, kv_heads, hd, start, 
         assert torch.equal(out.view(rows, width), want)
         assert (buf[:shift] == 3.0).all() and (buf[shift + rows * width:] == 3.0).all()
     assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd,start,rows,kind", [
+    (8, 8, 64, 192, 1, "nan"), (16, 8, 128, 448, 1, "nan"), (8, 8, 64, 192, 1, "inf"), (2, 1, 64, 0, 129, "nan"), (2, 1, 64, 0, 129, "inf"), (4, 2, 128, 256, 129, "nan")])
+def test_a_nan_score_alone_in_its_run_of_keys_reaches_the_result(heads, kv_heads, hd, start, rows, kind):
+    """The newest position's key makes a NaN score (a NaN, or infinities of both signs) and has a run of keys -- of the decode
+    kernel, of a cluster's CTA -- to itself: the rows that attend to it are NaN, the others as without it."""
+    rng = np.random.default_rng(heads + hd + start)
+    n, at = start + rows, start + rows - 1
+    k = torch.from_numpy((rng.standard_normal((n, kv_heads * hd)) * 0.5).astype(np.float16)).cuda()
+    v = torch.from_numpy(rng.standard_normal((n, kv_heads * hd)).astype(np.float16)).cuda()
+    q = torch.ones((rows, heads * hd), dtype=torch.float16, device="cuda")
+    clean, bad = (torch.empty((rows, heads * hd), dtype=torch.float32, device="cuda") for _ in range(2))
+    cache = sg.KvCache(heads, kv_heads, hd, n)
+    cache.extend(k, v)
+    cache.attend_causal(q, rows, clean)
+    k[at, 0] = float(kind)                                     # KV head 0
+    if kind == "inf":
+        k[at, 1] = -float("inf")
+    cache.clear()
+    cache.extend(k, v)
+    cache.attend_causal(q, rows, bad)
+    torch.cuda.synchronize()
+    hit = heads // kv_heads * hd
+    assert torch.isnan(bad[rows - 1, :hit]).all()
+    assert torch.equal(bad[rows - 1, hit:], clean[rows - 1, hit:]) and torch.equal(bad[:rows - 1], clean[:rows - 1])
+    assert sg.last_status() == 0
