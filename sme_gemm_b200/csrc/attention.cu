@@ -145,46 +145,110 @@ __device__ __forceinline__ void store8(const AttnArgs& p, size_t off, const floa
     }
 }
 
-// Eight depths of one (query row, head) by the scalar statement.  The products above are formed a key block at a time with
-// the probabilities in two parts, so an infinity or NaN among the values reaches rows that do not attend to it (0 * inf) and
-// an infinity turns into NaN (inf * 0 in the low part): a row whose result is not finite is formed again here.
-template <int QF32>
-__device__ __noinline__ void attend_exact8(const AttnArgs& p, int i, int head, int c, float (&v)[8]) {
+// Depths [c0, c1) of one (query row, head) by the scalar statement, a warp's work (all 32 lanes, the same arguments).  The
+// products above are formed a key block at a time with the probabilities in two parts, so an infinity or NaN among the
+// values reaches rows that do not attend to it (0 * inf) and an infinity turns into NaN (inf * 0 in the low part): a row
+// whose result is not finite although its probabilities are is formed again here.  (With a NaN score the probabilities'
+// sum is NaN and so is the scalar result: nothing to do.)  `base` is the row's maximum, to rounding.  A group of lanes takes
+// a key, a lane eight of its depths in K and V: four keys of every group are on their way at once, and nothing but the
+// score's reduction crosses lanes.  Every row formed again (an infinity at position 0):
+// 512 rows over 1024 keys, 32 heads of 128, 1.7 ms, one row 0.19 ms; the scalar kernel that this one replaced took 1.3 and 0.08
+// whatever the values, a thread per eight depths some hundreds.
+template <int QF32, int OUT16>
+__device__ __noinline__ void attend_exact_row(const AttnArgs& p, int i, int head, int c0, int c1, float base) {
+    constexpr int B = 4;
+    const int lane = threadIdx.x & 31;
     const int hd = p.head_dim, ld = p.kv_heads * hd, off = head / (p.heads / p.kv_heads) * hd, len = p.start + i + 1;
-    const size_t qo = (size_t)i * p.q_stride + (size_t)head * hd;
-    auto score = [&](int t) {
-        const uint16_t* kr = p.k + (size_t)t * ld + off;
-        float s = 0.0f;
-        for (int d = 0; d < hd; ++d) {
-            const float x = QF32 ? reinterpret_cast<const float*>(p.q)[qo + d] : __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(p.q)[qo + d]));
-            s = __fadd_rn(s, __fmul_rn(__half2float(__float2half_rn(__fmul_rn(x, p.scale))), __half2float(__ushort_as_half(kr[d]))));
+    int per = 1;                                               // lanes of a key
+    while (per * 8 < hd) per *= 2;
+    const int d = (lane & (per - 1)) * 8, keys = 32 / per;
+    const bool in_k = d < hd, in_v = d >= c0 && d < c1;
+    float q[8], acc[8], sum = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const size_t qo = (size_t)i * p.q_stride + (size_t)head * hd + d + e;
+        float x = 0.0f;
+        if (in_k) x = QF32 ? reinterpret_cast<const float*>(p.q)[qo] : __half2float(__ushort_as_half(reinterpret_cast<const uint16_t*>(p.q)[qo]));
+        q[e] = __half2float(__float2half_rn(__fmul_rn(x, p.scale)));
+        acc[e] = 0.0f;
+    }
+    for (int t0 = lane / per; __any_sync(0xffffffffu, t0 < len); t0 += keys * B) {
+        uint4 k[B], v[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            const size_t at = (size_t)min(t0 + b * keys, len - 1) * ld + off + d;
+            k[b] = v[b] = make_uint4(0, 0, 0, 0);
+            if (in_k) k[b] = *reinterpret_cast<const uint4*>(p.k + at);
+            if (in_v) v[b] = *reinterpret_cast<const uint4*>(p.v + at);
         }
-        return s;
-    };
-    float mx = -INFINITY, sum = 0.0f;
-    for (int t = 0; t < len; ++t) mx = fmaxf(mx, score(t));
+        // (the keys' chains side by side)
+        float s[B];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = 0.0f;
-    for (int t = 0; t < len; ++t) {
-        const float pt = expf(__fsub_rn(score(t), mx));
-        sum += pt;
-        const uint4 x = *reinterpret_cast<const uint4*>(p.v + (size_t)t * ld + off + c);
-        const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+        for (int b = 0; b < B; ++b) {
+            const uint32_t w[4] = {k[b].x, k[b].y, k[b].z, k[b].w};
+            s[b] = 0.0f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
-            v[2 * e] = __fadd_rn(v[2 * e], __fmul_rn(pt, f.x));
-            v[2 * e + 1] = __fadd_rn(v[2 * e + 1], __fmul_rn(pt, f.y));
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                s[b] = __fadd_rn(s[b], __fmul_rn(q[2 * e], f.x));
+                s[b] = __fadd_rn(s[b], __fmul_rn(q[2 * e + 1], f.y));
+            }
+        }
+        for (int o = per >> 1; o; o >>= 1)
+#pragma unroll
+            for (int b = 0; b < B; ++b) s[b] += __shfl_xor_sync(0xffffffffu, s[b], o);
+#pragma unroll
+        for (int b = 0; b < B; ++b) s[b] = expf(__fsub_rn(s[b], base));
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+            if (t0 + b * keys >= len) break;
+            const uint32_t w[4] = {v[b].x, v[b].y, v[b].z, v[b].w};
+            sum += s[b];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
+                acc[2 * e] = __fadd_rn(acc[2 * e], __fmul_rn(s[b], f.x));
+                acc[2 * e + 1] = __fadd_rn(acc[2 * e + 1], __fmul_rn(s[b], f.y));
+            }
         }
     }
+    __syncwarp();
+    for (int o = per; o < 32; o <<= 1) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(v[e], sum);
+        for (int e = 0; e < 8; ++e) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+    }
+    if (!in_v || lane >= per) return;
+    const size_t dst = ((size_t)i * p.heads + head) * hd + d;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        const float r = __fdiv_rn(acc[e], sum);
+        if (OUT16) reinterpret_cast<uint16_t*>(p.out)[dst + e] = __half_as_ushort(__float2half_rn(r));
+        else reinterpret_cast<float*>(p.out)[dst + e] = r;
+    }
 }
 __device__ __forceinline__ bool all_finite(const float (&v)[8]) {
     bool ok = true;
 #pragma unroll
     for (int e = 0; e < 8; ++e) ok = ok && fabsf(v[e]) <= 3.402823466e38f;
     return ok;
+}
+
+// Behind a pass in which every lane stored eight results (`mask`: the lanes whose are not finite, with a good sum) at depth c of the tile's row r:
+// the rows of the warp's bad results again, over the depths the warp holds of each (lanes of a row are neighbours, depths
+// ascending; r < 0: no result).
+template <int QF32, int OUT16>
+__device__ __noinline__ void redo_bad(const AttnArgs& p, unsigned mask, int r, int c, float base, int row0, int kvh) {
+    const int group = p.heads / p.kv_heads;
+    while (mask) {
+        const int first_bad = __ffs(mask) - 1, rr = __shfl_sync(0xffffffffu, r, first_bad);
+        const unsigned same = __ballot_sync(0xffffffffu, r == rr);
+        const int c0 = __shfl_sync(0xffffffffu, c, __ffs(same) - 1), c1 = __shfl_sync(0xffffffffu, c, 31 - __clz(same)) + 8;
+        const int i = (row0 + rr) / group, g = (row0 + rr) - i * group;
+        __syncwarp();
+        attend_exact_row<QF32, OUT16>(p, i, kvh * group + g, c0, c1, __shfl_sync(0xffffffffu, base, first_bad));
+        mask &= ~same;
+    }
 }
 
 // Grid: (CTAs per tile, tiles of 128 query rows x heads of a group, KV heads); the CTAs of a tile are a cluster.
@@ -196,6 +260,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     __shared__ __align__(8) uint64_t bars[2 * kAtMaxSlots + 9];
     __shared__ float red_m[2][128], red_l[2][128];             // per half of the softmax warps and row: maximum, sum
     __shared__ float part_m[128], part_l[128];                 // of this CTA's key range
+    __shared__ unsigned bad_rows[2][4];                        // per half and quarter: rows whose result is not finite
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_word;
     volatile int* abort_flag = &abort_word;
@@ -398,6 +463,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
         if (splits == 1) {
             const int i = (row0 + row) / group, g = (row0 + row) - i * group;
             const size_t dst = (size_t)i * p.heads * hd + (size_t)(kvh * group + g) * hd;
+            bool bad = false;
             for (int c = c_begin; ok && live && c < c_end; c += 8) {
                 uint32_t r[8];
                 tmem_ld8(tmem + ((uint32_t)(q4 * 32) << 16) + kAtOCol + c, r);
@@ -406,9 +472,17 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(__uint_as_float(r[e]) * (1.0f / kAtPScale), sum);
                 if (row < nrow) {
-                    if (!all_finite(v)) attend_exact8<QF32>(p, i, kvh * group + g, c, v);
+                    bad = bad || (sum > 0.0f && !all_finite(v));
                     store8<OUT16>(p, dst + c, v);
                 }
+            }
+            // rows to form again: the two warps that hold a row's halves take every other one, whole
+            const unsigned mine = __ballot_sync(0xffffffffu, bad);
+            if (lane == 0) bad_rows[half][q4] = mine;
+            named_barrier_sync(1, 256);
+            for (unsigned mask = (bad_rows[0][q4] | bad_rows[1][q4]) & (half ? 0xaaaaaaaau : 0x55555555u); mask; mask &= mask - 1) {
+                const int l = __ffs(mask) - 1, tr = row0 + q4 * 32 + l;
+                attend_exact_row<QF32, OUT16>(p, tr / group, kvh * group + tr % group, 0, hd, __shfl_sync(0xffffffffu, mx_e, l));
             }
         } else {
             if (half == 0) { part_m[row] = nb > 0 ? mx : -INFINITY; part_l[row] = sum; }
@@ -430,8 +504,11 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
         cluster_sync_all();
         const uint32_t o_a = smem_u32(smem), m_a = smem_u32(part_m), l_a = smem_u32(part_l);
         const int items = nrow * (hd / 8);
-        for (int it = rank * kAtThreads + tid; it < items && *abort_flag == 0; it += splits * kAtThreads) {
-            const int r = it / (hd / 8), c = (it - r * (hd / 8)) * 8;
+        // (warp by warp: `it0` is the warp's first item; a lane past the last one repeats it without a store)
+        const bool sound = __all_sync(0xffffffffu, *abort_flag == 0);
+        for (int it0 = rank * kAtThreads + (tid & ~31); sound && it0 < items; it0 += splits * kAtThreads) {
+            const bool mine = it0 + lane < items;
+            const int it = mine ? it0 + lane : items - 1, r = it / (hd / 8), c = (it - r * (hd / 8)) * 8;
             float m[8], l[8];
             float4 o[8][2];
 #pragma unroll
@@ -459,8 +536,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(v[e] * (1.0f / kAtPScale), sum);
             const int i = (row0 + r) / group, g = (row0 + r) - i * group;
-            if (!all_finite(v)) attend_exact8<QF32>(p, i, kvh * group + g, c, v);
-            store8<OUT16>(p, (size_t)i * p.heads * hd + (size_t)(kvh * group + g) * hd + c, v);
+            if (mine) store8<OUT16>(p, (size_t)i * p.heads * hd + (size_t)(kvh * group + g) * hd + c, v);
+            const unsigned mask = __ballot_sync(0xffffffffu, mine && sum > 0.0f && !all_finite(v));
+            if (mask) redo_bad<QF32, OUT16>(p, mask, mine ? r : -1, c, mx, row0, kvh);
         }
         tc_fence_before();
         cluster_sync_all();                                    // nobody leaves while its shared memory is read
@@ -507,7 +585,7 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
 }
 
 template <int QF32, int OUT16>
-__global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const __grid_constant__ AttnArgs p, int kc) {
+__global__ void __launch_bounds__(kAdThreads, 1) attn_decode_kernel(const __grid_constant__ AttnArgs p, int kc) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float part_m[16], part_l[16];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -626,8 +704,10 @@ __global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const __grid_co
     if (splits > 1) cluster_sync_all();
     else __syncthreads();
     const uint32_t o_a = smem_u32(o_s), m_a = smem_u32(part_m), l_a = smem_u32(part_l);
-    for (int it = rank * kAdThreads + tid; it < nrow * (hd / 8); it += splits * kAdThreads) {
-        const int r = it / (hd / 8), c = (it - r * (hd / 8)) * 8;
+    const int items = nrow * (hd / 8);
+    for (int it0 = rank * kAdThreads + (tid & ~31); it0 < items; it0 += splits * kAdThreads) {
+        const bool mine = it0 + lane < items;                  // (a lane past the last item repeats it without a store)
+        const int it = mine ? it0 + lane : items - 1, r = it / (hd / 8), c = (it - r * (hd / 8)) * 8;
         float m[8], l[8], mx = -INFINITY;
         float4 o[8][2];
 #pragma unroll
@@ -654,8 +734,9 @@ __global__ void __launch_bounds__(kAdThreads) attn_decode_kernel(const __grid_co
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(v[e] * (1.0f / kAtPScale), sum);
         const int i = r / group, head = kvh * group + r - i * group;
-        if (!all_finite(v)) attend_exact8<QF32>(p, i, head, c, v);
-        store8<OUT16>(p, (size_t)i * p.heads * hd + (size_t)head * hd + c, v);
+        if (mine) store8<OUT16>(p, (size_t)i * p.heads * hd + (size_t)head * hd + c, v);
+        const unsigned mask = __ballot_sync(0xffffffffu, mine && sum > 0.0f && !all_finite(v));
+        if (mask) redo_bad<QF32, OUT16>(p, mask, mine ? r : -1, c, mx, 0, kvh);
     }
     if (splits > 1) cluster_sync_all();                        // nobody leaves while its shared memory is read
 }
