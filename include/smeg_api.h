@@ -261,9 +261,10 @@ int smeg_gemm_dense(const smeg_dense *w, const uint16_t *a, uint16_t *c, size_t 
  * smeg_attn_kv_causal_dev -- attention_kv_causal_f16 (src/kernels/kv_attention.rs:155-242; rows = 1, start = len - 1 is
  * attention_kv_f16, :29-139): query row i attends to keys 0..=start+i of caches that already hold start + rows rows;
  * q is f16 bits (q_f32 = 0) or f32 rows of heads * head_dim values q_stride elements apart, out f32 [rows][heads *
- * head_dim].  Per head softmax(f16(q * scale) . k) @ v with f32 sums and f32 probabilities.  head_dim a multiple of 8 in
+ * head_dim].  Per head softmax(f16(q * scale) . k) @ v with f32 sums in an order of the kernel's own and probabilities of 22
+ * significant bits: no further from the statement in 64 bits than f32 sums in key order are.  head_dim a multiple of 8 in
  * 8..=256 and heads a positive multiple of kv_heads (-4 otherwise, where the reference panics); -3 beyond 65535 rows or
- * heads and beyond ~50 k keys.
+ * heads and beyond ~50 k keys.  out may start at any element.
  * smeg_attn_kv_causal_f16_dev -- the same with the result rounded to f16, as the out projection takes it. */
 int smeg_kv_append_dev(uint16_t *k_cache, uint16_t *v_cache, const uint16_t *src, size_t src_stride, size_t k_off,
                        size_t v_off, size_t row_len, size_t pos, size_t rows, void *stream);

@@ -10,10 +10,14 @@
 // keys and values; a key block is 128 keys.  Two passes over the keys of a tile:
 //   1. S = Q K^T into tensor memory, the row maxima from it;
 //   2. S again (not where both blocks of a short range are still in tensor memory), p = exp(s - max), O += P V.
-// With the exact maximum known first, a probability is the reference's exp(s - max) whatever the order of the blocks, and the
-// accumulator in tensor memory is never rescaled; the second Q K^T costs a quarter of the tensor work, and the tensor pipe
-// waits for the exponentials anyway.  Operands are exact: q and k are f16 already, and the f32 probability travels as the sum
-// of two f16 numbers (p * 2^15 = hi + lo: 22 significant bits down to probabilities of 2^-29), two MMAs per step of P V.
+// With the exact maximum known first, a probability is the reference's exp(s - max) whatever the order of the blocks, and no
+// sum is ever rescaled; the second Q K^T costs a quarter of the tensor work, and the tensor pipe waits for the exponentials
+// anyway.  Operands are exact: q and k are f16 already, and the f32 probability travels as the sum of two f16 numbers (p * 2^15 =
+// hi + lo: 22 significant bits down to probabilities of 2^-29), two MMAs per step of P V.  The tensor core cuts its f32 sums off
+// where an addition would round them, which grows with the length of a chain; so tensor memory holds one block's sums (the low
+// parts', then the high parts'), and the softmax warps add them up in registers.  Error against 64 bits (2-norm), 512 rows over
+// 1024 keys of 128 depths, flat / sharp scores: 4.4e-7 / 6.3e-7; the scalar f32 statement 6.2e-7 / 13.8e-7; one chain over all
+// keys 20.1e-7 / 13.3e-7, at 31.5 us against 34.7.  (Two blocks a chain: 6.9e-7, 35.6 us.)
 //
 // Roles (320 threads): warps 0-7 (softmax; warp = 32 rows x 64 keys of a block, a thread one row), warp 8 (TMA: K and V
 // blocks as three-dimensional boxes, so that a head of less than 64 depths and the rows past the last key read as zero),
@@ -66,6 +70,10 @@ __device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t cluster_addr) {
     return v;
 }
 
+// (x, y) += (a, b) in one instruction
+__device__ __forceinline__ void add2(float& x, float& y, uint32_t a, uint32_t b) {
+    asm("{\n\t.reg .b64 u, v;\n\tmov.b64 u, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tadd.rn.f32x2 u, u, v;\n\tmov.b64 {%0, %1}, u;\n\t}" : "+f"(x), "+f"(y) : "r"(a), "r"(b));
+}
 // Largest of a warp's 64 scores per row; keys from `lim` on do not count.
 template <bool MASK>
 __device__ __forceinline__ float block_max(uint32_t taddr, int lim, float mx) {
@@ -83,24 +91,24 @@ __device__ __forceinline__ float block_max(uint32_t taddr, int lim, float mx) {
     return mx;
 }
 
-// p = exp(s - mx) of a warp's 64 scores per row, added to `sum`, and written over them as two f16 parts: columns 0..31 of
-// the 64 hold the high parts (two keys to a column), 32..63 the low ones.
+// p = exp(s - mx) of a warp's 64 scores per row, added to `sum`, and written over them as two f16 parts, 16 keys at a time: eight
+// columns of high parts (two keys to a column), eight of low ones.
 template <bool MASK>
 __device__ __forceinline__ float block_exp(uint32_t taddr, int lim, float mx, float sum) {
-    uint32_t r[2][32];
-    tmem_ld32(taddr, r[0]);
-    tmem_ld32(taddr + 32, r[1]);
-    tmem_ld_wait();
-    uint32_t hi[2][16], lo[2][16];
     float sum2 = 0.0f;
+    uint32_t r[2][16];
+    tmem_ld16(taddr, r[0]);
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < 4; ++h) {
+        uint32_t hi[8], lo[8];
+        tmem_ld_wait();
+        if (h < 3) tmem_ld16(taddr + 16 * (h + 1), r[(h + 1) & 1]);
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-            float e0 = expf(__uint_as_float(r[h][i]) - mx), e1 = expf(__uint_as_float(r[h][i + 1]) - mx);
+        for (int i = 0; i < 16; i += 2) {
+            float e0 = expf(__uint_as_float(r[h & 1][i]) - mx), e1 = expf(__uint_as_float(r[h & 1][i + 1]) - mx);
             if (MASK) {
-                e0 = 32 * h + i < lim ? e0 : 0.0f;
-                e1 = 32 * h + i + 1 < lim ? e1 : 0.0f;
+                e0 = 16 * h + i < lim ? e0 : 0.0f;
+                e1 = 16 * h + i + 1 < lim ? e1 : 0.0f;
             }
             sum += e0;
             sum2 += e1;
@@ -108,13 +116,12 @@ __device__ __forceinline__ float block_exp(uint32_t taddr, int lim, float mx, fl
             e1 *= kAtPScale;
             const uint32_t p = pack2_t<0>(e0, e1);
             const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&p));
-            hi[h][i / 2] = p;
-            lo[h][i / 2] = pack2_t<0>(e0 - f.x, e1 - f.y);
+            hi[i / 2] = p;
+            lo[i / 2] = pack2_t<0>(e0 - f.x, e1 - f.y);
         }
-    tmem_st16(taddr, hi[0]);
-    tmem_st16(taddr + 16, hi[1]);
-    tmem_st16(taddr + 32, lo[0]);
-    tmem_st16(taddr + 48, lo[1]);
+        tmem_st8(taddr + 16 * h, hi);
+        tmem_st8(taddr + 16 * h + 8, lo);
+    }
     tmem_st_wait();
     return sum + sum2;
 }
@@ -252,12 +259,13 @@ __device__ __noinline__ void redo_bad(const AttnArgs& p, unsigned mask, int r, i
 }
 
 // Grid: (CTAs per tile, tiles of 128 query rows x heads of a group, KV heads); the CTAs of a tile are a cluster.
-template <int QF32, int OUT16>
+// NO: depths a softmax thread sums, half a head's, 64 or 128.
+template <int QF32, int OUT16, int NO>
 __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap tk, const __grid_constant__ CUtensorMap tv,
                                                                 const __grid_constant__ AttnArgs p) {
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
-    __shared__ __align__(8) uint64_t bars[2 * kAtMaxSlots + 9];
+    __shared__ __align__(8) uint64_t bars[2 * kAtMaxSlots + 11];
     __shared__ float red_m[2][128], red_l[2][128];             // per half of the softmax warps and row: maximum, sum
     __shared__ float part_m[128], part_l[128];                 // of this CTA's key range
     __shared__ unsigned bad_rows[2][4];                        // per half and quarter: rows whose result is not finite
@@ -265,7 +273,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     __shared__ int abort_word;
     volatile int* abort_flag = &abort_word;
     uint64_t *full = bars, *empty = full + kAtMaxSlots, *q_full = empty + kAtMaxSlots, *s_full = q_full + 1, *s_free = s_full + 2,
-             *p_full = s_free + 2, *pv_done = p_full + 2;
+             *p_full = s_free + 2, *pv_done = p_full + 2, *o_free = pv_done + 2;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hd = p.head_dim, group = p.heads / p.kv_heads, kvh = blockIdx.z;
     const int tile = gridDim.y - 1 - blockIdx.y;               // the tiles with the most keys first
@@ -285,7 +293,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
         abort_word = 0;
         for (int i = 0; i < nslots; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
         mbar_init(q_full, 256);
-        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 8); mbar_init(&p_full[i], 8); mbar_init(&pv_done[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 8); mbar_init(&p_full[i], 8); mbar_init(&pv_done[i], 1); mbar_init(&o_free[i], 8); }
         fence_barrier_init();
     }
     pdl_wait();                                                // (before the allocation: the kernel ahead may still hold tensor memory)
@@ -364,17 +372,20 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             if (!resident && j + 1 < nb) again(j + 1);
             const int b = j & 1;
             ok = ok && __all_sync(0xffffffffu, mbar_wait(&p_full[b], (j >> 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            // the sums of the block before (two blocks before, where tensor memory holds two) are in registers
+            if (NO == 64 ? j >= 2 : j >= 1)
+                ok = ok && __all_sync(0xffffffffu, NO == 64 ? mbar_wait(&o_free[b], ((j >> 1) - 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT)
+                                                            : mbar_wait(&o_free[0], (j - 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
             uint32_t addr;
             int slot;
             take(addr, slot);
             if (!ok) break;
             if (elect_one()) {
-                for (int s = 0; s < kAtKeys / 16; ++s) {
-                    const uint32_t a = tmem + 128 * b + (s >> 2) * 64 + (s & 3) * 8;
-                    const uint64_t bd = umma_desc_sw128_mn(addr + s * 2048);
-                    umma_f16_ts(tmem + kAtOCol, a, bd, idesc_o, j > 0 || s > 0);
-                    umma_f16_ts(tmem + kAtOCol, a + 32, bd, idesc_o, 1);
-                }
+                const uint32_t o = tmem + kAtOCol + (NO == 64 ? 128 * b : 0);
+                for (int s = 0; s < kAtKeys / 16; ++s)           // the low parts first: small numbers
+                    umma_f16_ts(o, tmem + 128 * b + 16 * s + 8, umma_desc_sw128_mn(addr + s * 2048), idesc_o, s > 0);
+                for (int s = 0; s < kAtKeys / 16; ++s)
+                    umma_f16_ts(o, tmem + 128 * b + 16 * s, umma_desc_sw128_mn(addr + s * 2048), idesc_o, 1);
                 umma_commit(&empty[slot]);
                 umma_commit(&pv_done[b]);
             }
@@ -440,6 +451,36 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
         mx = fmaxf(mx, red_m[half ^ 1][row]);
         const float mx_e = mx == -INFINITY ? 0.0f : mx;                          // no key of this range counts for the row
         float sum = 0.0f;
+        // the two halves of the warps take a half of the depths each
+        const int c_begin = half ? ((hd / 8 + 1) / 2) * 8 : 0, c_end = half ? hd : ((hd / 8 + 1) / 2) * 8;
+        float o[NO];
+#pragma unroll
+        for (int c = 0; c < NO; ++c) o[c] = 0.0f;
+        auto add_block = [&](int j) {
+            ok = ok && __all_sync(0xffffffffu, mbar_wait(&pv_done[j & 1], (j >> 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
+            if (!ok) return;
+            tc_fence_after();
+            if (live) {
+                const uint32_t t_o = tmem + ((uint32_t)(q4 * 32) << 16) + kAtOCol + (NO == 64 ? 128 * (j & 1) : 0) + c_begin;
+#pragma unroll
+                for (int c = 0; c < NO; c += 32) {
+                    uint32_t r[4][8];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (c_begin + c + 8 * u < c_end) tmem_ld8(t_o + c + 8 * u, r[u]);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (c_begin + c + 8 * u < c_end) {
+#pragma unroll
+                            for (int e = 0; e < 8; e += 2) add2(o[c + 8 * u + e], o[c + 8 * u + e + 1], r[u][e], r[u][e + 1]);
+                        }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&o_free[NO == 64 ? j & 1 : 0]);
+        };
         for (int j = 0; ok && j < nb; ++j) {
             const int b = j & 1, key0 = (blk0 + j) * kAtKeys + 64 * half;
             if (!resident) {
@@ -452,28 +493,25 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&p_full[b]);
+            if (j > 0) add_block(j - 1);
         }
         red_l[half][row] = sum;
-        if (nb > 0) ok = ok && __all_sync(0xffffffffu, mbar_wait(&pv_done[(nb - 1) & 1], ((nb - 1) >> 1) & 1, abort_flag, p.status, STATUS_TMEM_TIMEOUT));
-        tc_fence_after();
+        if (nb > 0) add_block(nb - 1);
         named_barrier_sync(1, 256);
         sum = red_l[0][row] + red_l[1][row];
-        // the two halves of the warps take a half of the depths each
-        const int c_begin = half ? ((hd / 8 + 1) / 2) * 8 : 0, c_end = half ? hd : ((hd / 8 + 1) / 2) * 8;
         if (splits == 1) {
             const int i = (row0 + row) / group, g = (row0 + row) - i * group;
             const size_t dst = (size_t)i * p.heads * hd + (size_t)(kvh * group + g) * hd;
             bool bad = false;
-            for (int c = c_begin; ok && live && c < c_end; c += 8) {
-                uint32_t r[8];
-                tmem_ld8(tmem + ((uint32_t)(q4 * 32) << 16) + kAtOCol + c, r);
-                tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < NO; c += 8) {
+                if (!ok || c_begin + c >= c_end) break;
                 float v[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(__uint_as_float(r[e]) * (1.0f / kAtPScale), sum);
+                for (int e = 0; e < 8; ++e) v[e] = __fdiv_rn(o[c + e] * (1.0f / kAtPScale), sum);
                 if (row < nrow) {
                     bad = bad || (sum > 0.0f && !all_finite(v));
-                    store8<OUT16>(p, dst + c, v);
+                    store8<OUT16>(p, dst + c_begin + c, v);
                 }
             }
             // rows to form again: the two warps that hold a row's halves take every other one, whole
@@ -487,17 +525,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
         } else {
             if (half == 0) { part_m[row] = nb > 0 ? mx : -INFINITY; part_l[row] = sum; }
             float* o_s = reinterpret_cast<float*>(smem);                         // the operands are not needed any more
-            for (int c = c_begin; live && c < c_end; c += 8) {
-                uint32_t r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                if (nb > 0) {
-                    tmem_ld8(tmem + ((uint32_t)(q4 * 32) << 16) + kAtOCol + c, r);
-                    tmem_ld_wait();
-                }
-                if (row < nrow) {
-                    *reinterpret_cast<uint4*>(o_s + (size_t)row * (hd + 4) + c) = make_uint4(r[0], r[1], r[2], r[3]);
-                    *reinterpret_cast<uint4*>(o_s + (size_t)row * (hd + 4) + c + 4) = make_uint4(r[4], r[5], r[6], r[7]);
-                }
-            }
+#pragma unroll
+            for (int c = 0; c < NO; c += 4)
+                if (c_begin + c < c_end && row < nrow) *reinterpret_cast<float4*>(o_s + (size_t)row * (hd + 4) + c_begin + c) = make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
         }
     }
     if (splits > 1) {                                          // ---- the parts of a cluster meet ----
@@ -527,7 +557,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             float sum = 0.0f, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
             for (int s = 0; s < 8; ++s) {
-                if (s >= splits || (m[s] == -INFINITY && l[s] == 0.0f)) continue;   // no key of this part counts (a NaN score does: l is NaN)
+                if (s >= splits || (m[s] == -INFINITY && l[s] == 0.0f)) continue;       // no key of this run counts (a NaN score does: l is NaN)
                 const float f = expf(m[s] - mx);
                 sum = fmaf(f, l[s], sum);
                 v[0] = fmaf(f, o[s][0].x, v[0]); v[1] = fmaf(f, o[s][0].y, v[1]); v[2] = fmaf(f, o[s][0].z, v[2]); v[3] = fmaf(f, o[s][0].w, v[3]);
@@ -684,7 +714,8 @@ __global__ void __launch_bounds__(kAdThreads, 1) attn_decode_kernel(const __grid
     __syncthreads();
     // ---- values: a warp eight depths at a time ----
     for (int n0 = warp * 8; n0 < hd; n0 += 64) {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        // 64 keys' high parts at a time: the instruction cuts its sums off where f32 addition rounds them
+        float acc[4] = {0.f, 0.f, 0.f, 0.f}, low[4] = {0.f, 0.f, 0.f, 0.f}, run[4] = {0.f, 0.f, 0.f, 0.f};
         for (int k0 = 0; k0 < nk16; k0 += 16) {
             uint32_t b0, b1;
             asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
@@ -694,9 +725,18 @@ __global__ void __launch_bounds__(kAdThreads, 1) attn_decode_kernel(const __grid
             const uint16_t *h = hi_s + g * (kc + 8) + k0 + 2 * t, *l = lo_s + g * (kc + 8) + k0 + 2 * t;
             const int down = 8 * (kc + 8);
             auto w = [](const uint16_t* x) { return *reinterpret_cast<const uint32_t*>(x); };
-            mma_16816(acc, w(h), w(h + down), w(h + 8), w(h + down + 8), b0, b1);
-            mma_16816(acc, w(l), w(l + down), w(l + 8), w(l + down + 8), b0, b1);
+            mma_16816(run, w(h), w(h + down), w(h + 8), w(h + down + 8), b0, b1);
+            mma_16816(low, w(l), w(l + down), w(l + 8), w(l + down + 8), b0, b1);
+            if ((k0 & 48) == 48) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    acc[e] += run[e];
+                    run[e] = 0.0f;
+                }
+            }
         }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[e] += run[e] + low[e];
         *reinterpret_cast<float2*>(o_s + g * (hd + 4) + n0 + 2 * t) = make_float2(acc[0], acc[1]);
         *reinterpret_cast<float2*>(o_s + (g + 8) * (hd + 4) + n0 + 2 * t) = make_float2(acc[2], acc[3]);
     }
@@ -784,7 +824,7 @@ __global__ void kv_append_kernel(uint16_t* __restrict__ kc, uint16_t* __restrict
 
 template <int QF32, int OUT16>
 cudaError_t attn_tc_launch(const CUtensorMap& tk, const CUtensorMap& tv, const AttnArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
-    auto kern = attn_tc_kernel<QF32, OUT16>;
+    auto kern = a.head_dim <= 128 ? attn_tc_kernel<QF32, OUT16, 64> : attn_tc_kernel<QF32, OUT16, 128>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};

@@ -458,3 +458,30 @@ def test_an_early_non_finite_value_costs_a_pass_and_not_seconds(heads, kv_heads,
     assert ((got - want).abs()[ok] / (1 + want.abs()[ok])).max() <= (2e-5 + 2.0 ** -11 if out16 else 2e-5)
     assert ev[0].elapsed_time(ev[1]) < 25.0                   # (measured 1.7 at the largest; a thread per eight depths took hundreds)
     assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("q_scale", [1.0, 6.0])
+@pytest.mark.parametrize("heads,kv_heads,hd,start,rows", [(16, 2, 64, 300, 300), (16, 4, 128, 4000, 1), (12, 12, 32, 64, 100), (8, 2, 128, 700, 130)])
+def test_no_further_from_64_bits_than_the_scalar_statement(heads, kv_heads, hd, start, rows, q_scale):
+    """The error of the f32 result against the statement in 64 bits, beside the error of the scalar f32 statement itself, over
+    flat and sharp distributions: probabilities in two parts and tensor-core sums lose nothing against f32 in key order."""
+    n, err, err_scalar = start + rows, 0.0, 0.0
+    for seed in range(3):
+        rng = np.random.default_rng(heads + hd + start + 1000 * seed)
+        k16, v16 = (rng.standard_normal((n, kv_heads * hd)).astype(np.float16) for _ in range(2))
+        q32 = (rng.standard_normal((rows, heads * hd)) * q_scale).astype(np.float16).astype(np.float32)
+        cache = sg.KvCache(heads, kv_heads, hd, n)
+        cache.extend(torch.from_numpy(k16).cuda(), torch.from_numpy(v16).cuda())
+        out = torch.empty((rows, heads * hd), dtype=torch.float32, device="cuda")
+        cache.attend_causal(torch.from_numpy(q32.astype(np.float16)).cuda(), rows, out)
+        scalar = orc.attention_kv_causal(q32, k16.view(np.uint16), v16.view(np.uint16), start, rows, heads, kv_heads, hd, cache.scale())
+        qh = (q32 * np.float32(cache.scale())).astype(np.float16).astype(np.float64).reshape(rows, kv_heads, heads // kv_heads, hd)
+        kd, vd = (x.astype(np.float64).reshape(n, kv_heads, hd) for x in (k16, v16))
+        s = np.einsum("ikgd,tkd->kgit", qh, kd)
+        s[:, :, np.arange(n)[None, :] > start + np.arange(rows)[:, None]] = -np.inf
+        p = np.exp(s - s.max(-1, keepdims=True))
+        want = (np.einsum("kgit,tkd->ikgd", p, vd) / p.sum(-1).transpose(2, 0, 1)[..., None]).reshape(rows, heads * hd)
+        err += float(((out.cpu().numpy() - want) ** 2).sum())
+        err_scalar += float(((np.asarray(scalar).reshape(want.shape) - want) ** 2).sum())
+    # (a tenth for the draw: two orders of the same f32 sums differ by that much)
+    assert err ** 0.5 <= 1.1 * err_scalar ** 0.5 and sg.last_status() == 0
