@@ -452,7 +452,6 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
         *abort_flag = 0;
         fence_barrier_init();
     }
-    pdl_launch_dependents();
     pdl_wait();                                                // (before the allocation: the kernel ahead may still hold tensor memory)
     if (warp == 25) {
         tmem_alloc(tmem_slot, 512);
@@ -461,6 +460,7 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_launch_dependents();
     const uint32_t tmem = *tmem_slot;
 
     if (warp == 24) {                                          // ---- row tiles ----

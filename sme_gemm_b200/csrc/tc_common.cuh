@@ -18,6 +18,8 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---- tensor memory ----
+// A kernel with tensor memory lets its dependents go (pdl_launch_dependents) only behind the allocation and a barrier: the
+// dependent may allocate before it waits for this grid, and would hold columns this grid still asks for.
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols)
                  : "memory");
