@@ -844,9 +844,7 @@ cudaError_t attn_tc_launch(const CUtensorMap& tk, const CUtensorMap& tv, const A
     return cudaLaunchKernelEx(&cfg, kern, tk, tv, a);
 }
 
-}  // namespace
-
-cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream) {
+cudaError_t attn_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream) {
     a.out_vec = ((uintptr_t)a.out & 15) == 0;                  // (rows are heads * head_dim long: multiples of 16 bytes)
     if (a.rows * (a.heads / a.kv_heads) <= 16) {
         // runs of 64 keys and up; caches whose runs do not fit shared memory (about 4 k keys at 128 depths) stay below
@@ -873,7 +871,6 @@ cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStrea
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     const size_t tiles = ((size_t)a.rows * (a.heads / a.kv_heads) + 127) / 128, blocks = (len + kAtKeys - 1) / kAtKeys;
-    if (tiles > 65535) return cudaErrorInvalidValue;
     // a cluster shares a tile's key blocks while the machine has SMs to spare and every CTA keeps a block
     unsigned splits = 1;
     while (splits < 8 && splits * 2 <= blocks && tiles * a.kv_heads * splits * 2 <= (size_t)sm_count) splits *= 2;
@@ -888,6 +885,23 @@ cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStrea
     const dim3 grid(splits, (unsigned)tiles, (unsigned)a.kv_heads);
     if (a.out16) return q_f32 ? attn_tc_launch<1, 1>(tk, tv, a, grid, smem, stream) : attn_tc_launch<0, 1>(tk, tv, a, grid, smem, stream);
     return q_f32 ? attn_tc_launch<1, 0>(tk, tv, a, grid, smem, stream) : attn_tc_launch<0, 0>(tk, tv, a, grid, smem, stream);
+}
+
+}  // namespace
+
+cudaError_t attn_kv_causal_launch(AttnArgs a, int q_f32, int sm_count, cudaStream_t stream) {
+    // as many query rows to a launch as its grid has tiles of 128 rows x heads of a group (8.4 M of them)
+    const int most = 65535 * 128 / (a.heads / a.kv_heads), rows = a.rows;        // (heads are at most 65535)
+    for (int r = 0; r < rows; r += most) {
+        AttnArgs s = a;
+        s.start = a.start + r;
+        s.rows = rows - r < most ? rows - r : most;
+        s.q = static_cast<const char*>(a.q) + (size_t)r * a.q_stride * (q_f32 ? 4 : 2);
+        s.out = static_cast<char*>(a.out) + (size_t)r * a.heads * a.head_dim * (a.out16 ? 2 : 4);
+        const cudaError_t e = attn_launch(s, q_f32, sm_count, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t kv_append_launch(uint16_t* kc, uint16_t* vc, const uint16_t* src, size_t stride, size_t k_off, size_t v_off, size_t row_len,

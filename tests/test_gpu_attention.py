@@ -485,3 +485,21 @@ def test_no_further_from_64_bits_than_the_scalar_statement(heads, kv_heads, hd, 
         err_scalar += float(((np.asarray(scalar).reshape(want.shape) - want) ** 2).sum())
     # (a tenth for the draw: two orders of the same f32 sums differ by that much)
     assert err ** 0.5 <= 1.1 * err_scalar ** 0.5 and sg.last_status() == 0
+
+
+def test_more_query_rows_of_a_head_than_one_grid_has_tiles():
+    """8192 heads on one KV head x 1100 rows: 70400 tiles of 128 query rows, past the 65535 of a grid's dimension."""
+    heads, hd, rows = 8192, 8, 1100
+    g = torch.Generator(device="cuda").manual_seed(3)
+    k, v = (torch.randn(rows, hd, generator=g, device="cuda").half() for _ in range(2))
+    q = torch.randn(rows, heads * hd, generator=g, device="cuda").half()
+    out = torch.full((rows, heads * hd), 3.0, dtype=torch.float32, device="cuda")
+    cache = sg.KvCache(heads, 1, hd, rows)
+    cache.extend(k, v)
+    cache.attend_causal(q, rows, out)
+    for i in (0, 1, 511, 1022, 1023, 1024, 1025, rows - 1):    # 65535 tiles end in row 1023
+        qh = (q[i].float() * np.float32(cache.scale())).half().double().view(heads, hd)
+        p = torch.softmax(qh @ k[:i + 1].double().T, -1)
+        want = (p @ v[:i + 1].double()).reshape(-1)
+        assert ((out[i].double() - want).abs() / (1 + want.abs())).max() <= 2e-5
+    assert not (out == 3.0).all(1).any() and sg.last_status() == 0
