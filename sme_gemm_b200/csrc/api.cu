@@ -687,7 +687,7 @@ static bool q4_fuses_decode(const smeg_q4* w, const uint16_t* a, size_t m, int b
     return !w->affine && !q4_rows_want_tc(w, m) && w->d.log2_block >= 5 && w->d.ku >= 1 && !(glu && w->d.n % 64 != 0);
 }
 
-// A whose rows TMA and the bulk copies cannot take (k no multiple of 8, or a base off a 16-byte boundary) in a zero-padded
+// A whose rows TMA and the 16-byte copies cannot take (k no multiple of 8, or a base off a 16-byte boundary) in a zero-padded
 // copy [m][kd] out of the stream's pool; *out = nullptr where A is fine as it is.
 static int padded_rows(const uint16_t* a, size_t m, size_t k, size_t kd, cudaStream_t stream, uint16_t** out) {
     *out = nullptr;
@@ -697,7 +697,7 @@ static int padded_rows(const uint16_t* a, size_t m, size_t k, size_t kd, cudaStr
     return 0;
 }
 
-// glu / yacc: the fused forms of the MLP block (the tensor-core GEMM, and the one-wave decode kernel at up to four rows).
+// glu / yacc: the fused forms of the MLP block, on every kernel that takes whole gate/up chunks.
 struct TpPush { float* bufs[8]; int world, rank, rows; };
 // The passes around a projection that the one-wave decode kernel takes along: its activations as the norm of f32 rows, and
 // the key / value columns of a [q | k | v] projection to the caches' next rows.
@@ -722,13 +722,21 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     if ((norm || kv) && (c32 || !q4_takes_direct(w, a, m, bf16, glu))) return -3;
     DeviceState* ds = dev_state();
     if (!ds) return -5;
-    // Rows that are not whole 16-byte words: one or two rows are read as they are by the decode kernels; every other call
-    // moves A by TMA or bulk copies and takes a padded copy, a pass of ~2 us.  2051 x 1500 f16, us without and with it:
-    // 8 rows 8.4 / 5.5, 64 rows 67 / 16, 300 rows 299 / 20 (the kernel that reads A by halves walks the weights once per 16
-    // rows); 5001 x 4097 bf16: 1 row 17.6 / 20.3, 4 rows 23.3 / 21.6, 64 rows 478 / 27.
+    // Rows that are not whole 16-byte words: one or two are staged as they are by q4_mma_kernel's CTAs (f32 sums, where the
+    // one-wave kernel's are f16: these calls had f32 sums before they came off the ring-staged kernel); every other call moves
+    // A by TMA or in 16-byte pieces and takes a padded copy, a pass of ~2 us and a trip to the allocator (5001 x 4097 bf16, us:
+    // reading A by halves 8 rows 33, 40 rows 285, with the copy 9.4 and 21).
     uint16_t* a_pad = nullptr;
     size_t k = k0;
-    if (!q4_takes_direct(w, a, m, bf16, glu)) {
+    const bool direct = q4_takes_direct(w, a, m, bf16, glu), ragged = k0 != 0 && (k0 % 8 != 0 || ((uintptr_t)a & 15) != 0);
+    bool in_place = false;
+    if (ragged && !q4_rows_want_tc(w, m)) {
+        Q4GemvArgs r;
+        memset(&r, 0, sizeof(r));
+        r.m = (int)m; r.k64 = (int)w->d.ku; r.log2_block = w->d.log2_block;
+        in_place = q4_mma_supported(r);
+    }
+    if (!direct && !in_place) {
         const int prc = padded_rows(a, m, k0, (k0 + 7) / 8 * 8, stream, &a_pad);
         if (prc) return prc;
         if (a_pad) { a = a_pad; k = (k0 + 7) / 8 * 8; }
@@ -742,7 +750,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     g.m = (int)m; g.n = (int)n; g.k = (int)k;
     g.n16 = (int)w->d.n16; g.k64 = (int)w->d.ku; g.nb = (int)w->d.nb;
     g.log2_block = w->d.log2_block;
-    g.a_vec_ok = (k % 8 == 0) && ((uintptr_t)a % 16 == 0);
+    g.a_vec_ok = !ragged || a_pad;
     g.status = ds->status;
     cudaError_t e;
     if ((push || q4_rows_want_tc(w, m)) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a)) {
@@ -769,7 +777,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         t.ws = sc.ws;
         t.counters = sc.counters;
         e = gemm_tc_launch(t, bf16, grid, smem, stream);
-    } else if ((int)m <= q4_direct_rows() && q4_direct_supported(g, bf16)) {
+    } else if (direct) {
         g.glu = glu; g.yacc = yacc;
         if (norm) { g.nx = norm->x; g.nw = norm->weight; g.nbias = norm->bias; g.neps = norm->eps; g.nrms = norm->rms; }
         if (kv) { g.kc = kv->k; g.vc = kv->v; g.q_len = (int)kv->q_len; g.kv_len = (int)kv->kv_len; }

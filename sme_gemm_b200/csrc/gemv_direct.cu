@@ -20,7 +20,10 @@
 //     packed f16 sums over 8 depths (HFMA2, as the reference's SME kernel accumulates a K-block
 //     in f16, csrc/gemm_f16f16_q4.h:236-341); every 32 depths the pair sums are widened and folded into
 //     the f32 total with the block's scale.  Against the f32-accumulating oracle this differs by
-//     f16 rounding of four-term partial sums, far inside the 1e-2 bar;
+//     f16 rounding of four-term partial sums and of their product with the scale, far inside the
+//     1e-2 bar at the magnitudes activations have; but it is an f16 sum, which overflows beyond
+//     65504 (a code of -8 times an activation above 8188) and is on f16's subnormal grid below
+//     6e-5 -- calls that have f32 sums elsewhere (q4_mma_kernel) are not brought here for speed;
 //   * 2-bit / 1-bit: the activation rows are quantised to int8 in shared memory by the CTA itself
 //     (one or two rows; bit-exact quantize_row, src/kernels/lowbit/matmul.rs:354-371) or copied from
 //     act_quant_kernel's output (three or four rows); codes are expanded in registers (2-bit: byte
@@ -183,30 +186,13 @@ __global__ void __launch_bounds__(kDThreads, 3) q4_direct_kernel(const __grid_co
     __shared__ float norm_sh[8];
     if (GEN && p.nx) {
         for (int r = 0; r < M; ++r) stage_norm_row(As + (size_t)r * a_stride, p.nx + (size_t)r * p.k, p.nw, p.nbias, p.k, kpad, p.neps, p.nrms, norm_sh);
-    } else if (!p.a_vec_ok) {
-        // rows that are no whole 16-byte words, or start off a 16-byte boundary: a half at a time, eight loads in flight
+    } else {
+#pragma unroll
         for (int r = 0; r < M; ++r)
-            for (int d0 = tid; d0 < kpad; d0 += kDThreads * 8) {
-                uint16_t v[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] = d0 + e * kDThreads < p.k ? p.a[(size_t)r * p.k + d0 + e * kDThreads] : (uint16_t)0;
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (d0 + e * kDThreads < kpad) As[(size_t)r * a_stride + d0 + e * kDThreads] = v[e];
-            }
-    } else
-#pragma unroll
-    for (int r = 0; r < M; ++r)
-    for (int d = tid * 8; d < kpad; d += kDThreads * 8) {
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (d + 8 <= p.k) v = *reinterpret_cast<const uint4*>(p.a + (size_t)r * p.k + d);
-        else if (d < p.k) {
-            __align__(16) uint16_t tmp[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) tmp[e] = d + e < p.k ? p.a[(size_t)r * p.k + d + e] : (uint16_t)0;
-            v = *reinterpret_cast<uint4*>(tmp);
-        }
-        *reinterpret_cast<uint4*>(As + (size_t)r * a_stride + d) = v;
+#pragma unroll 2
+            for (int d = tid * 8; d < kpad; d += kDThreads * 8)        // (k is a multiple of 8)
+                *reinterpret_cast<uint4*>(As + (size_t)r * a_stride + d) =
+                    d < p.k ? *reinterpret_cast<const uint4*>(p.a + (size_t)r * p.k + d) : make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
 
@@ -584,6 +570,7 @@ int direct_grid(int n16, int sm_count, int max_groups, int* cpc, int per_sm) {
 // ---- Q4 ----
 bool q4_direct_supported(const Q4GemvArgs& a, int bf16) {
     if (bf16 || a.m < 1 || a.m > 2 || a.log2_block < 5 || a.k64 < 1) return false;
+    if (a.k % 8 != 0 || !a.a_vec_ok) return false;                // 128-bit activation loads
     const size_t smem = kQ4RingBytes + (size_t)a.m * ((size_t)a.k64 * 64 + 8) * 2;
     return smem <= 100 * 1024;
 }

@@ -30,7 +30,7 @@ constexpr int kMThreads = 32 * kMWarps;
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-// 16 bytes, or zeros (nothing is read) where `bytes` is 0
+// `bytes` bytes (0 to 16) and zeros behind them: nothing past them is read
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
@@ -91,25 +91,57 @@ __device__ __forceinline__ void word_codes(uint32_t w, uint32_t (&a)[4]) {
     a[2] = *reinterpret_cast<const uint32_t*>(&r2); a[3] = *reinterpret_cast<const uint32_t*>(&r3);
 }
 
-// Ring slot of a warp: [CG] codes (dense: [CG][column g, g + 8][2 halves] pieces of weights), [2 NT] activation pieces, 16 bytes a
-// lane each, then [CG][2 halves] scale words.
+// Ring slot of a warp: [CG] codes (dense: [CG][column g, g + 8][2 halves] pieces of weights), [2 NT] activation pieces (none where
+// the rows are staged, rows = 0), 16 bytes a lane each, then [CG][2 halves] scale words.
 constexpr int mma_w_bytes(int dense) { return dense ? 2048 : 512; }
-constexpr int mma_slot_bytes(int nt, int cg, int dense) { return mma_w_bytes(dense) * cg + 1024 * nt + (dense ? 0 : 256 * cg); }
+constexpr int mma_slot_bytes(int rows, int cg, int dense) { return mma_w_bytes(dense) * cg + 1024 * rows + (dense ? 0 : 256 * cg); }
 // As deep as two CTAs per SM leave room for.
 constexpr int mma_ring_slots(int nt, int cg, int dense) { return dense ? (nt == 1 ? 4 : 3) : (nt == 1 ? (cg == 1 ? 6 : 4) : (cg == 1 ? 4 : 3)); }
-constexpr size_t mma_smem(int nt, int cg, int dense) {
-    return (size_t)kMWarps * mma_ring_slots(nt, cg, dense) * mma_slot_bytes(nt, cg, dense) + (size_t)kMWarps * cg * nt * 512;
+constexpr size_t mma_smem(int nt, int cg, int dense, int staged) {
+    return (size_t)kMWarps * mma_ring_slots(nt, cg, dense) * mma_slot_bytes(staged ? 0 : nt, cg, dense) + (size_t)kMWarps * cg * nt * 512;
+}
+constexpr size_t kMmaStagedMost = 56 * 1024;
+inline size_t mma_staged_bytes(int m, int k64) { return (size_t)m * ((size_t)k64 * 64 + 8) * 2; }
+
+// A row to shared memory (16-byte aligned) in pieces as wide as its start allows, eight on their way a thread, and zeros behind
+// it up to kpad.
+template <typename T>
+__device__ __forceinline__ int stage_pieces(uint16_t* dst, const uint16_t* src, int k) {
+    constexpr int per = sizeof(T) / 2;
+    const int n = k / per;
+    for (int d0 = threadIdx.x; d0 < n; d0 += kMThreads * 8) {
+        T v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (d0 + e * kMThreads < n) v[e] = reinterpret_cast<const T*>(src)[d0 + e * kMThreads];
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (d0 + e * kMThreads < n) reinterpret_cast<T*>(dst)[d0 + e * kMThreads] = v[e];
+    }
+    return n * per;
+}
+__device__ __noinline__ void stage_row(uint16_t* dst, const uint16_t* src, int k, int kpad) {
+    const unsigned at = (unsigned)(uintptr_t)src;
+    const int done = (at & 15) == 0 ? stage_pieces<uint4>(dst, src, k) : (at & 7) == 0 ? stage_pieces<uint2>(dst, src, k)
+                     : (at & 3) == 0 ? stage_pieces<uint32_t>(dst, src, k) : stage_pieces<uint16_t>(dst, src, k);
+    for (int d = done + (int)threadIdx.x; d < kpad; d += kMThreads) dst[d] = d < k ? src[d] : (uint16_t)0;
 }
 
-// NT = tiles of eight rows per CTA, CG = column groups of a pass.  Grid: (CTAs over the passes, row tiles of 8 NT).
-template <int BF16, int NT, int CG, int DENSE>
+// NT = tiles of eight rows per CTA, CG = column groups of a pass.  Grid: (CTAs over the passes, row tiles of 8 NT).  STAGED: a few
+// rows that are no whole 16-byte words, copied to shared memory by every CTA instead of a padded copy in
+// front of the call (us on the device, with the copy / staged: 5001 x 4097 1 row 8.8 / 6.9, 2 rows 8.7 / 7.8, 4096 x 8190 2 rows
+// 9.7 / 8.8, 14336 x 4092 15.2 / 13.5; a pass from the host, 2051 x 1500 2 rows, 8.7 / 5.3; 700 x 8191 at 3 rows 6.6 / 7.1).
+template <int BF16, int NT, int CG, int DENSE, int STAGED>
 __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_constant__ Q4GemvArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int PF = mma_ring_slots(NT, CG, DENSE), SLOT = mma_slot_bytes(NT, CG, DENSE), WB = mma_w_bytes(DENSE), PER = CG * NT * 128;
+    constexpr int PF = mma_ring_slots(NT, CG, DENSE), RB = STAGED ? 0 : 1024 * NT, SLOT = mma_slot_bytes(STAGED ? 0 : NT, CG, DENSE);
+    constexpr int WB = mma_w_bytes(DENSE), PER = CG * NT * 128;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t ring = smem_u32(smem_raw) + (uint32_t)(warp * PF * SLOT);
     float* red = reinterpret_cast<float*>(smem_raw + (size_t)kMWarps * PF * SLOT);       // [8 warps][CG][NT][4][32 lanes]
+    uint16_t* rows_s = reinterpret_cast<uint16_t*>(red + kMWarps * PER);                 // STAGED: [m][k64 * 64 + 8]
+    const int rows_ld = p.k64 * 64 + 8;
     // this CTA's passes: an equal share of all of them
     const int first = (int)blockIdx.x * p.dq + min((int)blockIdx.x, p.dr);
     const int passes = p.dq + ((int)blockIdx.x < p.dr ? 1 : 0);
@@ -146,7 +178,7 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
             const size_t grp = (size_t)min(group_of(pass, c), p.n16 - 1);               // a tail pass may be one group short
             cp_async16(slot + (uint32_t)(512 * c + lane * 16), p.codes + q4_unit_offset(grp, (size_t)u, p.k64) + lane * 16);
             const uint16_t* s = p.scales + q4_scale_row(grp, 0, p.nb) + 2 * g;
-            const uint32_t d = slot + (uint32_t)(512 * CG + 1024 * NT + 256 * c + lane * 4);
+            const uint32_t d = slot + (uint32_t)(512 * CG + RB + 256 * c + lane * 4);
             cp_async4(d, s + (size_t)((u * 64) >> p.log2_block) * 16);
             cp_async4(d + 128, s + (size_t)((u * 64 + 32) >> p.log2_block) * 16);
         }
@@ -159,6 +191,7 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
         kend[nt] = row0 + 8 * nt + g < p.m ? p.k : 0;
     }
     auto issue_rows = [&](uint32_t slot, int u) {
+        if (STAGED) return;
         const int d = u * 64;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -184,6 +217,10 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
         if (i < total) { issue_rows(ring + (uint32_t)(i * SLOT), lu); advance(); }
         cp_async_commit();
     }
+    if (STAGED) {
+        for (int r = 0; r < p.m; ++r) stage_row(rows_s + (size_t)r * rows_ld, p.a + (size_t)r * p.k, p.k, p.k64 * 64);
+        __syncthreads();
+    }
 
     float tot[CG][NT][4];
 #pragma unroll
@@ -201,6 +238,12 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
             uint4 alo[NT], ahi[NT];
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
+                if (STAGED) {
+                    const uint16_t* ar = rows_s + (size_t)min(g, p.m - 1) * rows_ld + (u_begin + u) * 64 + 8 * t;
+                    alo[nt] = g < p.m ? *reinterpret_cast<const uint4*>(ar) : make_uint4(0, 0, 0, 0);
+                    ahi[nt] = g < p.m ? *reinterpret_cast<const uint4*>(ar + 32) : make_uint4(0, 0, 0, 0);
+                    continue;
+                }
                 alo[nt] = lds128(sb + (uint32_t)(WB * CG + 1024 * nt + lane * 16));
                 ahi[nt] = lds128(sb + (uint32_t)(WB * CG + 1024 * nt + 512 + lane * 16));
             }
@@ -211,8 +254,8 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
 #pragma unroll
                 for (int j = 0; j < (DENSE ? 4 : 1); ++j) wv[c][j] = lds128(sb + (uint32_t)(WB * c + 512 * j + lane * 16));
                 if (!DENSE) {
-                    sw[c][0] = lds32(sb + (uint32_t)(512 * CG + 1024 * NT + 256 * c + lane * 4));
-                    sw[c][1] = lds32(sb + (uint32_t)(512 * CG + 1024 * NT + 256 * c + 128 + lane * 4));
+                    sw[c][0] = lds32(sb + (uint32_t)(512 * CG + RB + 256 * c + lane * 4));
+                    sw[c][1] = lds32(sb + (uint32_t)(512 * CG + RB + 256 * c + 128 + lane * 4));
                 }
             }
             // the slot read in the step before is free: the unit PF - 1 steps on goes there
@@ -307,22 +350,27 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
     cp_async_wait<0>();
 }
 
-template <int BF16, int NT, int CG, int DENSE>
+template <int BF16, int NT, int CG, int DENSE, int STAGED = 0>
 cudaError_t launch(const Q4GemvArgs& a, dim3 grid, cudaStream_t stream) {
     static int attr_dev = -1;   // the opt-in is per device
     int dev = 0;
     cudaGetDevice(&dev);
     if (attr_dev != dev) {
-        const cudaError_t e = cudaFuncSetAttribute(q4_mma_kernel<BF16, NT, CG, DENSE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mma_smem(NT, CG, DENSE));
+        const cudaError_t e = cudaFuncSetAttribute(q4_mma_kernel<BF16, NT, CG, DENSE, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)(mma_smem(NT, CG, DENSE, STAGED) + (STAGED ? kMmaStagedMost : 0)));
         if (e != cudaSuccess) return e;
         attr_dev = dev;
     }
-    return launch_pdl(q4_mma_kernel<BF16, NT, CG, DENSE>, grid, dim3(kMThreads), mma_smem(NT, CG, DENSE), stream, a);
+    const size_t smem = mma_smem(NT, CG, DENSE, STAGED) + (STAGED ? mma_staged_bytes(a.m, a.k64) : 0);
+    return launch_pdl(q4_mma_kernel<BF16, NT, CG, DENSE, STAGED>, grid, dim3(kMThreads), smem, stream, a);
 }
 
 }  // namespace
 
-bool q4_mma_supported(const Q4GemvArgs& a) { return a.m >= 1 && a.log2_block >= 5 && a.k64 >= 1 && a.a_vec_ok; }
+// Rows that are no whole 16-byte words are taken up to two at a time, while they fit beside two CTAs' rings.
+bool q4_mma_supported(const Q4GemvArgs& a) {
+    return a.m >= 1 && a.log2_block >= 5 && a.k64 >= 1 && (a.a_vec_ok || (a.m <= 2 && mma_staged_bytes(a.m, a.k64) <= kMmaStagedMost));
+}
 
 cudaError_t q4_mma_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t stream) {
     const int n16 = (a.n + 15) / 16;
@@ -341,6 +389,10 @@ cudaError_t q4_mma_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t str
     if (a.wdense) {
         if (bf16) return nt == 1 ? launch<1, 1, 1, 1>(a, grid, stream) : launch<1, 2, 1, 1>(a, grid, stream);
         return nt == 1 ? launch<0, 1, 1, 1>(a, grid, stream) : launch<0, 2, 1, 1>(a, grid, stream);
+    }
+    if (!a.a_vec_ok) {
+        if (bf16) return cg == 2 ? launch<1, 1, 2, 0, 1>(a, grid, stream) : launch<1, 1, 1, 0, 1>(a, grid, stream);
+        return cg == 2 ? launch<0, 1, 2, 0, 1>(a, grid, stream) : launch<0, 1, 1, 0, 1>(a, grid, stream);
     }
 #define SMEG_QM(B, T)                                                                          \
     if (bf16 == B && nt == T) return cg == 2 ? launch<B, T, 2, 0>(a, grid, stream) : launch<B, T, 1, 0>(a, grid, stream);

@@ -55,6 +55,13 @@ def run_q4(m, n, k, block, bf16=False, ep_builder=None, seed=0, from_f32=True, h
     return g32, w32, (q, s, a_bits)
 
 
+def q4_exact(q, s, n, k, block):
+    """The weights themselves, code x scale without a rounding, [k][n] f64."""
+    nib = np.stack((q & 15, q >> 4), 1).reshape(-1)[:k * n].reshape(k, n).astype(np.int64)
+    scales = orc.f16_bits_to_f32(s).reshape(n, -1).astype(np.float64)
+    return np.where(nib < 8, nib, nib - 16) * scales.T[np.arange(k) // block]
+
+
 def bias_relu(rng, m, n, bf16):
     """add_col(bias).relu() (tests/correctness/gemv.rs Q4 epilogue case)."""
     b32 = (rng.standard_normal(n) * 0.1).astype(np.float32)
@@ -355,3 +362,24 @@ def test_gated_block_in_two_launches_is_its_separate_passes(m, d, f):
     want += out.float()
     torch.cuda.synchronize()
     assert sg.last_status() == 0 and torch.equal(y, want)
+
+
+@pytest.mark.parametrize("magnitude", [1e4, 1.0, 1e-4])
+@pytest.mark.parametrize("m,n,k,off", [(1, 130, 1027, 0), (1, 70, 96, 1), (2, 130, 1500, 0), (2, 2051, 1027, 1), (3, 130, 1500, 0)])
+def test_rows_off_the_16_byte_grid_keep_f32_sums(m, n, k, off, magnitude):
+    """Activations whose products leave f16's range on both sides: the product is the exact one to its store's rounding."""
+    rng = np.random.default_rng(m + n + k)
+    q, s = q4_logical(rng, n, k, 32)
+    w = sg.Q4Weights.with_params(q, s, None, n, k, sg.Q4Params(32))
+    a16 = (rng.standard_normal((m, k)) * magnitude).astype(np.float16)
+    room = torch.full((m * k + 64,), float("nan"), dtype=torch.float16, device="cuda")
+    a = room[off:off + m * k]
+    a.copy_(torch.from_numpy(a16.reshape(-1)).cuda())
+    c = torch.full((m, n), 9.0, dtype=torch.float16, device="cuda")
+    sg.matmul_q4(a, w, c, m)
+    torch.cuda.synchronize()
+    wt, a64 = q4_exact(q, s, n, k, 32), a16.astype(np.float64)
+    want, room = a64 @ wt, np.abs(a64) @ np.abs(wt)
+    # half a place of the f16 store (2^-25 on its subnormal grid), and f32 sums in any order: 2^-24 of the terms' sizes a few times over
+    assert (np.abs(c.cpu().numpy().astype(np.float64) - want) <= 2.0 ** -11 * np.abs(want) + 2.0 ** -25 + 2.0 ** -21 * room).all()
+    assert sg.last_status() == 0
