@@ -125,6 +125,11 @@ int tc_scratch(cudaStream_t stream, size_t floats, size_t ncounters, TcScratch* 
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(g_mu);
     TcScratch& s = g_tc_scratch[{dev, stream}];
+    if (s.floats < floats || s.ncounters < ncounters) {
+        // (an allocation would end the capture with an error of its own)
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return -2;
+    }
     if (s.floats < floats) {
         float* fresh = nullptr;
         if (cudaMalloc(&fresh, floats * sizeof(float)) != cudaSuccess) return -2;
@@ -726,6 +731,8 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     // one-wave kernel's are f16: these calls had f32 sums before they came off the ring-staged kernel); every other call moves
     // A by TMA or in 16-byte pieces and takes a padded copy, a pass of ~2 us and a trip to the allocator (5001 x 4097 bf16, us:
     // reading A by halves 8 rows 33, 40 rows 285, with the copy 9.4 and 21).
+    // None of them needs the workspace: K-blocks below 32 stay off the streaming form, and where the GEMM would split the depth
+    // inside a capture that finds no workspace they run on the kernel for few rows.
     uint16_t* a_pad = nullptr;
     size_t k = k0;
     const bool direct = q4_takes_direct(w, a, m, bf16, glu), ragged = k0 != 0 && (k0 % 8 != 0 || ((uintptr_t)a & 15) != 0);
@@ -734,7 +741,8 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         Q4GemvArgs r;
         memset(&r, 0, sizeof(r));
         r.m = (int)m; r.k64 = (int)w->d.ku; r.log2_block = w->d.log2_block;
-        in_place = q4_mma_supported(r);
+        // (K-blocks below 32: one row whose bulk copies end with its last whole 16 bytes)
+        in_place = q4_mma_supported(r) || (w->d.log2_block < 5 && m == 1 && ((uintptr_t)a & 15) == 0);
     }
     if (!direct && !in_place) {
         const int prc = padded_rows(a, m, k0, (k0 + 7) / 8 * 8, stream, &a_pad);
@@ -750,11 +758,14 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     g.m = (int)m; g.n = (int)n; g.k = (int)k;
     g.n16 = (int)w->d.n16; g.k64 = (int)w->d.ku; g.nb = (int)w->d.nb;
     g.log2_block = w->d.log2_block;
-    g.a_vec_ok = !ragged || a_pad;
+    g.a_vec_ok = !ragged || a_pad || w->d.log2_block < 5;
     g.status = ds->status;
     cudaError_t e;
-    if ((push || q4_rows_want_tc(w, m)) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a)) {
-        GemmTcArgs t;
+    bool tc = (push || q4_rows_want_tc(w, m)) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a);
+    GemmTcArgs t;
+    dim3 grid;
+    size_t smem = 0;
+    if (tc) {
         memset(&t, 0, sizeof(t));
         t.codes = w->codes; t.scales = w->scales; t.a = a; t.c = c; t.c32 = c32; t.glu = glu; t.yacc = yacc;
         t.m = (int)m; t.n = (int)n; t.k = (int)k;
@@ -765,17 +776,21 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
             for (int s = 0; s < push->world; ++s) t.push[s] = push->bufs[s];
             t.push_world = push->world; t.push_rank = push->rank; t.push_rows = push->rows;
         }
-        dim3 grid;
-        size_t smem = 0, ws_floats = 0, ncounters = 0;
+        size_t ws_floats = 0, ncounters = 0;
         gemm_tc_plan(t, ds->sm_count, &grid, &smem, &ws_floats, &ncounters);
         TcScratch sc;
         if (ws_floats && tc_scratch(stream, ws_floats, ncounters, &sc)) {
-            if (ext) cudaFreeAsync(ext, stream);
-            if (a_pad) cudaFreeAsync(a_pad, stream);
-            return -2;
+            if (!ragged || push || glu || yacc) {
+                if (ext) cudaFreeAsync(ext, stream);
+                if (a_pad) cudaFreeAsync(a_pad, stream);
+                return -2;
+            }
+            tc = false;
         }
         t.ws = sc.ws;
         t.counters = sc.counters;
+    }
+    if (tc) {
         e = gemm_tc_launch(t, bf16, grid, smem, stream);
     } else if (direct) {
         g.glu = glu; g.yacc = yacc;
@@ -787,7 +802,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         e = q4_mma_launch(g, bf16, ds->sm_count, stream);
     } else {
         size_t ws_floats = 0, ncounters = 0;
-        q4_gemv_stream_plan(g, bf16, ds->sm_count, &ws_floats, &ncounters);
+        if (!ragged) q4_gemv_stream_plan(g, bf16, ds->sm_count, &ws_floats, &ncounters);
         if (g.sgrid) {
             TcScratch sc;
             if (tc_scratch(stream, ws_floats, ncounters, &sc)) {

@@ -149,14 +149,14 @@ __global__ void __launch_bounds__(kThreads) q4_gemv_kernel(const __grid_constant
                 if (st % stages_per_chunk != 0) continue;
                 const int ch = st / stages_per_chunk, buf = ch & 1;
                 const int ka0 = ch * p.ka;
-                const unsigned bytes = (unsigned)(min(p.ka, p.k - ka0) * 2);
+                const unsigned bytes = (unsigned)(min(p.ka, p.k - ka0) * 2) & ~15u;   // (a single row may end inside 16 bytes)
                 bool ok = true;
                 if (lane == 0) {
                     if (ch >= 2) ok = mbar_wait(&a_empty[buf], ((ch >> 1) - 1) & 1, abort_flag, p.status);
                     if (ok) mbar_expect_tx(&a_full[buf], rows_used * bytes);
                 }
                 if (!__all_sync(0xffffffffu, ok)) return false;
-                for (int r = lane; r < rows_used; r += 32)
+                for (int r = lane; r < rows_used && bytes; r += 32)
                     bulk_g2s(As + buf * a_buf_halves + (size_t)r * a_stride, p.a + (size_t)(row0 + r) * p.k + ka0, bytes, &a_full[buf]);
             }
             return true;
@@ -210,10 +210,12 @@ __global__ void __launch_bounds__(kThreads) q4_gemv_kernel(const __grid_constant
         const int buf = ch & (nbuf - 1);
         uint16_t* Ab = As + buf * a_buf_halves;
         const int valid = min(chunk, p.k - ka0);                // depths that exist in A
-        if (valid < chunk) {
-            // zero the padded tail (the bulk copy writes only the first `valid` depths)
-            for (int idx = tid; idx < rows_used * (chunk - valid); idx += 32 * kConsumerWarps)
-                Ab[(size_t)(idx / (chunk - valid)) * a_stride + valid + idx % (chunk - valid)] = 0;
+        const int whole = valid & ~7, rest = chunk - whole;     // ... that the bulk copy brings, and what follows them
+        if (rest) {
+            for (int idx = tid; idx < rows_used * rest; idx += 32 * kConsumerWarps) {
+                const int r = idx / rest, d = whole + idx % rest;
+                Ab[(size_t)r * a_stride + d] = d < valid ? p.a[(size_t)(row0 + r) * p.k + ka0 + d] : (uint16_t)0;
+            }
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kConsumerWarps));
         }
         mbar_wait(&a_full[buf], (ch >> 1) & 1, abort_flag, p.status);
@@ -589,7 +591,7 @@ void q4_gemv_stream_plan(Q4GemvArgs& a, int bf16, int sm_count, size_t* ws_float
     // tuning knob, read per call: 0 keeps every call on the column-group-per-CTA kernel, 2 streams small matrices too
     const char* knob = getenv("SMEG_Q4_STREAM");
     const int enabled = knob ? atoi(knob) : 1;
-    if (!enabled || !a.a_vec_ok || a.m > 16 || a.k64 <= 0 || a.n16 <= 0 || sm_count <= 0) return;
+    if (!enabled || !a.a_vec_ok || a.k % 8 != 0 || a.m > 16 || a.k64 <= 0 || a.n16 <= 0 || sm_count <= 0) return;
     const int mt = a.m <= 8 ? 1 : 2;
     // two units per warp and stage when every CTA still gets a dozen stages or more
     const int upw = (long long)a.n16 * ((a.k64 + 2 * kSWarps - 1) / (2 * kSWarps)) >= 12ll * sm_count ? 2 : 1;

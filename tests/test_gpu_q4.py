@@ -383,3 +383,28 @@ def test_rows_off_the_16_byte_grid_keep_f32_sums(m, n, k, off, magnitude):
     # half a place of the f16 store (2^-25 on its subnormal grid), and f32 sums in any order: 2^-24 of the terms' sizes a few times over
     assert (np.abs(c.cpu().numpy().astype(np.float64) - want) <= 2.0 ** -11 * np.abs(want) + 2.0 ** -25 + 2.0 ** -21 * room).all()
     assert sg.last_status() == 0
+
+
+@pytest.mark.parametrize("m,block,k,off", [(64, 32, 4092, 0), (40, 32, 4096, 1), (8, 16, 4092, 0), (1, 16, 4091, 0), (40, 16, 4092, 0)])
+def test_rows_off_the_16_byte_grid_in_a_capture_without_a_warm_call(m, block, k, off):
+    """These calls need no workspace, so the first one on a stream may be inside a capture; the replay gives the bits the
+    captured kernels give, within the bar of the same call outside."""
+    n = 4096
+    rng = np.random.default_rng(m + k)
+    q, s = q4_logical(rng, n, k, block, from_f32=False)
+    w = sg.Q4Weights.with_params(q, s, None, n, k, sg.Q4Params(block))
+    a = torch.full((m * k + 64,), float("nan"), dtype=torch.float16, device="cuda")[off:off + m * k]
+    a.copy_(torch.from_numpy(rng.standard_normal(m * k).astype(np.float16)).cuda())
+    c, want = (torch.full((m, n), 9.0, dtype=torch.float16, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+        sg.matmul_q4(a, w, c, m)
+    graph.replay()
+    torch.cuda.synchronize()
+    sg.matmul_q4(a, w, want, m)
+    torch.cuda.synchronize()
+    assert max_rel(c.float().cpu().numpy(), want.float().cpu().numpy()) <= TOL and sg.last_status() == 0
+    a64, wt = a.cpu().numpy().astype(np.float64).reshape(m, k), q4_exact(q, s, n, k, block)
+    assert max_rel(c.float().cpu().numpy(), a64 @ wt) <= half_tol(1e-2, k)
+    del graph
