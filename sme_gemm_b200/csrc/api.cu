@@ -601,14 +601,23 @@ int smeg_host_q1_quantize(const float* w, int layout, size_t n, size_t k, size_t
 static int q4_direct_rows() { return g_direct_rows < 2 ? g_direct_rows : 2; }
 
 // Whether an m-row call on these weights is better off on the tensor-core GEMM than on the warp-level kernels.  Up to 16
-// rows never; above, it depends on the matrix: q4_mma_kernel takes about 1.6 us and 0.29 us per 1000 units (16 columns x 64
-// depths) and 16 rows, the GEMM about 11 us and 0.33 us per 1000 units (more from 128 rows up).  Measured, us, mma / tc:
-// 1536 x 1152 at 17 and 64 rows 2.6 / 14, 3.2 / 14; 4096 x 4096 at 17 rows 11 / 15, at 64 rows 19 / 15.6.
-static bool q4_rows_want_tc(const smeg_q4* w, size_t m) {
+// rows never; above, it depends on the matrix.  q4_mma_kernel's time goes with column groups x (64-deep units + 12) x pairs of
+// row tiles; the GEMM's is 5 us on short depths, 9 where it splits the depth, and little more for more rows.  The line is
+// where the two met on a grid of 12 matrices x 9 row counts x 2 types; on it the kernel taken is within 8 % of the better
+// one (mma / GEMM, us, f16: 2048 x 4096 at 32 rows 6.4 / 9.4, 33 rows 11.1 / 10.2; 4096 x 4096 17 rows 11.4 / 10.9, 48 rows
+// 17.2 / 12.1; 8192 x 512 32 rows 4.3 / 5.1, 64 rows 7.5 / 5.5; 2048 x 1504 128 rows 8.4 / 11.1, 256 rows 15.2 / 12.8).  It lies at
+// twice that (`dear`) for bf16 up to 32 rows, whose expansion costs the GEMM more (6144 x 4096 14.0 / 15.3), and under an
+// epilogue with an activation, which costs the GEMM's drain 7 us (2048 x 4096 at 64 rows, bias and GELU, 12.7 / 19.1).
+static bool q4_rows_want_tc(const smeg_q4* w, size_t m, bool dear = false) {
     if ((int)m <= g_tc_min_rows) return false;
     if (w->d.log2_block < 5) return true;
-    const size_t units = div_up(w->d.n, 16) * w->d.ku;
-    return units * (29 * div_up(m, 16) - 33) >= 900000;
+    return div_up(w->d.n, 16) * (w->d.ku + 12) * div_up(m, 32) >= (dear ? 40000 : 19000);
+}
+static bool q4_dear_on_tc(const EpParams& ep, size_t m, int bf16) {
+    if ((bf16 && m <= 32) || (ep.n_nodes > 0 && !fast_ep_eligible(ep))) return true;
+    for (int i = 0; i < ep.n_nodes; ++i)
+        if ((ep.nodes[i].op & 0xffu) == 8) return true;
+    return false;
 }
 static bool q4_uses_tc(const smeg_q4* w, const uint16_t* a, size_t m) {
     return q4_rows_want_tc(w, m) && gemm_tc_supported(4, (int)m, (int)w->d.k, w->d.log2_block, a);
@@ -761,7 +770,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     g.a_vec_ok = !ragged || a_pad || w->d.log2_block < 5;
     g.status = ds->status;
     cudaError_t e;
-    bool tc = (push || q4_rows_want_tc(w, m)) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a);
+    bool tc = (push || q4_rows_want_tc(w, m, q4_dear_on_tc(g.ep, m, bf16))) && gemm_tc_supported(4, (int)m, (int)k, w->d.log2_block, a);
     GemmTcArgs t;
     dim3 grid;
     size_t smem = 0;
