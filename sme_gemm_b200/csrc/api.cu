@@ -1095,10 +1095,11 @@ int smeg_gemm_dense_dev(const smeg_dense* w, const uint16_t* a, uint16_t* c, siz
     EpNodeDev* ext = nullptr;
     int rc = make_ep(ep, n, &t.ep, stream, &ext);
     if (rc) { if (ext) cudaFreeAsync(ext, stream); if (a_pad) cudaFreeAsync(a_pad, stream); return rc; }
-    if (m <= 8 || div_up(n, 16) * ((k_run + 63) / 64) * div_up(m, 16) <= 20000) {
+    if (m <= 16 || div_up(n, 16) * ((k_run + 63) / 64) * div_up(m, 16) <= 20000) {
         // The warp-level kernel streams the weights once per 16 rows: about 1.6 us and 0.33 us per 1000 units (16 columns x 64
-        // depths) and 16 rows, where the GEMM takes 9 us and more (2048 x 1504 f16, us, GEMM / this: 1 row 9.4 / 2.1, 17 rows
-        // 8.5 / 3.3; 4096 x 2048: 1 row 9.1 / 3.1, 32 rows 11.4 / 7.2).
+        // depths) and 16 rows, where the GEMM takes 6 us and more: up to 16 rows whatever the matrix, above by the product (f16,
+        // us, GEMM / this: 1024 x 768 at 128 rows 7.5 / 4.3; 4096 x 2048 at 1 row 7.2 / 3.4, 32 rows 8.6 / 7.5, 64 rows 9.2 / 13.4;
+        // 4096 x 4096 at 16 rows 10.1 / 7.2, 17 rows 10.9 / 12.1; 14336 x 4096 at 16 rows 47.7 / 25.6; 32000 x 2048 49.7 / 30.2).
         Q4GemvArgs g;
         memset(&g, 0, sizeof(g));
         g.wdense = w->w; g.kd = (int)w->kd; g.a = a_run; g.c = c; g.beta = w->bf16 ? __uint_as_float_host((uint32_t)beta_bits << 16) : h2f(beta_bits);
