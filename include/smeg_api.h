@@ -174,7 +174,9 @@ int smeg_host_q1_quantize(const float *w, int layout, size_t n, size_t k, size_t
 /* ---- compute, device pointers (the timed paths) ------------------------------ */
 
 /* matmul_q4_ep / matmul_q4_bf16_ep (src/kernels/q4/matmul.rs:21-103, 178-271):
- * C[m][n] = ep(A[m][k] @ dequant(W)).  ep may be NULL. */
+ * C[m][n] = ep(A[m][k] @ dequant(W)).  ep may be NULL.  Up to 16 rows, and more on small matrices, a weight is code x
+ * scale unrounded (K-blocks of 32 and up); above, rounded to the operand type as the portable statement has it.  The
+ * reference's GEMV and MOPA kernels differ in the same way; the same rows move by 2.5e-3 (bf16) or 2e-4 (f16). */
 int smeg_matmul_q4_f16_dev(const smeg_q4 *w, const uint16_t *a, uint16_t *c, size_t m,
                            const ep_desc16 *ep, void *stream);
 int smeg_matmul_q4_bf16_dev(const smeg_q4 *w, const uint16_t *a, uint16_t *c, size_t m,

@@ -531,7 +531,8 @@ def matmul_q4_ep(a, w: Q4Weights, c, m: int, ep: Epilogue) -> None:
 
 
 def matmul_q4_bf16(a, w: Q4Weights, c, m: int) -> None:
-    """matmul_q4_bf16, src/kernels/q4/matmul.rs:178-186."""
+    """matmul_q4_bf16, src/kernels/q4/matmul.rs:178-186.  Up to 16 rows (more on small matrices) the weights are code x scale
+    unrounded, above that rounded to bf16 as the portable statement has them: the same rows move by about 2.5e-3 there."""
     _run_q4(a, w, c, m, None, True)
 
 

@@ -337,9 +337,14 @@ def test_warp_level_kernel(m, n, k, block, bf16):
     warps without a unit or end inside one, an epilogue on the product."""
     got, want, (q, s, a_bits) = run_q4(m, n, k, block, bf16, bias_relu, from_f32=False)
     assert max_rel(got, want) <= (2e-2 if bf16 else TOL)       # one bf16 place of the product can flip through the epilogue
-    # the product itself: f32 sums of unrounded weights, so nearer to the exact product than half a place of the store
-    got, want, _ = run_q4(m, n, k, block, bf16, None)
+    # the product itself: f32 sums (2^-24 of the terms' sizes a few times over) of the weights code x scale, unrounded, and one
+    # rounding of the store -- for bf16 as for f16, whatever the rows of the call
+    got, want, (q, s, a_bits) = run_q4(m, n, k, block, bf16, None)
     assert max_rel(got, want) <= TOL
+    if bf16 or m > 2:                                          # (one and two f16 rows run on the one-wave kernel)
+        a64, wt = orc.t_bits_to_f32(a_bits, bf16).reshape(m, k).astype(np.float64), q4_exact(q, s, n, k, block)
+        exact, room = a64 @ wt, np.abs(a64) @ np.abs(wt)
+        assert (np.abs(got.reshape(m, n) - exact) <= 2.0 ** (-8 if bf16 else -11) * np.abs(exact) + 2.0 ** -25 + 2.0 ** -21 * room).all()
 
 
 @pytest.mark.parametrize("m", [3, 8, 16, 17, 40, 64])
