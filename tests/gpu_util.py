@@ -1,4 +1,7 @@
 """Helpers shared by the GPU parity tests."""
+import os
+import re
+
 import numpy as np
 import torch
 
@@ -32,6 +35,17 @@ def max_rel(got_f32, want_f32):
 def half_tol(base, k):
     """tests/proptest.rs:83-85: max(base, base * sqrt(k) / 4)."""
     return max(base, base * (k ** 0.5) / 4.0)
+
+
+def takes_gemm(m, n, k, bf16=False, act=False, dense=False):
+    """Whether a call of these sizes (K-blocks of 32 and up) runs on the tensor-core GEMM: the library's rule, its limits read
+    from the source, so that a test written for that kernel fails when the line moves past its shapes."""
+    src = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "sme_gemm_b200", "csrc", "api.cu")).read()
+    if dense:
+        rows, units = map(int, re.search(r"if \(m <= (\d+) \|\| div_up\(n, 16\) \* \(\(k_run \+ 63\) / 64\) \* div_up\(m, 16\) <= (\d+)\)", src).groups())
+        return m > rows and -(-n // 16) * (-(-k // 64)) * -(-m // 16) > units
+    extra, dear, line = map(int, re.search(r"\* \(w->d\.ku \+ (\d+)\) \* div_up\(m, 32\) >= \(dear \? (\d+) : (\d+)\)", src).groups())
+    return m > 16 and -(-n // 16) * (-(-k // 64) + extra) * -(-m // 32) >= (dear if act or (bf16 and m <= 32) else line)
 
 
 def q4_logical(rng, n, k, block, from_f32=True):

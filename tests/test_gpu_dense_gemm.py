@@ -9,7 +9,7 @@ import torch
 
 import oracle as orc
 import sme_gemm_b200 as sg
-from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, max_rel
+from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, max_rel, takes_gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -23,9 +23,10 @@ def _case(m, n, k, bf16, seed):
     return a, b, bias
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 64, 64), (7, 100, 72), (33, 130, 512), (200, 1000, 256), (300, 384, 1024)])
+@pytest.mark.parametrize("m,n,k", [(1, 64, 64), (7, 100, 72), (33, 130, 512), (200, 1000, 256), (300, 384, 1024), (40, 2100, 4096), (200, 1100, 2048), (300, 1032, 1040)])
 @pytest.mark.parametrize("bf16", [False, True])
 def test_gemm_builder_matches_dense_reference(m, n, k, bf16):
+    assert takes_gemm(m, n, k, dense=True) == (n > 1000)           # the warp-level kernel below, the tensor-core one above
     a, b, bias = _case(m, n, k, bf16, m + n)
     tof = orc.bf16_bits_to_f32 if bf16 else orc.f16_bits_to_f32
     todev = bf16_bits_dev if bf16 else f16_bits_dev
@@ -49,22 +50,28 @@ def test_gemm_builder_matches_dense_reference(m, n, k, bf16):
     assert sg.last_status() == 0
 
 
-def test_beta_and_column_major_output():
-    m, n, k = 37, 96, 128
-    a, b, bias = _case(m, n, k, False, 3)
-    w = sg.prepack_f16(b, n, k)
-    ad = f16_bits_dev(a).reshape(m, k)
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("m,n,k", [(37, 96, 128), (40, 2050, 4096), (150, 8210, 256), (300, 1040, 2048)])
+def test_beta_and_column_major_output(m, n, k, bf16):
+    """On the warp-level kernel, the tensor-core one with a split depth (whose reduce stores) and without."""
+    assert takes_gemm(m, n, k, dense=True) == (n > 96)
+    a, b, bias = _case(m, n, k, bf16, 3)
+    to_f32, to_bits, to_dev = ((orc.bf16_bits_to_f32, orc.f32_to_bf16_bits, bf16_bits_dev) if bf16 else
+                               (orc.f16_bits_to_f32, orc.f32_to_f16_bits, f16_bits_dev))
+    w = (sg.prepack_bf16 if bf16 else sg.prepack_f16)(b, n, k)
+    ad = to_dev(a).reshape(m, k)
     # beta scales the f32 product before the store rounding: reference::gemm_f16 stores f16(beta * acc)
-    acc = orc.gemm16_f32(a, b, m, n, k)
-    want = orc.f32_to_f16_bits((np.float32(0.5) * acc).astype(np.float32)).reshape(m, n)
-    c = torch.zeros((m, n), dtype=torch.float16, device="cuda")
+    acc = (to_f32(a).reshape(m, k).astype(np.float64) @ to_f32(b).reshape(k, n).astype(np.float64)).astype(np.float32)
+    want = to_bits(np.float32(0.5) * acc).reshape(m, n)
+    c = torch.zeros((m, n), dtype=ad.dtype, device="cuda")
     sg.Gemm.new(ad, w, m).beta(0.5).run(c)
-    assert max_rel(orc.f16_bits_to_f32(bits_of(c)), orc.f16_bits_to_f32(want)) <= 1e-2
-    ccm = torch.zeros((n, m), dtype=torch.float16, device="cuda")      # c[i + j * m]
-    sg.Gemm.new(ad, w, m).beta(0.5).col_major_output().add_col(f16_bits_dev(bias)).run(ccm.view(m, n))
-    want_cm = orc.apply_ep(want, m, n, orc.Nodes([(4, 0, 0.0, bias, 0)]))
-    got = orc.f16_bits_to_f32(bits_of(ccm)).reshape(n, m).T
-    assert max_rel(got, orc.f16_bits_to_f32(want_cm).reshape(m, n)) <= 1e-2
+    assert max_rel(to_f32(bits_of(c)).reshape(m, n), to_f32(want).reshape(m, n)) <= 1e-2
+    ccm = torch.zeros((n, m), dtype=ad.dtype, device="cuda")           # c[i + j * m]
+    sg.Gemm.new(ad, w, m).beta(0.5).col_major_output().add_col(to_dev(bias)).run(ccm.view(m, n))
+    want_cm = orc.apply_ep(want, m, n, orc.Nodes([(4, 0, 0.0, bias, 0)]), bf16)
+    got = to_f32(bits_of(ccm)).reshape(n, m).T
+    assert max_rel(got, to_f32(want_cm).reshape(m, n)) <= (2e-2 if bf16 else 1e-2)
+    assert sg.last_status() == 0
 
 
 def test_host_pointer_entry_and_unsupported_depth():
@@ -97,6 +104,7 @@ def test_ragged_depth_runs_through_a_padded_copy(m, n, k):
 def test_handful_of_rows_on_dense_weights(m, n, k, bf16):
     """The warp-level kernel: row tiles of 8 and 16 with rows missing, a column group with columns missing, depths that leave
     warps without work or end inside a fragment, beta, a row operand and column-major output."""
+    assert not takes_gemm(m, n, k, dense=True)
     a, b, bias = _case(m, n, k, bf16, m * n)
     tof = orc.bf16_bits_to_f32 if bf16 else orc.f16_bits_to_f32
     w = (sg.prepack_bf16 if bf16 else sg.prepack_f16)(b, n, k)

@@ -5,7 +5,7 @@ import torch
 
 import oracle as orc
 import sme_gemm_b200 as sg
-from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, max_rel, q4_logical
+from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, max_rel, q4_logical, takes_gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -186,12 +186,14 @@ def test_mlp_equals_its_three_calls_and_the_oracle(m):
     assert torch.equal(y4, y)
 
 
-@pytest.mark.parametrize("m,d,f", [(65, 256, 1152), (130, 192, 2048), (300, 512, 1024)])
+@pytest.mark.parametrize("m,d,f", [(65, 256, 1152), (130, 192, 2048), (300, 512, 1024), (40, 832, 16384), (65, 832, 8192), (200, 832, 4096), (300, 832, 4096)])
 def test_prefill_mlp_with_fused_gate_and_residual_equals_its_three_calls(m, d, f):
-    """Above 64 rows the block runs as two tensor-core GEMMs -- the gated product formed in the
-    gate/up GEMM's store, the residual add in the down GEMM's -- and must give the bits of the
-    three separate calls plus add_f16 (tests/correctness/model.rs:447-510), also through the
-    tensor-parallel partial / finish pair."""
+    """The block runs as two GEMMs -- the gated product formed in the gate/up GEMM's store, the
+    residual add in the down GEMM's; the tensor-core ones on the larger matrices, the warp-level
+    ones on the small -- and must give the bits of the three separate calls plus add_f16
+    (tests/correctness/model.rs:447-510), also through the tensor-parallel partial / finish pair."""
+    # (832 deep: neither form of the gate/up GEMM splits the depth, so both sum in the same order)
+    assert d != 832 or (takes_gemm(m, 2 * f, d) and takes_gemm(m, d, f))
     rng = np.random.default_rng(m)
     wg = (rng.standard_normal(f * d) * 0.05).astype(np.float32)
     wu = (rng.standard_normal(f * d) * 0.05).astype(np.float32)
@@ -299,14 +301,15 @@ def test_converts_and_activation_passes_device_and_host_entries():
 
 def test_concurrent_host_threads_on_shapes_that_grow_the_scratch():
     """Host threads calling shapes with different scratch needs on one stream (the streaming decode kernel's shares and
-    counters, the depth-split GEMM's partial tiles): a block that is outgrown stays valid for the launch that read its
-    address, and every result equals the quiet run's bits (tests/concurrency.rs:130-180)."""
+    counters -- K-blocks of 16 -- and the depth-split GEMM's partial tiles): a block that is outgrown stays valid for the
+    launch that read its address, and every result equals the quiet run's bits (tests/concurrency.rs:130-180)."""
     import threading
     rng = np.random.default_rng(77)
     cases = []
-    for (m, n, k) in ((1, 4096, 2048), (5, 9216, 4096), (40, 256, 8192), (1, 12288, 4096), (33, 512, 4096)):
-        q, s = q4_logical(rng, n, k, 32, from_f32=False)
-        w = sg.Q4Weights.new(q, s, n, k)
+    for (m, n, k, block) in ((33, 4096, 4096, 32), (5, 14336, 4096, 16), (70, 2048, 4096, 64), (1, 16384, 4096, 16), (300, 512, 8192, 32)):
+        assert block == 16 or takes_gemm(m, n, k)                  # (few column tiles: the depth is split)
+        q, s = q4_logical(rng, n, k, block, from_f32=False)
+        w = sg.Q4Weights.with_params(q, s, None, n, k, sg.Q4Params(block))
         a = f16_bits_dev(orc.f32_to_f16_bits(rng.standard_normal((m, k)).astype(np.float32)))
         c = torch.zeros((m, n), dtype=torch.float16, device="cuda")
         sg.matmul_q4(a, w, c, m)

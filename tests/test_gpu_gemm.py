@@ -1,6 +1,7 @@
-"""Prefill GEMM (tcgen05 / TMEM) on the GPU against the CPU oracle, through the C ABI.
+"""Prefill calls on the GPU against the CPU oracle, through the C ABI.
 
-Rows above the decode kernel's row cap run the tensor-core kernel.  Tolerance as
+Above 16 rows a call runs on the tensor-core kernel (tcgen05 / TMEM) or, on small matrices, on the
+warp-level one: tests of the former say so (takes_gemm).  Tolerance as
 for the decode path: max |g-w|/(1+|w|) <= 1e-2 against the oracle (same f32
 accumulation over the same rounded weights; only the summation order differs)."""
 import numpy as np
@@ -9,7 +10,7 @@ import torch
 
 import oracle as orc
 import sme_gemm_b200 as sg
-from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, max_rel, q4_logical
+from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, max_rel, q4_logical, takes_gemm
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-2
@@ -61,14 +62,28 @@ def test_q4_gemm_matches_oracle(m, n, k, block, bf16):
     assert mr <= TOL, f"{m}x{n}x{k} block {block} bf16={bf16}: max_rel {mr}"
 
 
+@pytest.mark.parametrize("m,n,k,block", [(33, 4200, 2048, 64), (64, 4130, 2048, 128), (48, 4200, 2056, 256), (65, 2400, 2048, 64), (100, 2066, 2048, 128),
+                                         (257, 1040, 2048, 256), (300, 520, 4096, 128), (513, 1032, 576, 64), (800, 1040, 512, 32), (512, 1040, 1000, 512)])
 @pytest.mark.parametrize("bf16", [False, True])
-def test_q4_gemm_epilogue_graph(bf16):
-    assert run(100, 300, 512, 32, bf16, ep="cfg4") <= (TOL_BF16_EP if bf16 else TOL)
+def test_tensor_core_gemm_k_blocks(m, n, k, block, bf16):
+    """K-blocks of 64 and up on the tensor-core kernel, whose stages then share scale rows: one- and two-unit stages, single
+    CTAs and pairs, depth splits."""
+    assert takes_gemm(m, n, k, bf16)
+    mr = run(m, n, k, block, bf16)
+    assert mr <= TOL, f"{m}x{n}x{k} block {block} bf16={bf16}: max_rel {mr}"
 
 
-def test_ragged_depth_falls_back_to_the_decode_kernel_rows():
-    """k % 8 != 0 cannot use a tensor map; the call still runs and matches."""
-    assert run(40, 200, 1030, 32, False) <= TOL
+@pytest.mark.parametrize("m,n,k", [(100, 300, 512), (100, 4120, 2048), (300, 2080, 2048)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_q4_gemm_epilogue_graph(m, n, k, bf16):
+    assert takes_gemm(m, n, k, bf16, act=True) == (n > 300)
+    assert run(m, n, k, 32, bf16, ep="cfg4") <= (TOL_BF16_EP if bf16 else TOL)
+
+
+def test_ragged_depth_runs_through_a_padded_copy():
+    """k % 8 != 0 cannot use a tensor map: the activations are copied to rows that can, on either kernel."""
+    assert run(40, 200, 1030, 32, False) <= TOL and not takes_gemm(40, 200, 1030)
+    assert run(70, 2400, 2045, 32, False) <= TOL and takes_gemm(70, 2400, 2045)
     assert run(96, 130, 1027, 1, False) <= TOL
 
 
@@ -126,6 +141,7 @@ def test_tensor_core_gemm_on_large_matrices(n, k):
     rng = np.random.default_rng(n)
     w, dense = _big_q4(rng, n, k)
     for bf16 in (False, True):
+        assert takes_gemm(33, n, k, bf16)
         dt = torch.bfloat16 if bf16 else torch.float16
         rounded = dense.to(dt).float()
         bias = torch.randn(n, device="cuda").mul(0.1).to(dt)
@@ -157,6 +173,7 @@ def test_gated_block_on_large_matrices(m):
     """Gate and up columns in the two accumulator sets of every token tile, the residual add behind a depth split."""
     rng = np.random.default_rng(m)
     d, f = 4096, 9408
+    assert takes_gemm(m, 2 * f, d) and takes_gemm(m, d, f)
     up, wu = _big_q4(rng, 2 * f, d)
     down, wd = _big_q4(rng, d, f)
     x = torch.randn(m, d, device="cuda").half()
