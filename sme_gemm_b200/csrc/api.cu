@@ -1362,7 +1362,7 @@ int smeg_block_accumulate_dev(const smeg_block_args* b, void* stream_v) {
     // that take them (up to 1024 wide: every CTA repeats the norm, 384 wide 1.5 us less a norm than a launch of its own, 4096
     // wide 3 us more) -- five launches a layer instead of eight.
     const NormIn n1 = {b->x, b->norm1_w, b->norm1_b, b->norm1_eps, b->norm1_rms ? 1 : 0}, n2 = {b->x, b->norm2_w, b->norm2_b, b->norm2_eps, b->norm2_rms ? 1 : 0};
-    const bool direct = q4_takes_direct(b->qkv, h, m, 0, 0), norm_in = direct && d <= 1024;
+    const bool direct = q4_takes_direct(b->qkv, h, m, 0, 0), norm_in = direct && d <= kNormInMost;
     int rc = norm_in ? 0 : smeg_norm_rows_dev(h, nullptr, b->x, b->norm1_w, b->norm1_b, m, d, b->norm1_eps, b->norm1_rms, stream);
     if (direct) {
         const KvOut kv = {b->k_cache + b->pos * kv_len, b->v_cache + b->pos * kv_len, q_len, kv_len};
@@ -1373,7 +1373,7 @@ int smeg_block_accumulate_dev(const smeg_block_args* b, void* stream_v) {
     }
     if (!rc) rc = smeg_attn_kv_causal_f16_dev(att, qkv, 0, w, b->k_cache, b->v_cache, b->pos, m, b->heads, b->kv_heads, b->head_dim, b->scale, stream);
     if (!rc) rc = q4_accumulate(b->out, att, b->x, out, m, stream);
-    const bool norm_in_up = d <= 1024 && q4_takes_direct(up, nullptr, m, 0, b->mlp ? (int)b->mlp->act : 0) && (!b->mlp || up->d.n == 2 * hidden);
+    const bool norm_in_up = d <= kNormInMost && q4_takes_direct(up, nullptr, m, 0, b->mlp ? (int)b->mlp->act : 0) && (!b->mlp || up->d.n == 2 * hidden);
     if (!rc && !norm_in_up) rc = smeg_norm_rows_dev(h, nullptr, b->x, b->norm2_w, b->norm2_b, m, d, b->norm2_eps, b->norm2_rms, stream);
     if (!rc) {
         const NormIn* norm = norm_in_up ? &n2 : nullptr;

@@ -93,7 +93,7 @@ __device__ __forceinline__ float cta_sum(float v, float* sh) {
 // same bits), repeated by every CTA -- a row is a few KB out of L2 against a launch of its own in front of the projection.
 __device__ __noinline__ void stage_norm_row(uint16_t* dst, const float* xr, const float* weight, const float* bias, int dim, int kpad, float eps,
                                             int rms, float* sh) {
-    constexpr int KEEP = 16;               // values a thread keeps in registers between the passes (rows of up to 4096)
+    constexpr int KEEP = kNormInMost / kDThreads;              // values a thread keeps in registers between the passes
     const int tid = threadIdx.x;
     float x[KEEP];
 #pragma unroll
@@ -105,7 +105,6 @@ __device__ __noinline__ void stage_norm_row(uint16_t* dst, const float* xr, cons
 #pragma unroll
         for (int i = 0; i < KEEP; ++i)
             if (tid + i * kDThreads < dim) s += x[i];
-        for (int j = tid + KEEP * kDThreads; j < dim; j += kDThreads) s += xr[j];
         mean = __fdiv_rn(cta_sum(s, sh), fdim);
     }
     float ss = 0.0f;
@@ -115,10 +114,6 @@ __device__ __noinline__ void stage_norm_row(uint16_t* dst, const float* xr, cons
             const float d = __fsub_rn(x[i], mean);
             ss = __fmaf_rn(d, d, ss);
         }
-    for (int j = tid + KEEP * kDThreads; j < dim; j += kDThreads) {
-        const float d = __fsub_rn(xr[j], mean);
-        ss = __fmaf_rn(d, d, ss);
-    }
     const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(cta_sum(ss, sh), fdim), eps)));
     auto put = [&](int j, float v) {
         dst[j] = __half_as_ushort(__float2half_rn(__fadd_rn(__fmul_rn(__fmul_rn(__fsub_rn(v, mean), r), weight[j]), bias ? bias[j] : 0.0f)));
@@ -126,7 +121,6 @@ __device__ __noinline__ void stage_norm_row(uint16_t* dst, const float* xr, cons
 #pragma unroll
     for (int i = 0; i < KEEP; ++i)
         if (tid + i * kDThreads < dim) put(tid + i * kDThreads, x[i]);
-    for (int j = tid + KEEP * kDThreads; j < dim; j += kDThreads) put(j, xr[j]);
     for (int j = dim + tid; j < kpad; j += kDThreads) dst[j] = 0;
 }
 

@@ -10,6 +10,7 @@
 namespace smeg {
 
 // ---- Q4 GEMV (q4_gemv.cu) ----
+constexpr int kNormInMost = 1024;   // widest rows whose norm the one-wave kernel forms
 struct Q4GemvArgs {
     const unsigned char* codes;   // packed units, [n16][k64][512 B]
     const uint16_t* scales;       // f16 bits, [n16][nb][16]
@@ -21,7 +22,7 @@ struct Q4GemvArgs {
                                   // receives f16(act(f16(gate)) * f16(up)); a CTA then owns (gate group, up group) pairs
     float* yacc;                  // if set: y[m][n] += f32(f16(acc)) instead of storing c (the residual add)
     // one-wave kernel only -- the passes around a layer's projections at decode size:
-    const float *nx, *nw, *nbias; // if nx: the activations are norm(nx) (f32 rows of k, weight nw, bias nbias or null), formed by every CTA
+    const float *nx, *nw, *nbias; // if nx: the activations are norm(nx) (f32 rows of k <= kNormInMost, weight nw, bias nbias or null), formed by every CTA
     float neps;
     int nrms;                     // rms_norm (else layer_norm)
     // q4_mma_kernel on dense weights
