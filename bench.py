@@ -328,6 +328,23 @@ def run_profile_case(args):
         a = torch.randn(m, k, device="cuda", dtype=torch.float16)
         c = torch.zeros(m, n, device="cuda", dtype=torch.float16)
         fn, nsets = (lambda i: sg.matmul_q4(a, ws[i], c, m)), 3
+    elif name == "q4_rows8_bf16":
+        n, k = INTER, HIDDEN
+        q, s, _ = orc_quant(sg, (np.random.default_rng(8).standard_normal(n * k) * 0.02).astype(np.float32), 0, n, k)
+        ws = [sg.Q4Weights.new(q, s, n, k) for _ in range(6)]
+        a = torch.randn(8, k, device="cuda", dtype=torch.bfloat16)
+        c = torch.zeros(8, n, device="cuda", dtype=torch.bfloat16)
+        fn, nsets = (lambda i: sg.matmul_q4_bf16(a, ws[i], c, 8)), 6
+    elif name in ("attn_prefill", "attn_decode"):
+        rows = 512 if name == "attn_prefill" else 1          # over 1024 keys, 32 heads of 128 on 8 KV heads
+        caches = []
+        for _ in range(6):
+            cache = sg.KvCache(32, 8, 128, 1024)
+            cache.extend(torch.randn(1024, 1024, device="cuda").half(), torch.randn(1024, 1024, device="cuda").half())
+            caches.append(cache)
+        q = torch.randn(rows, 4096, device="cuda", dtype=torch.float16)
+        out = torch.zeros(rows, 4096, device="cuda")
+        fn, nsets = (lambda i: caches[i].attend_causal(q, rows, out)), 6
     else:
         fn, nsets, _ = kernel_cases(torch, sg, orc)[name]()
     for i in range(6):
@@ -738,7 +755,8 @@ def main():
     ap.add_argument("--collective", default="peer", choices=["peer", "nccl"],
                     help="N > 1: fused sum + finish over peer memory (this library's kernel) or NCCL all-reduce + finishing pass")
     ap.add_argument("--profile-case", default=None,
-                    choices=["q4_gemv", "q2_gemv", "q1_gemv", "q4_prefill", "q1_prefill", "mlp_gate_up", "mlp_down"],
+                    choices=["q4_gemv", "q2_gemv", "q1_gemv", "q4_prefill", "q1_prefill", "mlp_gate_up", "mlp_down", "q4_rows8_bf16",
+                             "attn_prefill", "attn_decode"],
                     help="run six plain launches of one kernel and exit (for profiler captures)")
     args = ap.parse_args()
     if args.profile_case:
