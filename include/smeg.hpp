@@ -689,7 +689,7 @@ public:
 };
 
 // y += down(act(x @ W_gate) * (x @ W_up)) -- Mlp::gated and Mlp::accumulate, src/mlp.rs:80-146, as one library call
-// (fused kernels above 64 rows, the one-wave decode kernels at a few rows).  x: m x k f16 bits, y: m x d f32.
+// (the gated product and the residual add in the products' stores).  x: m x k f16 bits, y: m x d f32.
 class Mlp {
     GatedLinear up_;
     Linear down_;

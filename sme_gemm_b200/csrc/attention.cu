@@ -24,8 +24,9 @@
 // warp 9 (MMA).  P goes back into the S columns it was read from (A operand in tensor memory), V is taken as it lies in the
 // cache ([key][depth]: an MN-major B operand).
 //
-// What bounds it: the exponentials -- about 14 instructions for each of a block's 16384 scores, ~1900 cycles per block on
-// the four schedulers against ~1500 cycles of tensor time.  A short prompt or a decode step has too few (tile, KV head)
+// What bounds it: the chain of hand-offs of one CTA per SM -- about 14 instructions for each of a block's 16384 scores are
+// ~1900 cycles per block on the four schedulers against ~1500 of tensor time, but a block takes ~4900: at 512 rows over 1024
+// keys the issue slots are 32 % busy, the tensor pipe 15 %, and waits for tensor-memory loads lead the stalls.  A short prompt or a decode step has too few (tile, KV head)
 // pairs for the machine: there a cluster of 2, 4 or 8 CTAs shares one tile's key blocks, each against the maximum of its own
 // range, and the parts meet over distributed shared memory (out = sum_c e^(m_c - m) O_c / sum_c e^(m_c - m) l_c, in rank
 // order).

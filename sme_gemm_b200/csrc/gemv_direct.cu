@@ -1,6 +1,7 @@
-// Decode GEMV for one to four activation rows, straight from global memory (sm_100a):
+// Decode GEMV for a few activation rows, straight from global memory (sm_100a):
 //   q4_direct_kernel      C[m][n] = ep( A[m][k] @ dequant(W) ), Q4 weights, f16, K-blocks of 32 and up, one or two rows
-//   lowbit_direct_kernel  2-bit / 1-bit weights against int8-quantised activations (matmul_q2 / matmul_q1)
+//                         of whole 16-byte words
+//   lowbit_direct_kernel  2-bit / 1-bit weights against int8-quantised activations (matmul_q2 / matmul_q1), one to four rows
 //
 // They replace the reference's SME GEMV kernels for the batch sizes a decode step has
 // (run_q4_gemv1 / run_q4_gemv, csrc/gemm_f16f16_q4.h:236-431; run_q2_gemv, csrc/gemm_q2.cc:300-404).

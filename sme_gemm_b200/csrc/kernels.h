@@ -51,7 +51,7 @@ struct Q4GemvArgs {
 // scratch the caller must provide in ws / counters).  Leaves sgrid = 0 otherwise.
 void q4_gemv_stream_plan(Q4GemvArgs& a, int bf16, int sm_count, size_t* ws_floats, size_t* ncounters);
 cudaError_t q4_gemv_launch(Q4GemvArgs a, int bf16, int sm_count, cudaStream_t stream);
-// One or two rows, f16, K-blocks of 32 and up: plain 128-bit loads, packed f16 multiply-adds (gemv_direct.cu).
+// One or two rows of whole 16-byte words, f16, K-blocks of 32 and up: 128-bit loads, packed f16 multiply-adds (gemv_direct.cu).
 bool q4_direct_supported(const Q4GemvArgs& a, int bf16);
 cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream);
 

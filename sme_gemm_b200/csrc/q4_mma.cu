@@ -13,10 +13,10 @@
 // f16 / bf16 integers (one lop3 per pair and a subtraction), the tensor core sums 32 depths in f32 and the block's f32
 // scale folds the sum into the total: no weight is rounded on the way, for bf16 either.
 //
-// What bounds it: instruction issue (about 60 per unit and column group) and the m16n8k16 rate of 32 cycles per scheduler.
-// Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 13.7 (2.4 TB/s), 16 rows
-// 67 -> 17; bf16 4096 x 4096 1 row 15.8 -> 5.6, 16 rows 28.5 -> 6.3; f16 8 rows 9.8 -> 4.6, 16 rows 14.0 -> 6.3; against
-// q4_direct_kernel at 4 rows 8.5 -> 5.0, at 2 rows 5.6 -> 6.3 (which therefore keeps one and two).
+// What bounds it: instruction issue (135 warp instructions a unit at eight bf16 rows, issue slots two thirds busy, the tensor
+// pipe a tenth).  Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 13.7 (2.4 TB/s),
+// 16 rows 67 -> 17.5; bf16 4096 x 4096 1 row 15.8 -> 4.9, 16 rows 28.5 -> 6.3; f16 8 rows 9.8 -> 4.6, 16 rows 14.0 -> 6.2; against
+// q4_direct_kernel, which keeps one and two rows (4.0 and 5.3), at 4 rows 8.5 -> 4.5.
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"

@@ -894,8 +894,9 @@ class GatedLinear:
 
 class Mlp:
     """y += down(act(up(x))) (Mlp::new) or y += down(act(x @ W_gate) * (x @ W_up)) (Mlp::gated); accumulate,
-    src/mlp.rs:67-146.  The gated Q4 form without biases or folded norms runs as one library call (fused kernels
-    above 64 rows); every other form runs its layers one after the other exactly as the reference's three-call path."""
+    src/mlp.rs:67-146.  The gated Q4 form without biases or folded norms runs as one library call (the gated product and
+    the residual add in the products' stores); every other form runs its layers one after the other exactly as the
+    reference's three-call path."""
 
     def __init__(self, up, down: Linear, act: "Gate | None" = None):
         gated = isinstance(up, GatedLinear)
