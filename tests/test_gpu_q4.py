@@ -347,11 +347,11 @@ def test_warp_level_kernel(m, n, k, block, bf16):
         assert (np.abs(got.reshape(m, n) - exact) <= 2.0 ** (-8 if bf16 else -11) * np.abs(exact) + 2.0 ** -25 + 2.0 ** -21 * room).all()
 
 
-@pytest.mark.parametrize("m", [3, 8, 16, 17, 40, 64])
-@pytest.mark.parametrize("d,f", [(256, 640), (1024, 3072)])
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 16, 17, 40, 64])
+@pytest.mark.parametrize("d,f", [(256, 640), (1024, 3072), (252, 672)])
 def test_gated_block_in_two_launches_is_its_separate_passes(m, d, f):
-    """The gated product and the residual add in the stores of the products, at every row count that fuses them: the bits of
-    product, gate pass, product, add."""
+    """The gated product and the residual add in the stores of the products, at every row count that fuses them, on whole and
+    on ragged rows: the bits of product, gate pass, product, add."""
     rng = np.random.default_rng(m + d)
     w = [(rng.standard_normal((f, d)) * 0.05).astype(np.float32) for _ in range(2)]
     up = sg.GatedLinear.quantize(w[0], w[1], sg.WeightLayout.OutIn, f, d, sg.Gate.Silu)
@@ -370,9 +370,11 @@ def test_gated_block_in_two_launches_is_its_separate_passes(m, d, f):
 
 
 @pytest.mark.parametrize("magnitude", [1e4, 1.0, 1e-4])
-@pytest.mark.parametrize("m,n,k,off", [(1, 130, 1027, 0), (1, 70, 96, 1), (2, 130, 1500, 0), (2, 2051, 1027, 1), (3, 130, 1500, 0)])
+@pytest.mark.parametrize("m,n,k,off", [(1, 130, 1027, 0), (1, 70, 96, 1), (2, 130, 1500, 0), (2, 2051, 1027, 1), (3, 130, 1500, 0),
+                                       (1, 9600, 66, 0), (2, 9700, 523, 0), (2, 9600, 258, 1), (2, 64, 8190, 0), (2, 40, 20001, 0)])
 def test_rows_off_the_16_byte_grid_keep_f32_sums(m, n, k, off, magnitude):
-    """Activations whose products leave f16's range on both sides: the product is the exact one to its store's rounding."""
+    """Activations whose products leave f16's range on both sides: the product is the exact one to its store's rounding.  Rows
+    that start on every boundary, passes of one and two column groups, depths whose rows are staged and too long for it."""
     rng = np.random.default_rng(m + n + k)
     q, s = q4_logical(rng, n, k, 32)
     w = sg.Q4Weights.with_params(q, s, None, n, k, sg.Q4Params(32))
