@@ -695,10 +695,11 @@ static bool q4_takes_direct(const smeg_q4* w, const uint16_t* a, size_t m, int b
     return q4_direct_supported(g, bf16);
 }
 
-// Can a call of m rows carry the fused stores of the MLP block (gated product, residual add) on a decode kernel?
+// Does q4_mma_kernel have the fused stores of the MLP block (gated product, residual add) for this matrix?
+static bool q4_mma_fuses(const smeg_q4* w, int glu) { return !w->affine && w->d.log2_block >= 5 && w->d.ku >= 1 && !(glu && w->d.n % 64 != 0); }
+// Can a call of m rows carry them on a decode kernel?
 static bool q4_fuses_decode(const smeg_q4* w, const uint16_t* a, size_t m, int bf16, int glu) {
-    if (q4_takes_direct(w, a, m, bf16, glu)) return true;
-    return !w->affine && !q4_rows_want_tc(w, m) && w->d.log2_block >= 5 && w->d.ku >= 1 && !(glu && w->d.n % 64 != 0);
+    return q4_takes_direct(w, a, m, bf16, glu) || (!q4_rows_want_tc(w, m) && q4_mma_fuses(w, glu));
 }
 
 // A whose rows TMA and the 16-byte copies cannot take (k no multiple of 8, or a base off a 16-byte boundary) in a zero-padded
@@ -741,7 +742,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     // A by TMA or in 16-byte pieces and takes a padded copy, a pass of ~2 us and a trip to the allocator (5001 x 4097 bf16, us:
     // reading A by halves 8 rows 33, 40 rows 285, with the copy 9.4 and 21).
     // None of them needs the workspace: K-blocks below 32 stay off the streaming form, and where the GEMM would split the depth
-    // inside a capture that finds no workspace they run on the kernel for few rows.
+    // (of aligned rows too) inside a capture that finds no workspace, the kernel for few rows takes the call.
     uint16_t* a_pad = nullptr;
     size_t k = k0;
     const bool direct = q4_takes_direct(w, a, m, bf16, glu), ragged = k0 != 0 && (k0 % 8 != 0 || ((uintptr_t)a & 15) != 0);
@@ -789,7 +790,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         gemm_tc_plan(t, ds->sm_count, &grid, &smem, &ws_floats, &ncounters);
         TcScratch sc;
         if (ws_floats && tc_scratch(stream, ws_floats, ncounters, &sc)) {
-            if (!ragged || push || glu || yacc) {
+            if (push || ((glu || yacc) && !q4_mma_fuses(w, glu))) {
                 if (ext) cudaFreeAsync(ext, stream);
                 if (a_pad) cudaFreeAsync(a_pad, stream);
                 return -2;

@@ -14,7 +14,7 @@ import torch
 
 import oracle as orc
 import sme_gemm_b200 as sg
-from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, half_tol, max_rel, q4_logical
+from gpu_util import bf16_bits_dev, bits_of, f16_bits_dev, half_tol, max_rel, q4_logical, takes_gemm
 from refgen import Lcg
 
 pytestmark = pytest.mark.gpu
@@ -414,4 +414,47 @@ def test_rows_off_the_16_byte_grid_in_a_capture_without_a_warm_call(m, block, k,
     assert max_rel(c.float().cpu().numpy(), want.float().cpu().numpy()) <= TOL and sg.last_status() == 0
     a64, wt = a.cpu().numpy().astype(np.float64).reshape(m, k), q4_exact(q, s, n, k, block)
     assert max_rel(c.float().cpu().numpy(), a64 @ wt) <= half_tol(1e-2, k)
+    del graph
+
+
+@pytest.mark.parametrize("form", ["f16", "bf16", "bias", "accumulate", "gated"])
+def test_tensor_core_calls_in_a_capture_without_a_warm_call(form):
+    """Rows and matrices on which the tensor-core GEMM splits the depth: the first such call on a stream may be inside a
+    capture, where its workspace cannot be allocated, and runs on the kernel for few rows there."""
+    m, n, k, block = 40, 4096, 4096, 32
+    rng = np.random.default_rng(51)
+    q, s = q4_logical(rng, n, k, block, from_f32=False)
+    w = sg.Q4Weights.with_params(q, s, None, n, k, sg.Q4Params(block))
+    assert takes_gemm(m, n, k, form == "bf16")
+    dtype = torch.bfloat16 if form == "bf16" else torch.float16
+    a = torch.from_numpy((rng.standard_normal((m, k)) * 0.1).astype(np.float32)).cuda().to(dtype)
+    ep = sg.Epilogue("f16").add_col(torch.from_numpy(rng.standard_normal(n).astype(np.float16)).cuda())
+    if form == "gated":
+        wg, wu, wd = ((rng.standard_normal(n // 2 * k) * 0.02).astype(np.float32) for _ in range(3))
+        mlp = sg.Mlp.gated(sg.GatedLinear.quantize(wg, wu, sg.WeightLayout.OutIn, n // 2, k, sg.Gate.Silu),
+                           sg.Linear.quantize(wd, sg.WeightLayout.OutIn, n, n // 2))
+
+    def call(c):
+        if form == "f16":
+            sg.matmul_q4(a, w, c, m)
+        elif form == "bf16":
+            sg.matmul_q4_bf16(a, w, c, m)
+        elif form == "bias":
+            sg.matmul_q4_ep(a, w, c, m, ep)
+        elif form == "accumulate":
+            sg.Linear.from_q4(w).accumulate(a, c, m)
+        else:
+            mlp.accumulate(a, c, m)
+
+    f32 = form in ("accumulate", "gated")
+    got, want = (torch.ones((m, n), dtype=torch.float32 if f32 else dtype, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream(priority=-1)):
+        call(got)
+    graph.replay()
+    torch.cuda.synchronize()
+    call(want)
+    torch.cuda.synchronize()
+    assert max_rel(got.float().cpu().numpy(), want.float().cpu().numpy()) <= TOL and sg.last_status() == 0
     del graph
