@@ -118,6 +118,9 @@ struct TcScratch {
     size_t ncounters = 0;
 };
 std::map<std::pair<int, cudaStream_t>, TcScratch> g_tc_scratch;
+// Held from the launch of a depth-split GEMM to that of the pass that adds its slices: both use the stream's block, so another
+// host thread's call on the stream must not come between them (its GEMM would overwrite the slices before they are added).
+std::mutex g_split_mu;
 std::vector<void*> g_retired;        // outgrown blocks, never freed
 
 int tc_scratch(cudaStream_t stream, size_t floats, size_t ncounters, TcScratch* out) {
@@ -801,6 +804,8 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         t.counters = sc.counters;
     }
     if (tc) {
+        std::unique_lock<std::mutex> both(g_split_mu, std::defer_lock);
+        if (t.ws) both.lock();
         e = gemm_tc_launch(t, bf16, grid, smem, stream);
     } else if (direct) {
         g.glu = glu; g.yacc = yacc;
@@ -1128,7 +1133,10 @@ int smeg_gemm_dense_dev(const smeg_dense* w, const uint16_t* a, uint16_t* c, siz
     }
     t.ws = sc.ws;
     t.counters = sc.counters;
+    std::unique_lock<std::mutex> both(g_split_mu, std::defer_lock);
+    if (t.ws) both.lock();
     cudaError_t e = gemm_tc_launch(t, w->bf16, grid, smem, stream);
+    if (both.owns_lock()) both.unlock();
     if (ext) cudaFreeAsync(ext, stream);
     if (a_pad) cudaFreeAsync(a_pad, stream);
     return e == cudaSuccess ? 0 : -6;

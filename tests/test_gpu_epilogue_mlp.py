@@ -338,3 +338,38 @@ def test_concurrent_host_threads_on_shapes_that_grow_the_scratch():
         t.join()
     assert not errors, errors[:5]
     assert sg.last_status() == 0
+
+
+def test_depth_split_calls_of_host_threads_do_not_mix_their_slices():
+    """Two host threads on one stream, each a GEMM whose depth slices a second launch adds up out of the stream's block: no
+    launch of the other thread comes between the two."""
+    import threading
+    rng = np.random.default_rng(78)
+    cases = []
+    for (m, n, k) in ((33, 4096, 4096), (70, 2048, 4096)):
+        assert takes_gemm(m, n, k)
+        q, s = q4_logical(rng, n, k, 32, from_f32=False)
+        w = sg.Q4Weights.new(q, s, n, k)
+        a = f16_bits_dev(orc.f32_to_f16_bits(rng.standard_normal((m, k)).astype(np.float32)))
+        c = torch.zeros((m, n), dtype=torch.float16, device="cuda")
+        sg.matmul_q4(a, w, c, m)
+        cases.append((m, w, a, c))
+    torch.cuda.synchronize()
+    wrong = [0, 0]
+
+    def worker(i):
+        torch.cuda.set_device(0)
+        m, w, a, want = cases[i]
+        out = [torch.zeros((m, w.n()), dtype=torch.float16, device="cuda") for _ in range(64)]
+        for _ in range(10):
+            for c in out:
+                sg.matmul_q4(a, w, c, m)
+            torch.cuda.synchronize()
+            wrong[i] += sum(not torch.equal(c.view(torch.int16), want.view(torch.int16)) for c in out)
+
+    threads = [threading.Thread(target=worker, args=(i,)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert wrong == [0, 0] and sg.last_status() == 0
