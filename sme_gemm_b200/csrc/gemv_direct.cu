@@ -1,6 +1,7 @@
 // Decode GEMV for a few activation rows, straight from global memory (sm_100a):
-//   q4_direct_kernel      C[m][n] = ep( A[m][k] @ dequant(W) ), Q4 weights, f16, K-blocks of 32 and up, one or two rows
-//                         of whole 16-byte words
+//   q4_stage_kernel       C[m][n] = ep( A[m][k] @ dequant(W) ), Q4 weights, f16, K-blocks of 32 and up, one or two rows
+//                         of whole 16-byte words, on warp-level tensor-core instructions
+//   q4_direct_kernel      the same in packed f16 arithmetic, for depths below 1793, and the form that norms its rows
 //   lowbit_direct_kernel  2-bit / 1-bit weights against int8-quantised activations (matmul_q2 / matmul_q1), one to four rows
 //
 // They replace the reference's SME GEMV kernels for the batch sizes a decode step has
@@ -17,7 +18,7 @@
 //     copied itself, so cp.async.wait_group is all the synchronisation the ring needs;
 //   * one CTA owns whole column groups over the whole depth, its eight warps split the depth, so
 //     a column's result never depends on the grid and nothing crosses CTAs;
-//   * Q4: nibbles become exact f16 integers with one lop3 per pair, and are multiplied into
+//   * Q4, q4_direct_kernel: nibbles become exact f16 integers with one lop3 per pair, and are multiplied into
 //     packed f16 sums over 8 depths (HFMA2, as the reference's SME kernel accumulates a K-block
 //     in f16, csrc/gemm_f16f16_q4.h:236-341); every 32 depths the pair sums are widened and folded into
 //     the f32 total with the block's scale.  Against the f32-accumulating oracle this differs by
@@ -123,6 +124,48 @@ __device__ __noinline__ void stage_norm_row(uint16_t* dst, const float* xr, cons
     for (int i = 0; i < KEEP; ++i)
         if (tid + i * kDThreads < dim) put(tid + i * kDThreads, x[i]);
     for (int j = dim + tid; j < kpad; j += kDThreads) dst[j] = 0;
+}
+
+// The warps' shares [8][cpc][M][16] in warp order, epilogue, store: `share` column groups (gated form: pairs of them) from `first`.
+template <int M>
+__device__ __forceinline__ void q4_store_cells(const Q4GemvArgs& p, const float* red, int CPC, int first, int share, int ncg) {
+    const int tid = threadIdx.x;
+    if (p.glu) {
+        // a hidden unit's gate and up sums lie in neighbouring local groups: out = f16(act(f16(gate)) * f16(up)), the
+        // arithmetic of the separate gate pass (glu, src/linear.rs:804-835) on the rounded projections
+        const int hn = p.n >> 1;
+        for (int o = tid; o < share * M * 16; o += kDThreads) {
+            const int col16 = o & 15, r = (o >> 4) % M, ul = o / (16 * M);
+            float ag = 0.0f, au = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kDWarps; ++w) {
+                ag += red[(((size_t)w * CPC + 2 * ul) * M + r) * 16 + col16];
+                au += red[(((size_t)w * CPC + 2 * ul + 1) * M + r) * 16 + col16];
+            }
+            const float gv = __half2float(__float2half_rn(ag)), uv = __half2float(__float2half_rn(au));
+            const int hcol = (first + ul) * 16 + col16;
+            if (hcol < hn) p.c[(size_t)r * hn + hcol] = __half_as_ushort(__float2half_rn(__fmul_rn(glu_gate((uint32_t)p.glu, gv), uv)));
+        }
+        return;
+    }
+    for (int o = tid; o < ncg * M * 16; o += kDThreads) {
+        const int col16 = o & 15, r = (o >> 4) % M, c = o / (16 * M);
+        float acc = 0.0f;
+#pragma unroll
+        for (int w = 0; w < kDWarps; ++w) acc += red[(((size_t)w * CPC + c) * M + r) * 16 + col16];
+        const int col = (first + c) * 16 + col16;
+        if (col < p.n) {
+            if (p.c32) p.c32[(size_t)r * p.n + col] = acc;
+            else if (p.yacc) p.yacc[(size_t)r * p.n + col] = __fadd_rn(p.yacc[(size_t)r * p.n + col], __half2float(__float2half_rn(acc)));
+            else if (p.kc && col >= p.q_len) {
+                const int kv = col - p.q_len;
+                const uint16_t v = __half_as_ushort(__float2half_rn(acc));
+                if (kv < p.kv_len) p.kc[(size_t)r * p.kv_len + kv] = v;
+                else p.vc[(size_t)r * p.kv_len + kv - p.kv_len] = v;
+            }
+            else p.c[(size_t)r * p.n + col] = ep_store_value<0>(p.ep, acc, (size_t)r, (size_t)col);
+        }
+    }
 }
 
 // GEN: the activations may be the norm of f32 rows (p.nx).
@@ -250,43 +293,292 @@ __global__ void __launch_bounds__(kDThreads, 3) q4_direct_kernel(const __grid_co
         for (int o = lane; o < ncg * M * 16; o += 32) red[(size_t)warp * CPC * M * 16 + o] = 0.0f;
     }
     __syncthreads();
-    // ---- the warps' shares in warp order, epilogue, store ----
-    if (p.glu) {
-        // a hidden unit's gate and up sums lie in neighbouring local groups: out = f16(act(f16(gate)) * f16(up)), the
-        // arithmetic of the separate gate pass (glu, src/linear.rs:804-835) on the rounded projections
-        const int hn = p.n >> 1;
-        for (int o = tid; o < share * M * 16; o += kDThreads) {
-            const int col16 = o & 15, r = (o >> 4) % M, ul = o / (16 * M);
-            float ag = 0.0f, au = 0.0f;
-#pragma unroll
-            for (int w = 0; w < kDWarps; ++w) {
-                ag += red[(((size_t)w * CPC + 2 * ul) * M + r) * 16 + col16];
-                au += red[(((size_t)w * CPC + 2 * ul + 1) * M + r) * 16 + col16];
-            }
-            const float gv = __half2float(__float2half_rn(ag)), uv = __half2float(__float2half_rn(au));
-            const int hcol = (first + ul) * 16 + col16;
-            if (hcol < hn) p.c[(size_t)r * hn + hcol] = __half_as_ushort(__float2half_rn(__fmul_rn(glu_gate((uint32_t)p.glu, gv), uv)));
-        }
-        return;
-    }
-    for (int o = tid; o < ncg * M * 16; o += kDThreads) {
+    q4_store_cells<M>(p, red, CPC, first, share, ncg);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Q4, f16, M rows (1 or 2), K-blocks >= 32, on warp-level tensor-core instructions: depths of eight stages and more.
+//
+// What q4_direct_kernel spends is instructions: 128 a unit of 1024 weights, of them 36 to make signed numbers of the codes, 32
+// packed multiply-adds, 16 to widen and fold two K-blocks; 66 MB of a gate/up matrix were bound by them at 3.3 TB/s.  Here
+//   * a code is not converted at all: four bits where they lie in a half word are the f16 subnormal u 2^-24 or u 2^-20 (u = code + 8),
+//     one AND a pair; the products are exact in f32 and 8 sum(a) comes off through the accumulators' start values;
+//   * mma.m16n8k16 has room for eight columns where there is one row, so the columns stand for K-blocks: a stage is four units,
+//     lane (g, t) takes vectors of unit t, B is zero but where its column's K-block meets its depths, and after sixteen MMAs
+//     the accumulators are the sums of eight K-blocks, folded at once (12 instructions instead of 128);
+//   * the copies are coalesced a unit at a time and read back across the lanes, under an XOR of the unit's number.
+// 67 warp instructions a unit (us, graph replays; q4_direct_kernel / this): 1 row, 28672 x 4096 18.2 / 13.0 (5.1 TB/s), 4096 x 14336
+// 11.6 / 8.3, 4096 x 4096 3.95 / 3.35; 2 rows, 14336 x 4096 14.1 / 11.7.  From 14336 to 28672 columns it adds 33 MB in 5.4 us, 6.0 TB/s:
+// what is left is the time to the first byte and the last wave's end.  Sums are f32 throughout (q4_direct_kernel: f16 over 8 depths).
+// Shared memory: ring [8 warps][PF] of a stage's codes and scale words | A rows [M][units * 72] f16 (a unit's 64 depths
+// and 8 halves of padding) | the blocks' start values [stages][8 M] f32 | the cross-warp exchange [8 warps][CPC][M][16] f32.
+// ---------------------------------------------------------------------------------------------
+// Zeros where `bytes` is 0 (nothing is read then).
+__device__ __forceinline__ void cp_async16z(uint32_t dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async4z(uint32_t dst, const void* src, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async16s(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4s(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+    return v;
+}
+// D (16 weight columns x 8, f32) += A (16 x 16 f16) * B (16 x 8 f16)
+__device__ __forceinline__ void mma_f16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+constexpr int kQ4StageUnits = 4;                                   // 256 depths
+constexpr int kQ4AUnit = 72;                                       // halves from one unit of an activation row to the next
+__host__ __device__ constexpr int q4_slot_bytes(int m) { return kQ4StageUnits * 512 + 256 * m; }
+__host__ __device__ constexpr int q4_stages(int k64) { return (k64 + kQ4StageUnits - 1) / kQ4StageUnits; }
+__host__ __device__ constexpr size_t q4_rows_bytes(int m, int stages) { return (size_t)m * stages * (kQ4StageUnits * kQ4AUnit * 2 + 32); }
+// Where depth d lies in a staged row: the second and third pair of each run of eight change places, so that the pairs of one
+// MMA's B operand are neighbours.
+__device__ __forceinline__ int q4_a_index(int d) { return (d >> 6) * kQ4AUnit + (d & 57) + ((d & 2) << 1) + ((d & 4) >> 1); }
+
+// Rows with an infinity or a NaN among their activations, again: the kernel's sums would carry them to columns whose code
+// there is zero or make a NaN of them (it multiplies code + 8 and takes 8 times the row's sum off).  A thread a column, code
+// by code; f32 sums of a K-block, folded with its scale.
+template <int M>
+__device__ __noinline__ void q4_exact_cells(const Q4GemvArgs& p, const uint16_t* As, int a_stride, float* red, int cpc, int ncg, int first) {
+    for (int o = threadIdx.x; o < ncg * M * 16; o += kDThreads) {
         const int col16 = o & 15, r = (o >> 4) % M, c = o / (16 * M);
-        float acc = 0.0f;
-#pragma unroll
-        for (int w = 0; w < kDWarps; ++w) acc += red[(((size_t)w * CPC + c) * M + r) * 16 + col16];
-        const int col = (first + c) * 16 + col16;
-        if (col < p.n) {
-            if (p.c32) p.c32[(size_t)r * p.n + col] = acc;
-            else if (p.yacc) p.yacc[(size_t)r * p.n + col] = __fadd_rn(p.yacc[(size_t)r * p.n + col], __half2float(__float2half_rn(acc)));
-            else if (p.kc && col >= p.q_len) {
-                const int kv = col - p.q_len;
-                const uint16_t v = __half_as_ushort(__float2half_rn(acc));
-                if (kv < p.kv_len) p.kc[(size_t)r * p.kv_len + kv] = v;
-                else p.vc[(size_t)r * p.kv_len + kv - p.kv_len] = v;
+        const int u0 = first + (c >> 1);
+        const int cg = p.glu ? 4 * (u0 >> 1) + (u0 & 1) + 2 * (c & 1) : first + c;
+        float tot = 0.0f;
+        for (int d0 = 0; d0 < p.k64 * 64; d0 += 32) {
+            float part = 0.0f;
+            for (int d = d0; d < d0 + 32; ++d) {
+                size_t at;
+                int nib;
+                q4_locate((size_t)d, (size_t)cg * 16 + col16, (size_t)p.k64, &at, &nib);
+                const int code = (int)((*reinterpret_cast<const uint32_t*>(p.codes + at) >> (4 * nib)) & 15u) - 8;
+                if (d < p.k) part = fmaf((float)code, __half2float(__ushort_as_half(As[(size_t)r * a_stride + q4_a_index(d)])), part);
             }
-            else p.c[(size_t)r * p.n + col] = ep_store_value<0>(p.ep, acc, (size_t)r, (size_t)col);
+            const uint16_t s = p.scales[q4_scale_row((size_t)cg, (size_t)(d0 >> p.log2_block), p.nb) + scale_slot(col16)];
+            if (d0 < p.k) tot = fmaf(part, __half2float(__ushort_as_half(s)), tot);
+        }
+        for (int w = 0; w < kDWarps; ++w) red[((size_t)w * cpc + c) * M * 16 + r * 16 + col16] = w ? 0.0f : tot;
+    }
+}
+
+// PF: ring slots per warp, a stage in work and the others on their way.
+template <int M, int PF>
+__global__ void __launch_bounds__(kDThreads, PF > 3 ? 2 : 3) q4_stage_kernel(const __grid_constant__ Q4GemvArgs p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int SLOT = q4_slot_bytes(M), NC = M;              // NC accumulator pairs
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int ns = q4_stages(p.k64), a_stride = ns * kQ4StageUnits * kQ4AUnit;
+    const uint32_t ring = smem_u32(smem_raw) + (uint32_t)(warp * PF * SLOT);
+    uint16_t* As = reinterpret_cast<uint16_t*>(smem_raw + (size_t)kDWarps * PF * SLOT);
+    float* start = reinterpret_cast<float*>(As + (size_t)M * a_stride);     // [stage][8 M]
+    float* red = start + (size_t)ns * 8 * M;
+    const int CPC = p.cg;                                          // most column groups a CTA takes
+    // this CTA's column groups: an equal share of all of them
+    // (gated form: the share is counted in pairs of a gate group 4q + e and its up group 4q + 2 + e, e = 0, 1 -- the
+    // matrix interleaves 32 gate and 32 up columns -- and the CTA walks gate, up, gate, up, ...)
+    const int first = (int)blockIdx.x * p.dq + min((int)blockIdx.x, p.dr);
+    const int share = p.dq + ((int)blockIdx.x < p.dr ? 1 : 0);
+    const int ncg = p.glu ? 2 * share : share;
+    auto group_of = [&](int c) -> int {
+        if (!p.glu) return first + c;
+        const int u = first + (c >> 1);
+        return 4 * (u >> 1) + (u & 1) + 2 * (c & 1);
+    };
+    // the eight warps split the depth: by the depth alone, so that a column's sum does not depend on the call's form
+    const int s_begin = (warp * ns) >> 3, s_end = ((warp + 1) * ns) >> 3, mine = s_end - s_begin;
+    const int total = ncg * mine;                                  // stages this warp walks
+
+    // K-blocks (of the stage's eight) whose scales this lane folds: see below
+    const int blk_a = M == 1 ? 4 * (t & 1) + (t >> 1) : 4 * (t & 1);
+    // load cursor
+    int ls = s_begin, lc = 0;
+    const unsigned char* lp = p.codes;
+    const unsigned char* lsc = p.codes;
+    const uint32_t cg_codes = (uint32_t)p.k64 * kUnitBytes, cg_scales = (uint32_t)p.nb * 32, sc_shift = (uint32_t)p.log2_block - 5;
+    auto load_from = [&](int c) {
+        const uint32_t cg = (uint32_t)group_of(c);
+        lp = p.codes + (uint64_t)cg * cg_codes + (uint32_t)(s_begin * kQ4StageUnits * kUnitBytes + lane * 16);
+        lsc = reinterpret_cast<const unsigned char*>(p.scales) + (uint64_t)cg * cg_scales + (uint32_t)(4 * g);
+    };
+    const uint32_t wr = (uint32_t)(g * 64), wx = (uint32_t)(t << 4);
+    auto issue = [&](uint32_t sb) {
+        const uint32_t ss = sb + kQ4StageUnits * 512 + (uint32_t)(lane * 8 * M), sw = sb + wr;
+        const uint32_t blk = (uint32_t)(ls * 8 + blk_a);           // counted in 32 depths
+        if (ls * kQ4StageUnits + kQ4StageUnits <= p.k64) {
+#pragma unroll
+            for (int j = 0; j < kQ4StageUnits; ++j) cp_async16s(sw + (wx ^ (uint32_t)(j << 4)) + j * 512, lp + j * kUnitBytes);
+#pragma unroll
+            for (int e = 0; e < 2 * M; ++e) cp_async4s(ss + 4 * e, lsc + (((blk + (M == 1 ? 2 : 1) * e) >> sc_shift) << 5));
+        } else {                                                   // the last stage of a depth that is no whole number of them: zeros
+            const int left = p.k64 - ls * kQ4StageUnits;
+#pragma unroll
+            for (int j = 0; j < kQ4StageUnits; ++j)
+                cp_async16z(sw + (wx ^ (uint32_t)(j << 4)) + j * 512, j < left ? lp + j * kUnitBytes : lp, j < left ? 16u : 0u);
+#pragma unroll
+            for (int e = 0; e < 2 * M; ++e) {
+                const uint32_t be = blk + (M == 1 ? 2 : 1) * e;
+                const bool in = be < (uint32_t)p.k64 * 2;
+                cp_async4z(ss + 4 * e, in ? lsc + ((be >> sc_shift) << 5) : lsc, in ? 4u : 0u);
+            }
+        }
+        lp += kQ4StageUnits * kUnitBytes;
+        if (++ls == s_end) {
+            ls = s_begin;
+            if (++lc < ncg) load_from(lc);
+        }
+    };
+    if (total) load_from(0);
+#pragma unroll
+    for (int i = 0; i < PF - 1; ++i) {
+        if (i < total) issue(ring + (uint32_t)(i * SLOT));
+        cp_async_commit();
+    }
+    pdl_launch_dependents();
+    pdl_wait();                                                    // the activations may come from the kernel ahead
+
+    // ---- stage the activation rows (zero past k), a warp a stage of 256 depths, and the blocks' start values: what the
+    // products with code + 8 have too much, -8 sum(a) 2^-24 ----
+    int bad = 0;
+#pragma unroll
+    for (int r = 0; r < M; ++r)
+        for (int st0 = warp; st0 < ns; st0 += kDWarps * 4) {       // four loads on their way
+            uint4 v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int st = st0 + e * kDWarps, d = st * 256 + lane * 8;
+                v[e] = make_uint4(0, 0, 0, 0);
+                if (st < ns && d < p.k) v[e] = *reinterpret_cast<const uint4*>(p.a + (size_t)r * p.k + d);        // (k is a multiple of 8)
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int st = st0 + e * kDWarps, d = st * 256 + lane * 8;
+                if (st >= ns) break;                               // (the same in all lanes)
+                *reinterpret_cast<uint4*>(As + (size_t)r * a_stride + q4_a_index(d)) = make_uint4(v[e].x, v[e].z, v[e].y, v[e].w);
+                const float2 f0 = __half22float2(as_h2(v[e].x)), f1 = __half22float2(as_h2(v[e].y)), f2 = __half22float2(as_h2(v[e].z)), f3 = __half22float2(as_h2(v[e].w));
+                float sum = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                bad |= !(fabsf(sum) <= 3.0e38f);                   // 32 finite f16 values sum to 2.1e6 at most
+                // block 2 tb + h of the stage is column h * 4 + tb of the products (one row), r * 4 + tb of those of half h (two)
+                const int tb = lane >> 3, h = (lane >> 2) & 1;
+                if (t == 0) start[(size_t)st * 8 * M + (M == 1 ? h * 4 + tb : h * 8 + r * 4 + tb)] = sum * -4.76837158203125e-07f;
+            }
+        }
+    bad = __syncthreads_or(bad);
+
+    // ---- the products ----
+    // Lane (g, t) multiplies the codes of unit t of the stage (of the lanes (g, 0..3) of that unit in turn), so the depths of
+    // an MMA are those of four units, and column n of its B operand is zero but for the unit (and half, or row) n stands for:
+    // an accumulator's column is one K-block's sum, and eight blocks are folded at once.
+    const uint32_t a_base = smem_u32(As) + (uint32_t)(((M == 1 ? t * kQ4AUnit + (g >> 2) * 32 : (g >> 2) * a_stride + t * kQ4AUnit)) * 2);
+    const bool on0 = (g & 3) == t && (M == 2 || g < 4), on1 = (g & 3) == t && (M == 2 || g >= 4);
+    const uint32_t s_base = smem_u32(start) + (uint32_t)(8 * t);
+    uint32_t rd[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) rd[i] = (uint32_t)(t * 512 + g * 64) + (wx ^ (uint32_t)(i << 4));
+    uint4 b0[2], b1[2];                                            // (zero in the lanes that never load them)
+    b0[0] = b0[1] = b1[0] = b1[1] = make_uint4(0, 0, 0, 0);
+    float tot0 = 0.0f, tot1 = 0.0f;
+    int cc = 0, cs = s_begin;                                     // compute cursor
+    const uint32_t ring_end = ring + PF * SLOT;
+    uint32_t sb = ring, fill = ring_end - SLOT;                    // the slot in work and the one before it
+    uint32_t aa = a_base + (uint32_t)(s_begin * kQ4StageUnits * kQ4AUnit * 2), sa = s_base + (uint32_t)(s_begin * M * 32);
+    for (int j = 0; j < total; ++j) {
+        cp_async_wait<PF - 2>();
+        __syncwarp();                                              // every lane's copies of the stage have landed, and the slot before is read
+        if (j + PF - 1 < total) issue(fill);
+        cp_async_commit();
+        float lo[NC][4], hi[NC][4];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const uint2 s = lds64(sa + (uint32_t)(c * 32));
+            lo[c][0] = lo[c][2] = __uint_as_float(s.x);
+            lo[c][1] = lo[c][3] = __uint_as_float(s.y);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) hi[c][q] = 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint4 wv = lds128(sb + rd[i]);
+            if (on0) b0[i & 1] = lds128(aa + 16 * i);
+            if (on1) b1[i & 1] = lds128(aa + (M == 1 ? 0 : 64) + 16 * i);
+            // a nibble where it lies is the f16 subnormal u 2^-24 (low ones) or u 2^-20
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t w0 = h ? wv.z : wv.x, w1 = h ? wv.w : wv.y, v0 = w0 >> 8, v1 = w1 >> 8;
+                const uint4& b = h ? b1[i & 1] : b0[i & 1];
+                const int c = M == 1 ? 0 : h;
+                mma_f16(lo[c], w0 & 0x000f000fu, v0 & 0x000f000fu, w1 & 0x000f000fu, v1 & 0x000f000fu, b.x, b.y);
+                mma_f16(hi[c], w0 & 0x00f000f0u, v0 & 0x00f000f0u, w1 & 0x00f000f0u, v1 & 0x00f000f0u, b.z, b.w);
+            }
+        }
+        uint32_t sw[2 * M];
+        const uint32_t ss = sb + kQ4StageUnits * 512 + (uint32_t)(lane * 8 * M);
+        if (M == 1) {
+            const uint2 v = lds64(ss);
+            sw[0] = v.x; sw[1] = v.y;
+        } else {
+            const uint4 v = lds128(ss);
+            sw[0] = v.x; sw[2 * M - 2] = v.z; sw[1] = v.y; sw[2 * M - 1] = v.w;
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            // columns 2t, 2t + 1 of the products: blocks blk_a and blk_a + 2 (one row); of half c: blk_a + c and blk_a + 2 + c (two)
+            const float2 fa = __half22float2(as_h2(M == 1 ? sw[0] : sw[c])), fc = __half22float2(as_h2(M == 1 ? sw[1] : sw[(2 + c) % (2 * M)]));
+            tot0 = fmaf(fmaf(hi[c][0], 0.0625f, lo[c][0]), fa.x, tot0);
+            tot1 = fmaf(fmaf(hi[c][2], 0.0625f, lo[c][2]), fa.y, tot1);
+            tot0 = fmaf(fmaf(hi[c][1], 0.0625f, lo[c][1]), fc.x, tot0);
+            tot1 = fmaf(fmaf(hi[c][3], 0.0625f, lo[c][3]), fc.y, tot1);
+        }
+        fill = sb;
+        sb = sb + SLOT == ring_end ? ring : sb + SLOT;
+        aa += kQ4StageUnits * kQ4AUnit * 2;
+        sa += M * 32;
+        if (++cs == s_end) {
+            // end of this warp's share of a column group: the lanes of a column (and row) hold different blocks
+            tot0 += __shfl_xor_sync(0xffffffffu, tot0, 1);
+            tot1 += __shfl_xor_sync(0xffffffffu, tot1, 1);
+            if (M == 1) {
+                tot0 += __shfl_xor_sync(0xffffffffu, tot0, 2);
+                tot1 += __shfl_xor_sync(0xffffffffu, tot1, 2);
+            }
+            if ((t & (M == 1 ? 3 : 1)) == 0) {
+                float* to = red + ((warp * CPC + cc) * M + (M == 1 ? 0 : t >> 1)) * 16;
+                to[g] = tot0 * 16777216.0f;
+                to[g + 8] = tot1 * 16777216.0f;
+            }
+            tot0 = tot1 = 0.0f;
+            aa -= (uint32_t)(mine * kQ4StageUnits * kQ4AUnit * 2);
+            sa -= (uint32_t)(mine * M * 32);
+            cs = s_begin;
+            ++cc;
         }
     }
+    cp_async_wait<0>();
+    __syncthreads();
+    if (bad) {
+        q4_exact_cells<M>(p, As, a_stride, red, CPC, ncg, first);
+        __syncthreads();
+    }
+    q4_store_cells<M>(p, red, CPC, first, share, ncg);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -571,7 +863,7 @@ bool q4_direct_supported(const Q4GemvArgs& a, int bf16) {
 }
 
 cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream) {
-    const int n16 = (a.n + 15) / 16;
+    const int n16 = (a.n + 15) / 16, ns = q4_stages(a.k64);
     a.n16 = n16;
     // three CTAs per SM when the matrix gives every SM that many, else two (and then never three on one SM
     // while another has one: the shared-memory request is padded past a third of an SM's)
@@ -588,6 +880,24 @@ cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream) {
         grid_x = direct_grid(n16, sm_count, 16, &a.cg, per_sm);
         a.dq = n16 / grid_x; a.dr = n16 % grid_x;
     }
+    cudaError_t e;
+    if (ns >= kDWarps && !a.nx) {
+        // At least a stage of 256 depths for each warp.  (Shorter depths stay with the kernel below, whose warps have a unit each
+        // where a stage would have one warp in work: us, this / that, 1 row: 1536 x 384 2.06 / 1.72, 4096 x 1024 2.40 / 2.06,
+        // 3072 x 2048 2.57 / 2.58, 1024 x 4096 2.7 / 3.2.)
+        // Ring: three slots where three CTAs share an SM; of two, each takes what its rows leave of half an SM, up to five.
+        const size_t slot = (size_t)kDWarps * q4_slot_bytes(a.m), rest = q4_rows_bytes(a.m, ns) + (size_t)kDWarps * a.cg * a.m * 16 * sizeof(float);
+        const int pf = per_sm > 2 ? 3 : 5 * slot + rest <= 112 * 1024 ? 5 : 4 * slot + rest <= 112 * 1024 ? 4 : 3;
+        size_t bytes = pf * slot + rest;
+        if (per_sm == 2 && bytes < 80 * 1024) bytes = 80 * 1024;
+#define SMEG_QS(MM, PP)                                                               \
+    if (a.m == MM && pf == PP) {                                                      \
+        e = opt_in_smem(q4_stage_kernel<MM, PP>, bytes);                              \
+        return e != cudaSuccess ? e : launch_pdl(q4_stage_kernel<MM, PP>, dim3(grid_x), dim3(kDThreads), bytes, stream, a); \
+    }
+        SMEG_QS(1, 3) SMEG_QS(1, 4) SMEG_QS(1, 5) SMEG_QS(2, 3) SMEG_QS(2, 4) SMEG_QS(2, 5)
+#undef SMEG_QS
+    }
     a.dupw = (a.k64 + kDWarps - 1) / kDWarps;
     size_t smem = kQ4RingBytes + (size_t)a.m * ((size_t)a.k64 * 64 + 8) * 2 + (size_t)kDWarps * a.cg * a.m * 16 * sizeof(float);
     if (per_sm == 2 && smem < 80 * 1024) smem = 80 * 1024;
@@ -595,7 +905,6 @@ cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream) {
     // from one kernel's code to another's costs a fetch of it each time (six 384-wide layers 96 us a step, 111 with two kernels)
     const bool gen = a.nx || (size_t)n16 * a.k64 <= 4096;
     const dim3 grid(grid_x);
-    cudaError_t e;
 #define SMEG_QD(MM)                                                                   \
     case MM:                                                                          \
         e = gen ? opt_in_smem(q4_direct_kernel<MM, 1>, smem) : opt_in_smem(q4_direct_kernel<MM, 0>, smem); \

@@ -458,3 +458,36 @@ def test_tensor_core_calls_in_a_capture_without_a_warm_call(form):
     torch.cuda.synchronize()
     assert max_rel(got.float().cpu().numpy(), want.float().cpu().numpy()) <= TOL and sg.last_status() == 0
     del graph
+
+
+# One and two rows on the kernel that takes stages of four units: depths from its first (29 units, a last stage of one unit) up,
+# depths that end in a stage's middle, K-blocks of a half unit up to longer than the depth, several column groups a CTA.
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("n,k,block", [(33, 1800, 32), (389, 2056, 64), (16, 2304, 128), (7001, 1856, 32), (100, 11008, 512), (48, 4096, 8192), (20, 14400, 32)])
+def test_one_and_two_rows_by_stages_of_four_units(m, n, k, block):
+    """Against the product in 64 bits of the weights themselves: an f16 store (2^-11 of the value) and f32 sums, whose terms
+    code x a are exact: at most 16 roundings of 2^-24 of the largest partial sum of |code + 8| |a| scale per 256 depths."""
+    g, _, (q, s, a_bits) = run_q4(m, n, k, block, seed=k)
+    a = orc.f16_bits_to_f32(a_bits).astype(np.float64).reshape(m, k)
+    want = a @ q4_exact(q, s, n, k, block)
+    big = np.abs(a) @ np.abs(orc.f16_bits_to_f32(s).reshape(n, -1).astype(np.float64).T[np.arange(k) // block]) * 16
+    assert np.all(np.abs(g - want) <= 2.0 ** -11 * np.abs(want) + 2.0 ** -24 + 16 * 2.0 ** -24 * big)
+
+
+@pytest.mark.parametrize("m", [1, 2])
+def test_rows_with_infinities_by_stages_of_four_units(m):
+    """An infinity meets a code of zero as a NaN and any other as an infinity, and leaves other rows alone."""
+    n, k = 200, 2048
+    rng = np.random.default_rng(4)
+    q, s = q4_logical(rng, n, k, 32, from_f32=False)
+    w = sg.Q4Weights.new(q, s, n, k)
+    a = rng.standard_normal((m, k)).astype(np.float16)
+    a[0, 1234] = np.inf
+    c = torch.zeros((m, n), dtype=torch.float16, device="cuda")
+    sg.matmul_q4(torch.from_numpy(a).cuda(), w, c, m)
+    exact = q4_exact(q, s, n, k, 32)
+    with np.errstate(invalid="ignore"):
+        want = a.astype(np.float64) @ exact
+    got = c.float().cpu().numpy()
+    assert np.array_equal(np.isnan(got[0]), exact[1234] == 0) and np.array_equal(np.isposinf(got[0]), exact[1234] > 0)
+    assert np.all(np.isfinite(got[1:])) and max_rel(got[1:], want[1:]) <= 1e-3
