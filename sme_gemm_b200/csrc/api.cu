@@ -871,7 +871,13 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
     // above that every CTA would repeat too much work, and a separate pass over the rows is faster
     static const size_t fuse_max_rows = []() { const char* e = getenv("SMEG_LB_FUSE_MAX_ROWS"); return e ? (size_t)atoi(e) : (size_t)4; }();
     g.a_vec_ok = (k % 8 == 0) && ((uintptr_t)a % 16 == 0);
-    if (k > 0 && (int)m <= g_direct_rows && m <= 2 && (g.a = a, lowbit_direct_supported(g, true))) {
+    const bool rows_kernel = m <= 16 && lowbit_rows_supported(g, w->bits, ds->sm_count);
+    if (rows_kernel && m * k <= kRowsFused) {
+        // up to 16 rows, K-blocks of 32 and up: one launch that quantises the rows, multiplies and folds
+        g.a = a;
+        g.q_out = q_out; g.sa_out = sa_out;
+        e = lowbit_rows_launch(g, w->bits, ds->sm_count, stream);
+    } else if (!rows_kernel && k > 0 && (int)m <= g_direct_rows && m <= 2 && (g.a = a, lowbit_direct_supported(g, true))) {
         // one or two rows: the direct kernel quantises the rows itself in every CTA
         g.q_out = q_out; g.sa_out = sa_out;
         e = lowbit_direct_launch(g, w->bits, ds->sm_count, stream);
@@ -889,7 +895,7 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
         // to the staged dp4a kernel
         static const int use_mma = []() { const char* e = getenv("SMEG_LOWBIT_MMA"); return e ? atoi(e) : 1; }();
         bool mma = false;
-        if (!tc && use_mma && (int)m > g_direct_rows && m <= 16) {
+        if (!rows_kernel && !tc && use_mma && (int)m > g_direct_rows && m <= 16) {
             LowbitGemvArgs probe = g;
             probe.qh = (const uint16_t*)1; probe.sa = (const float*)1; probe.qsum = (const int32_t*)1;   // set below
             mma = lowbit_mma_supported(probe, ds->sm_count);
@@ -930,7 +936,8 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
                 t.n16 = (int)w->d.n16; t.ku = (int)w->d.ku; t.nb = (int)nb; t.nb_real = (int)w->d.nb_real;
                 t.log2_block = w->d.log2_block; t.bits = w->bits; t.lut = w->lut ^ 0x80808080u; t.status = ds->status; t.ep = g.ep;
                 e = lowbit_tc_launch(t, ds->sm_count, stream);
-            } else if (mma) e = lowbit_mma_launch(g, w->bits, ds->sm_count, stream);
+            } else if (rows_kernel) e = lowbit_rows_launch(g, w->bits, ds->sm_count, stream);
+            else if (mma) e = lowbit_mma_launch(g, w->bits, ds->sm_count, stream);
             else if ((int)m <= g_direct_rows && lowbit_direct_supported(g, false)) e = lowbit_direct_launch(g, w->bits, ds->sm_count, stream);
             else e = lowbit_gemv_launch(g, w->bits, ds->sm_count, stream);
         }

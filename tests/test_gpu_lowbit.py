@@ -251,3 +251,44 @@ def test_row_tiles_of_the_block_kernel(kind, m, n, k, block):
     want = orc.lowbit_matmul(a_bits, kind, wbits, 1 if kind == 2 else 0, scales, book if kind == 2 else None, n, k, block, m)
     want = want[0] if isinstance(want, tuple) else want
     assert np.array_equal(_canon16(bits_of(c)).reshape(-1), _canon16(want).reshape(-1))
+
+
+# The kernel of one to sixteen rows: depths in one part, in four and in eight, K-blocks longer than a part's share, a depth that
+# ends inside a unit, a part without a whole K-block, more column groups than a round of a CTA's warps, rows past a tile of eight, and
+# more values than a CTA quantises for itself.
+@pytest.mark.parametrize("m,n,k,block", [(1, 40, 3000, 32), (2, 300, 12500, 128), (3, 70, 1000, 1024), (5, 33, 8200, 64), (8, 2400, 700, 256),
+                                         (9, 100, 4500, 128), (11, 64, 2049, 512), (16, 50, 2600, 128), (1, 40000, 256, 128), (16, 37900, 160, 32)])
+@pytest.mark.parametrize("kind", [1, 2])
+def test_parts_and_tiles_of_the_kernel_for_few_rows(kind, m, n, k, block):
+    rng = np.random.default_rng(m * 1000 + k)
+    scales = orc.f32_to_f16_bits(rng.uniform(-0.05, 0.05, n * -(-k // block)).astype(np.float32))
+    a_bits = orc.f32_to_f16_bits(rng.standard_normal(m * k).astype(np.float32))
+    wbits = rng.integers(0, 256, (k * n * kind + 7) // 8).astype(np.uint8)
+    if kind == 2:
+        w = sg.Q2Weights.new(wbits, scales, n, k, sg.Q2Params(block).with_codebook(BOOKS[2]))
+        check_bits(w, 2, wbits, 1, scales, BOOKS[2], n, k, block, m, a_bits, "q2")
+    else:
+        w = sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block)
+        check_bits(w, 1, wbits, 0, scales, None, n, k, block, m, a_bits, "q1")
+
+
+@pytest.mark.parametrize("m", [1, 6, 12])
+def test_resolved_graphs_of_the_kernel_for_few_rows(m):
+    """Scalars and column vectors without an activation, node by node on the f16 product: the interpreter's bits (numpy's f32)."""
+    n, k = 131, 512
+    rng = np.random.default_rng(m)
+    scales = orc.f32_to_f16_bits(rng.uniform(0.01, 0.05, n * 4).astype(np.float32))
+    w = sg.Q1Weights.new(rng.integers(0, 256, k * n // 8).astype(np.uint8), scales, sg.WeightLayout.OutIn, n, k, 128)
+    a = f16_bits_dev(orc.f32_to_f16_bits(rng.standard_normal(m * k).astype(np.float32)))
+    v = [rng.standard_normal(n).astype(np.float16) for _ in range(4)]
+    d = [torch.from_numpy(x).cuda() for x in v]
+    f = [x.astype(np.float32) for x in v]
+    plain = torch.empty((m, n), dtype=torch.float16, device="cuda")
+    sg.matmul_q1(a, w, plain, m)
+    x = plain.cpu().numpy().astype(np.float32)
+    for ep, want in ((sg.Epilogue().mul_col(d[0]).add_col(d[1]).sub_col(d[2]).max_col(d[3]), np.maximum((x * f[0] + f[1]) - f[2], f[3])),
+                     (sg.Epilogue().add_scalar(0.5).mul_scalar(3.0).sub_scalar(0.25).min(1.5), np.minimum((x + np.float32(0.5)) * 3 - np.float32(0.25), np.float32(1.5))),
+                     (sg.Epilogue().max(-0.5).min_col(d[0]), np.minimum(np.maximum(x, np.float32(-0.5)), f[0]))):
+        c = torch.empty_like(plain)
+        sg.matmul_q1_ep(a, w, c, m, ep)
+        assert np.array_equal(c.cpu().numpy().view(np.uint16), want.astype(np.float16).view(np.uint16))
