@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     volatile int* abort_flag = &abort_word;
     uint64_t *full = bars, *empty = full + kAtMaxSlots, *q_full = empty + kAtMaxSlots, *s_full = q_full + 1, *s_free = s_full + 2,
              *p_full = s_free + 2, *pv_done = p_full + 2, *o_free = pv_done + 2;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int hd = p.head_dim, group = p.heads / p.kv_heads, kvh = blockIdx.z;
     const int tile = gridDim.y - 1 - blockIdx.y;               // the tiles with the most keys first
     const int splits = gridDim.x, rank = blockIdx.x;
@@ -619,7 +619,7 @@ template <int QF32, int OUT16>
 __global__ void __launch_bounds__(kAdThreads, 1) attn_decode_kernel(const __grid_constant__ AttnArgs p, int kc) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float part_m[16], part_l[16];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int hd = p.head_dim, hd32 = (hd + 31) & ~31, group = p.heads / p.kv_heads, kvh = blockIdx.z;
     const int splits = gridDim.x, rank = blockIdx.x, nrow = p.rows * group;
     const int len = p.start + p.rows;

@@ -27,6 +27,12 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
+// The calling warp's index in its CTA, by a shuffle: the compiler then knows that it is one value in all lanes, so that the branches and
+// addresses of a warp's role are uniform -- no reconvergence points, address arithmetic on the uniform pipe (us, threadIdx.x >> 5 / this:
+// 1-bit prefill 512 x 4096 x 14336 109.3 / 97.3, MLP block at 256 rows 101.7 / 96.2, at one row 23.7 / 23.0, bf16 Q4 8 x 4096 x
+// 14336 13.7 / 13.2).  Called where all lanes of the warp are.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
     extern __shared__ unsigned char smem_dyn[];
     // the swizzled operands need 1024-byte aligned tiles: align the window by hand
     unsigned char* smem_raw = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int NT = p.nt, NK = p.nk, O = p.no, NW = p.nw, PU = p.pu;
     // CG == 2: the CTA is one of a pair (cluster of two along x).  Each CTA expands its own columns and loads half of
     // the token rows; the even CTA issues MMAs of 256 weight columns that read both CTAs' shared memory and write both

@@ -173,7 +173,7 @@ template <int M, int GEN>
 __global__ void __launch_bounds__(kDThreads, 3) q4_direct_kernel(const __grid_constant__ Q4GemvArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int PF = kQ4PF;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const int kpad = p.k64 * 64, a_stride = kpad + 8;
     uint4* ring_w = reinterpret_cast<uint4*>(smem_raw) + (size_t)warp * PF * 32 + lane;                     // + slot * 32
@@ -383,7 +383,7 @@ template <int M, int PF>
 __global__ void __launch_bounds__(kDThreads, PF > 3 ? 2 : 3) q4_stage_kernel(const __grid_constant__ Q4GemvArgs p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int SLOT = q4_slot_bytes(M), NC = M;              // NC accumulator pairs
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int ns = q4_stages(p.k64), a_stride = ns * kQ4StageUnits * kQ4AUnit;
     const uint32_t ring = smem_u32(smem_raw) + (uint32_t)(warp * PF * SLOT);

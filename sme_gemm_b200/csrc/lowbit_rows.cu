@@ -117,7 +117,7 @@ __device__ __noinline__ void codes_out(const LowbitGemvArgs& p, int r, int d, ui
 // LB: log2 of the K-block where the kernel is of one.
 template <int BITS, int PAIRED, int RB, int LB>
 __device__ __forceinline__ void quantise_rows(const LowbitGemvArgs& p, unsigned char* Qs, float* SQ, float* AMX, int m8) {
-    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int m = p.m, kq = p.kq, lb = LB ? LB : p.log2_block, chunks = (kq + 255) >> 8;
     // warps to a run of rows: the rows are dealt out where there are fewer runs of depths than warps
     const int deal = RB == 1 || chunks > 8 ? 1 : chunks > 4 ? 2 : 4, runs = chunks < kRWarps ? chunks : kRWarps;   // (deal x runs <= 16)
@@ -231,8 +231,7 @@ __global__ void __launch_bounds__(kRThreads, 1) lowbit_rows_kernel(const __grid_
     constexpr int NA = PAIRED ? 4 : LONG ? 2 : 1;                   // accumulators of a block
     constexpr int UB = LONG == 2 ? UD / 128 : 1;                    // K-blocks of a unit (whose sums are taken together)
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // (the shuffle lets the compiler know that a warp's index is one value: its branches need no reconvergence)
-    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31, g = lane >> 2, t = lane & 3;
     const int m = p.m, nb = p.nb, ku = p.ku, lb = p.log2_block;
     const int lparts = p.ns, parts = 1 << lparts, at_once = kRWarps >> lparts;      // parts of a column group's depth, column groups in work
     const int part = warp & (parts - 1), grp = warp >> lparts;

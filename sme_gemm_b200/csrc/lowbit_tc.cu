@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kLtThreads, 1) lowbit_tc_kernel(const __grid_c
     constexpr int BTILE = NT * 128;
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem_raw = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
 
     unsigned char* ring_a = smem_raw;                                          // [NA][16 KB]
     unsigned char* ring_b = ring_a + (size_t)NA * kLtATile;                 // [NB][BTILE], tiles 1024-byte aligned
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
              *f_full = acc_empty + 2, *f_empty = f_full + kLbNF;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(f_empty + kLbNF);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int col0 = blockIdx.x * 128, cg0 = blockIdx.x * 8, tok0 = blockIdx.y * NT;
     // depths that belong to a real K-block and are staged (>= k: what lies past k multiplies zero activations)
     const int k_end = (int)min((long long)p.nb_real << p.log2_block, (long long)p.kq);

@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int PF = mma_ring_slots(NT, CG, DENSE), RB = STAGED ? 0 : 1024 * NT, SLOT = mma_slot_bytes(STAGED ? 0 : NT, CG, DENSE);
     constexpr int WB = mma_w_bytes(DENSE), PER = CG * NT * 128;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t ring = smem_u32(smem_raw) + (uint32_t)(warp * PF * SLOT);
     float* red = reinterpret_cast<float*>(smem_raw + (size_t)kMWarps * PF * SLOT);       // [8 warps][CG][NT][4][32 lanes]
