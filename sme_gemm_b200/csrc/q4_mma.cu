@@ -13,8 +13,8 @@
 // f16 / bf16 integers (one lop3 per pair and a subtraction), the tensor core sums 32 depths in f32 and the block's f32
 // scale folds the sum into the total: no weight is rounded on the way, for bf16 either.
 //
-// What bounds it: instruction issue (135 warp instructions a unit at eight bf16 rows, issue slots two thirds busy, the tensor
-// pipe a tenth).  Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 13.7 (2.4 TB/s),
+// What bounds it: instruction issue (about 115 warp instructions a unit at eight bf16 rows, 44 of them the expansion; with the copies'
+// addresses formed from indexes for each unit 135: 8 x 4096 x 14336 13.5 us, now 12.15, 16 rows 16.7 and 15.6, f16 12.0 and 11.3).  Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 13.7 (2.4 TB/s),
 // 16 rows 67 -> 17.5; bf16 4096 x 4096 1 row 15.8 -> 4.9, 16 rows 28.5 -> 6.3; f16 8 rows 9.8 -> 4.6, 16 rows 14.0 -> 6.2; against
 // q4_direct_kernel, which keeps one and two rows (4.0 and 5.3), at 4 rows 8.5 -> 4.5.
 #include "epilogue.cuh"
@@ -155,16 +155,31 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
     const int u_begin = min(warp * upw, p.k64), u_end = min(u_begin + upw, p.k64), nu = u_end - u_begin;
     const int total = passes * nu;
 
-    // load cursor
+    // load cursor: where the unit's codes and scales (dense: pieces of weights) and its rows start, as pointers that a unit moves on.
+    // (Formed from the indexes for each unit they were a third of the loop's instructions.)
     int lu = u_begin, lpass = first;
-    auto issue_weights = [&](uint32_t slot, int pass, int u) {
+    // (Dense weights and passes of one column group on sixteen rows keep the indexes: 64 x 2048 x 2048 dense with pointers 7.0 us, without
+    // 6.84, 16 x 4096 x 4096 6.13 and 5.99.)
+    constexpr bool PTR = !DENSE && !(NT == 2 && CG == 1);
+    const unsigned char *wp[CG], *sp[CG];
+    const uint32_t sc_shift = DENSE ? 0u : (uint32_t)p.log2_block - 5;
+    auto weights_from = [&](int pass) {
+        if (!PTR) return;
+#pragma unroll
+        for (int c = 0; c < CG; ++c) {
+            const uint32_t grp = (uint32_t)min(group_of(pass, c), p.n16 - 1);           // a tail pass may be one group short
+            wp[c] = p.codes + (uint64_t)grp * (uint32_t)(p.k64 * kUnitBytes) + (uint32_t)(u_begin * kUnitBytes + lane * 16);
+            sp[c] = reinterpret_cast<const unsigned char*>(p.scales) + (uint64_t)grp * (uint32_t)(p.nb * 32) + (uint32_t)(4 * g);
+        }
+    };
+    auto issue_weights = [&](uint32_t slot, int u) {
         if (DENSE) {
             const int d = u * 64 + 8 * t;                          // (kd is a multiple of 8; columns past n and depths past kd are zeros)
 #pragma unroll
             for (int c = 0; c < CG; ++c)
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
-                    const int col = group_of(pass, c) * 16 + g + 8 * j;
+                    const int col = group_of(lpass, c) * 16 + g + 8 * j;
                     const uint16_t* src = p.wdense + (size_t)min(col, p.n - 1) * p.kd + d;
                     const uint32_t lo = col < p.n && d < p.kd ? 16u : 0u, hi = col < p.n && d + 32 < p.kd ? 16u : 0u;
                     const uint32_t dst = slot + (uint32_t)(WB * c + 1024 * j + lane * 16);
@@ -173,49 +188,90 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
                 }
             return;
         }
+        if (!PTR) {
+#pragma unroll
+            for (int c = 0; c < CG; ++c) {
+                const size_t grp = (size_t)min(group_of(lpass, c), p.n16 - 1);
+                cp_async16(slot + (uint32_t)(512 * c + lane * 16), p.codes + q4_unit_offset(grp, (size_t)u, p.k64) + lane * 16);
+                const uint16_t* s = p.scales + q4_scale_row(grp, 0, p.nb) + 2 * g;
+                const uint32_t d = slot + (uint32_t)(512 * CG + RB + 256 * c + lane * 4);
+                cp_async4(d, s + (size_t)((u * 64) >> p.log2_block) * 16);
+                cp_async4(d + 128, s + (size_t)((u * 64 + 32) >> p.log2_block) * 16);
+            }
+            return;
+        }
+        const uint32_t ra = ((uint32_t)(2 * u) >> sc_shift) * 32, rb = ((uint32_t)(2 * u + 1) >> sc_shift) * 32;
 #pragma unroll
         for (int c = 0; c < CG; ++c) {
-            const size_t grp = (size_t)min(group_of(pass, c), p.n16 - 1);               // a tail pass may be one group short
-            cp_async16(slot + (uint32_t)(512 * c + lane * 16), p.codes + q4_unit_offset(grp, (size_t)u, p.k64) + lane * 16);
-            const uint16_t* s = p.scales + q4_scale_row(grp, 0, p.nb) + 2 * g;
+            cp_async16(slot + (uint32_t)(512 * c + lane * 16), wp[c]);
+            wp[c] += kUnitBytes;
             const uint32_t d = slot + (uint32_t)(512 * CG + RB + 256 * c + lane * 4);
-            cp_async4(d, s + (size_t)((u * 64) >> p.log2_block) * 16);
-            cp_async4(d + 128, s + (size_t)((u * 64 + 32) >> p.log2_block) * 16);
+            cp_async4(d, sp[c] + ra);
+            cp_async4(d + 128, sp[c] + rb);
         }
     };
     const uint16_t* arow[NT];
-    int kend[NT];                                                  // rows past the batch are zeros, without a read
+    int kend[NT];
+    uint32_t a_sz[NT];                                             // rows past the batch are zeros, without a read
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        arow[nt] = p.a + (size_t)min(row0 + 8 * nt + g, p.m - 1) * p.k + 8 * t;
+        arow[nt] = p.a + (size_t)min(row0 + 8 * nt + g, p.m - 1) * p.k + (PTR ? u_begin * 64 : 0) + 8 * t;
+        a_sz[nt] = row0 + 8 * nt + g < p.m ? 16u : 0u;
         kend[nt] = row0 + 8 * nt + g < p.m ? p.k : 0;
     }
+    const int whole = p.k >> 6;                                    // units without a depth past the rows' end
     auto issue_rows = [&](uint32_t slot, int u) {
         if (STAGED) return;
-        const int d = u * 64;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            const uint32_t lo = d + 8 * t < kend[nt] ? 16u : 0u, hi = d + 32 + 8 * t < kend[nt] ? 16u : 0u;   // k is a multiple of 8
             const uint32_t dst = slot + (uint32_t)(WB * CG + 1024 * nt + lane * 16);
-            cp_async16_zfill(dst, lo ? arow[nt] + d : p.a, lo);
-            cp_async16_zfill(dst + 512, hi ? arow[nt] + d + 32 : p.a, hi);
+            if (!PTR) {
+                const int d = u * 64;
+                const uint32_t lo = d + 8 * t < kend[nt] ? 16u : 0u, hi = d + 32 + 8 * t < kend[nt] ? 16u : 0u;   // k is a multiple of 8
+                cp_async16_zfill(dst, lo ? arow[nt] + d : p.a, lo);
+                cp_async16_zfill(dst + 512, hi ? arow[nt] + d + 32 : p.a, hi);
+                continue;
+            }
+            if (u < whole) {                                       // (a size of zero reads nothing)
+                cp_async16_zfill(dst, arow[nt], a_sz[nt]);
+                cp_async16_zfill(dst + 512, arow[nt] + 32, a_sz[nt]);
+            } else {
+                const uint32_t lo = u * 64 + 8 * t < p.k ? a_sz[nt] : 0u, hi = u * 64 + 32 + 8 * t < p.k ? a_sz[nt] : 0u;   // k is a multiple of 8
+                cp_async16_zfill(dst, lo ? arow[nt] : p.a, lo);
+                cp_async16_zfill(dst + 512, hi ? arow[nt] + 32 : p.a, hi);
+            }
+            arow[nt] += 64;
         }
     };
-    auto advance = [&]() {
-        if (++lu == u_end) { lu = u_begin; ++lpass; }
+    auto rows_back = [&]() {
+        if (!PTR) return;
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) arow[nt] -= (size_t)nu * 64;
     };
     // the weights of the first ring-full do not depend on the kernel ahead in the stream; the activations may
+    if (total > 0) weights_from(first);
     {
-        const int lu0 = lu, lpass0 = lpass;
-        for (int i = 0; i < PF - 1 && i < total; ++i) { issue_weights(ring + (uint32_t)(i * SLOT), lpass, lu); advance(); }
-        lu = lu0; lpass = lpass0;
+        const int ahead = total < PF - 1 ? total : PF - 1;
+        for (int i = 0; i < ahead; ++i) {
+            issue_weights(ring + (uint32_t)(i * SLOT), lu);
+            if (++lu == u_end) {
+                lu = u_begin;
+                if (++lpass < first + passes) weights_from(lpass);
+            }
+        }
     }
     pdl_launch_dependents();
     pdl_wait();
+    {
+        int ru = u_begin;
 #pragma unroll
-    for (int i = 0; i < PF - 1; ++i) {
-        if (i < total) { issue_rows(ring + (uint32_t)(i * SLOT), lu); advance(); }
-        cp_async_commit();
+        for (int i = 0; i < PF - 1; ++i) {
+            if (i < total) {
+                issue_rows(ring + (uint32_t)(i * SLOT), ru);
+                if (++ru == u_end) { ru = u_begin; rows_back(); }
+            }
+            cp_async_commit();
+        }
     }
     if (STAGED) {
         for (int r = 0; r < p.m; ++r) stage_row(rows_s + (size_t)r * rows_ld, p.a + (size_t)r * p.k, p.k, p.k64 * 64);
@@ -262,9 +318,13 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
             const int fill = slot == 0 ? PF - 1 : slot - 1;
             if (lpass < first + passes) {
                 const uint32_t fb = ring + (uint32_t)(fill * SLOT);
-                issue_weights(fb, lpass, lu);
+                issue_weights(fb, lu);
                 issue_rows(fb, lu);
-                advance();
+                if (++lu == u_end) {
+                    lu = u_begin;
+                    rows_back();
+                    if (++lpass < first + passes) weights_from(lpass);
+                }
             }
             cp_async_commit();
             slot = slot + 1 == PF ? 0 : slot + 1;
