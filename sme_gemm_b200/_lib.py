@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libsmeg_b200.so")
@@ -46,6 +47,10 @@ class BlockArgs(C.Structure):
                 ("act", C.c_uint32)]
 
 
+# The same fields, packed by one call (0.3 us where filling a structure takes 1.6, of some 25 us of host work a layer at one row).
+BLOCK_ARGS = struct.Struct("@PNNPPPPffiiPPNNNPPNPPPfI")
+
+assert BLOCK_ARGS.size == C.sizeof(BlockArgs) and BlockArgs.act.offset == BLOCK_ARGS.size - 4
 assert C.sizeof(EpNode) == 32 and EpNode.ptr.offset == 16 and EpNode.ld.offset == 24
 
 _sz, _vp, _u32, _i = C.c_size_t, C.c_void_p, C.c_uint32, C.c_int
@@ -118,7 +123,7 @@ SIGNATURES = {
     "smeg_mlp_partial_dev": (_i, [_vp, _vp, _vp, _sz, _vp]),
     "smeg_matmul_q4_partial_dev": (_i, [_vp, _vp, _vp, _sz, _vp]),
     "smeg_matmul_q4_accumulate_dev": (_i, [_vp, _vp, _vp, _sz, _vp]),
-    "smeg_block_accumulate_dev": (_i, [C.POINTER(BlockArgs), _vp]),
+    "smeg_block_accumulate_dev": (_i, [_vp, _vp]),
     "smeg_kv_append_dev": (_i, [_vp, _vp, _vp, _sz, _sz, _sz, _sz, _sz, _sz, _vp]),
     "smeg_attn_kv_causal_dev": (_i, [_vp, _vp, _i, _sz, _vp, _vp, _sz, _sz, _sz, _sz, _sz, C.c_float, _vp]),
     "smeg_attn_kv_causal_f16_dev": (_i, [_vp, _vp, _i, _sz, _vp, _vp, _sz, _sz, _sz, _sz, _sz, C.c_float, _vp]),

@@ -495,8 +495,7 @@ __global__ void __launch_bounds__(kThreadsLb, 1) lowbit_gemv_kernel(const __grid
 #pragma unroll 1
                         for (int s = 0; s < STEPS; ++s) {
                             if (DP) {
-                                // at most four rows: dot products on the integer units instead of the tensor cores
-                                // (an int8 mma.sync issues about once per 85 cycles per scheduler on this part).
+                                // at most four rows: dot products on the integer units instead of the tensor cores.
                                 // The lane's bytes are columns g and g + 8 at depths 8t .. 8t + 7.
                                 uint2 aq[DP ? DP : 1];
 #pragma unroll

@@ -1,15 +1,14 @@
-// 2-bit / 1-bit matmul for five to sixteen activation rows (sm_100a): the exact int32 block sums of
+// 2-bit / 1-bit matmul for five to sixteen activation rows whose codes and K-blocks do not fit one CTA's shared memory beside its rings
+// (lowbit_rows.cu takes the others; 16 rows of 8192 depths, say, come here) (sm_100a): the exact int32 block sums of
 // matmul_q2 / matmul_q1 (run_q2_gemv, csrc/gemm_q2.cc:300-404; block_sums, src/kernels/lowbit/matmul.rs:373-421)
 // formed by warp-level tensor-core instructions, then the reference's ordered fold.
 //
-// Between the one-wave dp4a kernels (one to four rows, gemv_direct.cu) and the tcgen05 kernel (seventeen rows
-// up, lowbit_tc.cu) a call is still a few microseconds of weight streaming, but dp4a would need a
+// Below the tcgen05 kernel (seventeen rows up, lowbit_tc.cu) a call is still a few microseconds of weight streaming, but dp4a would need a
 // multiply-add instruction per four weights and row: eight rows of a 4096 x 14336 sign matrix are 117 M dp4a,
 // longer than the stream.  mma.m16n8k16 takes the packed unit's lane vector as its A fragment as it lies in
 // memory (16 weight columns = M, up to 8 activation rows = N), so the cost per weight no longer grows with the rows.
 //
-// Exactness.  The int8 tensor path of this part is slow, so the products run in f16 with f32 accumulation and are
-// still exact integers: an activation code q (|q| <= 128) is the f16 number q; a weight is the f16 SUBNORMAL whose
+// Exactness.  The products run in f16 with f32 accumulation and are exact integers all the same: an activation code q (|q| <= 128) is the f16 number q; a weight is the f16 SUBNORMAL whose
 // bit pattern is u (1-bit: the sign bit itself, u in {0,1}; 2-bit: codebook value + 128, u in 0..255), i.e. u * 2^-24.
 // Every product u q 2^-24 and every partial sum of up to 512 depths (|sum| < 2^24 units) is exact in f32, so
 // S = (int)(acc * 2^24) = sum u q, and the block sum is 2 S - sum q (1-bit) or S - 128 sum q (2-bit).  Accumulators are

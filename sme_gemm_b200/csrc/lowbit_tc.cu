@@ -15,8 +15,8 @@
 // f32 accumulator holds their sum exactly while it stays below 2^24 units -- which a run of at
 // most 256 depths guarantees (255 * 128 * 256 < 2^24).  A K-block longer than that is accumulated
 // in runs of 256 depths whose integer sums are added in the fold.  (tcgen05.mma.kind::i8 gives the
-// same integers, and an earlier form of this kernel used it, but the int8 tensor path of this
-// part sustains only ~135 TOP/s against ~1500 TFLOP/s for f16.)  The 1-bit form does not even move
+// same integers, and an earlier form of this kernel used it, but in it tcgen05's int8 kind
+// sustained only ~135 TOP/s against ~1500 TFLOP/s for f16.)  The 1-bit form does not even move
 // its sign bits: bit b of a half word is the f16 number 2^(b-24) for b < 12, so an operand register
 // is the packed word under one mask, and act_quant_kernel leaves the codes of the matching depths
 // in the matching order, scaled by the inverse power of two (2^8, 1, 2^6, 2^-2: still exact f16

@@ -19,7 +19,7 @@ from enum import IntEnum
 
 import numpy as np
 
-from ._lib import BlockArgs, EpDesc16, EpNode, SmegError, check, lib
+from ._lib import BLOCK_ARGS, EpDesc16, EpNode, SmegError, check, lib
 
 try:  # torch is plumbing for device memory and streams only
     import torch
@@ -109,10 +109,11 @@ def _ptr(x) -> int:
     return x.ctypes.data
 
 
-if torch is not None and hasattr(torch._C, "_cuda_getCurrentRawStream"):
+if torch is not None and hasattr(torch._C, "_cuda_getCurrentRawStream") and hasattr(torch._C, "_cuda_getDevice"):
     def _stream() -> int:
-        """The handle of torch's current stream on the current device (without building a Stream object: 2 us a call)."""
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        """The handle of torch's current stream on the current device (without building a Stream object: 2 us a call).  The device is
+        asked for directly: every caller has a CUDA tensor in hand, so CUDA is up."""
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 else:
     def _stream() -> int:
         return torch.cuda.current_stream().cuda_stream
@@ -353,6 +354,9 @@ def _round_scalar(v: float, dtype: str) -> float:
         return float(np.float32(np.float16(v)))
 
 
+_EP_ARRAYS: dict = {}                                          # length -> ctypes array type of a graph's nodes
+
+
 class Epilogue:
     """The fused epilogue as an ordered op-graph (src/epilogue/graph.rs:33-432).
 
@@ -466,22 +470,26 @@ class Epilogue:
         items = self.resolved()
         if not items:
             return None, []
-        arr = (EpNode * len(items))()
+        array = _EP_ARRAYS.get(len(items))                      # (an array type a length; its memory is the call's own)
+        if array is None:
+            array = _EP_ARRAYS[len(items)] = EpNode * len(items)
+        arr = array()
         keep = [arr]
-        for i, (op, aux, scalar, operand, ld) in enumerate(items):
-            p = None
+        want = torch.bfloat16 if device and self.dtype == "bf16" else torch.float16 if device else None
+        for node, (op, aux, scalar, operand, ld) in zip(arr, items):
+            node.op, node.aux, node.scalar, node.ld = op, aux, scalar, ld
             if operand is not None:
                 if device:
                     assert _is_torch(operand) and operand.is_cuda, "device call needs CUDA tensor operands"
-                    operand = operand.contiguous()
-                    want = torch.bfloat16 if self.dtype == "bf16" else torch.float16
+                    if not operand.is_contiguous():
+                        operand = operand.contiguous()
                     assert operand.dtype == want, f"operand dtype {operand.dtype} != {want}"
+                    node.ptr = operand.data_ptr()
                 else:
                     assert not _is_torch(operand), "host call needs numpy operands"
                     operand = _np_bits(operand, "epilogue operand")
+                    node.ptr = operand.ctypes.data
                 keep.append(operand)
-                p = _ptr(operand)
-            arr[i] = EpNode(op, aux, scalar, p, ld)
         desc = EpDesc16(len(items), arr)
         keep.append(desc)
         return desc, keep
@@ -495,7 +503,7 @@ def _check_io(a, c, m, n, k):
 
 
 def _run_q4(a, w: Q4Weights, c, m: int, ep: Epilogue | None, bf16: bool) -> None:
-    n, k = w.n(), w.k()
+    n, k = w._n, w._k
     _check_io(a, c, m, n, k)
     if ep is not None:
         assert ep.dtype == ("bf16" if bf16 else "f16")
@@ -507,9 +515,11 @@ def _run_q4(a, w: Q4Weights, c, m: int, ep: Epilogue | None, bf16: bool) -> None
         assert a.is_cuda and c.is_cuda and a.is_contiguous() and c.is_contiguous()
         want = torch.bfloat16 if bf16 else torch.float16
         assert a.dtype == want and c.dtype == want
-        desc, keep = ep._desc(True) if ep is not None else (None, [])
+        desc, keep = ep._desc(True) if ep is not None else (None, None)
         fn = L.smeg_matmul_q4_bf16_dev if bf16 else L.smeg_matmul_q4_f16_dev
-        check(fn.__name__, fn(w._h, _ptr(a), _ptr(c), m, C.byref(desc) if desc else None, _stream()))
+        rc = fn(w._h, a.data_ptr(), c.data_ptr(), m, C.byref(desc) if desc else None, _stream())
+        if rc:
+            check("smeg_matmul_q4_bf16_dev" if bf16 else "smeg_matmul_q4_f16_dev", rc)
         del keep
     else:
         ab = _np_bits(a, "a")
@@ -542,7 +552,7 @@ def matmul_q4_bf16_ep(a, w: Q4Weights, c, m: int, ep: Epilogue) -> None:
 
 
 def _run_lowbit(a, w: _LowbitWeights, c, m: int, ep: Epilogue | None, mopa: bool = False) -> None:
-    n, k = w.n(), w.k()
+    n, k = w._n, w._k
     _check_io(a, c, m, n, k)
     if ep is not None:
         assert ep.dtype == "f16"
@@ -553,9 +563,11 @@ def _run_lowbit(a, w: _LowbitWeights, c, m: int, ep: Epilogue | None, mopa: bool
     if _is_torch(a):
         assert a.is_cuda and c.is_cuda and a.is_contiguous() and c.is_contiguous()
         assert a.dtype == torch.float16 and c.dtype == torch.float16
-        desc, keep = ep._desc(True) if ep is not None else (None, [])
-        name = "smeg_matmul_lowbit_f16_dev" if mopa else "smeg_matmul_lowbit_dev"
-        check(name, getattr(L, name)(w._h, _ptr(a), _ptr(c), m, C.byref(desc) if desc else None, _stream()))
+        desc, keep = ep._desc(True) if ep is not None else (None, None)
+        fn = L.smeg_matmul_lowbit_f16_dev if mopa else L.smeg_matmul_lowbit_dev
+        rc = fn(w._h, a.data_ptr(), c.data_ptr(), m, C.byref(desc) if desc else None, _stream())
+        if rc:
+            check("smeg_matmul_lowbit_f16_dev" if mopa else "smeg_matmul_lowbit_dev", rc)
         del keep
     else:
         ab = _np_bits(a, "a")
@@ -1056,10 +1068,10 @@ class KvCache:
         self._len = min(self._len, n)
 
     def keys(self):
-        return self._k[: self._len]
+        return self._k.narrow(0, 0, self._len)               # (the slice, at half its cost)
 
     def values(self):
-        return self._v[: self._len]
+        return self._v.narrow(0, 0, self._len)
 
     def extend_from(self, src, stride: int, k_off: int, v_off: int, rows: int) -> None:
         """Appends `rows` key and value rows taken from rows of the f16 device tensor `src` (stride elements apart,
@@ -1180,22 +1192,31 @@ class Block:
         n1, attn, n2, mlp = self.norm1, self.attn, self.norm2, self.mlp
         if type(attn) is not SelfAttention or type(mlp) is not Mlp or type(n1) is not Norm or type(n2) is not Norm:
             return False
-        up = mlp.up.inner if type(mlp.up) is GatedLinear else mlp.up
-        for lin in (attn.qkv, attn.out, up, mlp.down):
+        up = mlp.up
+        gated = type(up) is GatedLinear
+        if gated:
+            up = up.inner
+        qkv, out, down = attn.qkv, attn.out, mlp.down
+        for lin in (qkv, out, up, down):
             if type(lin) is not Linear or lin.q4 is None or lin.bias is not None or lin.rms_eps is not None:
                 return False
-        if (mlp.up is not up and mlp._h is None) or not (x.is_cuda and x.is_contiguous()) or rows <= 0:
+        if (gated and mlp._h is None) or not (x.is_cuda and x.is_contiguous()) or rows <= 0:
             return False
-        d = self.width()
+        w1, w2, b1, b2 = n1.weight, n2.weight, n1.bias, n2.bias
+        d = w2.numel()
         heads, kv_heads, hd = attn._heads, attn._kv_heads, attn._head_dim
-        if n1.weight.numel() != d or type(cache) is not KvCache:
+        if w1.numel() != d or type(cache) is not KvCache:
             return False
         assert cache._heads == heads and cache._kv_heads == kv_heads and cache._head_dim == hd, "the cache's heads match the block's"
-        assert cache._len + rows <= cache._capacity, f"{rows} rows do not fit in the cache"
-        args = BlockArgs(x.data_ptr(), rows, d, n1.weight.data_ptr(), _ptr(n1.bias), n2.weight.data_ptr(), _ptr(n2.bias), n1.eps, n2.eps,
-                         n1.is_rms, n2.is_rms, attn.qkv.q4._h, attn.out.q4._h, heads, kv_heads, hd, cache._k.data_ptr(), cache._v.data_ptr(),
-                         cache._len, mlp._h if mlp.up is not up else None, up.q4._h, mlp.down.q4._h, cache._scale, int(mlp.act or 0))
-        check("smeg_block_accumulate_dev", lib().smeg_block_accumulate_dev(C.byref(args), _stream()))
+        pos = cache._len
+        assert pos + rows <= cache._capacity, f"{rows} rows do not fit in the cache"
+        args = BLOCK_ARGS.pack(x.data_ptr(), rows, d, w1.data_ptr(), b1.data_ptr() if b1 is not None else 0, w2.data_ptr(),
+                               b2.data_ptr() if b2 is not None else 0, n1.eps, n2.eps, n1.is_rms, n2.is_rms, qkv.q4._h.value, out.q4._h.value,
+                               heads, kv_heads, hd, cache._k.data_ptr(), cache._v.data_ptr(), pos, mlp._h.value if gated else 0, up.q4._h.value,
+                               down.q4._h.value, cache._scale, mlp.act or 0)
+        rc = lib().smeg_block_accumulate_dev(args, _stream())
+        if rc:
+            check("smeg_block_accumulate_dev", rc)
         cache._len += rows
         return True
 
