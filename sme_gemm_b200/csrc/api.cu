@@ -48,8 +48,8 @@ int g_tc_min_rows = []() {
 }();
 
 // Rows up to which the decode calls take the direct kernels of gemv_direct.cu (plain loads, packed
-// f16 / dp4a arithmetic; Q4 at most two rows: from three on its arithmetic per row costs more than q4_mma_kernel's
-// instructions); 0 keeps them on the other kernels.  SMEG_DIRECT_ROWS is a tuning knob.
+// f16 / dp4a arithmetic, or MMAs whose columns are K-blocks; Q4 at most two rows: from three on the arithmetic per row costs more than
+// q4_mma_kernel's instructions); 0 keeps them on the other kernels.  SMEG_DIRECT_ROWS is a tuning knob.
 int g_direct_rows = []() {
     const char* e = getenv("SMEG_DIRECT_ROWS");
     const int v = e ? atoi(e) : 4;
@@ -741,7 +741,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     DeviceState* ds = dev_state();
     if (!ds) return -5;
     // Rows that are not whole 16-byte words: one or two are staged as they are by q4_mma_kernel's CTAs (f32 sums, where the
-    // one-wave kernel's are f16: these calls had f32 sums before they came off the ring-staged kernel); every other call moves
+    // one-wave kernel's are f16 up to 1792 depths: these calls had f32 sums before they came off the ring-staged kernel); every other call moves
     // A by TMA or in 16-byte pieces and takes a padded copy, a pass of ~2 us and a trip to the allocator (5001 x 4097 bf16, us:
     // reading A by halves 8 rows 33, 40 rows 285, with the copy 9.4 and 21).
     // None of them needs the workspace: K-blocks below 32 stay off the streaming form, and where the GEMM would split the depth

@@ -3,7 +3,7 @@
 //                   DENSE: C = ep( T(beta * (A @ W)) ) on K-major 16-bit weights, whose 16-byte pieces are fragments as they lie
 //
 // Replaces the reference's SME Q4 GEMV (run_q4_gemv1 / run_q4_gemv, csrc/gemm_f16f16_q4.h:236-431, and the bf16 twin
-// csrc/gemm_b16b16_q4.h:171-268) above the rows of q4_direct_kernel, and for bf16 from one row.
+// csrc/gemm_b16b16_q4.h:171-268) above the rows of gemv_direct.cu's kernels, and for bf16 from one row.
 //
 // Laid out like q4_direct_kernel: a packed unit (16 columns x 64 depths) is one 16-byte asynchronous copy per lane into
 // the lane's own slot of a ring, a lane reads back only what it copied itself, so the loop has no barrier and no producer;
@@ -16,7 +16,7 @@
 // What bounds it: instruction issue (about 115 warp instructions a unit at eight bf16 rows, 44 of them the expansion; with the copies'
 // addresses formed from indexes for each unit 135: 8 x 4096 x 14336 13.5 us, now 12.15, 16 rows 16.7 and 15.6, f16 12.0 and 11.3).  Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 13.7 (2.4 TB/s),
 // 16 rows 67 -> 17.5; bf16 4096 x 4096 1 row 15.8 -> 4.9, 16 rows 28.5 -> 6.3; f16 8 rows 9.8 -> 4.6, 16 rows 14.0 -> 6.2; against
-// q4_direct_kernel, which keeps one and two rows (4.0 and 5.3), at 4 rows 8.5 -> 4.5.
+// q4_direct_kernel at 4 rows 8.5 -> 4.5 (one and two rows stay with the kernels of gemv_direct.cu: 3.4 and 4.1).
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"
