@@ -828,6 +828,9 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
             g.ws = sc.ws;
             g.counters = sc.counters;
         }
+        // (the streaming form's shares lie in the same block as a depth-split GEMM's slices)
+        std::unique_lock<std::mutex> alone(g_split_mu, std::defer_lock);
+        if (g.sgrid) alone.lock();
         e = q4_gemv_launch(g, bf16, ds->sm_count, stream);
     }
     if (ext) cudaFreeAsync(ext, stream);

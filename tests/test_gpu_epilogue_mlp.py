@@ -341,21 +341,21 @@ def test_concurrent_host_threads_on_shapes_that_grow_the_scratch():
 
 
 def test_depth_split_calls_of_host_threads_do_not_mix_their_slices():
-    """Two host threads on one stream, each a GEMM whose depth slices a second launch adds up out of the stream's block: no
-    launch of the other thread comes between the two."""
+    """Host threads on one stream: two with a GEMM whose depth slices a second launch adds up out of the stream's block, one with
+    the streaming kernel (K-blocks of 16), whose shares lie in that block: no launch that uses it comes between the two."""
     import threading
     rng = np.random.default_rng(78)
     cases = []
-    for (m, n, k) in ((33, 4096, 4096), (70, 2048, 4096)):
-        assert takes_gemm(m, n, k)
-        q, s = q4_logical(rng, n, k, 32, from_f32=False)
-        w = sg.Q4Weights.new(q, s, n, k)
+    for (m, n, k, block) in ((33, 4096, 4096, 32), (70, 2048, 4096, 32), (5, 14336, 4096, 16)):
+        assert block == 16 or takes_gemm(m, n, k)
+        q, s = q4_logical(rng, n, k, block, from_f32=False)
+        w = sg.Q4Weights.with_params(q, s, None, n, k, sg.Q4Params(block))
         a = f16_bits_dev(orc.f32_to_f16_bits(rng.standard_normal((m, k)).astype(np.float32)))
         c = torch.zeros((m, n), dtype=torch.float16, device="cuda")
         sg.matmul_q4(a, w, c, m)
         cases.append((m, w, a, c))
     torch.cuda.synchronize()
-    wrong = [0, 0]
+    wrong = [0, 0, 0]
 
     def worker(i):
         torch.cuda.set_device(0)
@@ -367,9 +367,9 @@ def test_depth_split_calls_of_host_threads_do_not_mix_their_slices():
             torch.cuda.synchronize()
             wrong[i] += sum(not torch.equal(c.view(torch.int16), want.view(torch.int16)) for c in out)
 
-    threads = [threading.Thread(target=worker, args=(i,)) for i in (0, 1)]
+    threads = [threading.Thread(target=worker, args=(i,)) for i in (0, 1, 2)]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
-    assert wrong == [0, 0] and sg.last_status() == 0
+    assert wrong == [0, 0, 0] and sg.last_status() == 0
