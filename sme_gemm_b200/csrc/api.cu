@@ -116,11 +116,13 @@ struct TcScratch {
     size_t floats = 0;
     int* counters = nullptr;
     size_t ncounters = 0;
+    // Held from the launch of a depth-split GEMM to that of the pass that adds its slices: both use the stream's block, so another
+    // host thread's call on the stream must not come between them (its GEMM would overwrite the slices before they are added).
+    // The block's own, since a launch into a full queue waits until its stream drains: calls that share nothing do not wait with it.
+    // (On one device the driver then holds the other streams' launches up itself; those of another device go on.)
+    std::mutex* launches = nullptr;
 };
 std::map<std::pair<int, cudaStream_t>, TcScratch> g_tc_scratch;
-// Held from the launch of a depth-split GEMM to that of the pass that adds its slices: both use the stream's block, so another
-// host thread's call on the stream must not come between them (its GEMM would overwrite the slices before they are added).
-std::mutex g_split_mu;
 std::vector<void*> g_retired;        // outgrown blocks, never freed
 
 int tc_scratch(cudaStream_t stream, size_t floats, size_t ncounters, TcScratch* out) {
@@ -128,6 +130,7 @@ int tc_scratch(cudaStream_t stream, size_t floats, size_t ncounters, TcScratch* 
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(g_mu);
     TcScratch& s = g_tc_scratch[{dev, stream}];
+    if (!s.launches) s.launches = new std::mutex;                  // (kept, like the blocks, until the process ends)
     if (s.floats < floats || s.ncounters < ncounters) {
         // (an allocation would end the capture with an error of its own)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -778,6 +781,7 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
     GemmTcArgs t;
     dim3 grid;
     size_t smem = 0;
+    std::mutex* launches = nullptr;
     if (tc) {
         memset(&t, 0, sizeof(t));
         t.codes = w->codes; t.scales = w->scales; t.a = a; t.c = c; t.c32 = c32; t.glu = glu; t.yacc = yacc;
@@ -802,10 +806,11 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
         }
         t.ws = sc.ws;
         t.counters = sc.counters;
+        launches = sc.launches;
     }
     if (tc) {
-        std::unique_lock<std::mutex> both(g_split_mu, std::defer_lock);
-        if (t.ws) both.lock();
+        std::unique_lock<std::mutex> both;
+        if (t.ws) both = std::unique_lock<std::mutex>(*launches);
         e = gemm_tc_launch(t, bf16, grid, smem, stream);
     } else if (direct) {
         g.glu = glu; g.yacc = yacc;
@@ -827,10 +832,11 @@ static int q4_dev(const smeg_q4* w, const uint16_t* a, uint16_t* c, size_t m, co
             }
             g.ws = sc.ws;
             g.counters = sc.counters;
+            launches = sc.launches;
         }
         // (the streaming form's shares lie in the same block as a depth-split GEMM's slices)
-        std::unique_lock<std::mutex> alone(g_split_mu, std::defer_lock);
-        if (g.sgrid) alone.lock();
+        std::unique_lock<std::mutex> alone;
+        if (g.sgrid) alone = std::unique_lock<std::mutex>(*launches);
         e = q4_gemv_launch(g, bf16, ds->sm_count, stream);
     }
     if (ext) cudaFreeAsync(ext, stream);
@@ -1143,8 +1149,8 @@ int smeg_gemm_dense_dev(const smeg_dense* w, const uint16_t* a, uint16_t* c, siz
     }
     t.ws = sc.ws;
     t.counters = sc.counters;
-    std::unique_lock<std::mutex> both(g_split_mu, std::defer_lock);
-    if (t.ws) both.lock();
+    std::unique_lock<std::mutex> both;
+    if (t.ws) both = std::unique_lock<std::mutex>(*sc.launches);
     cudaError_t e = gemm_tc_launch(t, w->bf16, grid, smem, stream);
     if (both.owns_lock()) both.unlock();
     if (ext) cudaFreeAsync(ext, stream);

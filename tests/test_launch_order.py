@@ -33,3 +33,24 @@ def test_dependents_are_let_go_only_with_tensor_memory_held():
             between = body[max(allocs):m.start()] if m.start() > max(allocs) else ""
             assert re.search(r"__syncthreads\(\)|cluster_sync_all\(\)", between), f"{name}: {kernel} lets its dependents go before its CTAs hold tensor memory"
     assert {"gemm_tc_kernel", "attn_tc_kernel", "lowbit_tc_kernel", "lowbit_tc_block_kernel"} <= set(seen)
+
+
+def test_no_lock_of_the_whole_process_is_held_over_a_launch():
+    """A launch waits on the host while its stream's queue is full.  What two launches must be kept together by is the lock of the
+    workspace they share (one per device and stream); a lock of the process would keep the threads of every other device waiting."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "api.cu")).read())
+    everyones = set(re.findall(r"^(?:static\s+)?std::mutex\s+(\w+);", text, re.M))
+    assert everyones
+    held = 0
+    for m in re.finditer(r"std::(?:lock_guard|unique_lock)<std::mutex>\s+(\w+)\b", text):
+        depth, i = 1, m.end()                                      # the rest of the block the lock lives in
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        block = text[m.start():i]
+        if not re.search(r"\w+_launch\(", block):
+            continue
+        held += 1
+        locked = re.match(r"[^;]*;[^;]*;", block).group(0)          # the declaration and the statement that locks
+        assert not everyones & set(re.findall(r"\w+", locked)), f"{locked.strip()!r} is held over a launch"
+    assert held == 3
