@@ -53,4 +53,4 @@ def test_no_lock_of_the_whole_process_is_held_over_a_launch():
         held += 1
         locked = re.match(r"[^;]*;[^;]*;", block).group(0)          # the declaration and the statement that locks
         assert not everyones & set(re.findall(r"\w+", locked)), f"{locked.strip()!r} is held over a launch"
-    assert held == 3
+    assert held >= 3
