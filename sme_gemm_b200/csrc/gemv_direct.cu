@@ -352,13 +352,14 @@ __host__ __device__ constexpr size_t q4_rows_bytes(int m, int stages) { return (
 // MMA's B operand are neighbours.
 __device__ __forceinline__ int q4_a_index(int d) { return (d >> 6) * kQ4AUnit + (d & 57) + ((d & 2) << 1) + ((d & 4) >> 1); }
 
-// Rows with an infinity or a NaN among their activations, again: the kernel's sums would carry them to columns whose code
-// there is zero or make a NaN of them (it multiplies code + 8 and takes 8 times the row's sum off).  A thread a column, code
-// by code; f32 sums of a K-block, folded with its scale.
+// Rows with an infinity or a NaN among their activations (bits of `rows`), again: the kernel's sums would carry them to columns
+// whose code there is zero or make a NaN of them (it multiplies code + 8 and takes 8 times the row's sum off).  A thread a column,
+// code by code; f32 sums of a K-block, folded with its scale.
 template <int M>
-__device__ __noinline__ void q4_exact_cells(const Q4GemvArgs& p, const uint16_t* As, int a_stride, float* red, int cpc, int ncg, int first) {
+__device__ __noinline__ void q4_exact_cells(const Q4GemvArgs& p, const uint16_t* As, int a_stride, float* red, int cpc, int ncg, int first, int rows) {
     for (int o = threadIdx.x; o < ncg * M * 16; o += kDThreads) {
         const int col16 = o & 15, r = (o >> 4) % M, c = o / (16 * M);
+        if (!((rows >> r) & 1)) continue;                          // (a finite row's result does not depend on its neighbour's)
         const int u0 = first + (c >> 1);
         const int cg = p.glu ? 4 * (u0 >> 1) + (u0 & 1) + 2 * (c & 1) : first + c;
         float tot = 0.0f;
@@ -476,13 +477,13 @@ __global__ void __launch_bounds__(kDThreads, PF > 3 ? 2 : 3) q4_stage_kernel(con
                 float sum = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
                 sum += __shfl_xor_sync(0xffffffffu, sum, 1);
                 sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-                bad |= !(fabsf(sum) <= 3.0e38f);                   // 32 finite f16 values sum to 2.1e6 at most
+                bad |= (int)!(fabsf(sum) <= 3.0e38f) << r;         // 32 finite f16 values sum to 2.1e6 at most
                 // block 2 tb + h of the stage is column h * 4 + tb of the products (one row), r * 4 + tb of those of half h (two)
                 const int tb = lane >> 3, h = (lane >> 2) & 1;
                 if (t == 0) start[(size_t)st * 8 * M + (M == 1 ? h * 4 + tb : h * 8 + r * 4 + tb)] = sum * -4.76837158203125e-07f;
             }
         }
-    bad = __syncthreads_or(bad);
+    __syncthreads();
 
     // ---- the products ----
     // Lane (g, t) multiplies the codes of unit t of the stage (of the lanes (g, 0..3) of that unit in turn), so the depths of
@@ -573,9 +574,11 @@ __global__ void __launch_bounds__(kDThreads, PF > 3 ? 2 : 3) q4_stage_kernel(con
         }
     }
     cp_async_wait<0>();
-    __syncthreads();
-    if (bad) {
-        q4_exact_cells<M>(p, As, a_stride, red, CPC, ncg, first);
+    if (__syncthreads_or(bad)) {
+        int rows = 0;
+#pragma unroll
+        for (int r = 0; r < M; ++r) rows |= __syncthreads_or((bad >> r) & 1) ? 1 << r : 0;
+        q4_exact_cells<M>(p, As, a_stride, red, CPC, ncg, first, rows);
         __syncthreads();
     }
     q4_store_cells<M>(p, red, CPC, first, share, ncg);

@@ -491,3 +491,20 @@ def test_rows_with_infinities_by_stages_of_four_units(m):
     got = c.float().cpu().numpy()
     assert np.array_equal(np.isnan(got[0]), exact[1234] == 0) and np.array_equal(np.isposinf(got[0]), exact[1234] > 0)
     assert np.all(np.isfinite(got[1:])) and max_rel(got[1:], want[1:]) <= 1e-3
+
+
+@pytest.mark.parametrize("other", [0, 1])
+@pytest.mark.parametrize("what", [np.inf, np.nan])
+def test_a_finite_row_keeps_its_bits_beside_one_with_infinities(other, what):
+    """Two rows by stages of four units: the finite one's result is that of the same call with a finite neighbour, bit for bit."""
+    n, k = 200, 2048
+    rng = np.random.default_rng(5)
+    q, s = q4_logical(rng, n, k, 32, from_f32=False)
+    w = sg.Q4Weights.new(q, s, n, k)
+    a = rng.standard_normal((2, k)).astype(np.float16)
+    c = [torch.zeros((2, n), dtype=torch.float16, device="cuda") for _ in range(2)]
+    sg.matmul_q4(torch.from_numpy(a).cuda(), w, c[0], 2)
+    a[other, 77] = what
+    sg.matmul_q4(torch.from_numpy(a).cuda(), w, c[1], 2)
+    assert not torch.isfinite(c[1][other]).all()
+    assert torch.equal(c[0][1 - other].view(torch.int16), c[1][1 - other].view(torch.int16))
