@@ -115,7 +115,7 @@ struct LowbitGemvArgs {
     int log2_block;
     uint32_t lut;                 // 2-bit codebook, byte c = value of code c
     int ns, gpt, kc, kqc;         // launcher-filled: ring depth, column groups per task, fold chunk, staged activation chunk
-    int ntasks, rows_s, u_bytes;  // launcher-filled: tasks along n, rows kept in the shared sums, bytes of the sums / f16-rows region
+    int ntasks, rows_s, u_bytes;  // launcher-filled: tasks along n, rows kept in the shared sums, bytes of the sums / f16-rows region (rows kernel: of a column group's area)
     int dq, dr, dupw, dsc;        // direct kernel: column groups per CTA (quotient, remainder), units per warp, scales staged in shared memory
     unsigned* status;
     EpParams ep;

@@ -159,7 +159,9 @@ __device__ __forceinline__ void quantise_rows(const LowbitGemvArgs& p, unsigned 
                             const uint32_t a0 = amax8(h[0]), a1 = amax8(h[1 % RB]), a2 = amax8(h[2 % RB]), a3 = amax8(h[3 % RB]);
                             uint32_t m01 = max2(__byte_perm(a0, a1, 0x5410), __byte_perm(a0, a1, 0x7632));
                             uint32_t m23 = max2(__byte_perm(a2, a3, 0x5410), __byte_perm(a2, a3, 0x7632));
-                            for (int o = 1; o < lanes; o <<= 1) {
+#pragma unroll
+                            for (int o = 1; o < 32; o <<= 1) {
+                                if (o >= lanes) break;
                                 m01 = max2(m01, __shfl_xor_sync(0xffffffffu, m01, o));
                                 m23 = max2(m23, __shfl_xor_sync(0xffffffffu, m23, o));
                             }
@@ -196,7 +198,9 @@ __device__ __forceinline__ void quantise_rows(const LowbitGemvArgs& p, unsigned 
                     } else if (BITS == 1) {
                         // sums of at most 256 codes, two rows to a word
                         int s01 = qs[0] + qs[1 % RB] * 65536, s23 = qs[2 % RB] + qs[3 % RB] * 65536;
-                        for (int o = 1; o < lanes; o <<= 1) {
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            if (o >= lanes) break;
                             s01 += __shfl_xor_sync(0xffffffffu, s01, o);
                             s23 += __shfl_xor_sync(0xffffffffu, s23, o);
                         }
@@ -236,24 +240,26 @@ __global__ void __launch_bounds__(kRThreads, 1) lowbit_rows_kernel(const __grid_
     const int lparts = p.ns, parts = 1 << lparts, at_once = kRWarps >> lparts;      // parts of a column group's depth, column groups in work
     const int part = warp & (parts - 1), grp = warp >> lparts;
     unsigned char* at = smem_raw;
-    const uint4* ring = reinterpret_cast<const uint4*>(at) + warp * PF * 32 + lane;
-    at += (size_t)kRWarps * PF * kUnitBytes;
     unsigned char* Qs = at;
     at += (size_t)m * p.kq;
-    uint16_t* SCs = reinterpret_cast<uint16_t*>(at) + (size_t)grp * nb * 16;      // [at_once][nb][16]
-    at += (size_t)at_once * nb * 32;
     float* SQ = reinterpret_cast<float*>(at);                       // [nb][activation scales, sums of codes][M8]
     at += (size_t)nb * M8 * 8;
     float* AMX = reinterpret_cast<float*>(at);                      // [nb][M8] (K-blocks longer than 256)
     if (lb > 8) at += (size_t)nb * M8 * 4;
-    float* hand = reinterpret_cast<float*>(at) + grp * NT * 128 + lane * 4;       // [at_once][NT][32] x 4: the totals between parts
-    at += parts > 1 ? (size_t)at_once * NT * 512 : 0;
+    // then an area for each column group in work (a CTA with fewer groups than its warps could take has no more areas than groups)
+    at += (size_t)grp * p.u_bytes;
+    const uint4* ring = reinterpret_cast<const uint4*>(at) + part * PF * 32 + lane;
+    at += (size_t)PF * kUnitBytes << lparts;
+    uint16_t* SCs = reinterpret_cast<uint16_t*>(at);               // [nb][16]
+    at += (size_t)nb * 32;
+    float* hand = reinterpret_cast<float*>(at) + lane * 4;         // [NT][32] x 4: the totals between parts
+    at += NT * 512;
     // this warp's run of the depth, whole K-blocks
     const int lbu = max(lb - (BITS == 2 ? 7 : 8), 0), nbu = (ku + (1 << lbu) - 1) >> lbu;
     const int u_begin = ((part * nbu) >> lparts) << lbu, u_end = min((((part + 1) * nbu) >> lparts) << lbu, ku), mine = u_end - u_begin;
     const int blk0 = (int)(((size_t)u_begin * UD) >> lb);
-    // the sums of the parts behind the first, lane-private: [at_once][parts - 1][gpt blocks][NT][32]
-    float4* keep = reinterpret_cast<float4*>(at) + ((size_t)(grp * (parts - 1) + part - 1) * p.gpt) * NT * 32 + lane;
+    // the sums of the parts behind the first, lane-private: [parts - 1][gpt blocks][NT][32]
+    float4* keep = reinterpret_cast<float4*>(at) + (size_t)((part - 1) * p.gpt) * NT * 32 + lane;
     // this CTA's column groups
     const int first = (int)blockIdx.x * p.dq + min((int)blockIdx.x, p.dr), share = p.dq + ((int)blockIdx.x < p.dr ? 1 : 0);
 
@@ -553,21 +559,32 @@ __global__ void __launch_bounds__(kRThreads, 1) lowbit_rows_kernel(const __grid_
     cpa_wait<0>();
 }
 
-// Column groups of a CTA, parts of their depth and K-blocks of a part, and the shared memory they take (0: too much).
-size_t rows_plan(const LowbitGemvArgs& a, int bits, int sm_count, int* grid, int* parts, int* keep_blocks) {
+// Column groups of a CTA, parts of their depth and K-blocks of a part, the bytes of a column group's area and the shared memory of it
+// all (0: too much, or better left to the kernels for what does not fit).  Only what is at work is counted: a ring a warp that has a
+// part, an area a column group in work.  (With rings and areas for sixteen warps whatever the share, a CTA of one or two groups ran
+// out of memory for its parts' sums and one warp a group did the work; us, that / this, and the kernels before in brackets: 2-bit
+// blocks of 64, 1 row 4096 x 14336 27.6 / 18.3 (17.6), 1-bit 8 rows 1024 x 8192 22.3 / 14.1 (15.3), blocks of 256, 16 rows 1024 x 8192
+// 18.2 / 12.6 (12.9), blocks of 32, 2-bit 1 row 1024 x 8192 19.3 / 10.6 (13.7).)
+size_t rows_plan(const LowbitGemvArgs& a, int bits, int sm_count, int* grid, int* parts, int* keep_blocks, int* area) {
     const int lu = bits == 2 ? 7 : 8, nt = a.m > 8 ? 2 : 1;
     const int bu = a.log2_block > lu ? 1 << (a.log2_block - lu) : 1, nbu = (a.ku + bu - 1) / bu;
     *grid = a.n16 < sm_count ? a.n16 : sm_count;
     const int share = (a.n16 + *grid - 1) / *grid;
-    size_t fixed = (size_t)kRWarps * kRowsRing * kUnitBytes + (size_t)a.m * a.kq + (size_t)a.nb * 8 * nt * 4 * (a.log2_block > 8 ? 3 : 2);
+    const size_t rows = (size_t)a.m * a.kq + (size_t)a.nb * 8 * nt * 4 * (a.log2_block > 8 ? 3 : 2);
     // Four parts at most, eight for long depths: every part's fold waits for the one before it (us with up to 2 / 4 / 8 / 16 parts: 2-bit
     // 1 row 512 x 2048 3.1 / 2.7 / 3.3 / 3.8, 1-bit 1024 x 4096 3.6 / 3.3 / 3.6 / 4.6, 4096 x 14336 12.0 / 11.8 / 9.9 / 9.9).
     for (int q = a.ku >= 48 ? 8 : 4; q >= 1; q >>= 1) {
         if (q > 1 && (q * share > kRWarps || q > nbu)) continue;
         // the most K-blocks of a part: of ceil(nbu / q) runs of bu units
         const size_t blocks = q > 1 ? (((size_t)((nbu + q - 1) / q) * bu << lu) >> a.log2_block) + 1 : 0;
-        const size_t bytes = fixed + (size_t)(kRWarps / q) * a.nb * 32 + (q > 1 ? (size_t)(kRWarps / q) * nt * 512 * (1 + (q - 1) * blocks) : 0);
+        const size_t group = (size_t)q * kRowsRing * kUnitBytes + (size_t)a.nb * 32 + nt * 512 + (q - 1) * blocks * nt * 512;
+        const size_t bytes = rows + (size_t)(kRWarps / q < share ? kRWarps / q : share) * group;
         if (bytes > kRSmemMost) continue;
+        // More than eight rows in one part, with one group a CTA (or two, of K-blocks whose sums lowbit_mma_kernel has room for): one or
+        // two of sixteen warps would do all the work (us, this / the other kernels: 1-bit 16 rows 1024 x 8192 blocks of 64 31.8 / 29.1, 12 rows
+        // 1024 x 16384 blocks of 512 26.2 / 19.5, 4096 x 14336 blocks of 256 26.3 / 25.0; but blocks of 64, 4096 x 8192 30.3 / 33.6).
+        if (q == 1 && nt == 2 && nbu >= 4 && (share == 1 || (share == 2 && a.log2_block >= 8))) return 0;
+        *area = (int)group;
         *parts = q;
         *keep_blocks = (int)blocks;
         return bytes;
@@ -578,15 +595,15 @@ size_t rows_plan(const LowbitGemvArgs& a, int bits, int sm_count, int* grid, int
 }  // namespace
 
 bool lowbit_rows_supported(const LowbitGemvArgs& a, int bits, int sm_count) {
-    int grid, parts, blocks;
-    return a.m >= 1 && a.m <= 16 && a.ku >= 1 && a.k >= 1 && a.log2_block >= 5 && rows_plan(a, bits, sm_count, &grid, &parts, &blocks) != 0;
+    int grid, parts, blocks, area;
+    return a.m >= 1 && a.m <= 16 && a.ku >= 1 && a.k >= 1 && a.log2_block >= 5 && rows_plan(a, bits, sm_count, &grid, &parts, &blocks, &area) != 0;
 }
 
 cudaError_t lowbit_rows_launch(LowbitGemvArgs a, int bits, int sm_count, cudaStream_t stream) {
-    int grid_x = 1, parts = 1, blocks = 0;
-    const size_t smem = rows_plan(a, bits, sm_count, &grid_x, &parts, &blocks);
+    int grid_x = 1, parts = 1, blocks = 0, area = 0;
+    const size_t smem = rows_plan(a, bits, sm_count, &grid_x, &parts, &blocks, &area);
     if (!smem) return cudaErrorInvalidValue;
-    a.ns = 0; a.gpt = blocks;
+    a.ns = 0; a.gpt = blocks; a.u_bytes = area;
     while ((1 << a.ns) < parts) ++a.ns;
     // Graphs of up to four scalars and column vectors without an activation or a division are resolved once a lane: a byte a
     // node, its operation and 8 for a vector.

@@ -292,3 +292,21 @@ def test_resolved_graphs_of_the_kernel_for_few_rows(m):
         c = torch.empty_like(plain)
         sg.matmul_q1_ep(a, w, c, m, ep)
         assert np.array_equal(c.cpu().numpy().view(np.uint16), want.astype(np.float16).view(np.uint16))
+
+
+# Depths whose parts have room only because no more is laid out than is at work (one and two column groups a CTA), for one and
+# two tiles of rows; the last ones are left to other kernels (one part of sixteen, one group a CTA).
+@pytest.mark.parametrize("m,n,k,block", [(1, 70, 14336, 64), (1, 4800, 8192, 32), (2, 64, 16384, 128), (7, 70, 8192, 64), (6, 4800, 4096, 32), (13, 33, 8192, 256),
+                                         (10, 2500, 3000, 64), (16, 70, 4096, 64), (16, 40, 8192, 64), (12, 40, 16384, 512)])
+@pytest.mark.parametrize("kind", [1, 2])
+def test_deep_parts_of_the_kernel_for_few_rows(kind, m, n, k, block):
+    rng = np.random.default_rng(m * 1000 + k)
+    scales = orc.f32_to_f16_bits(rng.uniform(-0.05, 0.05, n * -(-k // block)).astype(np.float32))
+    a_bits = orc.f32_to_f16_bits(rng.standard_normal(m * k).astype(np.float32))
+    wbits = rng.integers(0, 256, (k * n * kind + 7) // 8).astype(np.uint8)
+    if kind == 2:
+        w = sg.Q2Weights.new(wbits, scales, n, k, sg.Q2Params(block).with_codebook(BOOKS[1]))
+        check_bits(w, 2, wbits, 1, scales, BOOKS[1], n, k, block, m, a_bits, "q2")
+    else:
+        w = sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block)
+        check_bits(w, 1, wbits, 0, scales, None, n, k, block, m, a_bits, "q1")
