@@ -880,8 +880,9 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
     // above that every CTA would repeat too much work, and a separate pass over the rows is faster
     static const size_t fuse_max_rows = []() { const char* e = getenv("SMEG_LB_FUSE_MAX_ROWS"); return e ? (size_t)atoi(e) : (size_t)4; }();
     g.a_vec_ok = (k % 8 == 0) && ((uintptr_t)a % 16 == 0);
-    const bool rows_kernel = m <= 16 && lowbit_rows_supported(g, w->bits, ds->sm_count);
-    if (rows_kernel && m * k <= kRowsFused) {
+    const bool rows_kernel = m <= 16 && lowbit_rows_supported(g, w->bits, ds->sm_count) &&
+                             !((int)m <= g_direct_rows && lowbit_direct_shorter(g, w->bits, ds->sm_count));
+    if (rows_kernel && lowbit_rows_quantises(g)) {
         // up to 16 rows, K-blocks of 32 and up: one launch that quantises the rows, multiplies and folds
         g.a = a;
         g.q_out = q_out; g.sa_out = sa_out;

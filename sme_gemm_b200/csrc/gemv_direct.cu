@@ -936,6 +936,17 @@ bool lowbit_direct_supported(const LowbitGemvArgs& a, bool fused) {
     return lowbit_direct_smem(a, 1) <= 110 * 1024;
 }
 
+// lowbit_rows_kernel reads K-blocks above 256 twice before its products, and sixteen warps that hand parts of a depth on have little to do
+// on short ones.  us, there / here: blocks of 512, 1-bit, 1 row 2048 x 512 3.3 / 2.7, 8192 x 1024 5.9 / 5.1, 1024 x 6144 2.8 / 2.6 (but 4096 x
+// 4096 4.3 / 4.8), 2-bit 2 rows 512 x 256 4.0 / 3.3; blocks of 256, 2-bit, 1 row 2048 x 512 3.0 / 2.7 (3072 x 512 3.3 / 3.3), 1-bit 2 rows 1024 x 512
+// 3.8 / 3.5; blocks of 128, 2-bit, 2 rows 512 x 256 3.4 / 3.1 (2048 x 512 4.1 / 4.2; 1-bit 3.3 / 4.1); blocks of 64, 2-bit, 1 row 1024 x 512 2.8 / 2.7.
+bool lowbit_direct_shorter(const LowbitGemvArgs& a, int bits, int sm_count) {
+    if (a.m > 2 || !lowbit_direct_supported(a, true)) return false;
+    const bool one_group = a.n16 <= sm_count;                      // of columns a CTA of that kernel
+    if (a.log2_block > 8) return one_group ? (size_t)a.m * a.k <= 12288 : a.n16 <= 3 * sm_count && a.k <= 4096 - 1024 * a.m;
+    return one_group && a.k > 256 && (a.log2_block == 8 ? a.k <= 2048 : bits == 2 && a.log2_block >= 6 && a.k <= 1024);
+}
+
 cudaError_t lowbit_direct_launch(LowbitGemvArgs a, int bits, int sm_count, cudaStream_t stream) {
     int cpc = 1, maxg = 16;
     int grid_x = direct_grid(a.n16, sm_count, maxg, &cpc, 3);

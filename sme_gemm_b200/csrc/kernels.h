@@ -126,12 +126,13 @@ bool lowbit_gemv_fuses_quant(LowbitGemvArgs a, int bits, int sm_count);
 // itself (a.a set, at most two rows); otherwise a.q / a.sa / a.qsum come from act_quant_kernel.
 bool lowbit_direct_supported(const LowbitGemvArgs& a, bool fused);
 cudaError_t lowbit_direct_launch(LowbitGemvArgs a, int bits, int sm_count, cudaStream_t stream);
+// Is a call of one or two rows that quantises them itself shorter there than on lowbit_rows_kernel?
+bool lowbit_direct_shorter(const LowbitGemvArgs& a, int bits, int sm_count);
 // One to sixteen rows, K-blocks of 32 and up, on int8 warp-level tensor-core instructions (lowbit_rows.cu): quantises the f16 rows
 // itself (a.a set) or takes a.q / a.sa / a.qsum (1-bit) from act_quant_kernel.
 constexpr int kRowsRing = 8;                                       // units on their way per warp
-// Most values (rows x depth) that every CTA quantises for itself; above, act_quant_kernel runs in front (us, together / in front: 8 x
-// 14336 x 4096 13.7 / 14.4, 9 x 8192 x 6144 16.4 / 14.4, 6 x 1024 x 8192 10.1 / 9.1, 16 x 256 x 512 3.4 / 4.8).
-constexpr size_t kRowsFused = 40960;
+// Does every CTA quantise the rows for itself?  Else act_quant_kernel runs in front.
+bool lowbit_rows_quantises(const LowbitGemvArgs& a);
 bool lowbit_rows_supported(const LowbitGemvArgs& a, int bits, int sm_count);
 cudaError_t lowbit_rows_launch(LowbitGemvArgs a, int bits, int sm_count, cudaStream_t stream);
 // Up to sixteen rows on warp-level tensor-core instructions, exact block sums (lowbit_mma.cu); a.q / a.sa / a.qsum from

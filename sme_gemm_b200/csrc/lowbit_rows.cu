@@ -10,7 +10,7 @@
 // weight 2^0, 2^2, 2^4, 2^6 (twice that for columns g + 8), and 4-fold adds and one shift at a block's end make the sum of them.
 //
 // One CTA of sixteen warps per SM.  It quantises the rows into shared memory itself, in the order of the B fragments (or copies
-// the codes act_quant_kernel made, for more than kRowsFused values: every CTA repeats it), while its weights are on their way: a lane copies its own 16 bytes of every unit into its own ring slots (cp.async).  A warp takes a column group, or a part of
+// the codes act_quant_kernel made, where lowbit_rows_quantises says no: every CTA repeats it), while its weights are on their way: a lane copies its own 16 bytes of every unit into its own ring slots (cp.async).  A warp takes a column group, or a part of
 // its depth where a CTA has fewer groups than warps; block sums are whole in a warp, so the first part folds them in registers as
 // they come, in K order (total = fmaf((float)sum, scale * sa, total), the reference's bits), and each later one keeps its sums in
 // lane-private shared memory until the part before hands its totals on.
@@ -597,6 +597,16 @@ size_t rows_plan(const LowbitGemvArgs& a, int bits, int sm_count, int* grid, int
 bool lowbit_rows_supported(const LowbitGemvArgs& a, int bits, int sm_count) {
     int grid, parts, blocks, area;
     return a.m >= 1 && a.m <= 16 && a.ku >= 1 && a.k >= 1 && a.log2_block >= 5 && rows_plan(a, bits, sm_count, &grid, &parts, &blocks, &area) != 0;
+}
+
+// Up to 40960 values (us, in the CTAs / in front, 1-bit blocks of 128: 16 rows 512 x 256 3.8 / 4.9, 8 rows 4096 x 14336 8.5 / 9.6, 9 rows 4096 x
+// 4096 9.0 / 9.2; rows of 8192 depths and more meet earlier, 5 of 8192 x 1024 9.4 / 8.3).  K-blocks longer than a warp's run are read twice,
+// for their maxima first: one round of sixteen runs of eight rows, or two of one row (blocks of 512, 1-bit: 8 rows 4096 x 4096 7.3 / 7.5, 1 row
+// 8192 x 4096 6.3 / 7.0; 9 rows 4096 x 4096 9.9 / 8.4, 2 rows 8192 x 4096 9.3 / 7.8, 6 rows 6144 x 8192 11.8 / 9.4).
+bool lowbit_rows_quantises(const LowbitGemvArgs& a) {
+    if (a.log2_block <= 8) return (size_t)a.m * a.k <= 40960;
+    const int chunks = (a.kq + 255) / 256, deal = a.m == 1 || chunks > 8 ? 1 : chunks > 4 ? 2 : 4;      // (as in quantise_rows)
+    return (chunks + kRWarps - 1) / kRWarps * ((a.m + 8 * deal - 1) / (8 * deal)) <= (a.m == 1 ? 2 : 1);
 }
 
 cudaError_t lowbit_rows_launch(LowbitGemvArgs a, int bits, int sm_count, cudaStream_t stream) {

@@ -310,3 +310,21 @@ def test_deep_parts_of_the_kernel_for_few_rows(kind, m, n, k, block):
     else:
         w = sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block)
         check_bits(w, 1, wbits, 0, scales, None, n, k, block, m, a_bits, "q1")
+
+
+# Either side of the lines between the kernel for few rows and the one for one and two (whose long K-blocks are longer than a unit), and
+# between quantising in the CTAs and in front for K-blocks above 256.
+@pytest.mark.parametrize("m,n,k,block", [(1, 100, 2048, 256), (2, 100, 2050, 256), (1, 64, 257, 64), (2, 40, 1024, 128), (1, 70, 12288, 512), (1, 2400, 3000, 1024), (2, 40, 6144, 4096),
+                                         (2, 40, 6400, 1024), (8, 64, 4096, 512), (9, 64, 3000, 512), (16, 40, 2048, 2048), (3, 40, 4200, 8192)])
+@pytest.mark.parametrize("kind", [1, 2])
+def test_lines_of_the_dispatch_at_few_rows(kind, m, n, k, block):
+    rng = np.random.default_rng(m * 1000 + k)
+    scales = orc.f32_to_f16_bits(rng.uniform(-0.05, 0.05, n * -(-k // block)).astype(np.float32))
+    a_bits = orc.f32_to_f16_bits(rng.standard_normal(m * k).astype(np.float32))
+    wbits = rng.integers(0, 256, (k * n * kind + 7) // 8).astype(np.uint8)
+    if kind == 2:
+        w = sg.Q2Weights.new(wbits, scales, n, k, sg.Q2Params(block).with_codebook(BOOKS[2]))
+        check_bits(w, 2, wbits, 1, scales, BOOKS[2], n, k, block, m, a_bits, "q2")
+    else:
+        w = sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block)
+        check_bits(w, 1, wbits, 0, scales, None, n, k, block, m, a_bits, "q1")
