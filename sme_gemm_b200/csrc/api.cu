@@ -56,8 +56,8 @@ int g_direct_rows = []() {
     return v < 0 ? 0 : (v > 4 ? 4 : v);
 }();
 
-// Rows from which 2-bit / 1-bit calls form their block sums on the tensor cores (lowbit_tc.cu); below it, and above
-// the direct kernels' rows, the warp-level kernel runs.  SMEG_LOWBIT_TC_MIN_ROWS is a tuning knob (0 = never).
+// Rows from which 2-bit / 1-bit calls form their block sums on tcgen05 (lowbit_tc.cu); below it, and always up to g_direct_rows, the
+// kernels for few rows run.  SMEG_LOWBIT_TC_MIN_ROWS is a tuning knob (0 = never).
 int g_lowbit_tc = []() {
     const char* e = getenv("SMEG_LOWBIT_TC_MIN_ROWS");
     return e ? atoi(e) : 17;
@@ -876,11 +876,11 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
     g.log2_block = w->d.log2_block; g.lut = w->lut; g.status = ds->status;
     cudaError_t e = cudaSuccess;
     char* ws = nullptr;
-    // up to four rows the kernel stages and quantises the activations itself (one launch, no scratch);
-    // above that every CTA would repeat too much work, and a separate pass over the rows is faster
+    // (SMEG_LB_FUSE_MAX_ROWS: rows that the staged dp4a kernel quantises itself, where SMEG_DIRECT_ROWS=0 and lowbit_rows_kernel leave it a call)
     static const size_t fuse_max_rows = []() { const char* e = getenv("SMEG_LB_FUSE_MAX_ROWS"); return e ? (size_t)atoi(e) : (size_t)4; }();
     g.a_vec_ok = (k % 8 == 0) && ((uintptr_t)a % 16 == 0);
-    const bool rows_kernel = m <= 16 && lowbit_rows_supported(g, w->bits, ds->sm_count) &&
+    const bool tc = (int)m > g_direct_rows && g_lowbit_tc > 0 && (int)m >= g_lowbit_tc && lowbit_tc_supported(w->bits, (int)m, (int)k, w->d.log2_block);
+    const bool rows_kernel = !tc && m <= 16 && lowbit_rows_supported(g, w->bits, ds->sm_count) &&
                              !((int)m <= g_direct_rows && lowbit_direct_shorter(g, w->bits, ds->sm_count));
     if (rows_kernel && lowbit_rows_quantises(g)) {
         // up to 16 rows, K-blocks of 32 and up: one launch that quantises the rows, multiplies and folds
@@ -898,11 +898,9 @@ static int lowbit_dev(const smeg_lowbit* w, const uint16_t* a, uint16_t* c, size
         g.q_out = q_out; g.sa_out = sa_out;
         e = lowbit_gemv_launch(g, w->bits, ds->sm_count, stream);
     } else {
-        // quantise first, into stream-ordered scratch; above the direct kernels' rows the block sums run on the
-        // tensor cores (lowbit_tc.cu), which wants the per-block scales and sums block-major as well
-        const bool tc = (int)m > g_direct_rows && g_lowbit_tc > 0 && (int)m >= g_lowbit_tc && lowbit_tc_supported(w->bits, (int)m, (int)k, w->d.log2_block);
-        // between the two, warp-level tensor-core instructions (lowbit_mma.cu); SMEG_LOWBIT_MMA=0 leaves those row counts
-        // to the staged dp4a kernel
+        // quantise first, into stream-ordered scratch (tcgen05's kernel wants the per-block scales and sums block-major as well).  Five to
+        // sixteen rows that lowbit_rows_kernel has no room for: f16 warp-level instructions (lowbit_mma.cu); SMEG_LOWBIT_MMA=0 leaves
+        // those to the staged dp4a kernel
         static const int use_mma = []() { const char* e = getenv("SMEG_LOWBIT_MMA"); return e ? atoi(e) : 1; }();
         bool mma = false;
         if (!rows_kernel && !tc && use_mma && (int)m > g_direct_rows && m <= 16) {

@@ -3,6 +3,8 @@ oracle (quantize_row + reference, src/kernels/lowbit/matmul.rs:354-398) --
 int8 activation codes, per-block activation scales, int32 block sums and the f16
 output, for the reference's own shape / block / codebook / layout grid
 (src/kernels/lowbit/matmul.rs:419-494), through the C ABI."""
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -328,3 +330,44 @@ def test_lines_of_the_dispatch_at_few_rows(kind, m, n, k, block):
     else:
         w = sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block)
         check_bits(w, 1, wbits, 0, scales, None, n, k, block, m, a_bits, "q1")
+
+
+_COUNT_NODES = r"""
+import numpy as np, torch
+import sme_gemm_b200 as sg
+from cuda.bindings import runtime as rt
+rng = np.random.default_rng(0)
+n, k = 64, 512
+w = sg.Q1Weights.new(rng.integers(0, 256, n * k // 8).astype(np.uint8), np.full(n * k // 128, 0.01, np.float16).view(np.uint16), sg.WeightLayout.OutIn, n, k, 128)
+s = torch.cuda.Stream()
+for m in (4, 7, 9):
+    a = torch.ones((m, k), dtype=torch.float16, device="cuda")
+    c = torch.empty((m, n), dtype=torch.float16, device="cuda")
+    with torch.cuda.stream(s):
+        sg.matmul_q1(a, w, c, m)
+        s.synchronize()
+        assert rt.cudaStreamBeginCapture(s.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal)[0] == 0
+        sg.matmul_q1(a, w, c, m)
+        err, graph = rt.cudaStreamEndCapture(s.cuda_stream)
+    assert err == 0
+    err, _, count = rt.cudaGraphGetNodes(graph)
+    err, nodes, count = rt.cudaGraphGetNodes(graph, count)
+    kinds = [rt.cudaGraphNodeGetType(x)[1] for x in nodes[:count]]
+    print(m, sum(x == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for x in kinds))
+    rt.cudaGraphDestroy(graph)
+"""
+
+
+@pytest.mark.parametrize("knob,launches", [(None, {4: 1, 7: 1, 9: 1}), ("8", {4: 1, 7: 1, 9: 2})])
+def test_rows_from_which_tcgen05_takes_a_call(knob, launches):
+    """SMEG_LOWBIT_TC_MIN_ROWS holds for calls of any size: from its rows on a call is the quantisation and the tcgen05 kernel, two
+    launches, where the kernel for few rows is one."""
+    import subprocess
+    import sys
+    env = {x: v for x, v in os.environ.items() if x != "SMEG_LOWBIT_TC_MIN_ROWS"}
+    if knob:
+        env["SMEG_LOWBIT_TC_MIN_ROWS"] = knob
+    env["PYTHONPATH"] = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _COUNT_NODES], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    assert dict(map(int, line.split()) for line in r.stdout.splitlines()) == launches
