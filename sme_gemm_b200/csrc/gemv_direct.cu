@@ -930,6 +930,7 @@ static size_t lowbit_direct_smem(const LowbitGemvArgs& a, int cpc) {
 
 bool lowbit_direct_supported(const LowbitGemvArgs& a, bool fused) {
     if (a.m < 1 || a.m > 4 || a.ku < 1 || a.k < 1) return false;
+    if (a.m > 2 && a.log2_block > 4) return false;               // (lowbit_rows_kernel has room for whatever this kernel has)
     if (fused && a.m > 2) return false;                          // every CTA repeats the quantisation
     // in-kernel quantisation walks a row in rounds of 8192 depths: a K-block must lie inside one round
     if (fused && a.kq > 8192 && ((1 << a.log2_block) > 8192 || 8192 % (1 << a.log2_block) != 0)) return false;
@@ -959,19 +960,15 @@ cudaError_t lowbit_direct_launch(LowbitGemvArgs a, int bits, int sm_count, cudaS
     cudaError_t e;
     const int ud = bits == 2 ? kQ2UnitDepth : kQ1UnitDepth;
     const bool big = (1 << a.log2_block) >= ud;
-#define SMEG_LD(BB, MM)                                                                   \
-    if (bits == BB && a.m == MM) {                                                        \
-        if (big) {                                                                        \
-            e = opt_in_smem(lowbit_direct_kernel<BB, MM, 1>, smem);                       \
-            if (e != cudaSuccess) return e;                                               \
-            return launch_pdl(lowbit_direct_kernel<BB, MM, 1>, grid, dim3(kDThreads), smem, stream, a); \
-        }                                                                                 \
-        e = opt_in_smem(lowbit_direct_kernel<BB, MM, 0>, smem);                           \
+#define SMEG_LD(BB, MM, GG)                                                               \
+    if (bits == BB && a.m == MM && big == (GG == 1)) {                                    \
+        e = opt_in_smem(lowbit_direct_kernel<BB, MM, GG>, smem);                          \
         if (e != cudaSuccess) return e;                                                   \
-        return launch_pdl(lowbit_direct_kernel<BB, MM, 0>, grid, dim3(kDThreads), smem, stream, a); \
+        return launch_pdl(lowbit_direct_kernel<BB, MM, GG>, grid, dim3(kDThreads), smem, stream, a); \
     }
-    SMEG_LD(2, 1) SMEG_LD(2, 2) SMEG_LD(2, 3) SMEG_LD(2, 4)
-    SMEG_LD(1, 1) SMEG_LD(1, 2) SMEG_LD(1, 3) SMEG_LD(1, 4)
+    // (three and four rows come here under K-blocks of 16 alone)
+    SMEG_LD(2, 1, 0) SMEG_LD(2, 2, 0) SMEG_LD(2, 3, 0) SMEG_LD(2, 4, 0) SMEG_LD(2, 1, 1) SMEG_LD(2, 2, 1)
+    SMEG_LD(1, 1, 0) SMEG_LD(1, 2, 0) SMEG_LD(1, 3, 0) SMEG_LD(1, 4, 0) SMEG_LD(1, 1, 1) SMEG_LD(1, 2, 1)
 #undef SMEG_LD
     return cudaErrorInvalidValue;
 }

@@ -371,3 +371,40 @@ def test_rows_from_which_tcgen05_takes_a_call(knob, launches):
     r = subprocess.run([sys.executable, "-c", _COUNT_NODES], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
     assert dict(map(int, line.split()) for line in r.stdout.splitlines()) == launches
+
+
+# Five to sixteen rows whose codes do not fit a CTA, or would be one part of one group's depth: the kernel on f16 instructions, one and
+# two tiles of rows, K-blocks of a unit and longer and (two tiles, 1-bit) shorter ones; the last is left to the staged kernel.
+@pytest.mark.parametrize("kind,m,n,k,block", [(1, 8, 40, 28672, 256), (2, 8, 40, 28672, 256), (2, 5, 24, 60000, 1024), (1, 12, 40, 16384, 512), (2, 12, 40, 16384, 512),
+                                              (2, 12, 33, 16000, 256), (1, 9, 40, 15360, 128), (1, 16, 40, 8192, 64), (2, 16, 24, 8192, 32)])
+def test_deep_rows_of_the_kernels_behind(kind, m, n, k, block):
+    rng = np.random.default_rng(m * 1000 + k)
+    scales = orc.f32_to_f16_bits(rng.uniform(-0.05, 0.05, n * -(-k // block)).astype(np.float32))
+    a_bits = orc.f32_to_f16_bits(rng.standard_normal(m * k).astype(np.float32))
+    wbits = rng.integers(0, 256, (k * n * kind + 7) // 8).astype(np.uint8)
+    if kind == 2:
+        w = sg.Q2Weights.new(wbits, scales, n, k, sg.Q2Params(block).with_codebook(BOOKS[2]))
+        check_bits(w, 2, wbits, 1, scales, BOOKS[2], n, k, block, m, a_bits, "q2")
+    else:
+        w = sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block)
+        check_bits(w, 1, wbits, 0, scales, None, n, k, block, m, a_bits, "q1")
+
+
+@pytest.mark.parametrize("kind,m,k,block", [(1, 5, 6464, 32), (2, 5, 6560, 32), (2, 9, 7520, 64)])
+def test_wide_matrices_of_the_kernel_behind(kind, m, k, block):
+    """K-blocks shorter than a unit reach the kernel on f16 instructions where a CTA has sixteen groups whose scale rows leave its codes
+    no room: each row's bits are those of a call of that row alone, which runs on the kernel for few rows."""
+    n = 35600
+    rng = np.random.default_rng(k)
+    scales = orc.f32_to_f16_bits(rng.uniform(-0.05, 0.05, n * -(-k // block)).astype(np.float32))
+    wbits = rng.integers(0, 256, (k * n * kind + 7) // 8, dtype=np.uint8)
+    if kind == 2:
+        w, f = sg.Q2Weights.new(wbits, scales, n, k, sg.Q2Params(block).with_codebook(BOOKS[1])), sg.matmul_q2
+    else:
+        w, f = sg.Q1Weights.new(wbits, scales, sg.WeightLayout.OutIn, n, k, block), sg.matmul_q1
+    a = f16_bits_dev(orc.f32_to_f16_bits(rng.standard_normal(m * k).astype(np.float32))).reshape(m, k)
+    c, one = torch.zeros((m, n), dtype=torch.float16, device="cuda"), torch.zeros((1, n), dtype=torch.float16, device="cuda")
+    f(a, w, c, m)
+    for r in range(m):
+        f(a[r:r + 1].contiguous(), w, one, 1)
+        assert np.array_equal(_canon16(bits_of(c[r:r + 1])), _canon16(bits_of(one)))
