@@ -870,26 +870,38 @@ cudaError_t q4_direct_launch(Q4GemvArgs a, int sm_count, cudaStream_t stream) {
     a.n16 = n16;
     // three CTAs per SM when the matrix gives every SM that many, else two (and then never three on one SM
     // while another has one: the shared-memory request is padded past a third of an SM's)
-    const int per_sm = n16 > 2 * sm_count ? 3 : 2;
+    int per_sm = n16 > 2 * sm_count ? 3 : 2;
     int grid_x;
-    if (a.glu) {
-        // shares are (gate group, up group) pairs: n16 / 2 of them, at most 8 (16 groups) per CTA
-        const int pairs = n16 / 2;
-        int cpp = 1;
-        grid_x = direct_grid(pairs, sm_count, 8, &cpp, per_sm);
-        a.cg = 2 * cpp;
-        a.dq = pairs / grid_x; a.dr = pairs % grid_x;
-    } else {
-        grid_x = direct_grid(n16, sm_count, 16, &a.cg, per_sm);
-        a.dq = n16 / grid_x; a.dr = n16 % grid_x;
-    }
+    auto split = [&]() {
+        if (a.glu) {
+            // shares are (gate group, up group) pairs: n16 / 2 of them, at most 8 (16 groups) per CTA
+            const int pairs = n16 / 2;
+            int cpp = 1;
+            grid_x = direct_grid(pairs, sm_count, 8, &cpp, per_sm);
+            a.cg = 2 * cpp;
+            a.dq = pairs / grid_x; a.dr = pairs % grid_x;
+        } else {
+            grid_x = direct_grid(n16, sm_count, 16, &a.cg, per_sm);
+            a.dq = n16 / grid_x; a.dr = n16 % grid_x;
+        }
+    };
+    split();
     cudaError_t e;
     if (ns >= kDWarps && !a.nx) {
         // At least a stage of 256 depths for each warp.  (Shorter depths stay with the kernel below, whose warps have a unit each
         // where a stage would have one warp in work: us, this / that, 1 row: 1536 x 384 2.06 / 1.72, 4096 x 1024 2.40 / 2.06,
         // 3072 x 2048 2.57 / 2.58, 1024 x 4096 2.7 / 3.2.)
+        // As many CTAs per SM as have room with three slots (of 228 KB, each with 1 KB of the system's): one more would be the half wave
+        // behind (us, three or two whatever their size / this: 2 rows 28672 x 4096 18.2 / 13.4, 5120 x 5120 8.4 / 5.7, 1 row 5120 x 13824
+        // 12.6 / 9.4, 28672 x 8192 26.4 / 21.5).
         // Ring: three slots where three CTAs share an SM; of two, each takes what its rows leave of half an SM, up to five.
-        const size_t slot = (size_t)kDWarps * q4_slot_bytes(a.m), rest = q4_rows_bytes(a.m, ns) + (size_t)kDWarps * a.cg * a.m * 16 * sizeof(float);
+        const size_t slot = (size_t)kDWarps * q4_slot_bytes(a.m);
+        auto rest_bytes = [&]() { return q4_rows_bytes(a.m, ns) + (size_t)kDWarps * a.cg * a.m * 16 * sizeof(float); };
+        while (per_sm > 1 && 3 * slot + rest_bytes() > (per_sm == 3 ? 75 : 113) * (size_t)1024) {
+            --per_sm;
+            split();
+        }
+        const size_t rest = rest_bytes();
         const int pf = per_sm > 2 ? 3 : 5 * slot + rest <= 112 * 1024 ? 5 : 4 * slot + rest <= 112 * 1024 ? 4 : 3;
         size_t bytes = pf * slot + rest;
         if (per_sm == 2 && bytes < 80 * 1024) bytes = 80 * 1024;

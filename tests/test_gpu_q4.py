@@ -508,3 +508,36 @@ def test_a_finite_row_keeps_its_bits_beside_one_with_infinities(other, what):
     sg.matmul_q4(torch.from_numpy(a).cuda(), w, c[1], 2)
     assert not torch.isfinite(c[1][other]).all()
     assert torch.equal(c[0][1 - other].view(torch.int16), c[1][1 - other].view(torch.int16))
+
+
+# As many CTAs an SM as have room: three become two (one and two rows), two become one.
+@pytest.mark.parametrize("m,n,k,glu", [(2, 4752, 4096, False), (1, 4752, 9216, False), (2, 2400, 11008, False), (1, 2384, 24000, False), (2, 1024, 14336, False),
+                                       (2, 33, 14400, False), (2, 4800, 4096, True), (2, 4800, 11008, True)])
+def test_one_and_two_rows_where_fewer_ctas_fit(m, n, k, glu):
+    """Against the same rows one at a time in f32 sums of the weights themselves (an f16 store, 2^-11, and f32 sums as above)."""
+    rng = np.random.default_rng(n + k)
+    q = rng.integers(0, 256, n * k // 2, dtype=np.uint8)
+    s = rng.uniform(0.002, 0.01, n * (k // 32)).astype(np.float16)
+    w = sg.Q4Weights.new(q, s.view(np.uint16), n, k)
+    a = rng.standard_normal((m, k)).astype(np.float16)
+    codes = torch.from_numpy(np.stack([q & 15, q >> 4], 1).astype(np.int8).reshape(k, n)).cuda()
+    codes = (codes - 16 * (codes > 7)).float()
+    scale = torch.from_numpy(s.astype(np.float32)).cuda().view(n, k // 32).t()
+    blocks = torch.einsum("mbd,bdn->mbn", torch.from_numpy(a).cuda().double().view(m, k // 32, 32), codes.view(k // 32, 32, n).double())
+    want = (blocks * scale.double()).sum(1)
+    if not glu:
+        c = torch.zeros((m, n), dtype=torch.float16, device="cuda")
+        sg.matmul_q4(torch.from_numpy(a).cuda(), w, c, m)
+        big = torch.from_numpy(np.abs(a)).cuda().double() @ (16 * scale.double().repeat_interleave(32, 0))
+        assert torch.all((c.double() - want).abs() <= 2.0 ** -11 * want.abs() + 2.0 ** -24 + 16 * 2.0 ** -24 * big)
+        return
+    # gate and up columns interleaved by 32: the block's hidden units, rounded as the separate passes round them
+    down = sg.Linear.from_q4(sg.Q4Weights.new(*q4_logical(rng, 64, n // 2, 32, from_f32=False), 64, n // 2))
+    mlp = sg.Mlp.gated(sg.GatedLinear(sg.Linear.from_q4(w), sg.Gate.Silu), down)
+    y = torch.zeros((m, 64), device="cuda")
+    mlp.accumulate(torch.from_numpy(a).cuda(), y, m)
+    v = want.view(m, n // 64, 2, 32).half().double()
+    hidden = (v[:, :, 0] * torch.sigmoid(v[:, :, 0]) * v[:, :, 1]).reshape(m, n // 2).half()
+    got = torch.zeros((m, 64), dtype=torch.float16, device="cuda")
+    sg.matmul_q4(hidden, down.q4, got, m)
+    assert max_rel(y.cpu().numpy(), got.float().cpu().numpy()) <= TOL
