@@ -2,7 +2,8 @@
 //   q4_stage_kernel       C[m][n] = ep( A[m][k] @ dequant(W) ), Q4 weights, f16, K-blocks of 32 and up, one or two rows
 //                         of whole 16-byte words, on warp-level tensor-core instructions
 //   q4_direct_kernel      the same in packed f16 arithmetic, for depths below 1793, and the form that norms its rows
-//   lowbit_direct_kernel  2-bit / 1-bit weights against int8-quantised activations (matmul_q2 / matmul_q1), one to four rows
+//   lowbit_direct_kernel  2-bit / 1-bit weights against int8-quantised activations (matmul_q2 / matmul_q1): one to four rows under
+//                         K-blocks of 16, short calls of one and two rows (lowbit_direct_shorter)
 //
 // They replace the reference's SME GEMV kernels for the batch sizes a decode step has
 // (run_q4_gemv1 / run_q4_gemv, csrc/gemm_f16f16_q4.h:236-431; run_q2_gemv, csrc/gemm_q2.cc:300-404).
@@ -28,7 +29,7 @@
 //     6e-5 -- calls that have f32 sums elsewhere (q4_mma_kernel) are not brought here for speed;
 //   * 2-bit / 1-bit: the activation rows are quantised to int8 in shared memory by the CTA itself
 //     (one or two rows; bit-exact quantize_row, src/kernels/lowbit/matmul.rs:354-371) or copied from
-//     act_quant_kernel's output (three or four rows); codes are expanded in registers (2-bit: byte
+//     act_quant_kernel's output (more); codes are expanded in registers (2-bit: byte
 //     permute of the 4-entry codebook, 1-bit: {0,1} bytes with sum = 2S - sum(q)), dot products
 //     run on dp4a, exact int32 block sums meet in shared memory and one thread per output cell
 //     folds them in K order with fmaf((float)sum, scale * sa, total) -- the reference's bits.
@@ -307,9 +308,13 @@ __global__ void __launch_bounds__(kDThreads, 3) q4_direct_kernel(const __grid_co
 //     lane (g, t) takes vectors of unit t, B is zero but where its column's K-block meets its depths, and after sixteen MMAs
 //     the accumulators are the sums of eight K-blocks, folded at once (12 instructions instead of 128);
 //   * the copies are coalesced a unit at a time and read back across the lanes, under an XOR of the unit's number.
-// 67 warp instructions a unit (us, graph replays; q4_direct_kernel / this): 1 row, 28672 x 4096 18.2 / 13.0 (5.1 TB/s), 4096 x 14336
-// 11.6 / 8.3, 4096 x 4096 3.95 / 3.35; 2 rows, 14336 x 4096 14.1 / 11.7.  From 14336 to 28672 columns it adds 33 MB in 5.4 us, 6.0 TB/s:
-// what is left is the time to the first byte and the last wave's end.  Sums are f32 throughout (q4_direct_kernel: f16 over 8 depths).
+// 61 warp instructions a unit (us, graph replays; q4_direct_kernel / this): 1 row, 28672 x 4096 17.8 / 12.3 (5.4 TB/s), 4096 x 14336
+// 10.8 / 7.5, 4096 x 4096 3.95 / 3.25; 2 rows, 14336 x 4096 14.0 / 8.4 (but 1024 x 14336 7.9 / 8.5: rows that leave an SM room for one CTA).
+// From 14336 to 28672 columns it adds 33 MB in 5.3 us, 6.2 TB/s: what is left is the time to the first byte and the last wave's end.
+// Sums are f32 throughout (q4_direct_kernel: f16 over 8 depths): 2-norm of the error against 64 bits 2.1e-4 of the result, an exact
+// product's f16 store, where q4_direct_kernel has 4.9e-4 (1 and 2 rows, 1024 to 14336 columns, 2048 to 14336 depths, blocks of 32 to 128).
+// What a K-block's sum loses goes with 8 sum|a|, whatever its codes: columns of nothing but zero codes under nonzero scales are not
+// exactly zero (up to 1.4e-6 with scales of 0.01 over 4096 normal activations, under the f16 store of any other column).
 // Shared memory: ring [8 warps][PF] of a stage's codes and scale words | A rows [M][units * 72] f16 (a unit's 64 depths
 // and 8 halves of padding) | the blocks' start values [stages][8 M] f32 | the cross-warp exchange [8 warps][CPC][M][16] f32.
 // ---------------------------------------------------------------------------------------------

@@ -122,7 +122,7 @@ struct LowbitGemvArgs {
 };
 cudaError_t lowbit_gemv_launch(LowbitGemvArgs a, int bits, int sm_count, cudaStream_t stream);
 bool lowbit_gemv_fuses_quant(LowbitGemvArgs a, int bits, int sm_count);
-// One to four rows: plain 128-bit loads and dp4a (gemv_direct.cu).  fused: the kernel quantises the f16 rows
+// K-blocks of 16 at one to four rows, any at one and two: plain 128-bit loads and dp4a (gemv_direct.cu).  fused: the kernel quantises the f16 rows
 // itself (a.a set, at most two rows); otherwise a.q / a.sa / a.qsum come from act_quant_kernel.
 bool lowbit_direct_supported(const LowbitGemvArgs& a, bool fused);
 cudaError_t lowbit_direct_launch(LowbitGemvArgs a, int bits, int sm_count, cudaStream_t stream);

@@ -1,5 +1,6 @@
-// 2-bit / 1-bit matmul for five to sixteen activation rows whose codes and K-blocks do not fit one CTA's shared memory beside its rings
-// (lowbit_rows.cu takes the others; 16 rows of 8192 depths, say, come here) (sm_100a): the exact int32 block sums of
+// 2-bit / 1-bit matmul for five to sixteen activation rows that lowbit_rows.cu leaves (sm_100a): codes and K-blocks that do not fit one CTA's
+// shared memory beside its rings (8 rows of 28672 depths, say), or more than eight rows that would be one part of one column group's
+// depth (12 of 16384 under K-blocks of 512).  The exact int32 block sums of
 // matmul_q2 / matmul_q1 (run_q2_gemv, csrc/gemm_q2.cc:300-404; block_sums, src/kernels/lowbit/matmul.rs:373-421)
 // formed by warp-level tensor-core instructions, then the reference's ordered fold.
 //

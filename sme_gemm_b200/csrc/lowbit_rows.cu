@@ -18,8 +18,9 @@
 // What bounds it: instruction issue and, at its ends, latency (350 warp instructions a 1-bit unit at eight rows, 110 of them the
 // quantisation, issue slots half busy; of 16000 cycles of an 8 x 4096 x 14336 call 5200 go into the quantisation, 6700 into the
 // products, 2600 into the second parts' folds and the stores).  Against act_quant_kernel and the kernels that took these calls
-// before (dp4a to four rows, f16 MMAs on subnormal weights above; us, graph replays): 1-bit 8 x 4096 x 14336 15.9 -> 8.4, 1 row 4096 x
-// 4096 6.1 -> 3.3, 1 row 14336 x 4096 11.3 -> 5.8, 16 rows 27.3 -> 13.3; 2-bit 1 row 11008 x 4096 7.75 -> 6.2, 3 rows 14336 x 4096 16.4 -> 8.7.
+// before (dp4a to four rows, f16 MMAs on subnormal weights above; us, graph replays; rows x depth x columns): 1-bit 8 x 4096 x 14336 15.9 ->
+// 8.4, 1 x 4096 x 4096 6.1 -> 3.9, 1 x 4096 x 14336 11.3 -> 5.8, 16 x 4096 x 14336 27.3 -> 13.7; 2-bit 1 x 4096 x 11008 7.75 -> 6.1, 3 x 4096 x 14336
+// 16.4 -> 8.5.
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"
@@ -562,9 +563,9 @@ __global__ void __launch_bounds__(kRThreads, 1) lowbit_rows_kernel(const __grid_
 // Column groups of a CTA, parts of their depth and K-blocks of a part, the bytes of a column group's area and the shared memory of it
 // all (0: too much, or better left to the kernels for what does not fit).  Only what is at work is counted: a ring a warp that has a
 // part, an area a column group in work.  (With rings and areas for sixteen warps whatever the share, a CTA of one or two groups ran
-// out of memory for its parts' sums and one warp a group did the work; us, that / this, and the kernels before in brackets: 2-bit
-// blocks of 64, 1 row 4096 x 14336 27.6 / 18.3 (17.6), 1-bit 8 rows 1024 x 8192 22.3 / 14.1 (15.3), blocks of 256, 16 rows 1024 x 8192
-// 18.2 / 12.6 (12.9), blocks of 32, 2-bit 1 row 1024 x 8192 19.3 / 10.6 (13.7).)
+// out of memory for its parts' sums and one warp a group did the work; us, that / this, and the kernels before in brackets: columns x depth: 2-bit
+// blocks of 64, 1 row 4096 x 14336 27.5 / 18.2 (17.6), 1-bit 8 rows 1024 x 8192 22.2 / 12.8 (15.3), blocks of 256, 16 rows 1024 x 8192
+// 18.1 / 12.4 (12.9), blocks of 32, 2-bit 1 row 1024 x 8192 19.2 / 9.6 (13.7).)
 size_t rows_plan(const LowbitGemvArgs& a, int bits, int sm_count, int* grid, int* parts, int* keep_blocks, int* area) {
     const int lu = bits == 2 ? 7 : 8, nt = a.m > 8 ? 2 : 1;
     const int bu = a.log2_block > lu ? 1 << (a.log2_block - lu) : 1, nbu = (a.ku + bu - 1) / bu;

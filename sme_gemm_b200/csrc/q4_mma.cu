@@ -13,9 +13,9 @@
 // f16 / bf16 integers (one lop3 per pair and a subtraction), the tensor core sums 32 depths in f32 and the block's f32
 // scale folds the sum into the total: no weight is rounded on the way, for bf16 either.
 //
-// What bounds it: instruction issue (about 115 warp instructions a unit at eight bf16 rows, 44 of them the expansion; with the copies'
-// addresses formed from indexes for each unit 135: 8 x 4096 x 14336 13.5 us, now 12.15, 16 rows 16.7 and 15.6, f16 12.0 and 11.3).  Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 13.7 (2.4 TB/s),
-// 16 rows 67 -> 17.5; bf16 4096 x 4096 1 row 15.8 -> 4.9, 16 rows 28.5 -> 6.3; f16 8 rows 9.8 -> 4.6, 16 rows 14.0 -> 6.2; against
+// What bounds it: instruction issue (109 warp instructions a unit at eight bf16 rows, 44 of them the expansion, issue slots 58 % busy; with the
+// copies' addresses formed from indexes for each unit 135: 8 x 4096 x 14336 13.5 us, now 12.1, 16 rows 16.7 and 15.6, f16 12.0 and 11.4).
+// Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 12.1 (2.8 TB/s), 16 rows 67 -> 15.6; bf16 4096 x 4096 1 row 15.8 -> 4.9, 16 rows 28.5 -> 6.3; f16 8 rows 9.8 -> 4.6, 16 rows 14.0 -> 6.2; against
 // q4_direct_kernel at 4 rows 8.5 -> 4.5 (one and two rows stay with the kernels of gemv_direct.cu: 3.4 and 4.1).
 #include "epilogue.cuh"
 #include "kernels.h"
