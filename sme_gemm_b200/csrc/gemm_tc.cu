@@ -29,6 +29,8 @@
 // leaves its f32 partial tile in a global workspace and splitk_reduce_kernel, launched right
 // behind, adds the slices in slice order (so the result does not depend on arrival order) and stores.
 // Every wait is bounded; a timed-out wait raises the status word and the kernel drains and exits.
+#include <atomic>
+
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"
@@ -905,13 +907,13 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const __grid_constan
 template <int BF16, int US, int DENSE, int CG>
 cudaError_t launch_tc(const CUtensorMap& tm, const CUtensorMap& tc, const CUtensorMap& tw, const CUtensorMap& ts, const GemmTcArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kern = gemm_tc_kernel<BF16, US, DENSE, CG>;
-    static int attr_dev = -1;
+    static std::atomic<int> attr_dev{-1};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
+    if (attr_dev.load(std::memory_order_acquire) != dev) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        attr_dev.store(dev, std::memory_order_release);
     }
     TcMaps<DENSE> maps;
     maps.tok = tm;

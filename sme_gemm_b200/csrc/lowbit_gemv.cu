@@ -16,6 +16,8 @@
 //   * the epilogue graph runs on the f16-rounded product.
 // Weights stream through shared memory with cp.async.bulk + mbarriers exactly
 // as in the Q4 kernel.
+#include <atomic>
+
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"
@@ -683,13 +685,13 @@ __global__ void __launch_bounds__(kThreadsLb, 1) lowbit_gemv_kernel(const __grid
 template <int BITS, int MT, int NCG, int B16, int DP>
 cudaError_t launch_lb(const LowbitGemvArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kern = lowbit_gemv_kernel<BITS, MT, NCG, B16, DP>;
-    static int attr_dev = -1;   // the opt-in is per device; set it once (to the maximum) per device
+    static std::atomic<int> attr_dev{-1};   // the opt-in is per device; set it once (to the maximum) per device
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
+    if (attr_dev.load(std::memory_order_acquire) != dev) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        attr_dev.store(dev, std::memory_order_release);
     }
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     return launch_pdl(kern, grid, dim3(kThreadsLb), smem, stream, a);

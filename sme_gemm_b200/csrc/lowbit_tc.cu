@@ -43,6 +43,8 @@
 //                       epilogue graph runs on the f16-rounded product and C is stored.
 // K-blocks of one run take lowbit_tc_block_kernel, further down.
 // Every wait is bounded; a timed-out wait raises the status word and the kernel drains and exits.
+#include <atomic>
+
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"
@@ -713,13 +715,13 @@ __global__ void __launch_bounds__(kLbThreads, 1) lowbit_tc_block_kernel(const __
 template <int BITS, int TPW, int DW>
 cudaError_t launch_lt(const CUtensorMap& tm, const LowbitTcArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kern = lowbit_tc_kernel<BITS, TPW, DW>;
-    static int attr_dev = -1;
+    static std::atomic<int> attr_dev{-1};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
+    if (attr_dev.load(std::memory_order_acquire) != dev) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        attr_dev.store(dev, std::memory_order_release);
     }
     kern<<<grid, kLtThreads, smem, stream>>>(tm, a);
     return cudaGetLastError();
@@ -746,13 +748,13 @@ cudaError_t launch_lb(const CUtensorMap& rows, const LowbitTcArgs& a, dim3 grid,
         !map(&maps.scales, CU_TENSOR_MAP_DATA_TYPE_UINT64, a.scales, sdim, sstride, sbox))
         return cudaErrorInvalidValue;
     auto kern = lowbit_tc_block_kernel<BITS, NT>;
-    static int attr_dev = -1;
+    static std::atomic<int> attr_dev{-1};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
+    if (attr_dev.load(std::memory_order_acquire) != dev) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lb_smem(NT));
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        attr_dev.store(dev, std::memory_order_release);
     }
     return launch_pdl(kern, grid, dim3(kLbThreads), lb_smem(NT), stream, maps, a);
 }

@@ -22,6 +22,8 @@
 //     epilogue graph runs on the rounded product, C is stored once.
 #include <algorithm>
 #include <cstdlib>
+#include <atomic>
+
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"
@@ -566,13 +568,13 @@ __global__ void __launch_bounds__(kSThreads, 1) q4_gemv_stream_kernel(const __gr
 template <int BF16, int MT>
 cudaError_t launch(const Q4GemvArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kern = q4_gemv_kernel<BF16, MT>;
-    static int attr_dev = -1;   // the opt-in is per device; set it once (to the maximum) per device
+    static std::atomic<int> attr_dev{-1};   // the opt-in is per device; set it once (to the maximum) per device
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
+    if (attr_dev.load(std::memory_order_acquire) != dev) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        attr_dev.store(dev, std::memory_order_release);
     }
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     return launch_pdl(kern, grid, dim3(kThreads), smem, stream, a);
@@ -624,13 +626,13 @@ void q4_gemv_stream_plan(Q4GemvArgs& a, int bf16, int sm_count, size_t* ws_float
 template <int BF16, int MT, int UPW>
 static cudaError_t launch_stream_u(const Q4GemvArgs& a, cudaStream_t stream) {
     auto kern = q4_gemv_stream_kernel<BF16, MT, UPW>;
-    static int attr_dev = -1;
+    static std::atomic<int> attr_dev{-1};
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
+    if (attr_dev.load(std::memory_order_acquire) != dev) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        attr_dev.store(dev, std::memory_order_release);
     }
     const size_t smem = 1024 + (size_t)a.sns * a.sslot + (size_t)a.a_rows * ((size_t)a.k64 * 64 + 8) * 2 +
                         (size_t)2 * kSWarps * 4 * MT * 32 * sizeof(float);

@@ -17,6 +17,8 @@
 // copies' addresses formed from indexes for each unit 135: 8 x 4096 x 14336 13.5 us, now 12.1, 16 rows 16.7 and 15.6, f16 12.0 and 11.4).
 // Against the ring-staged kernel that ran these calls before (us): bf16 8 x 4096 x 14336 28.0 -> 12.1 (2.8 TB/s), 16 rows 67 -> 15.6; bf16 4096 x 4096 1 row 15.8 -> 4.9, 16 rows 28.5 -> 6.3; f16 8 rows 9.8 -> 4.6, 16 rows 14.0 -> 6.2; against
 // q4_direct_kernel at 4 rows 8.5 -> 4.5 (one and two rows stay with the kernels of gemv_direct.cu: 3.4 and 4.1).
+#include <atomic>
+
 #include "epilogue.cuh"
 #include "kernels.h"
 #include "layout.h"
@@ -412,14 +414,14 @@ __global__ void __launch_bounds__(kMThreads, 2) q4_mma_kernel(const __grid_const
 
 template <int BF16, int NT, int CG, int DENSE, int STAGED = 0>
 cudaError_t launch(const Q4GemvArgs& a, dim3 grid, cudaStream_t stream) {
-    static int attr_dev = -1;   // the opt-in is per device
+    static std::atomic<int> attr_dev{-1};   // the opt-in is per device
     int dev = 0;
     cudaGetDevice(&dev);
-    if (attr_dev != dev) {
+    if (attr_dev.load(std::memory_order_acquire) != dev) {
         const cudaError_t e = cudaFuncSetAttribute(q4_mma_kernel<BF16, NT, CG, DENSE, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)(mma_smem(NT, CG, DENSE, STAGED) + (STAGED ? kMmaStagedMost : 0)));
         if (e != cudaSuccess) return e;
-        attr_dev = dev;
+        attr_dev.store(dev, std::memory_order_release);
     }
     const size_t smem = mma_smem(NT, CG, DENSE, STAGED) + (STAGED ? mma_staged_bytes(a.m, a.k64) : 0);
     return launch_pdl(q4_mma_kernel<BF16, NT, CG, DENSE, STAGED>, grid, dim3(kMThreads), smem, stream, a);

@@ -54,3 +54,17 @@ def test_no_lock_of_the_whole_process_is_held_over_a_launch():
         locked = re.match(r"[^;]*;[^;]*;", block).group(0)          # the declaration and the statement that locks
         assert not everyones & set(re.findall(r"\w+", locked)), f"{locked.strip()!r} is held over a launch"
     assert held >= 3
+
+
+def test_words_that_launchers_share_are_atomic():
+    """A launcher remembers the device it last raised its kernel's shared-memory limit on, and host threads on several devices read
+    and write that word: no function-local static that is written after its initialisation is a plain number."""
+    seen = 0
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cc")):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, name)).read())
+        for kind, word in re.findall(r"^[ \t]+static ([\w:<>]+(?: \w+)*?) (\w+)\s*(?:=\s*-?\d+|\{-?\d+\});", text, re.M):
+            seen += 1
+            assert kind.startswith("std::atomic<"), f"{name}: static {kind} {word}"
+    assert seen >= 7
